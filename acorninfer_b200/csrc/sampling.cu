@@ -9,7 +9,13 @@
 // u * total.  Rows do not interact, so the result does not depend on the batch.
 // temperature == 0 selects argmax (lowest index among equal maxima).
 // A row with a NaN or an infinite logit yields token -1 (the host raises).
+//
+// Two kernels.  `sample_cluster_kernel` takes every vocabulary that fits the shared memory of a cluster of eight CTAs;
+// `sample_kernel` walks the row in global memory and takes larger ones.
 #include "common.cuh"
+
+#include <cooperative_groups.h>
+namespace cg = cooperative_groups;
 
 #define SAMPLE_THREADS 1024
 
@@ -172,11 +178,313 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
     }
 }
 
+// ------------------------------------------------------------------ a cluster a row, the row in shared memory
+//
+// What bounds the walk above is one SM reading its row again for each of up to 64 bisection steps (64 rows of 151,936
+// with top-k and top-p: 701 us).  Here the CTAs of a cluster hold the row in shared memory, read from HBM once, and the
+// bounds of top-k and top-p are found digit by digit (11 + 11 + 10 bits of the ordered key): a histogram of the
+// candidates a level, summed over the cluster through distributed shared memory.  Both are one question: the smallest
+// key K with weight(lo_key <= key <= K) > limit, where a key weighs 1 and limit is V - k (the k-th largest), or weighs
+// its probability and limit is (1 - top_p) of the total.  Probabilities are summed as integers of 2^-44 of the largest
+// one (a sum's error is below that of float32 sums, and its order does not matter).
+#define SC_THREADS 512
+#define SC_WARPS (SC_THREADS / 32)
+#define SC_BINS 2048
+#define SC_MAX_CLUSTER 8
+#define SC_MAX_SLICE 45056          // floats of a row a CTA can hold beside the histogram
+typedef unsigned long long u64;
+
+struct alignas(16) ScShared {
+    u64 sums[SC_BINS];              // this CTA's share of a level's bins, summed over the cluster (bins / cluster of them)
+    unsigned int hist[3][SC_BINS];  // a level's weights: 16-bit pieces, so that 32-bit atomics cannot overflow
+    u64 total;                      // of `sums`
+    u64 kept;                       // this CTA's part of the kept set
+    u64 best;                       // largest (key, ~index) of this CTA's slice
+    unsigned int bad;
+    u64 warp_a[SC_WARPS];
+    u64 found_cum;                  // answer of a level: weight below the bin, the bin (SC_BINS: limit not exceeded)
+    unsigned int found_bin;
+};
+
+__device__ __forceinline__ u64 prob_fixed(float x, float gmax, float inv_t) {
+    return __float2ull_rn(expf((x - gmax) * inv_t) * 17592186044416.f);
+}
+
+__device__ __forceinline__ u64 warp_sum_u64(u64 v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ u64 block_sum_u64(u64 v, u64* scratch) {
+    v = warp_sum_u64(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return warp_sum_u64((threadIdx.x & 31) < SC_WARPS ? scratch[threadIdx.x & 31] : 0ull);
+}
+
+// The smallest key K of the row with weight(lo_key <= key <= K) > limit(total weight from lo_key on); 0xffffffff if there
+// is none.  Called by all threads of the cluster with the same arguments.
+template <bool MASS>
+__device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigned int lo_key, float gmax, float inv_t, u64 count_limit,
+                                  float drop) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const int c = (int)cluster.num_blocks(), tid = threadIdx.x, lane = tid & 31;
+    constexpr int PIECES = MASS ? 3 : 1;
+    unsigned int prefix = 0;        // the digits found so far
+    u64 limit = 0;
+#pragma unroll 1
+    for (int level = 0; level < 3; ++level) {
+        const int shift = level == 0 ? 21 : level == 1 ? 10 : 0;
+        const int bins = level == 2 ? 1024 : 2048, above = level == 0 ? 32 : level == 1 ? 21 : 10;
+        for (int i = tid; i < PIECES * SC_BINS; i += SC_THREADS) (&sh.hist[0][0])[i] = 0;
+        __syncthreads();
+        for (int i = tid; i < n; i += SC_THREADS) {
+            const float v = row[i];
+            const unsigned int key = float_key(v);
+            if (key < lo_key || (level > 0 && (key >> above) != prefix)) continue;
+            const int bin = (key >> shift) & (bins - 1);
+            if (MASS) {
+                const u64 w = prob_fixed(v, gmax, inv_t);
+                if (w == 0) continue;
+                atomicAdd(&sh.hist[0][bin], (unsigned int)w & 0xffffu);
+                if (w >> 16) atomicAdd(&sh.hist[1][bin], (unsigned int)(w >> 16) & 0xffffu);
+                if (w >> 32) atomicAdd(&sh.hist[2][bin], (unsigned int)(w >> 32));
+            } else {
+                atomicAdd(&sh.hist[0][bin], 1u);
+            }
+        }
+        cluster.sync();
+        // this CTA sums its share of the bins over the cluster
+        const int share = bins / c, first = (int)cluster.block_rank() * share;
+        u64 mine = 0;
+        for (int i = tid; i < share; i += SC_THREADS) {
+            u64 s = 0;
+            for (int r = 0; r < c; ++r) {
+                const unsigned int* h = cluster.map_shared_rank(&sh.hist[0][0], r) + first + i;
+                s += h[0];
+                if (MASS) s += ((u64)h[SC_BINS] << 16) + ((u64)h[2 * SC_BINS] << 32);
+            }
+            sh.sums[i] = s;
+            mine += s;
+        }
+        mine = block_sum_u64(mine, sh.warp_a);
+        if (tid == 0) sh.total = mine;
+        cluster.sync();
+        // one warp finds the bin: first the CTA whose share holds it, then the bin in that share
+        if (tid < 32) {
+            const u64 t = lane < c ? *cluster.map_shared_rank(&sh.total, lane) : 0ull;
+            u64 incl = t;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const u64 up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
+            }
+            const u64 all = __shfl_sync(0xffffffffu, incl, c - 1);
+            if (level == 0) limit = MASS ? (u64)((double)drop * (double)all) : count_limit;
+            const unsigned int over = __ballot_sync(0xffffffffu, lane < c && incl > limit);
+            if (over == 0) {
+                if (lane == 0) sh.found_bin = SC_BINS;
+            } else {
+                const int owner = __ffs(over) - 1;
+                u64 run = __shfl_sync(0xffffffffu, incl - t, owner);
+                const u64* sums = cluster.map_shared_rank(&sh.sums[0], owner);
+                const int per = (share + 31) / 32;
+                u64 part = 0;
+                for (int i = lane * per; i < min(share, (lane + 1) * per); ++i) part += sums[i];
+                u64 pin = part;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const u64 up = __shfl_up_sync(0xffffffffu, pin, o);
+                    if (lane >= o) pin += up;
+                }
+                const int who = __ffs(__ballot_sync(0xffffffffu, run + pin > limit)) - 1;
+                if (lane == who) {
+                    run += pin - part;
+                    int i = lane * per;
+                    while (run + sums[i] <= limit) run += sums[i++];
+                    sh.found_bin = owner * share + i;
+                    sh.found_cum = run;
+                }
+            }
+            __syncwarp();
+            limit = __shfl_sync(0xffffffffu, limit, 0);
+            if (sh.found_bin != SC_BINS) limit -= sh.found_cum;
+        }
+        __syncthreads();
+        if (sh.found_bin == SC_BINS) return 0xffffffffu;
+        prefix = (prefix << (level == 0 ? 11 : level == 1 ? 11 : 10)) | sh.found_bin;
+    }
+    return prefix;
+}
+
+__global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
+    const float* __restrict__ logits, int64_t ld, int V, int slice, const float* __restrict__ temperature,
+    const int* __restrict__ top_k, const float* __restrict__ top_p, const u64* __restrict__ seed,
+    const u64* __restrict__ counter, int* __restrict__ token_out, float* __restrict__ logprob_out) {
+    extern __shared__ __align__(16) unsigned char sc_smem[];
+    ScShared& sh = *reinterpret_cast<ScShared*>(sc_smem);
+    float* row = reinterpret_cast<float*>(sc_smem + sizeof(ScShared));
+    cg::cluster_group cluster = cg::this_cluster();
+    const int c = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int r = blockIdx.x / c, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_wait();
+    pdl_trigger();
+    const int i0 = min(V, rank * slice), n = min(V, i0 + slice) - i0;
+    const float* x = logits + (int64_t)r * ld + i0;
+    const float temp = temperature[r];
+
+    // the slice into shared memory; largest logit (first index among equals) and finiteness on the way
+    u64 best = 0;
+    unsigned int bad = 0;
+    auto take = [&](float v, int i) {
+        if (!(fabsf(v) <= 3.0e38f)) bad = 1;
+        // -0 and 0 are equal: the first of them wins
+        const u64 k = ((u64)float_key(v == 0.f ? 0.f : v) << 32) | (unsigned int)~(i0 + i);
+        best = k > best ? k : best;
+        row[i] = v;
+    };
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        const int n4 = n >> 2;
+#pragma unroll 4
+        for (int i = tid; i < n4; i += SC_THREADS) {
+            const float4 v = reinterpret_cast<const float4*>(x)[i];
+            take(v.x, 4 * i); take(v.y, 4 * i + 1); take(v.z, 4 * i + 2); take(v.w, 4 * i + 3);
+        }
+        for (int i = 4 * n4 + tid; i < n; i += SC_THREADS) take(x[i], i);
+    } else {
+#pragma unroll 4
+        for (int i = tid; i < n; i += SC_THREADS) take(x[i], i);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other > best ? other : best;
+    }
+    if (tid == 0) sh.bad = 0;
+    if (lane == 0) sh.warp_a[warp] = best;
+    __syncthreads();
+    if (bad) sh.bad = 1;
+    if (tid == 0) {
+        for (int w = 0; w < SC_WARPS; ++w) best = sh.warp_a[w] > best ? sh.warp_a[w] : best;
+        sh.best = best;
+    }
+    cluster.sync();
+    bad = 0;
+    for (int k = 0; k < c; ++k) {
+        const u64 b = *cluster.map_shared_rank(&sh.best, k);
+        best = k == 0 || b > best ? b : best;
+        bad |= *cluster.map_shared_rank(&sh.bad, k);
+    }
+    const int arg = (int)~(unsigned int)best;
+    if (bad || !(temp > 0.f)) {
+        if (rank == 0 && tid == 0) {
+            token_out[r] = bad ? -1 : arg;
+            if (logprob_out) logprob_out[r] = 0.f;
+        }
+        cluster.sync();              // a CTA's shared memory stays until all have read it
+        return;
+    }
+    const unsigned int gkey = (unsigned int)(best >> 32);
+    const float gmax = __uint_as_float((gkey & 0x80000000u) ? gkey & 0x7fffffffu : ~gkey);
+    const float inv_t = 1.f / temp;
+    unsigned int lo_key = 0u;
+    const int k = top_k[r];
+    if (k > 0 && k < V) lo_key = sc_select<false>(sh, row, n, 0u, 0.f, 0.f, (u64)(V - k), 0.f);
+    const float p_keep = top_p[r];
+    if (p_keep < 1.f) {
+        const unsigned int found = sc_select<true>(sh, row, n, lo_key, gmax, inv_t, 0ull, 1.f - p_keep);
+        lo_key = found < gkey ? found : gkey;        // the largest always stays
+    }
+    // inverse CDF in token order over the kept set; a thread owns a run of the slice (of odd length: no bank conflicts)
+    const int seg = ((n + SC_THREADS - 1) / SC_THREADS) | 1;
+    const int a = min(n, tid * seg), b = min(n, a + seg);
+    u64 mine = 0;
+    for (int i = a; i < b; ++i)
+        if (float_key(row[i]) >= lo_key) mine += prob_fixed(row[i], gmax, inv_t);
+    u64 incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+    }
+    __syncthreads();
+    if (lane == 31) sh.warp_a[warp] = incl;
+    __syncthreads();
+    u64 before = incl - mine;
+    u64 here = 0;
+    for (int w = 0; w < SC_WARPS; ++w) {
+        if (w < warp) before += sh.warp_a[w];
+        here += sh.warp_a[w];
+    }
+    if (tid == 0) sh.kept = here;
+    cluster.sync();
+    u64 total = 0;
+    for (int q = 0; q < c; ++q) {
+        const u64 t = *cluster.map_shared_rank(&sh.kept, q);
+        if (q < rank) before += t;
+        total += t;
+    }
+    // u = m / 2^24: the first token whose running sum exceeds floor(m total / 2^24)
+    const u64 m = (u64)(uniform_from(seed[r], counter[r]) * 16777216.f);
+    const u64 target = (__umul64hi(m, total) << 40) | ((m * total) >> 24);
+    if (target >= before && target < before + mine) {
+        int i = a;
+        for (;; ++i) {
+            if (float_key(row[i]) < lo_key) continue;
+            before += prob_fixed(row[i], gmax, inv_t);
+            if (before > target) break;
+        }
+        token_out[r] = i0 + i;
+        if (logprob_out) logprob_out[r] = (row[i] - gmax) * inv_t - logf((float)((double)total * 5.684341886080802e-14));
+    } else if (total == 0 && rank == 0 && tid == 0) {
+        token_out[r] = arg;
+        if (logprob_out) logprob_out[r] = 0.f;
+    }
+    cluster.sync();
+}
+
+static int launch_sample_cluster(const float* logits, int64_t ld, int rows, int V, int c, int slice, const float* temperature,
+                                 const int* top_k, const float* top_p, const u64* seed, const u64* counter, int* token_out,
+                                 float* logprob_out, cudaStream_t stream) {
+    static AcornPerDevice configured;
+    if (!configured.seen()) {
+        const int most = (int)(sizeof(ScShared) + SC_MAX_SLICE * sizeof(float));
+        cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return (int)e;
+        configured.mark();
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(rows * c));
+    cfg.blockDim = dim3(SC_THREADS);
+    cfg.dynamicSmemBytes = sizeof(ScShared) + (size_t)slice * sizeof(float);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = c;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = acorn_pdl_enabled() ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel, logits, ld, V, slice, temperature, top_k, top_p, seed, counter,
+                                       token_out, logprob_out);
+    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
 extern "C" int acorn_sample(const float* logits, int64_t ld, int rows, int V, const float* temperature,
                             const int* top_k, const float* top_p, const unsigned long long* seed,
                             const unsigned long long* counter, int* token_out, float* logprob_out,
                             cudaStream_t stream) {
     if (rows <= 0) return 0;
+    // small vocabularies fit one CTA; slices are multiples of four logits, so that they start on 16 bytes where the row does
+    const int c = V <= 4096 ? 1 : SC_MAX_CLUSTER;
+    const int slice = ((V + c - 1) / c + 3) & ~3;
+    if (slice <= SC_MAX_SLICE && rows <= 0x7fffffff / SC_MAX_CLUSTER)
+        return launch_sample_cluster(logits, ld, rows, V, c, slice, temperature, top_k, top_p, seed, counter, token_out,
+                                     logprob_out, stream);
     return acorn_launch(sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, temperature, top_k,
                         top_p, seed, counter, token_out, logprob_out);
 }

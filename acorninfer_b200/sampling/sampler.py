@@ -11,6 +11,7 @@ device-to-host copy per step.
 
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from ..kernels import ops
@@ -90,10 +91,15 @@ class Sampler:
         if all(p.greedy for p in params):
             temperature, top_k, top_p, seeds, ctrs = self._greedy_params(R)
         else:
-            dev = self.device
-            temperature = torch.tensor([p.temperature for p in params], dtype=torch.float32).to(dev, non_blocking=True)
-            top_k = torch.tensor([p.top_k for p in params], dtype=torch.int32).to(dev, non_blocking=True)
-            top_p = torch.tensor([p.top_p for p in params], dtype=torch.float32).to(dev, non_blocking=True)
-            seeds = torch.tensor([p.seed & (2 ** 63 - 1) for p in params], dtype=torch.int64).to(dev, non_blocking=True)
-            ctrs = torch.tensor([int(c) for c in counters], dtype=torch.int64).to(dev, non_blocking=True)
+            # one copy to the device for all five (each copy costs the host as much as the kernel takes)
+            block = np.empty(7 * R, dtype=np.int32)
+            wide = block[:4 * R].view(np.int64)
+            wide[:R] = [p.seed & (2 ** 63 - 1) for p in params]
+            wide[R:] = [int(c) for c in counters]
+            block[4 * R:6 * R].view(np.float32)[:] = [p.temperature for p in params] + [p.top_p for p in params]
+            block[6 * R:] = [p.top_k for p in params]
+            block = torch.from_numpy(block).to(self.device, non_blocking=True)
+            seeds, ctrs = block[:2 * R].view(torch.int64), block[2 * R:4 * R].view(torch.int64)
+            temperature, top_p = block[4 * R:5 * R].view(torch.float32), block[5 * R:6 * R].view(torch.float32)
+            top_k = block[6 * R:]
         return ops.sample(logits, temperature, top_k, top_p, seeds, ctrs, want_logprobs)

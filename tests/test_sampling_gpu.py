@@ -67,3 +67,39 @@ def test_draws_follow_the_distribution_and_do_not_depend_on_the_batch():
     assert (freq - x[0].double().softmax(-1)).abs().max() < 0.03
     alone, _ = run(x[:1], 1.0, 0, 1.0, 11, [123])
     assert alone[0] == toks[123]
+
+
+@pytest.mark.parametrize("vocab", [4095, 4096, 4097, 32771, 151936, 360448, 360449])
+def test_large_vocabularies_in_every_cut(vocab):
+    """Around the sizes where the kernel changes (one CTA, a cluster, the walk in global memory); rows of odd length, which
+    start on 16 bytes only every fourth time; a row of equal logits, one masked down to a few tokens, one with many ties."""
+    from acorninfer_b200.kernels import ops
+    R = 7
+    g = torch.Generator().manual_seed(vocab)
+    x = 2.5 * torch.randn(R, vocab, generator=g)
+    x[4] = 0.25
+    x[5, 9:] = -3.0e38
+    x[6] = (x[6] * 2).round() / 2           # many equal logits
+    temperature, top_k, top_p = [0.7, 1.0, 0.6, 0.0, 1.0, 1.0, 0.8], [0, 20, 50, 0, 0, 0, 1000], [0.95, 0.8, 1.0, 1.0, 0.5, 0.9, 0.9]
+    seeds, counters = list(range(50, 50 + R)), [3 * i for i in range(R)]
+    f = lambda v, dt: torch.tensor(v, dtype=dt, device=DEV)
+    toks, lps = ops.sample(x.to(DEV), f(temperature, torch.float32), f(top_k, torch.int32), f(top_p, torch.float32),
+                           f(seeds, torch.int64), f(counters, torch.int64), True)
+    toks, lps = toks.tolist(), lps.tolist()
+    checked = 0
+    for r in range(R):
+        if temperature[r] == 0:
+            assert toks[r] == int(x[r].argmax())
+            continue
+        processed = plain.process_logits(x[r], temperature[r], top_k[r], top_p[r])
+        # among equal logits at the bound of top-p the kernel keeps all, the plain one those that its sort puts last
+        scaled = x[r].double() / temperature[r]
+        processed = scaled.masked_fill(scaled < processed[torch.isfinite(processed)].min(), float("-inf"))
+        u = ops.uniform(seeds[r], counters[r])
+        want, want_lp, margin = plain.sample_with_uniform(processed, u)
+        # a kept set may differ by the token at the bound of top-p, whose mass moves the CDF by as much
+        if margin > 1e-6 and r != 4:
+            assert toks[r] == want
+            assert abs(lps[r] - want_lp) < 1e-4
+            checked += 1
+    assert 0 <= toks[4] < vocab and checked >= 3
