@@ -23,14 +23,10 @@
 //   linear_chunk_fold   per state entry along a row's chunks: the state every chunk starts from, the end state into the slot
 //   delta_chunk_out     as above, with Q' and v in place of q and U
 //
-// A row's chunks are counted from its first token of the step; chunk c of row r is number row_start[r] / 64 + r + c of the
-// step (distinct for all chunks; some numbers stay unused).
-#include "common.cuh"
+#include "chunk_helpers.cuh"
 
-#define DC 64                       // tokens a chunk
 #define DC_VT 16                    // value columns a block of delta_chunk_state
 #define DC_OT 64                    // value columns a block of delta_chunk_out
-#define DC_PAD 4                    // floats between rows in shared memory (16-byte reads of neighbouring rows hit distinct banks)
 
 struct DeltaChunkParams {
     const float* q;                 // [T, KH, dim]
@@ -66,39 +62,6 @@ template <typename T> struct LinearChunkParams {
     float* decay;                   // [chunk numbers, H, dim]
     int rows, H, dim, vdim;
 };
-
-// The row and chunk of a chunk number, or false for an unused one.
-__device__ __forceinline__ bool chunk_of(int id, const int* __restrict__ row_start, int rows, int& r, int& first, int& n) {
-    int lo = 0, hi = rows - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (row_start[mid] / DC + mid <= id) lo = mid;
-        else hi = mid - 1;
-    }
-    r = lo;
-    const int start = row_start[lo], c = id - (start / DC + lo);
-    first = start + c * DC;
-    n = min(DC, row_start[lo + 1] - first);
-    return n > 0;
-}
-
-__device__ __forceinline__ void dc_cp16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
-
-// n rows of `width` floats (a multiple of 4), ld apart, into DC rows of DP + DC_PAD; the rest zeros
-template <int DP> __device__ __forceinline__ void load_rows(float* dst, const float* src, int64_t ld, int n, int width) {
-    for (int e = threadIdx.x; e < DC * (DP / 4); e += blockDim.x) {
-        const int i = e / (DP / 4), c = (e % (DP / 4)) * 4;
-        float* d = dst + i * (DP + DC_PAD) + c;
-        if (i < n && c < width) dc_cp16(d, src + (int64_t)i * ld + c);
-        else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-}
-
-__device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
-    return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
-}
 
 template <int DP>
 __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(const DeltaChunkParams p) {

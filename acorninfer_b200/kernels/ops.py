@@ -114,6 +114,10 @@ class _Sigs:
     acorn_attention_plain = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
                              c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_int, c_void_p]
+    acorn_scan_chunk = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
+                        c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                        c_void_p]
+    acorn_scan_chunk_supported = [c_int, c_int]
     acorn_bigram_add = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                         c_int, c_int, c_int, c_int, c_void_p]
     acorn_rmsnorm_add = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]
@@ -2173,6 +2177,17 @@ def scan_segments(longest_row: int, num_rows: int, heads: int, n: int, v: int) -
     return -(-longest_row // nseg), nseg
 
 
+SCAN_CHUNK = 64                   # tokens a chunk of the chunked scan
+
+
+def scan_chunk_ok(longest_row: int, num_rows: int, b: torch.Tensor, c: torch.Tensor, x: torch.Tensor, heads: int, n: int, v: int) -> bool:
+    """Whether the scan of these rows runs over chunks of tokens: a row of a chunk or more, sizes and alignments the kernels
+    know (16-byte reads of b, c and x), and room for the chunks' states."""
+    return (longest_row >= SCAN_CHUNK and bool(lib().acorn_scan_chunk_supported(n, v)) and num_rows <= 65535 and heads <= 65535
+            and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in (b, c, x))
+            and 4 * (x.shape[0] // SCAN_CHUNK + num_rows) * heads * n * v <= DELTA_CHUNK_SCRATCH_BYTES)
+
+
 def linear_scan(b: torch.Tensor, c: torch.Tensor, x: torch.Tensor, decay: torch.Tensor, w: torch.Tensor | None,
                 skip32: torch.Tensor | None, state: torch.Tensor, state_off: int, row_start: torch.Tensor,
                 row_slot: torch.Tensor, num_rows: int, heads: int, groups: int, n: int, v: int,
@@ -2181,7 +2196,8 @@ def linear_scan(b: torch.Tensor, c: torch.Tensor, x: torch.Tensor, decay: torch.
     row's slot (``[heads, v, n]`` float32 at ``state_off``, updated in place).  ``b``, ``c`` [T, groups * n],
     ``x`` [T, heads * v] float32 (column slices allowed); ``decay`` [T, heads] per token or [heads] for all;
     ``w`` [T, heads] or None.  Returns float32 y [T, heads * v].  ``longest_row``: a bound on the tokens of a row
-    (a host number); long rows of a step with few rows are run in segments side by side (``scan_segments``)."""
+    (a host number); steps with a long row run over chunks of tokens (``scan_chunk_ok``) or, at sizes those kernels do not
+    take, with their rows in segments side by side (``scan_segments``)."""
     for t, name in ((b, "b"), (c, "c"), (x, "x")):
         _rows2(t, name, torch.float32)
     _check(state, "state", torch.float32, 2)
@@ -2199,6 +2215,16 @@ def linear_scan(b: torch.Tensor, c: torch.Tensor, x: torch.Tensor, decay: torch.
     if skip32 is not None:
         _check(skip32, "skip", torch.float32, 1)
     y = torch.empty((T, heads * v), dtype=torch.float32, device=x.device)
+    if scan_chunk_ok(int(longest_row), num_rows, b, c, x, heads, n, v):
+        ids = T // SCAN_CHUNK + num_rows
+        s0 = torch.empty((ids, heads, n, v), dtype=torch.float32, device=x.device)
+        dec = torch.empty((ids, heads), dtype=torch.float32, device=x.device)
+        _ok(lib().acorn_scan_chunk(b.data_ptr(), b.stride(0), c.data_ptr(), c.stride(0), x.data_ptr(), x.stride(0), decay.data_ptr(),
+                                   decay.stride(0) if decay.dim() == 2 else 0, _ptr(w), w.stride(0) if w is not None else 0,
+                                   _ptr(skip32), state.data_ptr() + 4 * int(state_off), state.stride(0), y.data_ptr(),
+                                   row_start.data_ptr(), row_slot.data_ptr(), T, num_rows, heads, groups, n, v, s0.data_ptr(),
+                                   dec.data_ptr(), _stream()), "linear_scan")
+        return y
     seg, nseg = scan_segments(int(longest_row), num_rows, heads, n, v)
     seg_state = seg_decay = None
     if seg:

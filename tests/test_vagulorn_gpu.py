@@ -424,6 +424,50 @@ def test_linear_scan_carries_state_across_steps_and_slots(H, G, N, V, long):
     assert float(state[1].min()) == 123.0 and float(state[3, :5].abs().max()) == 0.0      # other slots and the vector's head untouched
 
 
+@pytest.mark.parametrize("H,G,N,V,fixed", [(4, 2, 64, 64, False), (20, 2, 128, 64, False), (3, 3, 12, 8, True), (9, 1, 36, 100, False),
+                                           (2, 2, 128, 132, True)])
+def test_linear_scan_over_chunks(H, G, N, V, fixed):
+    """Rows around the chunk of 64 tokens, decays of zero and of one among them, more heads to a group than a block takes, sizes
+    that fill no tile; outputs and end states against the loop in 64 bits (float32 sums of up to 200 terms of about N^1/2: 2e-5
+    of the largest), from states that lie unaligned."""
+    o = ops()
+    g = torch.Generator().manual_seed(N + V)
+    lens, slots = [200, 1, 64, 65, 63, 128], [3, 0, 6, 2, 5, 1]
+    T = sum(lens)
+    decay = torch.rand(H, generator=g).double() * 0.3 + 0.7
+    decay[0], decay[1] = 1.0, 0.0
+    a = decay.float().double()[None].repeat(T, 1) if fixed else (torch.rand(T, H, generator=g) ** 0.3)
+    if not fixed:
+        a[7], a[70:72], a[90] = 0.0, 0.0, 1.0
+    a = a.double()
+    dt = torch.ones(T, H).double() if fixed else torch.rand(T, H, generator=g).double()
+    B, C = torch.randn(T, G, N, generator=g).double(), torch.randn(T, G, N, generator=g).double()
+    x, D = torch.randn(T, H, V, generator=g).double(), torch.randn(H, generator=g).double()
+    state = torch.randn(8, H * N * V + 11, generator=g).to(DEV)
+    before = state.double().cpu()
+    i32 = dict(dtype=torch.int32, device=DEV)
+    f = lambda t, *shape: t.float().reshape(*shape).contiguous().to(DEV)
+    bc = torch.cat([f(B, T, G * N), f(C, T, G * N)], 1).contiguous()
+    starts = np.cumsum([0] + lens)
+    b, c = bc[:, :G * N], bc[:, G * N:]
+    assert o.scan_chunk_ok(max(lens), len(lens), b, c, f(x, T, H * V), H, N, V)
+    y = o.linear_scan(b, c, f(x, T, H * V), f(decay, H) if fixed else f(a, T, H), None if fixed else f(dt, T, H), f(D, H), state, 5,
+                      torch.tensor(starts, **i32), torch.tensor(slots, **i32), len(lens), H, G, N, V, longest_row=max(lens))
+    y, after = y.double().cpu().view(T, H, V), state.double().cpu()
+    hg = torch.arange(H) // (H // G)
+    for r, (n, slot) in enumerate(zip(lens, slots)):
+        S = before[slot, 5:5 + H * N * V].view(H, V, N).transpose(1, 2).clone()
+        want = torch.zeros(n, H, V).double()
+        for i in range(n):
+            t = starts[r] + i
+            S = a[t][:, None, None] * S + (dt[t][:, None] * B[t, hg])[:, :, None] * x[t][:, None, :]
+            want[i] = torch.einsum("hnv,hn->hv", S, C[t, hg]) + D.float().double()[:, None] * x[t]
+        assert (y[starts[r]:starts[r + 1]] - want).abs().max() < 2e-5 * want.abs().max(), r
+        got = after[slot, 5:5 + H * N * V].view(H, V, N).transpose(1, 2)
+        assert (got - S).abs().max() < 2e-5 * S.abs().max(), r
+    assert torch.equal(after[[4, 7]], before[[4, 7]]) and torch.equal(after[:, :5], before[:, :5])
+
+
 def test_linear_scan_with_one_decay_per_head_and_no_step_sizes():
     o = ops()
     g = torch.Generator().manual_seed(1)
