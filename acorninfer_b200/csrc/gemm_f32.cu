@@ -1,33 +1,52 @@
 // C[M, N] = A[M, K] * W[N, K]^T in true float32: FMA on the CUDA cores, no tensor-core
 // mode of reduced precision.  It is the matrix product of the float32 path.
 //
-// Every kernel here computes an output element as one chain acc = fma(a[k], w[k], acc) over
-// k = 0, 1, 2, ... from acc = 0, so the result of a row is the same bits whichever kernel ran
-// and does not depend on M, on the other rows or on the tile sizes.
+// Every kernel here sums an output element in one order: K is cut into eight ranges of ceil(K / 128) * 16, a range is a
+// chain acc = fma(a[k], w[k], acc) from 0 in the order of k, and the result is T0 + T1 + ... + T7 from the left.  So a
+// row's bits do not depend on the kernel that ran, on M, on the other rows or on the tile sizes.  The ranges are what lets
+// eight warps (decode) or eight CTAs (prompts with few tiles) work on one output tile: one chain over all of K = 6,144
+// takes 12.5 us in dependent multiply-adds alone, where the weights of N = 2,048 columns stream in 7.6 us.
 //
 // A, W: float32 row-major, K contiguous, with row strides lda, ldw; C row stride ldc.
-//   rows kernel   up to 64 rows (decode): 16 rows x 32 columns a block, the weight tiles streamed
-//                 through a ring of cp.async stages (the product is bound by reading W once);
-//   tile kernel   more rows: 128 x 128 a block, 8 x 8 a thread, the next tile fetched into
-//                 registers while this one is multiplied;
+//   rows kernel   up to 16 rows (decode): a block takes 16 or 32 columns and all rows, a warp one range of K with a ring
+//                 of cp.async stages of its own (no block barrier): bound by reading W once;
+//   tile kernel   more rows: 64 x 64 a block; a cluster of eight shares a tile's ranges where the tiles
+//                 alone leave the device idle: bound by the multiply-adds and the reads of shared memory that feed them;
 //   plain kernel  64 x 64 a block, scalar loads: operands that are not 16-byte aligned.
 #include "mma_helpers.cuh"
 
+#include <cooperative_groups.h>
+namespace cg = cooperative_groups;
+
+// a range of K: a multiple of 16, so that no k-step of a kernel crosses from one into the next
+#define K_RANGES 8
+__host__ __device__ __forceinline__ int k_range(int K) { return (K + 16 * K_RANGES - 1) / (16 * K_RANGES) * 16; }
+
 // ------------------------------------------------------------------ plain kernel
 
-#define BM 64
-#define BN 64
-#define BK 16
+#define PL_BM 64
+#define PL_BN 64
+#define PL_BK 16
 
 __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__ A, int64_t lda,
                                                        const float* __restrict__ W, int64_t ldw,
                                                        float* __restrict__ C, int64_t ldc, int M, int N, int K) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    __shared__ float As[PL_BK][PL_BM + 4];
+    __shared__ float Ws[PL_BK][PL_BN + 4];
+    const int m0 = blockIdx.y * PL_BM, n0 = blockIdx.x * PL_BN;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 x 16 threads
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += BK) {
+    float acc[4][4] = {}, total[4][4] = {};
+    const int range = k_range(K);
+    for (int k0 = 0; k0 < K; k0 += PL_BK) {
+        if (k0 > 0 && k0 % range == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    total[i][j] += acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int idx = threadIdx.x + e * 256;
@@ -38,7 +57,7 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
         }
         __syncthreads();
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
+        for (int kk = 0; kk < PL_BK; ++kk) {
             float a[4], w[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
@@ -58,197 +77,315 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
-            if (n < N) C[(int64_t)m * ldc + n] = acc[i][j];
+            if (n < N) C[(int64_t)m * ldc + n] = total[i][j] + acc[i][j];
         }
     }
 }
 
 // ------------------------------------------------------------------ rows kernel
 
-#define RS_BN 32
-#define RS_BK 64
-#define RS_ROWS 16
-#define RS_STAGES 5
-#define RS_LD (RS_BK + 4)       // row stride in shared memory: 16-byte reads of 8 neighbouring rows hit 8 banks groups
-#define RS_THREADS 128
-#define RS_SMEM (RS_STAGES * (RS_BN + RS_ROWS) * RS_LD * sizeof(float))
+#define RS_BK 32
+#define RS_STAGES 4
+#define RS_LD (RS_BK + 4)       // row stride in shared memory: 16-byte reads of 8 neighbouring rows hit 8 groups of banks
+#define RS_THREADS (32 * K_RANGES)
 
-// Block b works on columns (b / mblocks) * 32 .. and rows (b % mblocks) * 16 ..: the blocks that
-// share a weight tile run next to each other and all but the first find it in L2.
+// R rows and CPL columns a lane, 2 R rows and 16 CPL columns a block.
+template <int R, int CPL> constexpr int rs_smem() { return K_RANGES * RS_STAGES * (16 * CPL + 2 * R) * RS_LD * (int)sizeof(float); }
+
+// Measured (B200): the 113 products of a decode step of 6 rows at Qwen3-1.7B sizes (6.9 GB), with one block for 32 columns and
+// 16 rows whose four warps walked K together 5.64 ms, this 2.09 ms.  At 6 rows the reads of A and W from shared memory that feed
+// the multiply-adds set the pace (3.6 TB/s at N = 12,288; 4.6 TB/s at one row).
+// With two columns a lane a row of A that was read serves two weights, but a block takes 32 columns: for wide matrices only.
+template <int R, int CPL>
 __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* __restrict__ A, int64_t lda,
                                                                    const float* __restrict__ W, int64_t ldw,
-                                                                   float* __restrict__ C, int64_t ldc, int M, int N,
-                                                                   int K, int mblocks) {
-    extern __shared__ __align__(16) float rs_smem[];
-    float* Ws = rs_smem;                                          // [stages][32][LD]
-    float* As = rs_smem + RS_STAGES * RS_BN * RS_LD;              // [stages][16][LD]
-    const int n0 = (blockIdx.x / mblocks) * RS_BN, m0 = (blockIdx.x % mblocks) * RS_ROWS;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;      // column of the tile; rows ty * 4 .. + 3
-    const int nk = (K + RS_BK - 1) / RS_BK;
+                                                                   float* __restrict__ C, int64_t ldc, int M, int N, int K) {
+    extern __shared__ __align__(16) float rs_buf[];
+    constexpr int BN = 16 * CPL, ROWS = BN + 2 * R, STAGE = ROWS * RS_LD;
+    const int n0 = blockIdx.x * BN;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int col = lane & 15, row0 = (lane >> 4) * R;
+    const int range = k_range(K), kbeg = min(K, warp * range), kend = min(K, kbeg + range);
+    const int nk = (kend - kbeg + RS_BK - 1) / RS_BK;
+    float* ring = rs_buf + warp * RS_STAGES * STAGE;
 
     auto load = [&](int stage, int kb) {
-        // chunks of 4 floats: 32 x 16 of W (4 a thread), 16 x 16 of A (2 a thread); outside the matrix: zeros
+        float* dst = ring + stage * STAGE;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int c = threadIdx.x + e * RS_THREADS, row = c >> 4, k = kb * RS_BK + (c & 15) * 4;
-            const bool valid = n0 + row < N && k < K;
-            const float* src = valid ? W + (int64_t)(n0 + row) * ldw + k : W;
-            cp_async_16(smem_addr(Ws + (stage * RS_BN + row) * RS_LD + (c & 15) * 4), src, valid);
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int c = threadIdx.x + e * RS_THREADS, row = c >> 4, k = kb * RS_BK + (c & 15) * 4;
-            const bool valid = m0 + row < M && k < K;
-            const float* src = valid ? A + (int64_t)(m0 + row) * lda + k : A;
-            cp_async_16(smem_addr(As + (stage * RS_ROWS + row) * RS_LD + (c & 15) * 4), src, valid);
+        for (int e = 0; e < ROWS / 4; ++e) {                     // rows of W, then of A; 8 lanes take 128 bytes of a row
+            const int row = e * 4 + (lane >> 3), seg = (lane & 7) * 4, k = kbeg + kb * RS_BK + seg;
+            const bool of_w = e < BN / 4;
+            const bool valid = k < kend && (of_w ? n0 + row < N : row - BN < M);
+            const float* src = of_w ? W + (int64_t)(n0 + row) * ldw + k : A + (int64_t)(row - BN) * lda + k;
+            cp_async_16(smem_addr(dst + row * RS_LD + seg), valid ? src : W, valid);
         }
     };
 
+    // the first weights on their way to L2 while the kernel before this one ends (W may be its result: not read yet)
+#pragma unroll
+    for (int e = 0; e < CPL * (RS_STAGES - 1) / 2; ++e) {
+        const int row = (lane + 32 * e) % BN, k = kbeg + ((lane + 32 * e) / BN) * RS_BK;
+        if (k < kend && n0 + row < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (int64_t)(n0 + row) * ldw + k));
+    }
+    pdl_wait();
+    pdl_trigger();
     for (int s = 0; s < RS_STAGES - 1; ++s) {
         if (s < nk) load(s, s);
         cp_async_commit();
     }
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int kb = 0; kb < nk; ++kb) {
-        cp_async_wait<RS_STAGES - 2>();          // this thread's copies of stage kb have landed
-        __syncthreads();                         // everyone's have, and everyone is done with stage kb - 1
-        if (kb + RS_STAGES - 1 < nk) load((kb + RS_STAGES - 1) % RS_STAGES, kb + RS_STAGES - 1);
-        cp_async_commit();
-        const int stage = kb % RS_STAGES;
-        const float* wrow = Ws + (stage * RS_BN + tx) * RS_LD;
-        const float* arow = As + (stage * RS_ROWS + ty * 4) * RS_LD;
-#pragma unroll 4
-        for (int kk = 0; kk < RS_BK; kk += 4) {
-            const float4 w = *reinterpret_cast<const float4*>(wrow + kk);
+    float acc[R][CPL];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) acc[i][c] = 0.f;
+    int stage = 0, fill = RS_STAGES - 1;
+    for (int kb = 0; kb < nk; ++kb) {
+        cp_async_wait<RS_STAGES - 2>();          // this lane's copies of stage kb have landed
+        __syncwarp();                            // all lanes' have, and all are done with stage kb - 1
+        if (kb + RS_STAGES - 1 < nk) load(fill, kb + RS_STAGES - 1);
+        cp_async_commit();
+        const float* wrow = ring + stage * STAGE + col * RS_LD;
+        const float* arow = ring + stage * STAGE + (BN + row0) * RS_LD;
+        stage = stage + 1 == RS_STAGES ? 0 : stage + 1;
+        fill = fill + 1 == RS_STAGES ? 0 : fill + 1;
+#pragma unroll
+        for (int kk = 0; kk < RS_BK; kk += 4) {
+            float4 w[CPL];
+#pragma unroll
+            for (int c = 0; c < CPL; ++c) w[c] = *reinterpret_cast<const float4*>(wrow + 16 * c * RS_LD + kk);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
                 const float4 a = *reinterpret_cast<const float4*>(arow + i * RS_LD + kk);
-                acc[i] = fmaf(a.x, w.x, acc[i]);
-                acc[i] = fmaf(a.y, w.y, acc[i]);
-                acc[i] = fmaf(a.z, w.z, acc[i]);
-                acc[i] = fmaf(a.w, w.w, acc[i]);
+#pragma unroll
+                for (int c = 0; c < CPL; ++c) {
+                    acc[i][c] = fmaf(a.x, w[c].x, acc[i][c]);
+                    acc[i][c] = fmaf(a.y, w[c].y, acc[i][c]);
+                    acc[i][c] = fmaf(a.z, w[c].z, acc[i][c]);
+                    acc[i][c] = fmaf(a.w, w[c].w, acc[i][c]);
+                }
             }
         }
     }
     cp_async_wait<0>();
-    if (n0 + tx < N) {
+    __syncthreads();                             // the rings are free: the ranges' sums meet there
+    float* parts = rs_buf;                       // [ranges][2 R][BN]
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int m = m0 + ty * 4 + i;
-            if (m < M) C[(int64_t)m * ldc + n0 + tx] = acc[i];
-        }
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) parts[(warp * 2 * R + row0 + i) * BN + 16 * c + col] = acc[i][c];
+    __syncthreads();
+    for (int o = threadIdx.x; o < 2 * R * BN; o += RS_THREADS) {
+        const int r = o / BN, c = o % BN;
+        if (r >= M || n0 + c >= N) continue;
+        float v = parts[o];
+#pragma unroll
+        for (int q = 1; q < K_RANGES; ++q) v += parts[q * 2 * R * BN + o];
+        C[(int64_t)r * ldc + n0 + c] = v;
     }
 }
 
 // ------------------------------------------------------------------ tile kernel
 
-#define TL_BM 128
-#define TL_BN 128
 #define TL_BK 16
-#define TL_LD (TL_BM + 4)
-#define TL_THREADS 256
+#define TL_LD (TL_BK + 4)       // row stride in shared memory: 16-byte reads of 8 neighbouring rows hit 8 groups of banks
+#define TL_THREADS 128
+#define TL_TM 4                 // a thread's rows and columns of the tile
+#define TL_TN 8
+#define TL_BM (16 * TL_TM)
+#define TL_BN (8 * TL_TN)
 
-__global__ void __launch_bounds__(TL_THREADS, 2) gemm_f32_tile_kernel(const float* __restrict__ A, int64_t lda,
+#define TL_SMEM ((2 * (TL_BM + TL_BN) * TL_LD + TL_BM * TL_BN) * (int)sizeof(float))
+
+// Rows of A and W lie in shared memory as in memory (16-byte copies), and a thread reads four k of a row at a time: twelve
+// reads feed 128 multiply-adds, and four blocks on an SM hide one another's loads.  (Tiles of 128 x 128 with 8 x 16 a thread:
+// the same 38 TFLOP/s at 2,048 rows and less where tiles are few; with operands transposed for multiply-adds in packed pairs
+// 40 TFLOP/s, 29 at 777 rows.  A loop of nothing but multiply-adds on three registers runs at 61 here.)
+// SPLIT: a cluster of eight CTAs shares an output tile, each takes one range of K, and each adds up and writes an eighth of
+// the tile's rows.
+// Measured (B200): the 112 products of a 777-token prompt at Qwen3-0.6B sizes, with one chain over K and tiles of 128 x 128
+// 32.8 ms, this 20.6 ms.
+template <bool SPLIT>
+__global__ void __launch_bounds__(TL_THREADS, 4) gemm_f32_tile_kernel(const float* __restrict__ A, int64_t lda,
                                                                       const float* __restrict__ W, int64_t ldw,
                                                                       float* __restrict__ C, int64_t ldc, int M, int N,
                                                                       int K) {
-    __shared__ __align__(16) float As[2][TL_BK][TL_LD];        // transposed: [k][row]
-    __shared__ __align__(16) float Ws[2][TL_BK][TL_LD];
-    const int m0 = blockIdx.y * TL_BM, n0 = blockIdx.x * TL_BN;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;      // columns tx * 4 .. + 3 and 64 + ..; rows ty * 4 .. likewise
-    const int nt = (K + TL_BK - 1) / TL_BK;
-    // a tile is 128 rows x 4 chunks of 4 floats: two chunks of A and two of W a thread
-    const int lrow = threadIdx.x >> 2, lseg = (threadIdx.x & 3) * 4;
-    float4 ra[2], rw[2];
+    constexpr int TM = TL_TM, TN = TL_TN, BM = TL_BM, BN = TL_BN;
+    extern __shared__ __align__(16) float tl_buf[];
+    float* ring = tl_buf;                                        // [2][BM + BN][LD]: rows of A, then of W
+    float* total = ring + 2 * (BM + BN) * TL_LD;                 // the ranges' sum so far, [element][thread]; SPLIT: [row][column]
+    const int part = SPLIT ? blockIdx.x % K_RANGES : 0;
+    const int m0 = blockIdx.y * BM, n0 = (SPLIT ? blockIdx.x / K_RANGES : blockIdx.x) * BN;
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;       // columns tx + 8 j, rows ty + 16 i
+    const int range = k_range(K);
+    const int kbeg = SPLIT ? min(K, part * range) : 0, kend = SPLIT ? min(K, kbeg + range) : K;
+    const int nt = (kend - kbeg + TL_BK - 1) / TL_BK;
 
-    auto fetch = [&](int t) {
-        const int k = t * TL_BK + lseg;
+    auto load = [&](int t) {
+        float* dst = ring + (t & 1) * (BM + BN) * TL_LD;
+        const int seg = (threadIdx.x & 3) * 4, k = kbeg + t * TL_BK + seg;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int row = lrow + e * 64;
-            ra[e] = (m0 + row < M && k < K) ? *reinterpret_cast<const float4*>(A + (int64_t)(m0 + row) * lda + k)
-                                            : make_float4(0.f, 0.f, 0.f, 0.f);
-            rw[e] = (n0 + row < N && k < K) ? *reinterpret_cast<const float4*>(W + (int64_t)(n0 + row) * ldw + k)
-                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int e = 0; e < (BM + BN) / 32; ++e) {
+            const int row = e * 32 + (threadIdx.x >> 2);
+            const bool of_a = e < BM / 32;
+            const int at = of_a ? m0 + row : n0 + row - BM;
+            const bool valid = k < kend && at < (of_a ? M : N);
+            const float* src = of_a ? A + (int64_t)at * lda + k : W + (int64_t)at * ldw + k;
+            cp_async_16(smem_addr(dst + row * TL_LD + seg), valid ? src : W, valid);
         }
-    };
-    auto stash = [&](int buf) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int row = lrow + e * 64;
-            As[buf][lseg + 0][row] = ra[e].x; As[buf][lseg + 1][row] = ra[e].y;
-            As[buf][lseg + 2][row] = ra[e].z; As[buf][lseg + 3][row] = ra[e].w;
-            Ws[buf][lseg + 0][row] = rw[e].x; Ws[buf][lseg + 1][row] = rw[e].y;
-            Ws[buf][lseg + 2][row] = rw[e].z; Ws[buf][lseg + 3][row] = rw[e].w;
-        }
+        cp_async_commit();
     };
 
-    float acc[8][8];
+    float acc[TM][TN];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    fetch(0);
-    stash(0);
-    __syncthreads();
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    pdl_wait();
+    pdl_trigger();
+    if (nt > 0) load(0);
+    bool folded = false;
     for (int t = 0; t < nt; ++t) {
-        const int buf = t & 1;
-        if (t + 1 < nt) fetch(t + 1);            // in flight while this tile is multiplied
+        cp_async_wait<0>();
+        __syncthreads();                         // tile t is there for all, and all are done with the one before it
+        if (t + 1 < nt) load(t + 1);
+        if (!SPLIT && t > 0 && (t * TL_BK) % range == 0) {
 #pragma unroll
-        for (int kk = 0; kk < TL_BK; ++kk) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][kk][64 + ty * 4]);
-            const float4 w0 = *reinterpret_cast<const float4*>(&Ws[buf][kk][tx * 4]);
-            const float4 w1 = *reinterpret_cast<const float4*>(&Ws[buf][kk][64 + tx * 4]);
-            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+                for (int j = 0; j < TN; ++j) {
+                    float* p = total + (i * TN + j) * TL_THREADS + threadIdx.x;
+                    *p = folded ? *p + acc[i][j] : acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+            folded = true;
         }
-        if (t + 1 < nt) stash(buf ^ 1);          // the other buffer was last read before the barrier below, a tile ago
-        __syncthreads();
+        const float* a_at = ring + (t & 1) * (BM + BN) * TL_LD + ty * TL_LD;
+        const float* w_at = ring + ((t & 1) * (BM + BN) + BM + tx) * TL_LD;
+#pragma unroll
+        for (int kk = 0; kk < TL_BK; kk += 4) {
+            float4 a[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(a_at + 16 * i * TL_LD + kk);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const float4 w = *reinterpret_cast<const float4*>(w_at + 8 * j * TL_LD + kk);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, w.x, acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].y, w.y, acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].z, w.z, acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, w.w, acc[i][j]);
+            }
+        }
+    }
+    if (SPLIT) {
+        cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) total[(ty + 16 * i) * BN + tx + 8 * j] = acc[i][j];
+        cluster.sync();
+        const float4* mine = reinterpret_cast<const float4*>(total);
+#pragma unroll 2
+        for (int o = threadIdx.x; o < BM / K_RANGES * BN / 4; o += TL_THREADS) {
+            const int row = part * (BM / K_RANGES) + o / (BN / 4), c = (o % (BN / 4)) * 4, at = (row * BN + c) / 4;
+            if (m0 + row >= M) break;
+            float4 p[K_RANGES];
+#pragma unroll
+            for (int q = 0; q < K_RANGES; ++q) p[q] = cluster.map_shared_rank(mine, q)[at];
+            float v[4] = {p[0].x, p[0].y, p[0].z, p[0].w};
+#pragma unroll
+            for (int q = 1; q < K_RANGES; ++q) { v[0] += p[q].x; v[1] += p[q].y; v[2] += p[q].z; v[3] += p[q].w; }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (n0 + c + e < N) C[(int64_t)(m0 + row) * ldc + n0 + c + e] = v[e];
+        }
+        cluster.sync();                          // a CTA's shared memory stays until all have read it
+        return;
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
-        if (m >= M) continue;
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + ty + 16 * i;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-            if (n < N) C[(int64_t)m * ldc + n] = acc[i][j];
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + tx + 8 * j;
+            if (m < M && n < N)
+                C[(int64_t)m * ldc + n] = folded ? total[(i * TN + j) * TL_THREADS + threadIdx.x] + acc[i][j] : acc[i][j];
         }
     }
 }
 
 // ------------------------------------------------------------------ host side
 
+template <int R, int CPL>
+static int launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
+                       cudaStream_t stream) {
+    static AcornPerDevice configured;
+    if (!configured.seen()) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<R, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, rs_smem<R, CPL>());
+        if (e != cudaSuccess) return (int)e;
+        configured.mark();
+    }
+    return acorn_launch(gemm_f32_rows_kernel<R, CPL>, dim3((N + 16 * CPL - 1) / (16 * CPL)), dim3(RS_THREADS), rs_smem<R, CPL>(), stream,
+                        A, lda, W, ldw, C, ldc, M, N, K);
+}
+
+template <bool SPLIT>
+static int launch_tile(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
+                       cudaStream_t stream) {
+    static AcornPerDevice configured;
+    if (!configured.seen()) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured.mark();
+    }
+    const int tn = (N + TL_BN - 1) / TL_BN, tm = (M + TL_BM - 1) / TL_BM;
+    if (tm > 65535 || (int64_t)tn * K_RANGES > 0x7fffffff) return ACORN_ERR_UNSUPPORTED;
+    if (!SPLIT)
+        return acorn_launch(gemm_f32_tile_kernel<SPLIT>, dim3(tn, tm), dim3(TL_THREADS), TL_SMEM, stream, A, lda, W, ldw,
+                            C, ldc, M, N, K);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tn * K_RANGES, tm);
+    cfg.blockDim = dim3(TL_THREADS);
+    cfg.dynamicSmemBytes = TL_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = K_RANGES;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = acorn_pdl_enabled() ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<SPLIT>, A, lda, W, ldw, C, ldc, M, N, K);
+    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
 extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, float* C,
                               int64_t ldc, int M, int N, int K, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     // the faster kernels move 16 bytes at a time along K
     const bool aligned = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
-    if (aligned && M <= 64) {
-        static AcornPerDevice configured;
-        if (!configured.seen()) {
-            cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM);
-            if (e != cudaSuccess) return (int)e;
-            configured.mark();
-        }
-        const int mblocks = (M + RS_ROWS - 1) / RS_ROWS;
-        const int64_t blocks = (int64_t)((N + RS_BN - 1) / RS_BN) * mblocks;
-        if (blocks > 0x7fffffff) return ACORN_ERR_UNSUPPORTED;
-        gemm_f32_rows_kernel<<<(unsigned)blocks, RS_THREADS, RS_SMEM, stream>>>(A, lda, W, ldw, C, ldc, M, N, K, mblocks);
-        return acorn_launch_status();
+    if (aligned && M <= 16) {
+        const bool wide = N >= 8192;             // blocks of 32 columns still cover the device
+        if (M <= 4)
+            return wide ? launch_rows<2, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<2, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+        if (M <= 8)
+            return wide ? launch_rows<4, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<4, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+        return wide ? launch_rows<8, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<8, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
     if (aligned) {
-        dim3 grid((N + TL_BN - 1) / TL_BN, (M + TL_BM - 1) / TL_BM);
-        if (grid.y > 65535) return ACORN_ERR_UNSUPPORTED;
-        gemm_f32_tile_kernel<<<grid, TL_THREADS, 0, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
-        return acorn_launch_status();
+        // A cluster to a tile where whole tiles would leave an SM fewer than four of them, which is what hides their loads'
+        // latency (777 rows, N = 1,024, K = 2,048, 208 tiles: 146 -> 98 us; N = 4,096, K = 1,024, 832 tiles: 203 against 199 us
+        // whole), and a range of K is worth its share of the exchange.
+        const int64_t tiles = (int64_t)((N + TL_BN - 1) / TL_BN) * ((M + TL_BM - 1) / TL_BM);
+        if (tiles < 4 * 148 && K >= 256) return launch_tile<true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+        return launch_tile<false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+    dim3 grid((N + PL_BN - 1) / PL_BN, (M + PL_BM - 1) / PL_BM);
     if (grid.y > 65535) return ACORN_ERR_UNSUPPORTED;
     gemm_f32_kernel<<<grid, 256, 0, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
     return acorn_launch_status();

@@ -1,6 +1,7 @@
 """Choice of the attention kernel for a step, behind one call.
 
-The float32 engine always runs the plain kernel.  The bfloat16 engine runs the split-K
+The float32 engine runs its own prefill and decode kernels (head sizes 64 and 128, causal masks with or without a
+window) and the plain kernel for everything else.  The bfloat16 engine runs the split-K
 decode kernel when every row of the step is a single token, the tensor-core prefill kernel
 otherwise (a single-token row is then a tile of one query), and the plain kernel for head
 sizes and group sizes the fast kernels do not take.
@@ -181,6 +182,22 @@ def paged_attention(qkv: torch.Tensor, inputs, group, cache, nq: int, nkv: int, 
                                      decode_splits(n_single, nkv, bound, d, sm_count(qkv.device),
                                                    _merge_free(nq, nkv, d, P) if windowed_only else 1),
                                      token_list=x["attention.single_tokens"], out=out, **mask)
+            return out
+    if qkv.dtype == torch.float32 and (value_dim is None or value_dim == d) and windowed_only and cache.k_pages.shape == cache.v_pages.shape:
+        # a row of one token goes to the decode kernel whatever else is in the step, so that its bits stay the same
+        n_single = inputs.num_tokens if inputs.plan.all_decode else int(inputs.plan.extra["attention.single_tokens"].size)
+        chunks = ops.f32_decode_chunks(_key_bound(group.block_table.shape[1] * P, window, None, 0), window)
+        if n_single <= 65535 and ops.attention_f32_supported(nq, nkv, d, n_single, chunks):
+            out = torch.empty((inputs.num_tokens, nq * d), dtype=qkv.dtype, device=qkv.device)
+            if n_single < inputs.num_tokens:
+                ops.attention_f32_prefill(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table, group.page_base,
+                                          inputs.row_start, inputs.row_pos, inputs.extra["attention.q_tiles"], nq, nkv, d, scale,
+                                          window, ops.f32_prefill_chunks(group.block_table.shape[1] * P, window), out)
+            if n_single:
+                ops.attention_f32_decode(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table, group.page_base,
+                                         inputs.token_row, inputs.positions,
+                                         None if inputs.plan.all_decode else inputs.extra["attention.single_tokens"], n_single, nq,
+                                         nkv, d, scale, window, chunks, out)
             return out
     return ops.attention_plain(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table,
                                group.page_base, inputs.token_row, inputs.positions, inputs.num_tokens,

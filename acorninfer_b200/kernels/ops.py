@@ -118,6 +118,11 @@ class _Sigs:
                         c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                         c_void_p]
     acorn_scan_chunk_supported = [c_int, c_int]
+    acorn_attention_f32_supported = [c_int, c_int, c_int]
+    acorn_attention_f32_prefill = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
+                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p]
+    acorn_attention_f32_decode = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
+                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p]
     acorn_bigram_add = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                         c_int, c_int, c_int, c_int, c_void_p]
     acorn_rmsnorm_add = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]
@@ -692,6 +697,75 @@ def _check_sink(sink32: torch.Tensor | None, num_heads: int) -> None:
     if sink32 is not None:
         _check(sink32, "sink", torch.float32, 1)
         if sink32.numel() != num_heads:
+F32_DECODE_KEYS = 128       # keys a block of the float32 decode kernel takes
+F32_Q_TILE = 64             # queries a tile of the float32 prefill kernel takes
+_F32_SCRATCH_MAX = 1 << 28  # floats of partial results (1 GB): beyond, the plain kernel
+
+
+F32_PREFILL_KEYS = 512      # keys a block of the float32 prefill kernel walks
+
+
+def f32_decode_chunks(key_bound: int, window: int | None) -> int:
+    """Blocks of keys that a single-token row of the float32 decode kernel can touch: its keys end anywhere in the bound,
+    and a window may start inside a block."""
+    return -(-key_bound // F32_DECODE_KEYS) + (1 if window else 0)
+
+
+def f32_prefill_chunks(table_keys: int, window: int | None) -> int:
+    """Runs of keys that a tile of the float32 prefill kernel can touch: its queries' windows lie one after the other."""
+    keys = min(table_keys, window + F32_Q_TILE) if window else table_keys
+    return -(-keys // F32_PREFILL_KEYS) + (1 if window else 0)
+
+
+def attention_f32_supported(num_heads: int, num_kv_heads: int, head_dim: int, num_tokens: int = 0, chunks: int = 0) -> bool:
+    """Whether the float32 prefill and decode kernels take these heads, and the decode kernel ``num_tokens`` rows of
+    ``chunks`` key blocks."""
+    return (bool(lib().acorn_attention_f32_supported(num_heads, num_kv_heads, head_dim)) and chunks <= 65535
+            and num_tokens * num_heads * chunks * (head_dim + 2) <= _F32_SCRATCH_MAX)
+
+
+def attention_f32_prefill(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
+                          page_base: torch.Tensor, row_start: torch.Tensor, row_pos: torch.Tensor, tiles: torch.Tensor, num_heads: int,
+                          num_kv_heads: int, head_dim: int, scale: float, window: int | None, chunks: int, out: torch.Tensor) -> torch.Tensor:
+    """Float32 causal attention of the query tiles listed in ``tiles`` (int32 [n, 2]: row, first token within the row;
+    64 tokens a tile at most), into their rows of ``out`` [tokens, nq * d].  ``chunks``: see ``f32_prefill_chunks``."""
+    for t, name in ((k_pages, "k_pages"), (v_pages, "v_pages")):
+        _check(t, name, torch.float32, 4)
+    _check(out, "out", torch.float32, 2)
+    # partial results of tiles whose keys are several blocks' work, of as many tiles at a time as fit the scratch
+    each = F32_Q_TILE * num_heads * chunks * (head_dim + 2)
+    at_once = tiles.shape[0] if chunks == 1 else max(1, min(tiles.shape[0], _F32_SCRATCH_MAX // each))
+    part = torch.empty(at_once * each if chunks > 1 else 0, dtype=torch.float32, device=q.device)
+    for at in range(0, tiles.shape[0], at_once):
+        n = min(at_once, tiles.shape[0] - at)
+        _ok(lib().acorn_attention_f32_prefill(q.data_ptr(), q_stride, out.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(),
+                                              block_table.data_ptr(), page_base.data_ptr(), block_table.stride(0), row_start.data_ptr(),
+                                              row_pos.data_ptr(), tiles.data_ptr() + 8 * at, n, num_heads, num_kv_heads, head_dim,
+                                              k_pages.shape[2], float(scale), int(window or 0), chunks, part.data_ptr(),
+                                              part.data_ptr() + 4 * n * F32_Q_TILE * num_heads * chunks * head_dim, _stream()),
+            "attention_plain")
+    return out
+
+
+def attention_f32_decode(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
+                         page_base: torch.Tensor, token_row: torch.Tensor, positions: torch.Tensor, token_list: torch.Tensor | None,
+                         num_rows: int, num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int | None,
+                         chunks: int, out: torch.Tensor) -> torch.Tensor:
+    """Float32 attention of single-token rows: tokens 0..num_rows-1, or the ``num_rows`` listed in ``token_list``.
+    ``chunks``: see ``f32_decode_chunks``."""
+    for t, name in ((k_pages, "k_pages"), (v_pages, "v_pages")):
+        _check(t, name, torch.float32, 4)
+    _check(out, "out", torch.float32, 2)
+    part_o = torch.empty((num_rows, num_heads, chunks, head_dim), dtype=torch.float32, device=q.device)
+    part_ml = torch.empty((num_rows, num_heads, chunks, 2), dtype=torch.float32, device=q.device)
+    _ok(lib().acorn_attention_f32_decode(q.data_ptr(), q_stride, out.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(),
+                                         block_table.data_ptr(), page_base.data_ptr(), block_table.stride(0), token_row.data_ptr(),
+                                         positions.data_ptr(), _ptr(token_list), num_rows, num_heads, num_kv_heads, head_dim,
+                                         k_pages.shape[2], float(scale), int(window or 0), chunks, part_o.data_ptr(),
+                                         part_ml.data_ptr(), _stream()), "attention_plain")
+    return out
+
+
             raise KernelError("sink must have one entry per query head")
 
 

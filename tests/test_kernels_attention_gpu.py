@@ -122,6 +122,55 @@ def test_attention_plain(dtype, nq, nkv, d, P, window):
     assert torch.allclose(out.double().cpu(), want, **tol)
 
 
+@pytest.mark.parametrize("nq,nkv,d,P,window", [(4, 2, 128, 16, None), (8, 1, 128, 4, None), (6, 2, 64, 16, None), (4, 4, 128, 32, 130),
+                                               (16, 4, 64, 8, 1)])
+def test_attention_float32_prefill_and_decode(nq, nkv, d, P, window):
+    """Rows around the kernels' tiles (64 queries, 64 and 128 keys, runs of 512 keys), decoded rows beside portions, one to eight query heads
+    to a kv head; a row's bits do not depend on the step's other rows or on tokens after it."""
+    before, qlens = [0, 300, 129, 0, 63, 127, 128, 1100, 490], [65, 1, 64, 2, 1, 1, 1, 3, 130]
+    num_pages = sum(-(-(b + n) // P) for b, n in zip(before, qlens)) + 7
+    lay = rows_layout(before, qlens, P, num_pages, seed=4)
+    scale = d ** -0.5
+    k_pages = torch.randn(num_pages, nkv, P, d, device=DEV)
+    v_pages = torch.randn_like(k_pages)
+    qs, wants = [], []
+    for r, (b, n) in enumerate(zip(before, qlens)):
+        k, v, q = torch.randn(b + n, nkv, d), torch.randn(b + n, nkv, d), 2 * torch.randn(n, nq, d)
+        scatter_to_pages(k_pages, lay["tables"][r], k.to(DEV), P)
+        scatter_to_pages(v_pages, lay["tables"][r], v.to(DEV), P)
+        qs.append(q)
+        wants.append(dense_attention(q.double(), k.double(), v.double(), scale, window, b))
+    q_all = torch.cat(qs).reshape(-1, nq * d).to(DEV)
+    wide = torch.cat([q_all, torch.randn(q_all.shape[0], 2 * nkv * d, device=DEV)], dim=1).contiguous()
+    starts = [0]
+    for n in qlens:
+        starts.append(starts[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    tiles = [(r, q0) for r, n in enumerate(qlens) if n > 1 for q0 in range(0, n, 64)]
+    single = [starts[r] for r, n in enumerate(qlens) if n == 1]
+    chunks = ops().f32_decode_chunks(min(window or 1 << 20, lay["block_table"].shape[1] * P), window)
+    common = (k_pages, v_pages, lay["block_table"], lay["page_base"])
+
+    def run(tiles, single):
+        out = torch.zeros(starts[-1], nq * d, device=DEV)
+        ops().attention_f32_prefill(wide, wide.stride(0), *common, i32(starts), i32(before), i32(tiles).view(-1, 2), nq, nkv, d, scale,
+                                    window, ops().f32_prefill_chunks(lay["block_table"].shape[1] * P, window), out)
+        ops().attention_f32_decode(wide, wide.stride(0), *common, lay["token_row"], lay["positions"], i32(single), len(single), nq,
+                                   nkv, d, scale, window, chunks, out)
+        return out
+
+    out = run(tiles, single)
+    want = torch.cat(wants).reshape(-1, nq * d)
+    assert torch.allclose(out.double().cpu(), want, atol=2e-5, rtol=1e-4)
+    alone = run(tiles[-1:], single[-1:])
+    last, (r, q0) = single[-1], tiles[-1]
+    assert torch.equal(alone[last], out[last])
+    assert torch.equal(alone[starts[r] + q0:starts[r + 1]], out[starts[r] + q0:starts[r + 1]])
+    # the same queries in tiles that start elsewhere: rows 1.. of the first row as tile (0, 1)
+    moved = run([(0, 1)], single[:1])
+    assert torch.equal(moved[1:starts[1]], out[1:starts[1]])
+
+
 def build_case(before, qlens, nq, nkv, d, P, window, num_pages, seed, standout_row=None):
     """Random paged K/V and queries for rows with ``before`` cached tokens and ``qlens`` new ones;
     returns the device inputs and the plain float64 result [tokens, nq * d]."""
