@@ -693,10 +693,6 @@ def attention_plain(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_pag
     return out
 
 
-def _check_sink(sink32: torch.Tensor | None, num_heads: int) -> None:
-    if sink32 is not None:
-        _check(sink32, "sink", torch.float32, 1)
-        if sink32.numel() != num_heads:
 F32_DECODE_KEYS = 128       # keys a block of the float32 decode kernel takes
 F32_Q_TILE = 64             # queries a tile of the float32 prefill kernel takes
 _F32_SCRATCH_MAX = 1 << 28  # floats of partial results (1 GB): beyond, the plain kernel
@@ -766,6 +762,10 @@ def attention_f32_decode(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, 
     return out
 
 
+def _check_sink(sink32: torch.Tensor | None, num_heads: int) -> None:
+    if sink32 is not None:
+        _check(sink32, "sink", torch.float32, 1)
+        if sink32.numel() != num_heads:
             raise KernelError("sink must have one entry per query head")
 
 
