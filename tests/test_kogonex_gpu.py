@@ -280,12 +280,47 @@ def test_router_choice_matches_plain(N, top, groups, keep):
         assert max(abs(float(a) - float(b)) for (_, a), b in zip(want, wts[t])) < 1e-6
 
 
+@pytest.mark.parametrize("N,K,scaled,limit", [(128, 64, False, 0.0), (600, 136, True, 0.0), (520, 1032, False, 7.0), (34, 72, True, 3.0)])
+@pytest.mark.parametrize("tcgen05", [True, False])
+def test_grouped_products_of_many_rows(N, K, scaled, limit, tcgen05, monkeypatch):
+    """The paired tcgen05 kernel (tiles of 256 rows) and the mma.sync one: experts with no row, one row, a tile
+    and a row more, hundreds; widths that fill no tile; factors by slot and the capped form in the epilogue.  Inputs are
+    bfloat16 numbers, sums float32, one rounding to bfloat16: 2^-8 of the result and float32 sums' 2e-5 of the operands'
+    norms."""
+    o = ops()
+    monkeypatch.setattr(o, "GROUPED_TCGEN05_MIN_ROWS", 1 if tcgen05 else 10 ** 9)
+    counts = [0, 1, 256, 257, 0, 130, 515, 3, 128]
+    E, slots = len(counts), sum(counts) + 9                     # nine rows of no expert at the end
+    g = torch.Generator().manual_seed(N)
+    rows = torch.randint(0, 700, (slots,), generator=g, dtype=torch.int32).to(DEV)
+    x = torch.randn(700, K, generator=g).bfloat16().to(DEV)
+    w = (torch.randn(E, N, K, generator=g) / K ** 0.5).bfloat16().to(DEV)
+    scale = (torch.rand(slots, generator=g) + 0.5).to(DEV) if scaled else None
+    offsets = torch.tensor([sum(counts[:e]) for e in range(E + 1)] + [slots], dtype=torch.int32, device=DEV)
+    for act in (False, True):
+        out = o.grouped_gemm(x, rows, w, offsets, slots, swiglu_pairs=act, slot_scale=scale,
+                             **(dict(activation="capped_swish", limit=limit) if act and limit else {}))
+        for e in range(E):
+            a, b = sum(counts[:e]), sum(counts[:e + 1])
+            want = x[rows[a:b].long()].double() @ w[e].double().T
+            if scaled:
+                want = want * scale[a:b, None].double()
+            if act:
+                gate, up = want[:, 0::2], want[:, 1::2]
+                if limit:
+                    gate, up = gate.clamp(max=limit), up.clamp(-limit, limit) + 1.0
+                want = gate * torch.sigmoid((1.702 if limit else 1.0) * gate) * up
+            got = out[a:b].double()
+            assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2e-4).all(), (e, act)
+    assert o.lib().acorn_gemm_tc_pair_error() == 0
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-4), (torch.bfloat16, 0.15)])
 @pytest.mark.parametrize("E,T,top,min_rows", [(7, 90, 2, None), (2, 300, 2, None), (12, 5, 2, None), (3, 400, 2, 10 ** 9)])
 def test_grouped_products_take_each_experts_own_rows(dtype, tol, E, T, top, min_rows, monkeypatch):
     """Rows scattered over experts, some experts with no rows and some with more than a tile: every
     row against its own expert's matrix.  In bfloat16 the second shape has enough rows an expert for the
-    tcgen05 kernel (tiles of 128 rows, an expert's last tile partly another's rows); the others, and the
+    tcgen05 kernel (tiles of 256 rows, an expert's last tile partly another's rows); the others, and the
     last with that kernel switched off, take the three tile heights of the mma.sync kernel (64, 16, 128)."""
     o = ops()
     if min_rows is not None:
