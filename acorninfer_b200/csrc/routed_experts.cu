@@ -805,10 +805,100 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const T* __restrict_
     }
 }
 
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[q]));
+        v[2 * q] = f.x;
+        v[2 * q + 1] = f.y;
+    }
+}
+__device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void store8(bf16* p, const float (&v)[8]) {
+    *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+}
+
+#define MC_TOP 8                    // choices of a token whose rows a thread fetches at once
+
+// The same with eight entries of the row a thread, which stay in registers between the sum and the norm; the choices' rows are
+// fetched together.  Bound by their latency and by 2-byte reads before: 2,000 tokens of 6 choices, rows of 2,048, 52 -> 18 us
+// (90 MB).  The sums run in the same order.
+template <typename T>
+__global__ void __launch_bounds__(512) moe_combine_vec_kernel(const T* __restrict__ y, const T* __restrict__ x, const int* __restrict__ slot_of,
+                                                               const int* __restrict__ idx, const float* __restrict__ wts, T* __restrict__ out,
+                                                               int H, int top, int E, float* __restrict__ resid32,
+                                                               const float* __restrict__ norm_w, float eps, const T* __restrict__ extra,
+                                                               const float* __restrict__ extra_z, int64_t ldz) {
+    __shared__ float scratch[32];
+    pdl_wait();
+    pdl_trigger();
+    const int64_t t = blockIdx.x;
+    const int i = threadIdx.x * 8;
+    const bool on = i < H;
+    const T* row[MC_TOP];
+    float w[MC_TOP];
+#pragma unroll
+    for (int k = 0; k < MC_TOP; ++k) {
+        const int64_t p = t * top + (k < top ? k : 0);
+        row[k] = idx[p] >= E ? x + t * H : y + (int64_t)slot_of[p] * H;
+        w[k] = wts ? wts[p] : 1.f;
+    }
+    float acc[8] = {};
+    if (on) {
+        float v[MC_TOP][8];
+#pragma unroll
+        for (int k = 0; k < MC_TOP; ++k)
+            if (k < top) load8(row[k] + i, v[k]);
+#pragma unroll
+        for (int k = 0; k < MC_TOP; ++k)
+            if (k < top)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[e] = fmaf(w[k], v[k][e], acc[e]);
+        if (extra) {
+            const float gate = extra_z ? 1.f / (1.f + expf(-extra_z[t * ldz])) : 1.f;
+            load8(extra + t * H + i, v[0]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] = fmaf(gate, v[0][e], acc[e]);
+        }
+        if (!resid32) store8(out + t * H + i, acc);
+    }
+    if (!resid32) return;
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += acc[e] * acc[e];
+    float r[8], nw[8];
+    if (on) {
+        load8(resid32 + t * H + i, r);
+        load8(norm_w + i, nw);
+    }
+    ss = block_sum(ss, scratch);
+    const float inv = rsqrtf(ss / (float)H + eps);
+    if (!on) return;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r[e] += acc[e] * inv * nw[e];
+    store8(resid32 + t * H + i, r);
+    if (out) store8(out + t * H + i, r);
+}
+
 extern "C" int acorn_moe_combine(const void* y, const void* x, const int* slot_of, const int* idx, const float* wts, void* out,
                                  int tokens, int H, int top, int E, int dtype, float* resid32, const float* norm_w, float eps,
                                  const void* extra, const float* extra_z, int64_t ldz, cudaStream_t stream) {
     if (tokens <= 0) return 0;
+    const uintptr_t rows = (uintptr_t)y | (uintptr_t)x | (uintptr_t)out | (uintptr_t)resid32 | (uintptr_t)norm_w | (uintptr_t)extra;
+    if (H % 8 == 0 && H <= 4096 && top <= MC_TOP && (rows & 15) == 0) {
+        ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(moe_combine_vec_kernel<T>, dim3(tokens), dim3((H / 8 + 31) / 32 * 32), 0, stream,
+                                                           (const T*)y, (const T*)x, slot_of, idx, wts, (T*)out, H, top, E, resid32,
+                                                           norm_w, eps, (const T*)extra, extra_z, ldz));
+    }
     const size_t smem = resid32 ? (size_t)H * sizeof(float) : 0;
     if (smem > 48 * 1024) return ACORN_ERR_UNSUPPORTED;
     ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(moe_combine_kernel<T>, dim3(tokens), dim3(256), smem, stream, (const T*)y,
