@@ -184,30 +184,39 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
 // with top-k and top-p: 701 us).  Here the CTAs of a cluster hold the row in shared memory, read from HBM once, and the
 // bounds of top-k and top-p are found digit by digit (11 + 11 + 10 bits of the ordered key): a histogram of the
 // candidates a level, summed over the cluster through distributed shared memory.  Both are one question: the smallest
-// key K with weight(lo_key <= key <= K) > limit, where a key weighs 1 and limit is V - k (the k-th largest), or weighs
-// its probability and limit is (1 - top_p) of the total.  Probabilities are summed as integers of 2^-44 of the largest
-// one (a sum's error is below that of float32 sums, and its order does not matter).
+// key K with weight(keys <= K) > limit, where a key weighs 1 and limit is the number of keys less k (the k-th largest), or
+// weighs its probability and limit is (1 - top_p) of the total.  Most keys are no candidates and cost no atomic: for k up
+// to the number of warps, those below the least of the warps' maxima; for top-p, those so improbable that all of them
+// together would stay within the limit.  Probabilities are summed as integers of 2^-44 of the largest one (a sum's error
+// is below that of float32 sums, and its order does not matter).
 #define SC_THREADS 512
 #define SC_WARPS (SC_THREADS / 32)
 #define SC_BINS 2048
-#define SC_MAX_CLUSTER 8
+#define SC_CLUSTER 8
 #define SC_MAX_SLICE 45056          // floats of a row a CTA can hold beside the histogram
 typedef unsigned long long u64;
 
 struct alignas(16) ScShared {
-    u64 sums[SC_BINS];              // this CTA's share of a level's bins, summed over the cluster (bins / cluster of them)
+    u64 sums[SC_BINS / SC_CLUSTER]; // this CTA's share of a level's bins, summed over the cluster
     unsigned int hist[3][SC_BINS];  // a level's weights: 16-bit pieces, so that 32-bit atomics cannot overflow
     u64 total;                      // of `sums`
     u64 kept;                       // this CTA's part of the kept set
     u64 best;                       // largest (key, ~index) of this CTA's slice
+    unsigned int low;               // key of the least of its warps' maxima
+    u64 z;                          // probability of its slice
     unsigned int bad;
     u64 warp_a[SC_WARPS];
     u64 found_cum;                  // answer of a level: weight below the bin, the bin (SC_BINS: limit not exceeded)
     unsigned int found_bin;
 };
 
+// e^((x - gmax) / t) in units of 2^-44, cut off below; by shifts of the mantissa (a conversion to 64 bits runs at a sixteenth
+// of their rate).  NaN, which 0 * inf gives, counts as 0.
 __device__ __forceinline__ u64 prob_fixed(float x, float gmax, float inv_t) {
-    return __float2ull_rn(expf((x - gmax) * inv_t) * 17592186044416.f);
+    const unsigned int b = __float_as_uint(expf((x - gmax) * inv_t));
+    const int shift = (int)(b >> 23) - 106;                     // 2^(exponent - 150 + 44) a unit of the mantissa; at most 21
+    const u64 m = (b & 0x7fffffu) | 0x800000u;
+    return shift > 21 || shift < -24 ? 0ull : shift >= 0 ? m << shift : m >> -shift;
 }
 
 __device__ __forceinline__ u64 warp_sum_u64(u64 v) {
@@ -224,13 +233,13 @@ __device__ __forceinline__ u64 block_sum_u64(u64 v, u64* scratch) {
     return warp_sum_u64((threadIdx.x & 31) < SC_WARPS ? scratch[threadIdx.x & 31] : 0ull);
 }
 
-// The smallest key K of the row with weight(lo_key <= key <= K) > limit(total weight from lo_key on); 0xffffffff if there
-// is none.  Called by all threads of the cluster with the same arguments.
+// The smallest key K of the row from `cut` on with weight(keys <= K) > limit; 0xffffffff if there is none.  MASS: keys from
+// lo_key on weigh their probability, the total is z, the limit (1 - top_p) z; else keys weigh 1 and the limit leaves k above
+// it.  No key below `cut` is K.  Called by all threads of the cluster with the same arguments.
 template <bool MASS>
-__device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigned int lo_key, float gmax, float inv_t, u64 count_limit,
-                                  float drop) {
+__device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigned int cut, float gmax, float inv_t, u64 z, u64 bound) {
     cg::cluster_group cluster = cg::this_cluster();
-    const int c = (int)cluster.num_blocks(), tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
     constexpr int PIECES = MASS ? 3 : 1;
     unsigned int prefix = 0;        // the digits found so far
     u64 limit = 0;
@@ -243,7 +252,7 @@ __device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigne
         for (int i = tid; i < n; i += SC_THREADS) {
             const float v = row[i];
             const unsigned int key = float_key(v);
-            if (key < lo_key || (level > 0 && (key >> above) != prefix)) continue;
+            if (key < cut || (level > 0 && (key >> above) != prefix)) continue;
             const int bin = (key >> shift) & (bins - 1);
             if (MASS) {
                 const u64 w = prob_fixed(v, gmax, inv_t);
@@ -256,15 +265,20 @@ __device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigne
             }
         }
         cluster.sync();
-        // this CTA sums its share of the bins over the cluster
-        const int share = bins / c, first = (int)cluster.block_rank() * share;
+        // this CTA sums its share of the bins over the cluster (all remote reads of a bin in flight at once)
+        const int share = bins / SC_CLUSTER, first = (int)cluster.block_rank() * share;
         u64 mine = 0;
         for (int i = tid; i < share; i += SC_THREADS) {
+            unsigned int h[SC_CLUSTER][PIECES];
+#pragma unroll
+            for (int r = 0; r < SC_CLUSTER; ++r)
+#pragma unroll
+                for (int q = 0; q < PIECES; ++q) h[r][q] = cluster.map_shared_rank(&sh.hist[q][0], r)[first + i];
             u64 s = 0;
-            for (int r = 0; r < c; ++r) {
-                const unsigned int* h = cluster.map_shared_rank(&sh.hist[0][0], r) + first + i;
-                s += h[0];
-                if (MASS) s += ((u64)h[SC_BINS] << 16) + ((u64)h[2 * SC_BINS] << 32);
+#pragma unroll
+            for (int r = 0; r < SC_CLUSTER; ++r) {
+                s += h[r][0];
+                if (MASS) s += ((u64)h[r][PIECES / 2] << 16) + ((u64)h[r][PIECES - 1] << 32);
             }
             sh.sums[i] = s;
             mine += s;
@@ -274,25 +288,30 @@ __device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigne
         cluster.sync();
         // one warp finds the bin: first the CTA whose share holds it, then the bin in that share
         if (tid < 32) {
-            const u64 t = lane < c ? *cluster.map_shared_rank(&sh.total, lane) : 0ull;
+            const u64 t = lane < SC_CLUSTER ? *cluster.map_shared_rank(&sh.total, lane) : 0ull;
             u64 incl = t;
 #pragma unroll
             for (int o = 1; o < 8; o <<= 1) {
                 const u64 up = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += up;
             }
-            const u64 all = __shfl_sync(0xffffffffu, incl, c - 1);
-            if (level == 0) limit = MASS ? (u64)((double)drop * (double)all) : count_limit;
-            const unsigned int over = __ballot_sync(0xffffffffu, lane < c && incl > limit);
+            const u64 all = __shfl_sync(0xffffffffu, incl, SC_CLUSTER - 1);
+            // counted from the cut on: less what lies below it
+            if (level == 0) limit = MASS ? bound - (z - all) : all - bound;
+            const unsigned int over = __ballot_sync(0xffffffffu, lane < SC_CLUSTER && incl > limit);
             if (over == 0) {
                 if (lane == 0) sh.found_bin = SC_BINS;
             } else {
                 const int owner = __ffs(over) - 1;
                 u64 run = __shfl_sync(0xffffffffu, incl - t, owner);
                 const u64* sums = cluster.map_shared_rank(&sh.sums[0], owner);
-                const int per = (share + 31) / 32;
-                u64 part = 0;
-                for (int i = lane * per; i < min(share, (lane + 1) * per); ++i) part += sums[i];
+                constexpr int PER = SC_BINS / SC_CLUSTER / 32;                // a lane's bins (the last level has half as many)
+                const int per = share / 32;
+                u64 own[PER], part = 0;
+#pragma unroll
+                for (int i = 0; i < PER; ++i) own[i] = i < per ? sums[lane * per + i] : 0ull;
+#pragma unroll
+                for (int i = 0; i < PER; ++i) part += own[i];
                 u64 pin = part;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
@@ -302,9 +321,14 @@ __device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigne
                 const int who = __ffs(__ballot_sync(0xffffffffu, run + pin > limit)) - 1;
                 if (lane == who) {
                     run += pin - part;
-                    int i = lane * per;
-                    while (run + sums[i] <= limit) run += sums[i++];
-                    sh.found_bin = owner * share + i;
+                    int i = 0;
+                    bool on = true;
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) {
+                        on = on && run + own[k] <= limit;
+                        if (on) { run += own[k]; ++i; }
+                    }
+                    sh.found_bin = owner * share + lane * per + i;
                     sh.found_cum = run;
                 }
             }
@@ -327,8 +351,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     ScShared& sh = *reinterpret_cast<ScShared*>(sc_smem);
     float* row = reinterpret_cast<float*>(sc_smem + sizeof(ScShared));
     cg::cluster_group cluster = cg::this_cluster();
-    const int c = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-    const int r = blockIdx.x / c, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = (int)cluster.block_rank();
+    const int r = blockIdx.x / SC_CLUSTER, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_wait();
     pdl_trigger();
     const int i0 = min(V, rank * slice), n = min(V, i0 + slice) - i0;
@@ -336,27 +360,28 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     const float temp = temperature[r];
 
     // the slice into shared memory; largest logit (first index among equals) and finiteness on the way
-    u64 best = 0;
+    float top = -INFINITY;
+    int top_i = -1;
     unsigned int bad = 0;
     auto take = [&](float v, int i) {
         if (!(fabsf(v) <= 3.0e38f)) bad = 1;
-        // -0 and 0 are equal: the first of them wins
-        const u64 k = ((u64)float_key(v == 0.f ? 0.f : v) << 32) | (unsigned int)~(i0 + i);
-        best = k > best ? k : best;
+        if (v > top) { top = v; top_i = i; }
         row[i] = v;
     };
     if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
         const int n4 = n >> 2;
-#pragma unroll 4
+#pragma unroll 8
         for (int i = tid; i < n4; i += SC_THREADS) {
             const float4 v = reinterpret_cast<const float4*>(x)[i];
             take(v.x, 4 * i); take(v.y, 4 * i + 1); take(v.z, 4 * i + 2); take(v.w, 4 * i + 3);
         }
         for (int i = 4 * n4 + tid; i < n; i += SC_THREADS) take(x[i], i);
     } else {
-#pragma unroll 4
+#pragma unroll 8
         for (int i = tid; i < n; i += SC_THREADS) take(x[i], i);
     }
+    // -0 and 0 are equal: the first of them wins
+    u64 best = top_i < 0 ? 0ull : ((u64)float_key(top == 0.f ? 0.f : top) << 32) | (unsigned int)~(i0 + top_i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
@@ -367,15 +392,23 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     __syncthreads();
     if (bad) sh.bad = 1;
     if (tid == 0) {
-        for (int w = 0; w < SC_WARPS; ++w) best = sh.warp_a[w] > best ? sh.warp_a[w] : best;
+        u64 least = best;
+        for (int w = 0; w < SC_WARPS; ++w) {
+            best = sh.warp_a[w] > best ? sh.warp_a[w] : best;
+            least = sh.warp_a[w] < least ? sh.warp_a[w] : least;
+        }
         sh.best = best;
+        sh.low = (unsigned int)(least >> 32);
     }
     cluster.sync();
     bad = 0;
-    for (int k = 0; k < c; ++k) {
+    unsigned int low = 0xffffffffu;
+#pragma unroll
+    for (int k = 0; k < SC_CLUSTER; ++k) {
         const u64 b = *cluster.map_shared_rank(&sh.best, k);
         best = k == 0 || b > best ? b : best;
         bad |= *cluster.map_shared_rank(&sh.bad, k);
+        low = min(low, *cluster.map_shared_rank(&sh.low, k));
     }
     const int arg = (int)~(unsigned int)best;
     if (bad || !(temp > 0.f)) {
@@ -391,10 +424,27 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     const float inv_t = 1.f / temp;
     unsigned int lo_key = 0u;
     const int k = top_k[r];
-    if (k > 0 && k < V) lo_key = sc_select<false>(sh, row, n, 0u, 0.f, 0.f, (u64)(V - k), 0.f);
+    if (k > 0 && k < V) {
+        // as many warps as k each hold a key from `low` on, so the k-th largest is one (a maximum of -0 counts as 0 there)
+        if (low == float_key(0.f)) low = float_key(-0.f);
+        lo_key = sc_select<false>(sh, row, n, k <= SC_CLUSTER * SC_WARPS ? low : 0u, 0.f, 0.f, 0ull, (u64)k);
+    }
     const float p_keep = top_p[r];
     if (p_keep < 1.f) {
-        const unsigned int found = sc_select<true>(sh, row, n, lo_key, gmax, inv_t, 0ull, 1.f - p_keep);
+        u64 part = 0;
+        for (int i = tid; i < n; i += SC_THREADS)
+            if (float_key(row[i]) >= lo_key) part += prob_fixed(row[i], gmax, inv_t);
+        part = block_sum_u64(part, sh.warp_a);
+        if (tid == 0) sh.z = part;
+        cluster.sync();
+        u64 z = 0;
+#pragma unroll
+        for (int q = 0; q < SC_CLUSTER; ++q) z += *cluster.map_shared_rank(&sh.z, q);
+        const u64 bound = (u64)((double)(1.f - p_keep) * (double)z);
+        // V keys of half of bound / V each stay within the bound
+        const float least = 0.5f * (float)((double)bound / V * 5.684341886080802e-14);
+        const unsigned int cut = least > 1e-12f ? float_key(gmax + temp * logf(least)) : 0u;
+        const unsigned int found = sc_select<true>(sh, row, n, max(cut, lo_key), gmax, inv_t, z, bound);
         lo_key = found < gkey ? found : gkey;        // the largest always stays
     }
     // inverse CDF in token order over the kept set; a thread owns a run of the slice (of odd length: no bank conflicts)
@@ -421,7 +471,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     if (tid == 0) sh.kept = here;
     cluster.sync();
     u64 total = 0;
-    for (int q = 0; q < c; ++q) {
+#pragma unroll
+    for (int q = 0; q < SC_CLUSTER; ++q) {
         const u64 t = *cluster.map_shared_rank(&sh.kept, q);
         if (q < rank) before += t;
         total += t;
@@ -445,7 +496,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     cluster.sync();
 }
 
-static int launch_sample_cluster(const float* logits, int64_t ld, int rows, int V, int c, int slice, const float* temperature,
+static int launch_sample_cluster(const float* logits, int64_t ld, int rows, int V, int slice, const float* temperature,
                                  const int* top_k, const float* top_p, const u64* seed, const u64* counter, int* token_out,
                                  float* logprob_out, cudaStream_t stream) {
     static AcornPerDevice configured;
@@ -456,13 +507,13 @@ static int launch_sample_cluster(const float* logits, int64_t ld, int rows, int 
         configured.mark();
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(rows * c));
+    cfg.gridDim = dim3((unsigned)(rows * SC_CLUSTER));
     cfg.blockDim = dim3(SC_THREADS);
     cfg.dynamicSmemBytes = sizeof(ScShared) + (size_t)slice * sizeof(float);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = c;
+    attr[0].val.clusterDim.x = SC_CLUSTER;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -479,12 +530,10 @@ extern "C" int acorn_sample(const float* logits, int64_t ld, int rows, int V, co
                             const unsigned long long* counter, int* token_out, float* logprob_out,
                             cudaStream_t stream) {
     if (rows <= 0) return 0;
-    // small vocabularies fit one CTA; slices are multiples of four logits, so that they start on 16 bytes where the row does
-    const int c = V <= 4096 ? 1 : SC_MAX_CLUSTER;
-    const int slice = ((V + c - 1) / c + 3) & ~3;
-    if (slice <= SC_MAX_SLICE && rows <= 0x7fffffff / SC_MAX_CLUSTER)
-        return launch_sample_cluster(logits, ld, rows, V, c, slice, temperature, top_k, top_p, seed, counter, token_out,
-                                     logprob_out, stream);
+    // slices are multiples of four logits, so that they start on 16 bytes where the row does
+    const int slice = ((V + SC_CLUSTER - 1) / SC_CLUSTER + 3) & ~3;
+    if (slice <= SC_MAX_SLICE && rows <= 0x7fffffff / SC_CLUSTER)
+        return launch_sample_cluster(logits, ld, rows, V, slice, temperature, top_k, top_p, seed, counter, token_out, logprob_out, stream);
     return acorn_launch(sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, temperature, top_k,
                         top_p, seed, counter, token_out, logprob_out);
 }

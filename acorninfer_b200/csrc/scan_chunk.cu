@@ -10,8 +10,8 @@
 //
 // What bounds it: multiply-adds fed from shared memory (register tiles of 4 x 4 by 4 and of 8 x 4).  The walk over tokens it
 // replaces for long rows is bound by the issue of dependent instructions, twice over in its two passes.  Measured (2,048
-// tokens, B200): 64 heads of 64 columns, keys of 128, 8 groups: 492 -> 185 us; 16 heads of 128 columns, keys of 128:
-// 277 -> 130 us.
+// tokens, B200): 64 heads of 64 columns, keys of 128, 8 groups: 492 -> 215 us; 16 heads of 128 columns, keys of 128:
+// 277 -> 135 us.
 #include "chunk_helpers.cuh"
 
 #define SCO_VT 64                   // columns a block
