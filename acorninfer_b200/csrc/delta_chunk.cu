@@ -13,6 +13,14 @@
 //                       every chunk starts from; the row's end state into its slot
 //   delta_chunk_out     all chunks side by side: O
 //
+// With a decay per key channel g_id the same holds with b_id per channel, the decays inside the sums over channels:
+//     A_ij = beta_i sum_d k_id k_jd exp(b_id - b_jd),   P_ij = sum_d q_id k_jd exp(b_id - b_jd),   W from diag(beta) (K exp(b)),
+//     O = (Q exp(b)) S_0 + P U,   S_end = diag(exp(b_n)) S_0 + sum_j (k_j exp(b_n - b_j)) u_j^T
+// (channel_chunk_solve in place of delta_chunk_solve; the other two kernels read its scaled q and k).  The walk over tokens that
+// it replaces for long rows is a chain of dependent instructions: 2,000 tokens, 16 heads of 128 x 128: 844 -> 340 us a layer
+// (B200).  b is kept as sums within blocks of 16 tokens, each as two floats, and the blocks' sums: differences lose nothing to a
+// strong decay that both sides have behind them.
+//
 // Gated linear attention, S_i = diag(a_i) S_(i-1) + k_i v_i^T, o_i = S_i^T q_i, with a decay per key channel: with b_i the sums of
 // the logarithms per channel up to i,
 //     O = Q' S_0 + P V,   Q'_i = q_i exp(b_i),   P_ij = sum_d q_id k_jd exp(b_id - b_jd) for j <= i
@@ -45,6 +53,10 @@ struct DeltaChunkParams {
     float* s0;                      // [chunk numbers, H, dim, vdim]
     float* out;                     // [T, H, vdim]
     int rows, H, KH, dim, vdim;
+    // decays per key channel: log_g is [T, H, dim], to base 2, and
+    float* qs;                      // [T, H, dim]: q exp(b)
+    float* kend;                    // [T, H, dim]: k exp(b_n - b)
+    float* decay;                   // [chunk numbers, H, dim]: exp(b_n)
 };
 
 template <typename T> struct LinearChunkParams {
@@ -62,6 +74,24 @@ template <typename T> struct LinearChunkParams {
     float* decay;                   // [chunk numbers, H, dim]
     int rows, H, dim, vdim;
 };
+
+// x <- (1 + A)^-1 x, A strictly lower triangular
+__device__ __forceinline__ void substitute(const float* sA, float (&x)[DC]) {
+    constexpr int LA = DC + DC_PAD;
+#pragma unroll
+    for (int i = 1; i < DC; ++i) {
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int j = 0; j < i; j += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(sA + i * LA + j);
+            s0 = fmaf(a.x, x[j], s0);
+            if (j + 1 < i) s1 = fmaf(a.y, x[j + 1], s1);
+            if (j + 2 < i) s0 = fmaf(a.z, x[j + 2], s0);
+            if (j + 3 < i) s1 = fmaf(a.w, x[j + 3], s1);
+        }
+        x[i] -= s0 + s1;
+    }
+}
 
 template <int DP>
 __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(const DeltaChunkParams p) {
@@ -150,19 +180,182 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(const DeltaCh
 #pragma unroll
             for (int i = 0; i < DC; ++i) x[i] *= sbeta[i];
         }
+        substitute(sA, x);
+        float* dst = is_w ? p.w + ((int64_t)first * p.H + h) * p.dim + col : p.u + ((int64_t)first * p.H + h) * p.vdim + col - p.dim;
+        const int64_t ld = (int64_t)p.H * (is_w ? p.dim : p.vdim);
 #pragma unroll
-        for (int i = 1; i < DC; ++i) {
-            float s0 = 0.f, s1 = 0.f;
+        for (int i = 0; i < DC; ++i)
+            if (i < n) dst[i * ld] = x[i];
+    }
+}
+
+__device__ __forceinline__ float4 at4(const float* q) { return *reinterpret_cast<const float4*>(q); }
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float4 sub4(const float4& a, const float4& b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
+__device__ __forceinline__ float4 mul4(const float4& a, const float4& b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+// 2^x for x <= 0 by the instruction that exp2f is made of, without its care for results below 2^-126 (they are 0 here)
+__device__ __forceinline__ float exp2_neg(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float4 exp2_4(const float4& a) { return make_float4(exp2_neg(a.x), exp2_neg(a.y), exp2_neg(a.z), exp2_neg(a.w)); }
+
+// Sums of a chunk's logarithms within blocks of 16 tokens, in place, and what they lack of the exact sums.
+template <int DP> __device__ __forceinline__ void block_sums(float* sB, float* sB2) {
+    constexpr int LD = DP + DC_PAD;
+    for (int e = threadIdx.x; e < 4 * DP; e += blockDim.x) {
+        float run = 0.f, rest = 0.f;
+        const int at = (e / DP) * 16 * LD + e % DP;
 #pragma unroll
-            for (int j = 0; j < i; j += 4) {            // entries from j = i on are zeros in A
-                const float4 a = *reinterpret_cast<const float4*>(sA + i * LA + j);
-                s0 = fmaf(a.x, x[j], s0);
-                if (j + 1 < i) s1 = fmaf(a.y, x[j + 1], s1);
-                if (j + 2 < i) s0 = fmaf(a.z, x[j + 2], s0);
-                if (j + 3 < i) s1 = fmaf(a.w, x[j + 3], s1);
-            }
-            x[i] -= s0 + s1;
+        for (int i = 0; i < 16; ++i) {
+            const float x = sB[at + i * LD], sum = run + x, back = sum - run;
+            rest += (run - (sum - back)) + (x - back);
+            run = sum;
+            sB[at + i * LD] = run;
+            sB2[at + i * LD] = rest;
         }
+    }
+}
+
+// Logarithms at channels c .. of the decays of a block of 16 up to its token i, of tokens j + 1 .. i of one block, of blocks
+// m0 .. m1 - 1.
+template <int DP> struct ChunkLogs {
+    static constexpr int LD = DP + DC_PAD;
+    const float* b;
+    const float* b2;
+    __device__ __forceinline__ float4 upto(int i, int c) const { return add4(at4(b + i * LD + c), at4(b2 + i * LD + c)); }
+    __device__ __forceinline__ float4 between(int j, int i, int c) const {
+        return add4(sub4(at4(b + i * LD + c), at4(b + j * LD + c)), sub4(at4(b2 + i * LD + c), at4(b2 + j * LD + c)));
+    }
+    __device__ __forceinline__ float4 span(int m0, int m1, int c) const {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int m = m0; m < m1; ++m) x = add4(x, upto(16 * m + 15, c));
+        return x;
+    }
+};
+
+// Decays per key channel.  A block of 16 tokens against an earlier one: both sides at the later block's start; within a block
+// entry by entry, the lower triangles of two blocks side by side on 16 x 16 threads.  No exponent is positive.
+#define CC_THREADS 512              // one block's shared memory fills an SM: its own warps have to hide their latencies
+
+template <int DP>
+__global__ void __launch_bounds__(CC_THREADS) channel_chunk_solve_kernel(const DeltaChunkParams p) {
+    constexpr int LD = DP + DC_PAD, LA = DC + DC_PAD, DQ = DP / 4;
+    extern __shared__ __align__(16) float sm[];
+    float* sK = sm;                                     // [DC][LD]
+    float* sQ = sK + DC * LD;                           // [DC][LD], later q at its block's start
+    float* sB = sQ + DC * LD;                           // [DC][LD] sums of the logarithms within blocks of 16 tokens
+    float* sB2 = sB + DC * LD;                          // [DC][LD] what they lack
+    float* sR = sB2 + DC * LD;                          // [48][LD] keys of the blocks before one, at its start
+    float* sE = sR + 48 * LD;                           // [16][LD] the block's own keys, at its start
+    float* sA = sE + 16 * LD;                           // [DC][LA]
+    __shared__ float sbeta[DC];
+    pdl_wait();
+    pdl_trigger();
+    const int h = blockIdx.y, kh = h / (p.H / p.KH), tid = threadIdx.x;
+    int r, first, n;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    load_rows<DP>(sB, p.log_g + ((int64_t)first * p.H + h) * p.dim, (int64_t)p.H * p.dim, n, p.dim);
+    asm volatile("cp.async.commit_group;\n" ::);
+    load_rows<DP>(sK, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
+    load_rows<DP>(sQ, p.q + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
+    asm volatile("cp.async.commit_group;\n" ::);
+    if (tid < DC) sbeta[tid] = tid < n ? p.beta[(int64_t)(first + tid) * p.H + h] : 0.f;
+    asm volatile("cp.async.wait_group 1;\n" ::);
+    __syncthreads();
+    block_sums<DP>(sB, sB2);
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    const ChunkLogs<DP> logs = {sB, sB2};
+    // entries within blocks of 16 tokens: a half of the threads two blocks, (ty, tx) of the first and (tx, ty) of the second
+    const int half = tid >> 8, tx = tid & 15, ty = (tid >> 4) & 15;
+    float* P = p.p + ((int64_t)first * p.H + h) * DC;
+    const int64_t ldp = (int64_t)p.H * DC;
+    {
+        const int lower = tx <= ty ? 32 * half : 32 * half + 16, upper = 64 * half + 16 - lower;
+        const int i = lower + max(tx, ty), j = lower + min(tx, ty);
+        float a = 0.f, q = 0.f;
+#pragma unroll 4
+        for (int d = 0; d < DP; d += 4) {
+            const float4 k = mul4(at4(sK + j * LD + d), exp2_4(logs.between(j, i, d)));
+            a = dot4(at4(sK + i * LD + d), k, a);
+            q = dot4(at4(sQ + i * LD + d), k, q);
+        }
+        sA[i * LA + j] = i > j ? sbeta[i] * a : 0.f;
+        if (i < n) P[i * ldp + j] = q;
+        if (tx != ty) {                                 // above the diagonal of the other block
+            if (upper + min(tx, ty) < n) P[(upper + min(tx, ty)) * ldp + upper + max(tx, ty)] = 0.f;
+        } else {                                        // the other block's diagonal
+            const int o = upper + tx;
+            float s = 0.f;
+#pragma unroll 4
+            for (int d = 0; d < DP; d += 4) s = dot4(at4(sQ + o * LD + d), at4(sK + o * LD + d), s);
+            sA[o * LA + o] = 0.f;
+            if (o < n) P[o * ldp + o] = s;
+        }
+    }
+    __syncthreads();
+    // q exp(b) and k exp(b_n - b) to memory; in shared memory q at its block's start
+    for (int e = tid; e < DC * DQ; e += CC_THREADS) {
+        const int i = e / DQ, c = (e % DQ) * 4, at = i * LD + c;
+        const float4 q = at4(sQ + at), b = logs.upto(i, c);
+        if (i < n && c < p.dim) {
+            const int64_t to = ((int64_t)(first + i) * p.H + h) * p.dim + c;
+            *reinterpret_cast<float4*>(p.qs + to) = mul4(q, exp2_4(add4(logs.span(0, i >> 4, c), b)));
+            *reinterpret_cast<float4*>(p.kend + to) = mul4(at4(sK + at), exp2_4(add4(logs.between(i, i | 15, c), logs.span((i >> 4) + 1, 4, c))));
+        }
+        if (i >= 16) *reinterpret_cast<float4*>(sQ + at) = mul4(q, exp2_4(b));
+    }
+    if (tid < DQ && 4 * tid < p.dim)
+        *reinterpret_cast<float4*>(p.decay + ((int64_t)blockIdx.x * p.H + h) * p.dim + 4 * tid) = exp2_4(logs.span(0, 4, 4 * tid));
+#pragma unroll
+    for (int I = 1; I < 4; ++I) {                       // entries against the blocks before
+        for (int e = tid; e < 16 * (I + 1) * DQ; e += CC_THREADS) {
+            const int j = e / DQ, c = (e % DQ) * 4;
+            const float4 k = at4(sK + j * LD + c);
+            if (j < 16 * I) *reinterpret_cast<float4*>(sR + j * LD + c) = mul4(k, exp2_4(add4(logs.between(j, j | 15, c), logs.span((j >> 4) + 1, I, c))));
+            else *reinterpret_cast<float4*>(sE + (j - 16 * I) * LD + c) = mul4(k, exp2_4(logs.upto(j, c)));
+        }
+        __syncthreads();
+        const int i = 16 * I + ty;
+        const float* rows = half == 0 ? sE + ty * LD : sQ + i * LD;      // half of the threads A, half P
+        float s[3] = {0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int d = 0; d < DP; d += 4) {
+            const float4 x = at4(rows + d);
+#pragma unroll
+            for (int J = 0; J < I; ++J) s[J] = dot4(x, at4(sR + (16 * J + tx) * LD + d), s[J]);
+        }
+#pragma unroll
+        for (int J = 0; J < I; ++J) {
+            if (half == 0) sA[i * LA + 16 * J + tx] = sbeta[i] * s[J];
+            else if (i < n) P[i * ldp + 16 * J + tx] = s[J];
+        }
+        __syncthreads();
+    }
+    // forward substitution: a thread a column of [W | Ubar], its 64 entries in registers
+    for (int c0 = 0; c0 < p.dim + p.vdim; c0 += CC_THREADS) {
+        const int col = c0 + tid;
+        if (col >= p.dim + p.vdim) break;
+        const bool is_w = col < p.dim;
+        float x[DC];
+        if (is_w) {
+#pragma unroll
+            for (int i = 0; i < DC; ++i) {
+                float before = 0.f;
+#pragma unroll
+                for (int m = 0; m < (i >> 4); ++m) before += sB[(16 * m + 15) * LD + col] + sB2[(16 * m + 15) * LD + col];
+                x[i] = sbeta[i] * exp2_neg(before + (sB[i * LD + col] + sB2[i * LD + col])) * sK[i * LD + col];
+            }
+        } else {
+            const float* v = p.v + ((int64_t)first * p.H + h) * p.vdim + col - p.dim;
+#pragma unroll
+            for (int i = 0; i < DC; ++i) x[i] = i < n ? v[(int64_t)i * p.H * p.vdim] : 0.f;
+#pragma unroll
+            for (int i = 0; i < DC; ++i) x[i] *= sbeta[i];
+        }
+        substitute(sA, x);
         float* dst = is_w ? p.w + ((int64_t)first * p.H + h) * p.dim + col : p.u + ((int64_t)first * p.H + h) * p.vdim + col - p.dim;
         const int64_t ld = (int64_t)p.H * (is_w ? p.dim : p.vdim);
 #pragma unroll
@@ -174,7 +367,8 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(const DeltaCh
 // Both products of a chunk have few outputs (64 x 16 and dim x 16) and a long sum, so a warp takes a slice of the sum for large
 // register tiles (8 x 4 a lane: three reads of shared memory for 32 multiply-adds) and the slices are added up through
 // shared memory: U over 8 slices of the key channels, the state over 4 slices of the tokens by 2 halves of the channels.
-template <int DP>
+// CHANNEL: decays per key channel (the keys come as k exp(b_n - b)).
+template <int DP, bool CHANNEL>
 __global__ void __launch_bounds__(256) delta_chunk_state_kernel(const DeltaChunkParams p) {
     constexpr int LD = DP + DC_PAD, LV = DC_VT + DC_PAD, SLICE = DP / 8, ND = DP / 64 > 0 ? DP / 64 : 1;
     constexpr int PARTS = 8 * DC > 4 * DP ? 8 * DC : 4 * DP;
@@ -216,7 +410,8 @@ __global__ void __launch_bounds__(256) delta_chunk_state_kernel(const DeltaChunk
     auto fetch = [&](int c) {
         const int first = start + c * DC, n = min(DC, L - c * DC);
         load_rows<DP>(sW + (c & 1) * DC * LD, p.w + ((int64_t)first * p.H + h) * p.dim, (int64_t)p.H * p.dim, n, p.dim);
-        load_rows<DP>(sK + (c & 1) * DC * LD, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
+        if (CHANNEL) load_rows<DP>(sK + (c & 1) * DC * LD, p.kend + ((int64_t)first * p.H + h) * p.dim, (int64_t)p.H * p.dim, n, p.dim);
+        else load_rows<DP>(sK + (c & 1) * DC * LD, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
     };
     auto axpy = [](float a, const float4& x, float4& y) {
         y.x = fmaf(a, x.x, y.x); y.y = fmaf(a, x.y, y.y); y.z = fmaf(a, x.z, y.z); y.w = fmaf(a, x.w, y.w);
@@ -227,11 +422,12 @@ __global__ void __launch_bounds__(256) delta_chunk_state_kernel(const DeltaChunk
     const int token = tid >> 2;                         // the token whose u this thread collects
     for (int c = 0; c < chunks; ++c) {
         const int first = start + c * DC, n = min(DC, L - c * DC);
-        const float bn = p.b[(int64_t)(first + n - 1) * p.H + h];
+        const float bn = CHANNEL ? 0.f : p.b[(int64_t)(first + n - 1) * p.H + h];
         const int64_t t = (int64_t)(first + min(token, n - 1)) * p.H + h;
         const bool live = token < n && on;
         const float4 ub = live ? *reinterpret_cast<const float4*>(p.u + t * p.vdim + c4) : zero;
-        const float bj = p.b[t];
+        const float bj = CHANNEL ? 0.f : p.b[t];
+        const float* gn_d = CHANNEL ? p.decay + ((int64_t)(id0 + c) * p.H + h) * p.dim : nullptr;
         if (c + 1 < chunks) fetch(c + 1);
         asm volatile("cp.async.commit_group;\n" ::);
         float* keep = p.s0 + ((int64_t)(id0 + c) * p.H + h) * p.dim * p.vdim;      // the state this chunk starts from
@@ -268,7 +464,7 @@ __global__ void __launch_bounds__(256) delta_chunk_state_kernel(const DeltaChunk
             for (int q = 0; q < 8; ++q) add(u, *reinterpret_cast<const float4*>(part + (q * DC + token) * LV + 4 * (tid & 3)));
             u = make_float4(ub.x - u.x, ub.y - u.y, ub.z - u.z, ub.w - u.w);
             if (live) *reinterpret_cast<float4*>(p.u + t * p.vdim + c4) = u;
-            const float G = token < n ? expf(bn - bj) : 0.f;
+            const float G = token < n ? (CHANNEL ? 1.f : expf(bn - bj)) : 0.f;
             *reinterpret_cast<float4*>(sU + token * LV + 4 * (tid & 3)) = make_float4(u.x * G, u.y * G, u.z * G, u.w * G);
         }
         __syncthreads();
@@ -297,11 +493,12 @@ __global__ void __launch_bounds__(256) delta_chunk_state_kernel(const DeltaChunk
             }
         }
         __syncthreads();
-        const float gn = expf(bn);
+        const float g_head = expf(bn);
 #pragma unroll
         for (int m = 0; m < ND; ++m) {
             const int d = (tid + 256 * m) >> 2;
             if (d >= DP) break;
+            const float gn = CHANNEL ? (d < p.dim ? gn_d[d] : 0.f) : g_head;
             S[m] = make_float4(S[m].x * gn, S[m].y * gn, S[m].z * gn, S[m].w * gn);
 #pragma unroll
             for (int q = 0; q < 4; ++q) add(S[m], *reinterpret_cast<const float4*>(part + (q * DP + d) * LV + 4 * (tid & 3)));
@@ -412,16 +609,39 @@ template <int DP> static int launch_delta_chunk(const DeltaChunkParams& p, int i
     static AcornPerDevice configured;
     if (!configured.seen()) {
         cudaError_t e = cudaFuncSetAttribute(delta_chunk_solve_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_state_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_state_kernel<DP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_out_kernel<DP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
         if (e != cudaSuccess) return (int)e;
         configured.mark();
     }
     int rc = acorn_launch(delta_chunk_solve_kernel<DP>, dim3(ids, p.H), dim3(256), solve, stream, p);
     if (rc) return rc;
-    rc = acorn_launch(delta_chunk_state_kernel<DP>, dim3((p.vdim + DC_VT - 1) / DC_VT, p.H, p.rows), dim3(256), walk, stream, p);
+    rc = acorn_launch(delta_chunk_state_kernel<DP, false>, dim3((p.vdim + DC_VT - 1) / DC_VT, p.H, p.rows), dim3(256), walk, stream, p);
     if (rc) return rc;
     return acorn_launch(delta_chunk_out_kernel<DP, false>, dim3(ids, p.H, (p.vdim + DC_OT - 1) / DC_OT), dim3(256), out, stream, p);
+}
+
+template <int DP> static int launch_channel_chunk(const DeltaChunkParams& p, int ids, cudaStream_t stream) {
+    constexpr int LD = DP + DC_PAD, LV = DC_VT + DC_PAD, PARTS = 8 * DC > 4 * DP ? 8 * DC : 4 * DP;
+    const size_t solve = (size_t)((4 * DC + 64) * LD + DC * (DC + DC_PAD)) * sizeof(float);
+    const size_t walk = (size_t)(4 * DC * LD + (DP + DC + PARTS) * LV) * sizeof(float);
+    const size_t out = (size_t)(DC * LD + DP * (DC_OT + DC_PAD) + DC * (DC_OT + DC_PAD) + DC * (DC + DC_PAD)) * sizeof(float);
+    static AcornPerDevice configured;
+    if (!configured.seen()) {
+        cudaError_t e = cudaFuncSetAttribute(channel_chunk_solve_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_state_kernel<DP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_out_kernel<DP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
+        if (e != cudaSuccess) return (int)e;
+        configured.mark();
+    }
+    int rc = acorn_launch(channel_chunk_solve_kernel<DP>, dim3(ids, p.H), dim3(CC_THREADS), solve, stream, p);
+    if (rc) return rc;
+    rc = acorn_launch(delta_chunk_state_kernel<DP, true>, dim3((p.vdim + DC_VT - 1) / DC_VT, p.H, p.rows), dim3(256), walk, stream, p);
+    if (rc) return rc;
+    DeltaChunkParams o = p;                             // the scaled queries are per head
+    o.q = p.qs;
+    o.KH = p.H;
+    return acorn_launch(delta_chunk_out_kernel<DP, true>, dim3(ids, p.H, (p.vdim + DC_OT - 1) / DC_OT), dim3(256), out, stream, o);
 }
 
 // ---------------------------------------------------------------- gated linear attention
@@ -674,6 +894,165 @@ extern "C" int acorn_linear_chunk(const void* in, int64_t ld, const float* z, in
     return ACORN_ERR_UNSUPPORTED;
 }
 
+// ---------------------------------------------------------------- time mixing
+
+// S_i = diag(g_i) S_(i-1) + k_i v_i^T, o_i = S_(i-1)^T q_i + (sum_d q_id bonus_d k_id) v_i: a token reads the state before its own decay
+// and write and sees itself through the bonus.  As gated linear attention over chunks, with the sums e_i = b_(i-1) up to the token
+// before on the reading side:
+//     Q'_i = q_i exp(e_i),   P_ij = sum_d q_id k_jd exp(e_id - b_jd) for j < i,   P_ii = sum_d q_id bonus_d k_id.
+// The walk over segments that it replaces for long rows went through every token twice: 1,800 tokens of 32 heads of 64 x 64
+// 203 -> 98 us (B200).
+template <int DP>
+__global__ void __launch_bounds__(256) mix_chunk_local_kernel(const DeltaChunkParams p, const float* __restrict__ bonus) {
+    constexpr int LD = DP + DC_PAD, LO = DC_OT + DC_PAD, DQ = DP / 4;
+    extern __shared__ __align__(16) float sm[];
+    float* sK = sm;                                     // [DC][LD], later keys at the chunk's end
+    float* sQ = sK + DC * LD;                           // [DC][LD], later q at its block's start
+    float* sB = sQ + DC * LD;                           // [DC][LD] sums of the logarithms within blocks of 16 tokens
+    float* sB2 = sB + DC * LD;                          // [DC][LD] what they lack
+    float* sR = sB2 + DC * LD;                          // [48][LD] keys of the blocks before one, at its start
+    float* sV = sR + 48 * LD;                           // [DC][LO]
+    pdl_wait();
+    pdl_trigger();
+    const int h = blockIdx.y, kh = h / (p.H / p.KH), tid = threadIdx.x;
+    int r, first, n;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    load_rows<DP>(sB, p.log_g + ((int64_t)first * p.H + h) * p.dim, (int64_t)p.H * p.dim, n, p.dim);
+    asm volatile("cp.async.commit_group;\n" ::);
+    load_rows<DP>(sK, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
+    load_rows<DP>(sQ, p.q + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
+    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.wait_group 1;\n" ::);
+    __syncthreads();
+    block_sums<DP>(sB, sB2);
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    const ChunkLogs<DP> logs = {sB, sB2};
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int tx = tid & 15, ty = tid >> 4;
+    float* P = p.p + ((int64_t)first * p.H + h) * DC;
+    const int64_t ldp = (int64_t)p.H * DC;
+    // entries within blocks of 16 tokens: two blocks at a time, (ty, tx) of the first and (tx, ty) of the second, then the diagonals
+    for (int I = 0; I < 4; I += 2) {
+        const int lower = tx < ty ? 16 * I : 16 * I + 16, upper = 32 * I + 16 - lower;
+        const int i = lower + max(tx, ty), j = lower + min(tx, ty);
+        if (tx != ty) {
+            float s = 0.f;
+#pragma unroll 4
+            for (int d = 0; d < DP; d += 4)
+                s = dot4(at4(sQ + i * LD + d), mul4(at4(sK + j * LD + d), exp2_4(logs.between(j, i - 1, d))), s);
+            if (i < n) P[i * ldp + j] = s;
+            if (upper + min(tx, ty) < n) P[(upper + min(tx, ty)) * ldp + upper + max(tx, ty)] = 0.f;
+        }
+    }
+    if (tid < DC && tid < n) {
+        float s = 0.f;
+#pragma unroll 4
+        for (int d = 0; d < DP; d += 4) {
+            const float4 u = d < p.dim ? make_float4(bonus[h * p.dim + d], bonus[h * p.dim + d + 1], bonus[h * p.dim + d + 2], bonus[h * p.dim + d + 3]) : zero;
+            s = dot4(at4(sQ + tid * LD + d), mul4(at4(sK + tid * LD + d), u), s);
+        }
+        P[tid * ldp + tid] = s;
+    }
+    __syncthreads();
+    for (int e = tid; e < DC * DQ; e += 256) {
+        const int i = e / DQ, c = (e % DQ) * 4, at = i * LD + c;
+        const float4 own = (i & 15) ? logs.upto(i - 1, c) : zero;
+        const float4 q = at4(sQ + at);
+        if (i < n && c < p.dim)
+            *reinterpret_cast<float4*>(p.qs + ((int64_t)(first + i) * p.H + h) * p.dim + c) = mul4(q, exp2_4(add4(logs.span(0, i >> 4, c), own)));
+        if (i >= 16) *reinterpret_cast<float4*>(sQ + at) = mul4(q, exp2_4(own));
+    }
+    if (tid < DQ && 4 * tid < p.dim)
+        *reinterpret_cast<float4*>(p.decay + ((int64_t)blockIdx.x * p.H + h) * p.dim + 4 * tid) = exp2_4(logs.span(0, 4, 4 * tid));
+#pragma unroll
+    for (int I = 1; I < 4; ++I) {                       // entries against the blocks before
+        for (int e = tid; e < 16 * I * DQ; e += 256) {
+            const int j = e / DQ, c = (e % DQ) * 4;
+            *reinterpret_cast<float4*>(sR + j * LD + c) = mul4(at4(sK + j * LD + c), exp2_4(add4(logs.between(j, j | 15, c), logs.span((j >> 4) + 1, I, c))));
+        }
+        __syncthreads();
+        const int i = 16 * I + ty;
+        float s[3] = {0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int d = 0; d < DP; d += 4) {
+            const float4 q = at4(sQ + i * LD + d);
+#pragma unroll
+            for (int J = 0; J < I; ++J) s[J] = dot4(q, at4(sR + (16 * J + tx) * LD + d), s[J]);
+        }
+        if (i < n)
+#pragma unroll
+            for (int J = 0; J < I; ++J) P[i * ldp + 16 * J + tx] = s[J];
+        __syncthreads();
+    }
+    // the keys at the chunk's end, and their sum with the values
+    for (int e = tid; e < DC * DQ; e += 256) {
+        const int j = e / DQ, c = (e % DQ) * 4, at = j * LD + c;
+        *reinterpret_cast<float4*>(sK + at) = mul4(at4(sK + at), exp2_4(add4(logs.between(j, j | 15, c), logs.span((j >> 4) + 1, 4, c))));
+    }
+    constexpr int ND = DP / 64 > 0 ? DP / 64 : 1;       // groups of 4 key channels a thread
+    for (int v0 = 0; v0 < p.vdim; v0 += DC_OT) {
+        for (int e = tid; e < DC * (DC_OT / 4); e += 256) {
+            const int j = e / (DC_OT / 4), c = (e % (DC_OT / 4)) * 4;
+            *reinterpret_cast<float4*>(sV + j * LO + c) =
+                j < n && v0 + c < p.vdim ? at4(p.v + ((int64_t)(first + j) * p.H + h) * p.vdim + v0 + c) : zero;
+        }
+        __syncthreads();
+        float4 acc[ND][4];
+#pragma unroll
+        for (int m = 0; m < ND; ++m)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[m][q] = zero;
+        if (4 * ty < DP) {
+#pragma unroll 4
+            for (int j = 0; j < DC; ++j) {
+                const float4 v = at4(sV + j * LO + 4 * tx);
+#pragma unroll
+                for (int m = 0; m < ND; ++m) {
+                    const float4 k = at4(sK + j * LD + 4 * ty + 64 * m);
+                    const float kk[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        acc[m][q].x = fmaf(kk[q], v.x, acc[m][q].x); acc[m][q].y = fmaf(kk[q], v.y, acc[m][q].y);
+                        acc[m][q].z = fmaf(kk[q], v.z, acc[m][q].z); acc[m][q].w = fmaf(kk[q], v.w, acc[m][q].w);
+                    }
+                }
+            }
+            float* E = p.s0 + ((int64_t)blockIdx.x * p.H + h) * p.dim * p.vdim;
+#pragma unroll
+            for (int m = 0; m < ND; ++m)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int d = 4 * ty + 64 * m + q;
+                    if (d < p.dim && v0 + 4 * tx < p.vdim) *reinterpret_cast<float4*>(E + (int64_t)d * p.vdim + v0 + 4 * tx) = acc[m][q];
+                }
+        }
+        __syncthreads();
+    }
+}
+
+template <int DP> static int launch_mix_chunk(const DeltaChunkParams& p, const float* bonus, int ids, cudaStream_t stream) {
+    constexpr int LD = DP + DC_PAD, LO = DC_OT + DC_PAD;
+    const size_t local = (size_t)((4 * DC + 48) * LD + DC * LO) * sizeof(float);
+    const size_t out = (size_t)(DC * LD + DP * LO + DC * LO + DC * (DC + DC_PAD)) * sizeof(float);
+    static AcornPerDevice configured;
+    if (!configured.seen()) {
+        cudaError_t e = cudaFuncSetAttribute(mix_chunk_local_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_out_kernel<DP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
+        if (e != cudaSuccess) return (int)e;
+        configured.mark();
+    }
+    int rc = acorn_launch(mix_chunk_local_kernel<DP>, dim3(ids, p.H), dim3(256), local, stream, p, bonus);
+    if (rc) return rc;
+    rc = acorn_launch(linear_chunk_fold_kernel, dim3((p.dim * (p.vdim / 4) + 255) / 256, p.H, p.rows), dim3(256), 0, stream, p.state,
+                      p.slot_stride, p.row_start, p.row_slot, p.s0, (const float*)p.decay, p.H, p.dim, p.vdim);
+    if (rc) return rc;
+    DeltaChunkParams o = p;                             // the scaled queries are per head
+    o.q = p.qs;
+    o.KH = p.H;
+    return acorn_launch(delta_chunk_out_kernel<DP, true>, dim3(ids, p.H, (p.vdim + DC_OT - 1) / DC_OT), dim3(256), out, stream, o);
+}
+
 extern "C" int acorn_delta_chunk_supported(int dim, int vdim) { return dim >= 4 && dim <= 128 && dim % 4 == 0 && vdim >= 4 && vdim % 4 == 0; }
 
 // chunk numbers of a step (what s0 must have room for)
@@ -690,4 +1069,38 @@ extern "C" int acorn_delta_chunk(const float* q, const float* k, const float* v,
     if (dim <= 32) return launch_delta_chunk<32>(p, ids, stream);
     if (dim <= 64) return launch_delta_chunk<64>(p, ids, stream);
     return launch_delta_chunk<128>(p, ids, stream);
+}
+
+// log2_g [T, H, dim]: the decays' logarithms to base 2, none positive
+extern "C" int acorn_channel_chunk(const float* q, const float* k, const float* v, const float* beta, const float* log2_g, float* state,
+                                   int64_t slot_stride, const int* row_start, const int* row_slot, float* w, float* u, float* pp,
+                                   float* qs, float* kend, float* decay, float* s0, float* out, int tokens, int rows, int H, int KH,
+                                   int dim, int vdim, cudaStream_t stream) {
+    if (tokens <= 0 || rows <= 0) return 0;
+    const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)log2_g | (uintptr_t)w | (uintptr_t)u | (uintptr_t)pp | (uintptr_t)qs |
+                          (uintptr_t)kend | (uintptr_t)decay | (uintptr_t)s0 | (uintptr_t)out;
+    if (!acorn_delta_chunk_supported(dim, vdim) || KH < 1 || H < 1 || H % KH || H > 65535 || rows > 65535 || (all & 15)) return ACORN_ERR_UNSUPPORTED;
+    DeltaChunkParams p = {q, k, v, beta, log2_g, state, slot_stride, row_start, row_slot, w, u, pp, nullptr, s0, out, rows, H, KH, dim, vdim,
+                          qs, kend, decay};
+    const int ids = acorn_delta_chunk_ids(tokens, rows);
+    if (dim <= 32) return launch_channel_chunk<32>(p, ids, stream);
+    if (dim <= 64) return launch_channel_chunk<64>(p, ids, stream);
+    return launch_channel_chunk<128>(p, ids, stream);
+}
+
+// v as it is; bonus [H, dim]; log2_g as above
+extern "C" int acorn_mix_chunk(const float* q, const float* k, const float* v, const float* bonus, const float* log2_g, float* state,
+                               int64_t slot_stride, const int* row_start, const int* row_slot, float* pp, float* qs, float* decay,
+                               float* s0, float* out, int tokens, int rows, int H, int KH, int dim, int vdim, cudaStream_t stream) {
+    if (tokens <= 0 || rows <= 0) return 0;
+    const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)log2_g | (uintptr_t)pp | (uintptr_t)qs | (uintptr_t)decay |
+                          (uintptr_t)s0 | (uintptr_t)out | (uintptr_t)state;
+    if (!acorn_delta_chunk_supported(dim, vdim) || KH < 1 || H < 1 || H % KH || H > 65535 || rows > 65535 || (all & 15) || slot_stride % 4)
+        return ACORN_ERR_UNSUPPORTED;
+    DeltaChunkParams p = {q, k, v, nullptr, log2_g, state, slot_stride, row_start, row_slot, nullptr, const_cast<float*>(v), pp, nullptr, s0, out,
+                          rows, H, KH, dim, vdim, qs, nullptr, decay};
+    const int ids = acorn_delta_chunk_ids(tokens, rows);
+    if (dim <= 32) return launch_mix_chunk<32>(p, bonus, ids, stream);
+    if (dim <= 64) return launch_mix_chunk<64>(p, bonus, ids, stream);
+    return launch_mix_chunk<128>(p, bonus, ids, stream);
 }

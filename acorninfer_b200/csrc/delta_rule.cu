@@ -9,7 +9,7 @@
 //   delta_prep          per token: the short causal convolution over time of the q, k, v channels
 //                       (inputs before the step's first token come from the request's state), silu,
 //                       unit norms, beta = sigmoid(.), g = exp(-exp(A_log) softplus(. + dt_bias)),
-//                       the output gate sigmoid(.); float32 outputs
+//                       (or its logarithm to base 2), the output gate sigmoid(.); float32 outputs
 //   conv_state_update   per row: the last taps - 1 convolution inputs into the request's state
 //   delta_rule          the recurrence over a row's tokens, state in registers
 //   delta_out           per token and head: o / rms(o) * w * gate
@@ -32,7 +32,7 @@ __global__ void delta_prep_kernel(const T* __restrict__ main_, int64_t ld, const
                                   const int* __restrict__ token_row, const int* __restrict__ row_start,
                                   const int* __restrict__ row_slot, float* __restrict__ qn, float* __restrict__ kn,
                                   float* __restrict__ vv, float* __restrict__ beta, float* __restrict__ g,
-                                  float* __restrict__ gate, int H, int KH, int dim, int vdim, int taps) {
+                                  float* __restrict__ gate, int H, int KH, int dim, int vdim, int taps, int logs) {
     extern __shared__ float act[];                      // [C] activations of the q, k, v channels
     __shared__ float inv_norm[2 * 64];                  // per q head, per k head (KH <= 64)
     pdl_wait();
@@ -70,19 +70,141 @@ __global__ void delta_prep_kernel(const T* __restrict__ main_, int64_t ld, const
         vv[(int64_t)t * H * vdim + c] = act[2 * KH * dim + c];
         gate[(int64_t)t * H * vdim + c] = sigmoidf_(up[(int64_t)t * ld_up + H * dim + c]);
     }
-    for (int c = threadIdx.x; c < H * dim; c += blockDim.x)
-        g[(int64_t)t * H * dim + c] = expf(-expf(A_log[c / dim]) * softplusf_(up[(int64_t)t * ld_up + c] + dt_bias[c]));
+    for (int c = threadIdx.x; c < H * dim; c += blockDim.x) {
+        const float lg = -expf(A_log[c / dim]) * softplusf_(up[(int64_t)t * ld_up + c] + dt_bias[c]);
+        g[(int64_t)t * H * dim + c] = logs ? lg * 1.4426950408889634f : expf(lg);
+    }
     for (int h = threadIdx.x; h < H; h += blockDim.x) beta[(int64_t)t * H + h] = sigmoidf_(to_float(main_[(int64_t)t * ld + C + h]));
+}
+
+// The same four channels a lane, 2^lph_log2 lanes a head, TPT consecutive tokens a lane (their inputs and those before them are
+// fetched at once): the heads of q, k and v through the convolution, then the heads' decays and gates.  One block a token with
+// 2-byte reads of four rows a channel was bound by its loads' latency: 2,000 tokens of 16 + 16 heads of 128 92 -> 50 us.
+template <typename T, int TAPS, int TPT>
+__global__ void __launch_bounds__(256) delta_prep_vec_kernel(const T* __restrict__ main_, int64_t ld, const float* __restrict__ up,
+                                                             int64_t ld_up, const float* __restrict__ conv_w,
+                                                             const float* __restrict__ state, int64_t slot_stride, int64_t conv_off,
+                                                             const float* __restrict__ A_log, const float* __restrict__ dt_bias,
+                                                             const int* __restrict__ token_row, const int* __restrict__ row_start,
+                                                             const int* __restrict__ row_slot, float* __restrict__ qn,
+                                                             float* __restrict__ kn, float* __restrict__ vv, float* __restrict__ beta,
+                                                             float* __restrict__ g, float* __restrict__ gate, int tokens, int H, int KH,
+                                                             int dim, int vdim, int logs, int lph_log2) {
+    constexpr int PAST = TAPS - 1;
+    const int conv_heads = 2 * KH + H, heads = conv_heads + 2 * H;
+    const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t item = gid >> lph_log2;
+    const int l = (int)(gid & ((1 << lph_log2) - 1));
+    const bool in_range = item < ((int64_t)tokens + TPT - 1) / TPT * heads;
+    const int t0 = in_range ? (int)(item / heads) * TPT : 0, h = in_range ? (int)(item % heads) : 0;
+    const int C = 2 * KH * dim + H * vdim;
+    pdl_wait();
+    pdl_trigger();
+    const bool conv = h < conv_heads, is_v = h >= 2 * KH && conv;
+    const int vh = h - 2 * KH, width = !conv ? (h - conv_heads < H ? dim : vdim) : (is_v ? vdim : dim);
+    const bool on = in_range && 4 * l < width;
+    if (conv) {                                             // alike for all lanes of a head
+        const int chan = on ? (is_v ? 2 * KH * dim + vh * vdim : h * dim) + 4 * l : 0;
+        const unsigned int head_lanes = (lph_log2 == 5 ? 0xffffffffu : (1u << (1 << lph_log2)) - 1u) << ((threadIdx.x & 31) & ~((1 << lph_log2) - 1));
+        float w[4 * TAPS];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(conv_w + (int64_t)chan * TAPS + 4 * j);
+            w[4 * j] = v.x; w[4 * j + 1] = v.y; w[4 * j + 2] = v.z; w[4 * j + 3] = v.w;
+        }
+        float4 in[TPT + PAST];
+#pragma unroll
+        for (int q = 0; q < TPT + PAST; ++q) in[q] = Vec4<T>::load(main_ + (int64_t)min(max(t0 + q - PAST, 0), tokens - 1) * ld + chan);
+#pragma unroll
+        for (int q = 0; q < TPT; ++q) {
+            const int t = min(t0 + q, tokens - 1), r = token_row[t], i0 = t - row_start[r];
+            const float* cstate = i0 < PAST ? state + (int64_t)row_slot[r] * slot_stride + conv_off + chan : nullptr;
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {                // index within the row i0 - PAST + j; negative: before the step
+                float4 u = in[q + j];
+                if (i0 - PAST + j < 0) {
+                    const float* c = cstate + (int64_t)(i0 + j) * C;
+                    u = make_float4(c[0], c[1], c[2], c[3]);
+                }
+                x.x = fmaf(w[j], u.x, x.x);
+                x.y = fmaf(w[TAPS + j], u.y, x.y);
+                x.z = fmaf(w[2 * TAPS + j], u.z, x.z);
+                x.w = fmaf(w[3 * TAPS + j], u.w, x.w);
+            }
+            x = make_float4(x.x * sigmoidf_(x.x), x.y * sigmoidf_(x.y), x.z * sigmoidf_(x.z), x.w * sigmoidf_(x.w));
+            float f = 1.f;
+            if (!is_v) {
+                float ss = on ? x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w : 0.f;
+                for (int o = (1 << lph_log2) >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(head_lanes, ss, o);
+                f = rsqrtf(ss + 1e-6f) * (h < KH ? rsqrtf((float)dim) : 1.f);
+            }
+            if (!on || t0 + q >= tokens) continue;
+            float* dst = is_v ? vv + ((int64_t)t * H + vh) * vdim
+                              : (h < KH ? qn + ((int64_t)t * KH + h) * dim : kn + ((int64_t)t * KH + h - KH) * dim);
+            *reinterpret_cast<float4*>(dst + 4 * l) = make_float4(x.x * f, x.y * f, x.z * f, x.w * f);
+            if (is_v && l == 0) beta[(int64_t)t * H + vh] = sigmoidf_(to_float(main_[(int64_t)t * ld + C + vh]));
+        }
+        return;
+    }
+    if (!on) return;
+    const bool is_gate = h - conv_heads >= H;
+    const int hh = (h - conv_heads) % H, col = hh * width + 4 * l;
+    const float A = is_gate ? 0.f : -expf(A_log[hh]) * (logs ? 1.4426950408889634f : 1.f);
+    const float4 bias = is_gate ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(dt_bias + col);
+    float4 z[TPT];
+#pragma unroll
+    for (int q = 0; q < TPT; ++q)
+        z[q] = *reinterpret_cast<const float4*>(up + (int64_t)min(t0 + q, tokens - 1) * ld_up + (is_gate ? H * dim : 0) + col);
+#pragma unroll
+    for (int q = 0; q < TPT; ++q) {
+        if (t0 + q >= tokens) break;
+        float4 o;
+        if (is_gate) {
+            o = make_float4(sigmoidf_(z[q].x), sigmoidf_(z[q].y), sigmoidf_(z[q].z), sigmoidf_(z[q].w));
+        } else {
+            o = make_float4(A * softplusf_(z[q].x + bias.x), A * softplusf_(z[q].y + bias.y), A * softplusf_(z[q].z + bias.z),
+                            A * softplusf_(z[q].w + bias.w));
+            if (!logs) o = make_float4(expf(o.x), expf(o.y), expf(o.z), expf(o.w));
+        }
+        *reinterpret_cast<float4*>((is_gate ? gate + (int64_t)(t0 + q) * H * vdim : g + (int64_t)(t0 + q) * H * dim) + col) = o;
+    }
+}
+
+template <typename T, int TAPS, typename... Args>
+static int launch_delta_prep_vec(int tokens, int H, int KH, int dim, int vdim, int logs, cudaStream_t stream, Args... args) {
+    int lph_log2 = 0;
+    while ((4 << lph_log2) < (dim > vdim ? dim : vdim)) ++lph_log2;
+    const int tpt = tokens > 256 ? 4 : 1;
+    const int64_t threads = (((int64_t)tokens + tpt - 1) / tpt * (2 * KH + 3 * H)) << lph_log2;
+    const dim3 grid((unsigned)((threads + 255) / 256));
+    if (tpt == 1)
+        return acorn_launch(delta_prep_vec_kernel<T, TAPS, 1>, grid, dim3(256), 0, stream, args..., tokens, H, KH, dim, vdim, logs, lph_log2);
+    return acorn_launch(delta_prep_vec_kernel<T, TAPS, 4>, grid, dim3(256), 0, stream, args..., tokens, H, KH, dim, vdim, logs, lph_log2);
 }
 
 extern "C" int acorn_delta_prep(const void* main_, int64_t ld, const float* up, int64_t ld_up, const float* conv_w,
                                 const float* state, int64_t slot_stride, int64_t conv_off, const float* A_log,
                                 const float* dt_bias, const int* token_row, const int* row_start, const int* row_slot,
                                 float* qn, float* kn, float* vv, float* beta, float* g, float* gate, int tokens, int H,
-                                int KH, int dim, int vdim, int taps, int dtype, cudaStream_t stream) {
+                                int KH, int dim, int vdim, int taps, int dtype, int logs, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     const int64_t C = 2 * (int64_t)KH * dim + (int64_t)H * vdim;
     if (KH < 1 || KH > 64 || H % KH || taps < 1 || taps > DELTA_MAX_TAPS || C * 4 > 160 * 1024) return ACORN_ERR_UNSUPPORTED;
+    // four channels at a time: heads of up to 128 channels whose rows start on vectors of four, 2 to 4 taps
+    const uintptr_t f32s = (uintptr_t)up | (uintptr_t)conv_w | (uintptr_t)dt_bias | (uintptr_t)qn | (uintptr_t)kn | (uintptr_t)vv |
+                           (uintptr_t)g | (uintptr_t)gate;
+    if (dim % 4 == 0 && vdim % 4 == 0 && dim <= 128 && vdim <= 128 && ld % 4 == 0 && ld_up % 4 == 0 && taps >= 2 && taps <= 4 &&
+        (f32s & 15) == 0 && ((uintptr_t)main_ & (dtype == ACORN_DTYPE_BF16 ? 7 : 15)) == 0) {
+#define DELTA_PREP_VEC(TAPS) return launch_delta_prep_vec<T, TAPS>(tokens, H, KH, dim, vdim, logs, stream, (const T*)main_, ld, up, ld_up, \
+                             conv_w, state, slot_stride, conv_off, A_log, dt_bias, token_row, row_start, row_slot, qn, kn, vv, beta, g, gate)
+        ACORN_DISPATCH_DTYPE(dtype, T, {
+            if (taps == 2) DELTA_PREP_VEC(2);
+            if (taps == 3) DELTA_PREP_VEC(3);
+            DELTA_PREP_VEC(4);
+        });
+#undef DELTA_PREP_VEC
+    }
     const size_t smem = (size_t)C * sizeof(float);
     if (smem > 48 * 1024) {
         static AcornPerDevice configured;
@@ -96,7 +218,7 @@ extern "C" int acorn_delta_prep(const void* main_, int64_t ld, const float* up, 
     ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(delta_prep_kernel<T>, dim3(tokens), dim3(256), smem, stream,
                                                        (const T*)main_, ld, up, ld_up, conv_w, state, slot_stride, conv_off,
                                                        A_log, dt_bias, token_row, row_start, row_slot, qn, kn, vv, beta, g,
-                                                       gate, H, KH, dim, vdim, taps));
+                                                       gate, H, KH, dim, vdim, taps, logs));
     return ACORN_ERR_UNSUPPORTED;
 }
 

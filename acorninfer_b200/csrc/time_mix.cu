@@ -100,7 +100,7 @@ template <typename T>
 __global__ void wkv_prep_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v,
                                 const T* __restrict__ g, int64_t ld, const float* __restrict__ z, int64_t ld_z,
                                 const float* __restrict__ w0, float* __restrict__ r32, float* __restrict__ k32,
-                                float* __restrict__ v32, float* __restrict__ decay, float* __restrict__ gate, int C) {
+                                float* __restrict__ v32, float* __restrict__ decay, float* __restrict__ gate, int C, int logs) {
     pdl_wait();
     pdl_trigger();
     const int64_t t = blockIdx.x;
@@ -112,17 +112,18 @@ __global__ void wkv_prep_kernel(const T* __restrict__ r, const T* __restrict__ k
     v32[o] = to_float(v[in]);
     const float gv = to_float(g[in]);
     gate[o] = gv / (1.f + expf(-gv));
-    decay[o] = expf(-expf(z[t * ld_z + c] + w0[c]));
+    const float lg = -expf(z[t * ld_z + c] + w0[c]);
+    decay[o] = logs ? lg * 1.4426950408889634f : expf(lg);
 }
 
 extern "C" int acorn_wkv_prep(const void* r, const void* k, const void* v, const void* g, int64_t ld, const float* z,
                               int64_t ld_z, const float* w0, float* r32, float* k32, float* v32, float* decay,
-                              float* gate, int tokens, int C, int dtype, cudaStream_t stream) {
+                              float* gate, int tokens, int C, int dtype, int logs, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if ((C + 127) / 128 > 65535) return ACORN_ERR_UNSUPPORTED;
     dim3 grid(tokens, (C + 127) / 128);
     ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(wkv_prep_kernel<T>, grid, dim3(128), 0, stream, (const T*)r,
                                                        (const T*)k, (const T*)v, (const T*)g, ld, z, ld_z, w0, r32, k32,
-                                                       v32, decay, gate, C));
+                                                       v32, decay, gate, C, logs));
     return ACORN_ERR_UNSUPPORTED;
 }

@@ -133,7 +133,9 @@ class _Sigs:
     acorn_token_shift = [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
                          c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_wkv_prep = [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
-                      c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
+                      c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
+    acorn_mix_chunk = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
+                       c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_latent_prep = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
                          c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
                          c_int, c_void_p, c_int64, c_void_p]
@@ -144,7 +146,9 @@ class _Sigs:
                          c_int, c_void_p]
     acorn_delta_prep = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p,
                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                        c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+                        c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+    acorn_channel_chunk = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
+                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_conv_state_update = [c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int, c_int, c_int,
                                c_int, c_int, c_void_p, c_void_p]
     acorn_delta_rule = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
@@ -1534,10 +1538,10 @@ def head_linear(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor) -> torch.Tens
 
 def delta_prep(main: torch.Tensor, up32: torch.Tensor, conv_w32: torch.Tensor, state: torch.Tensor, conv_off: int,
                a_log32: torch.Tensor, dt_bias32: torch.Tensor, token_row: torch.Tensor, row_start: torch.Tensor,
-               row_slot: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, taps: int):
+               row_slot: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, taps: int, log2_decays: bool = False):
     """Convolution + silu of the q, k, v channels, unit norms, write strength, decays and output gate of
     every token: returns float32 (q [T, KH, dim], k [T, KH, dim], v [T, H, vdim], beta [T, H],
-    g [T, H, dim], gate [T, H, vdim])."""
+    g [T, H, dim], gate [T, H, vdim]).  ``log2_decays``: g holds the decays' logarithms to base 2."""
     _check(main, "main", None, 2)
     _check(up32, "up", torch.float32, 2)
     _check(state, "state", torch.float32, 2)
@@ -1556,7 +1560,7 @@ def delta_prep(main: torch.Tensor, up32: torch.Tensor, conv_w32: torch.Tensor, s
                                state.data_ptr(), state.stride(0), int(conv_off), a_log32.data_ptr(), dt_bias32.data_ptr(),
                                token_row.data_ptr(), row_start.data_ptr(), row_slot.data_ptr(), q.data_ptr(), k.data_ptr(),
                                v.data_ptr(), beta.data_ptr(), g.data_ptr(), gate.data_ptr(), T, heads, kv_heads, dim, vdim,
-                               taps, dtype_code(main.dtype), _stream()), "delta_prep")
+                               taps, dtype_code(main.dtype), int(log2_decays), _stream()), "delta_prep")
     return q, k, v, beta, g, gate
 
 
@@ -1619,6 +1623,58 @@ def delta_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.T
                                 state.data_ptr() + 4 * int(state_off), state.stride(0), row_start.data_ptr(), row_slot.data_ptr(),
                                 w.data_ptr(), u.data_ptr(), p.data_ptr(), b.data_ptr(), s0.data_ptr(), out.data_ptr(), T, num_rows, H,
                                 KH, dim, vdim, _stream()), "delta_chunk")
+    return out
+
+
+def channel_chunk_ok(longest_row: int, tokens: int, num_rows: int, heads: int, dim: int, vdim: int) -> bool:
+    """Whether the delta rule with decays per key channel runs over chunks (``channel_chunk``) in a step of these rows."""
+    return (longest_row >= DELTA_CHUNK_MIN_ROW and bool(lib().acorn_delta_chunk_supported(dim, vdim)) and heads <= 65535
+            and num_rows <= 65535 and 4 * lib().acorn_delta_chunk_ids(tokens, num_rows) * heads * dim * vdim <= DELTA_CHUNK_SCRATCH_BYTES)
+
+
+def channel_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, log2_g: torch.Tensor, state: torch.Tensor,
+                  row_start: torch.Tensor, row_slot: torch.Tensor, num_rows: int, state_off: int = 0) -> torch.Tensor:
+    """The gated delta rule with a decay per key channel (``log2_g`` [T, H, dim], logarithms to base 2) over chunks of 64
+    tokens, as ``delta_chunk`` does with one per head.  Other arguments and result as for ``delta_rule``."""
+    T, H, vdim = v.shape
+    KH, dim = q.shape[1], q.shape[2]
+    for t, n in ((q, "q"), (k, "k"), (v, "v"), (beta, "beta"), (log2_g, "log2_g")):
+        _check(t, n, torch.float32)
+    _check(state, "state", torch.float32, 2)
+    if log2_g.shape != (T, H, dim) or beta.shape != (T, H) or state.shape[1] < state_off + H * dim * vdim:
+        raise KernelError(f"channel_chunk: log2_g {tuple(log2_g.shape)}, state {tuple(state.shape)} do not fit")
+    f = lambda *shape: torch.empty(shape, dtype=torch.float32, device=v.device)
+    ids = lib().acorn_delta_chunk_ids(T, num_rows)
+    w, u, p, qs, kend, out = f(T, H, dim), f(T, H, vdim), f(T, H, 64), f(T, H, dim), f(T, H, dim), f(T, H, vdim)
+    s0, decay = f(ids, H, dim, vdim), f(ids, H, dim)
+    _ok(lib().acorn_channel_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), log2_g.data_ptr(),
+                                  state.data_ptr() + 4 * int(state_off), state.stride(0), row_start.data_ptr(), row_slot.data_ptr(),
+                                  w.data_ptr(), u.data_ptr(), p.data_ptr(), qs.data_ptr(), kend.data_ptr(), decay.data_ptr(),
+                                  s0.data_ptr(), out.data_ptr(), T, num_rows, H, KH, dim, vdim, _stream()), "delta_rule")
+    return out
+
+
+def mix_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bonus32: torch.Tensor, log2_g: torch.Tensor, state: torch.Tensor,
+              row_start: torch.Tensor, row_slot: torch.Tensor, num_rows: int, state_off: int = 0) -> torch.Tensor:
+    """The form of ``delta_rule`` that reads the state first (``bonus32``) over chunks of 64 tokens; ``log2_g`` [T, H, dim]:
+    logarithms to base 2 of the decays.  Taken where ``channel_chunk_ok`` says so and the slots are aligned
+    (``state_off`` and the slots' stride multiples of four)."""
+    T, H, vdim = v.shape
+    KH, dim = q.shape[1], q.shape[2]
+    for t, n in ((q, "q"), (k, "k"), (v, "v"), (log2_g, "log2_g")):
+        _check(t, n, torch.float32, 3)
+    _check(bonus32, "bonus", torch.float32, 2)
+    _check(state, "state", torch.float32, 2)
+    if log2_g.shape != (T, H, dim) or bonus32.shape != (H, dim) or state.shape[1] < state_off + H * dim * vdim:
+        raise KernelError(f"mix_chunk: log2_g {tuple(log2_g.shape)}, bonus {tuple(bonus32.shape)}, state {tuple(state.shape)} do not fit")
+    f = lambda *shape: torch.empty(shape, dtype=torch.float32, device=v.device)
+    ids = lib().acorn_delta_chunk_ids(T, num_rows)
+    p, qs, out = f(T, H, 64), f(T, H, dim), f(T, H, vdim)
+    s0, decay = f(ids, H, dim, vdim), f(ids, H, dim)
+    _ok(lib().acorn_mix_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), bonus32.data_ptr(), log2_g.data_ptr(),
+                              state.data_ptr() + 4 * int(state_off), state.stride(0), row_start.data_ptr(), row_slot.data_ptr(),
+                              p.data_ptr(), qs.data_ptr(), decay.data_ptr(), s0.data_ptr(), out.data_ptr(), T, num_rows, H, KH, dim,
+                              vdim, _stream()), "delta_rule")
     return out
 
 
@@ -1844,9 +1900,9 @@ def token_shift(h: torch.Tensor, mu32: torch.Tensor, state: torch.Tensor, prev_o
 
 
 def wkv_prep(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, z32: torch.Tensor, w0_32: torch.Tensor,
-             heads: int):
-    """For the recurrence, float32 [T, H, dim] each: r, k, v as they are, the decay ``exp(-exp(z + w0))`` and the
-    gate ``silu(g)``.  r, k, v, g: [T, H dim] of the activation dtype with one row stride; z32 [T, H dim] float32."""
+             heads: int, log2_decays: bool = False):
+    """For the recurrence, float32 [T, H, dim] each: r, k, v as they are, the decay ``exp(-exp(z + w0))`` (``log2_decays``: its
+    logarithm to base 2) and the gate ``silu(g)``.  r, k, v, g: [T, H dim] of the activation dtype with one row stride; z32 [T, H dim] float32."""
     T, C = r.shape
     for t, n in ((r, "r"), (k, "k"), (v, "v"), (g, "g")):
         if not t.is_cuda or t.dtype != r.dtype or t.dim() != 2:
@@ -1860,7 +1916,7 @@ def wkv_prep(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor,
     outs = torch.empty((5, T, heads, C // heads), dtype=torch.float32, device=r.device)
     _ok(lib().acorn_wkv_prep(r.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), r.stride(0), z32.data_ptr(),
                              z32.stride(0), w0_32.data_ptr(), outs[0].data_ptr(), outs[1].data_ptr(), outs[2].data_ptr(),
-                             outs[3].data_ptr(), outs[4].data_ptr(), T, C, dtype_code(r.dtype), _stream()), "wkv_prep")
+                             outs[3].data_ptr(), outs[4].data_ptr(), T, C, dtype_code(r.dtype), int(log2_decays), _stream()), "wkv_prep")
     return outs[0], outs[1], outs[2], outs[3], outs[4]
 
 

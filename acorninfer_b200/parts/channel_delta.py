@@ -81,11 +81,13 @@ class ChannelDelta(Mixer):
         dt = self.ctx.dtype
         main = ops.linear(x, self.w_main, out_dtype=dt)
         up = ops.linear(ops.linear(x, self.w_low, out_dtype=dt), self.w_up, out_dtype=torch.float32)
+        # long rows over chunks of tokens, whose kernels want the decays' logarithms; other steps token by token
+        chunks = ops.channel_chunk_ok(inputs.plan.max_q_len, main.shape[0], inputs.num_rows, self.H, self.dim, self.vdim)
         q, k, v, beta, g, gate = ops.delta_prep(main, up, self.conv32, cache.state, self.state_s, self.a_log32,
                                                 self.dt_bias32, inputs.token_row, inputs.row_start, inputs.row_slot,
-                                                self.H, self.KH, self.dim, self.vdim, self.taps)
+                                                self.H, self.KH, self.dim, self.vdim, self.taps, log2_decays=chunks)
         ops.conv_state_update(main, cache.state, self.state_s, inputs.row_start, inputs.row_slot, inputs.num_rows,
                               self.channels, self.taps)
-        o = ops.delta_rule(q, k, v, beta, g, cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)
+        o = (ops.channel_chunk if chunks else ops.delta_rule)(q, k, v, beta, g, cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)
         y = ops.delta_out(o, gate, self.norm32, self.eps, dt)
         return ops.linear(y, self.w_o, out_dtype=dt)

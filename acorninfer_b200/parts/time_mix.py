@@ -77,8 +77,14 @@ class TimeMix(Mixer):
         r, k, v, g = ops.grouped_gemm(mixes[:4].view(4 * T, self.hidden_size), None, self.w_rkvg,
                                       inputs.extra["time_mix.blend_rows"], 4 * T).view(4, T, -1).unbind(0)
         z = ops.linear(ops.linear(mixes[4], w["w1"], out_dtype=dt, act="tanh"), w["w2"], out_dtype=torch.float32)
-        r32, k32, v32, decay, gate = ops.wkv_prep(r, k, v, g, z, self.w0_32, self.H)
-        o = ops.delta_rule(r32, k32, v32, None, decay, cache.state, inputs.row_start, inputs.row_slot,
-                           inputs.num_rows, bonus32=self.u32, longest_row=inputs.plan.max_q_len)
+        # long rows over chunks of tokens, whose kernels want the decays' logarithms; other steps token by token
+        d = r.shape[1] // self.H
+        chunks = cache.state.stride(0) % 4 == 0 and ops.channel_chunk_ok(inputs.plan.max_q_len, T, inputs.num_rows, self.H, d, d)
+        r32, k32, v32, decay, gate = ops.wkv_prep(r, k, v, g, z, self.w0_32, self.H, log2_decays=chunks)
+        if chunks:
+            o = ops.mix_chunk(r32, k32, v32, self.u32, decay, cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)
+        else:
+            o = ops.delta_rule(r32, k32, v32, None, decay, cache.state, inputs.row_start, inputs.row_slot,
+                               inputs.num_rows, bonus32=self.u32, longest_row=inputs.plan.max_q_len)
         y = ops.delta_out(o, gate, self.norm32, self.eps, dt)
         return ops.linear(y, w["o"], out_dtype=dt)

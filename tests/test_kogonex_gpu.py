@@ -457,3 +457,49 @@ def test_bigram_rows_carry_the_previous_token_between_steps():
         for s, (a, b) in cut.items():
             assert got[t:t + b - a] == want[s][a:b], (cut, s)
             t += b - a
+
+
+@pytest.mark.parametrize("H,KH,dim,vdim", [(4, 2, 8, 12), (3, 3, 32, 20), (2, 1, 64, 64), (6, 3, 96, 80), (2, 2, 128, 128), (1, 1, 128, 200)])
+def test_delta_rule_with_channel_decays_over_chunks(H, KH, dim, vdim):
+    """The recurrence over chunks of tokens against the loop over tokens in 64 bits and no further from it than three times the
+    kernel that walks them: rows that end on and around an edge of a chunk (64) and of a block in it (16), unequal rows in one step, keys that
+    repeat (a system far from the identity), channels from no decay to one that leaves nothing, states that were there before."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim + vdim)
+    rand = lambda *shape, scale=1.0: scale * torch.randn(*shape, generator=g)
+    unit = lambda t: t / torch.sqrt(t.pow(2).sum(-1, keepdim=True) + 1e-6)
+    for lens in ([64], [65, 1, 63], [1, 200, 2, 128, 129, 5, 64, 17], [330]):
+        T, slots = sum(lens), torch.randperm(10, generator=g)[:len(lens)].tolist()
+        k = unit((rand(T, KH, dim, scale=0.4) + rand(KH, dim)).double())
+        q = unit(rand(T, KH, dim).double()) * dim ** -0.5
+        v, beta = rand(T, H, vdim).double(), torch.rand(T, H, generator=g).double()
+        log2_g = -torch.exp(rand(T, H, dim, scale=2.0) - 2.0)
+        log2_g[:, :, 0] = 0.0
+        log2_g[T // 2, :, 1:5] = -130.0
+        state = rand(10, H * dim * vdim + 4)
+        f = lambda t: t.float().contiguous().to(DEV)
+        starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+        i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)
+        assert o.channel_chunk_ok(max(lens), T, len(lens), H, dim, vdim) == (max(lens) >= 64)
+        got, ends = {}, {}
+        for how in ("chunks", "walk"):
+            sd = state.to(DEV)
+            run, decays = (o.channel_chunk, log2_g) if how == "chunks" else (o.delta_rule, torch.exp2(log2_g.double()))
+            got[how] = run(f(q), f(k), f(v), f(beta), f(decays), sd, i32(starts), i32(slots), len(lens), state_off=4).double().cpu()
+            ends[how] = sd.double().cpu()
+        group = torch.arange(H) // (H // KH)
+        qf, kf, vf, bf = (t.float().double() for t in (q, k, v, beta))
+        for r, (n, slot) in enumerate(zip(lens, slots)):
+            S, want = state[slot, 4:].double().view(H, dim, vdim), []
+            for t in range(starts[r], starts[r] + n):
+                S = torch.exp2(log2_g[t].double())[:, :, None] * S
+                u = bf[t][:, None] * (vf[t] - torch.einsum("hdv,hd->hv", S, kf[t][group]))
+                S = S + kf[t][group][:, :, None] * u[:, None]
+                want.append(torch.einsum("hdv,hd->hv", S, qf[t][group]))
+            want = torch.stack(want)
+            rows = slice(starts[r], starts[r] + n)
+            err = {how: float((got[how][rows] - want).norm() / want.norm()) for how in got}
+            end = {how: float((ends[how][slot, 4:].view(H, dim, vdim) - S).norm() / S.norm()) for how in got}
+            assert err["chunks"] < max(3 * err["walk"], 1e-6) and end["chunks"] < max(3 * end["walk"], 1e-6), (lens, r, err, end)
+        untouched = [s for s in range(10) if s not in slots]
+        assert torch.equal(ends["chunks"][untouched], state[untouched].double()) and torch.equal(ends["chunks"][:, :4], state[:, :4].double())

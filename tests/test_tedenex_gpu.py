@@ -431,6 +431,46 @@ def test_recurrence_that_reads_the_state_first_across_steps_and_slots(H, dim, lo
     assert float(state[1].min()) == 123.0 and float(state[3, H * dim * dim:].min()) == 123.0
 
 
+@pytest.mark.parametrize("H,dim,vdim", [(3, 8, 12), (4, 32, 32), (2, 64, 64), (1, 100, 68), (2, 128, 132)])
+def test_recurrence_that_reads_the_state_first_over_chunks(H, dim, vdim):
+    """Over chunks of tokens against the loop in 64 bits, and no further from it than three times the kernel that walks the
+    tokens: rows around the edges of a chunk (64) and of a block in it (16), channels from no decay to one that leaves nothing."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim)
+    for lens in ([64], [65, 1, 63], [1, 200, 2, 128, 129, 5, 64, 17], [330]):
+        T, slots = sum(lens), torch.randperm(10, generator=g)[:len(lens)].tolist()
+        r, k, v = torch.randn(T, H, dim, generator=g), 0.5 * torch.randn(T, H, dim, generator=g), torch.randn(T, H, vdim, generator=g)
+        log2_g = -torch.exp(2.0 * torch.randn(T, H, dim, generator=g) - 2.0)
+        log2_g[:, :, 0] = 0.0
+        log2_g[T // 2, :, 1:5] = -130.0
+        u = torch.randn(H, dim, generator=g)
+        state = torch.randn(10, 4 + H * dim * vdim, generator=g)
+        i32 = dict(dtype=torch.int32, device=DEV)
+        starts = np.cumsum([0] + lens)
+        got, ends = {}, {}
+        for how in ("chunks", "walk"):
+            sd = state.to(DEV)
+            args = (sd, torch.tensor(starts, **i32), torch.tensor(slots, **i32), len(lens))
+            if how == "chunks":
+                out = o.mix_chunk(r.to(DEV), k.to(DEV), v.to(DEV), u.to(DEV), log2_g.to(DEV), *args, state_off=4)
+            else:
+                out = o.delta_rule(r.to(DEV), k.to(DEV), v.to(DEV), None, torch.exp2(log2_g.double()).float().to(DEV), *args,
+                                   bonus32=u.to(DEV), state_off=4)
+            got[how], ends[how] = out.double().cpu(), sd.double().cpu()
+        rd, kd, vd, ud = r.double(), k.double(), v.double(), u.double()
+        for row, (n, slot) in enumerate(zip(lens, slots)):
+            S, want = state[slot, 4:].double().view(H, dim, vdim), []
+            for t in range(starts[row], starts[row] + n):
+                kv = kd[t][:, :, None] * vd[t][:, None]
+                want.append(torch.einsum("hdv,hd->hv", S + ud[:, :, None] * kv, rd[t]))
+                S = torch.exp2(log2_g[t].double())[:, :, None] * S + kv
+            want, rows = torch.stack(want), slice(starts[row], starts[row] + n)
+            err = {how: float((got[how][rows] - want).norm() / want.norm()) for how in got}
+            end = {how: float((ends[how][slot, 4:].view(H, dim, vdim) - S).norm() / S.norm()) for how in got}
+            assert err["chunks"] < max(3 * err["walk"], 1e-6) and end["chunks"] < max(3 * end["walk"], 1e-6), (lens, row, err, end)
+        assert torch.equal(ends["chunks"][:, :4], state[:, :4].double())
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
 @pytest.mark.parametrize("W,off,tail,single", [(20, 7, 3, False), (20, 8, 4, False), (20, 8, 4, True), (520, 4, 0, True),
                                                (22, 8, 2, True)])
