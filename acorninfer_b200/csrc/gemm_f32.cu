@@ -10,7 +10,7 @@
 // A, W: float32 row-major, K contiguous, with row strides lda, ldw; C row stride ldc.
 //   rows kernel   up to 16 rows (decode): a block takes 16 or 32 columns and all rows, a warp one range of K with a ring
 //                 of cp.async stages of its own (no block barrier): bound by reading W once;
-//   tile kernel   more rows: 64 x 64 a block; a cluster of eight shares a tile's ranges where the tiles
+//   tile kernel   more rows: 64 x 128 a block; a cluster of eight shares a tile's ranges where the tiles
 //                 alone leave the device idle: bound by the multiply-adds and the reads of shared memory that feed them;
 //   plain kernel  64 x 64 a block, scalar loads: operands that are not 16-byte aligned.
 #include "mma_helpers.cuh"
@@ -186,106 +186,136 @@ __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* 
 
 // ------------------------------------------------------------------ tile kernel
 
+#define TL_BM 64
+#define TL_BN 128
 #define TL_BK 16
-#define TL_LD (TL_BK + 4)       // row stride in shared memory: 16-byte reads of 8 neighbouring rows hit 8 groups of banks
 #define TL_THREADS 128
-#define TL_TM 4                 // a thread's rows and columns of the tile
-#define TL_TN 8
-#define TL_BM (16 * TL_TM)
-#define TL_BN (8 * TL_TN)
+#define TL_SMEM ((2 * TL_BK * (TL_BM + TL_BN) + TL_BM * TL_BN) * (int)sizeof(float))
 
-#define TL_SMEM ((2 * (TL_BM + TL_BN) * TL_LD + TL_BM * TL_BN) * (int)sizeof(float))
+// acc += (a, a) * w on a pair of columns
+__device__ __forceinline__ void fma_pair(float2& acc, unsigned long long a, float2 w) {
+    unsigned long long r = *reinterpret_cast<unsigned long long*>(&acc);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(r) : "l"(a), "l"(*reinterpret_cast<unsigned long long*>(&w)));
+    acc = *reinterpret_cast<float2*>(&r);
+}
 
-// Rows of A and W lie in shared memory as in memory (16-byte copies), and a thread reads four k of a row at a time: twelve
-// reads feed 128 multiply-adds, and four blocks on an SM hide one another's loads.  (Tiles of 128 x 128 with 8 x 16 a thread:
-// the same 38 TFLOP/s at 2,048 rows and less where tiles are few; with operands transposed for multiply-adds in packed pairs
-// 40 TFLOP/s, 29 at 777 rows.  A loop of nothing but multiply-adds on three registers runs at 61 here.)
+// A thread holds 8 rows x 8 columns in packed pairs: four 16-byte reads of shared memory feed 64 multiply-adds, and the packed
+// instructions leave half of the issue slots to them.  Four lanes bring 64 bytes of a row; shared memory is [k][row], rows
+// exchanged in groups of eight by k / 4, so that neither those writes nor the reads meet in a bank.
 // SPLIT: a cluster of eight CTAs shares an output tile, each takes one range of K, and each adds up and writes an eighth of
 // the tile's rows.
-// Measured (B200): the 112 products of a 777-token prompt at Qwen3-0.6B sizes, with one chain over K and tiles of 128 x 128
-// 32.8 ms, this 20.6 ms.
+// Bound by the multiply-adds and the reads of shared memory about equally (2,048 rows, N = 4,096, K = 1,024: the multiply-add
+// pipe 67 % busy, the shared memory pipe 70 %; 47 TFLOP/s, where a loop of nothing but packed multiply-adds runs at 73).
+// Measured (B200): the 112 products of a 777-token prompt at Qwen3-0.6B sizes: with one chain over K and tiles of 128 x 128
+// 32.8 ms; tiles of 64 x 64, 4 x 8 a thread, one multiply-add an instruction, rows as in memory 20.6 ms; this 18.8 ms.
 template <bool SPLIT>
-__global__ void __launch_bounds__(TL_THREADS, 4) gemm_f32_tile_kernel(const float* __restrict__ A, int64_t lda,
+__global__ void __launch_bounds__(TL_THREADS, 3) gemm_f32_tile_kernel(const float* __restrict__ A, int64_t lda,
                                                                       const float* __restrict__ W, int64_t ldw,
                                                                       float* __restrict__ C, int64_t ldc, int M, int N,
                                                                       int K) {
-    constexpr int TM = TL_TM, TN = TL_TN, BM = TL_BM, BN = TL_BN;
+    constexpr int BM = TL_BM, BN = TL_BN;
     extern __shared__ __align__(16) float tl_buf[];
-    float* ring = tl_buf;                                        // [2][BM + BN][LD]: rows of A, then of W
-    float* total = ring + 2 * (BM + BN) * TL_LD;                 // the ranges' sum so far, [element][thread]; SPLIT: [row][column]
+    float* As = tl_buf;                                          // [2][BK][BM]
+    float* Ws = As + 2 * TL_BK * BM;                             // [2][BK][BN]
+    float* total = Ws + 2 * TL_BK * BN;                          // the ranges' sum so far, [element][thread]; SPLIT: [row][column]
     const int part = SPLIT ? blockIdx.x % K_RANGES : 0;
     const int m0 = blockIdx.y * BM, n0 = (SPLIT ? blockIdx.x / K_RANGES : blockIdx.x) * BN;
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;       // columns tx + 8 j, rows ty + 16 i
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);     // columns 4 tx .., 64 + ..; rows 4 ty .., 32 + ..
     const int range = k_range(K);
     const int kbeg = SPLIT ? min(K, part * range) : 0, kend = SPLIT ? min(K, kbeg + range) : K;
     const int nt = (kend - kbeg + TL_BK - 1) / TL_BK;
+    const int lrow = threadIdx.x >> 2, lseg = threadIdx.x & 3;   // brings k 4 lseg .. of rows lrow + 32 e
+    float4 ra[BM / 32], rw[BN / 32];
 
-    auto load = [&](int t) {
-        float* dst = ring + (t & 1) * (BM + BN) * TL_LD;
-        const int seg = (threadIdx.x & 3) * 4, k = kbeg + t * TL_BK + seg;
+    auto fetch = [&](int t) {                                    // rows beyond the matrix: another row's values, never written
+        const int k = kbeg + t * TL_BK + 4 * lseg;
 #pragma unroll
-        for (int e = 0; e < (BM + BN) / 32; ++e) {
-            const int row = e * 32 + (threadIdx.x >> 2);
-            const bool of_a = e < BM / 32;
-            const int at = of_a ? m0 + row : n0 + row - BM;
-            const bool valid = k < kend && at < (of_a ? M : N);
-            const float* src = of_a ? A + (int64_t)at * lda + k : W + (int64_t)at * ldw + k;
-            cp_async_16(smem_addr(dst + row * TL_LD + seg), valid ? src : W, valid);
+        for (int e = 0; e < BM / 32; ++e)
+            ra[e] = k < kend ? *reinterpret_cast<const float4*>(A + (int64_t)min(m0 + lrow + 32 * e, M - 1) * lda + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < BN / 32; ++e)
+            rw[e] = k < kend ? *reinterpret_cast<const float4*>(W + (int64_t)min(n0 + lrow + 32 * e, N - 1) * ldw + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto stash = [&](int buf) {
+        float* a = As + (buf * TL_BK + 4 * lseg) * BM + (lrow ^ (lseg << 3));
+        float* w = Ws + (buf * TL_BK + 4 * lseg) * BN + (lrow ^ (lseg << 3));
+#pragma unroll
+        for (int e = 0; e < BM / 32; ++e) {
+            a[32 * e] = ra[e].x; a[BM + 32 * e] = ra[e].y; a[2 * BM + 32 * e] = ra[e].z; a[3 * BM + 32 * e] = ra[e].w;
         }
-        cp_async_commit();
+#pragma unroll
+        for (int e = 0; e < BN / 32; ++e) {
+            w[32 * e] = rw[e].x; w[BN + 32 * e] = rw[e].y; w[2 * BN + 32 * e] = rw[e].z; w[3 * BN + 32 * e] = rw[e].w;
+        }
     };
 
-    float acc[TM][TN];
+    float2 acc[8][4];                            // [row][pair of columns]
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
     pdl_wait();
     pdl_trigger();
-    if (nt > 0) load(0);
+    if (nt > 0) {
+        fetch(0);
+        stash(0);
+    }
+    __syncthreads();
     bool folded = false;
     for (int t = 0; t < nt; ++t) {
-        cp_async_wait<0>();
-        __syncthreads();                         // tile t is there for all, and all are done with the one before it
-        if (t + 1 < nt) load(t + 1);
+        const int buf = t & 1;
+        if (t + 1 < nt) fetch(t + 1);            // in flight while this tile is multiplied
         if (!SPLIT && t > 0 && (t * TL_BK) % range == 0) {
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    float* p = total + (i * TN + j) * TL_THREADS + threadIdx.x;
-                    *p = folded ? *p + acc[i][j] : acc[i][j];
-                    acc[i][j] = 0.f;
+                for (int j = 0; j < 4; ++j) {
+                    float2* p = reinterpret_cast<float2*>(total) + (i * 4 + j) * TL_THREADS + threadIdx.x;
+                    float2 v = folded ? *p : make_float2(0.f, 0.f);
+                    v.x += acc[i][j].x;
+                    v.y += acc[i][j].y;
+                    *p = v;
+                    acc[i][j] = make_float2(0.f, 0.f);
                 }
             folded = true;
         }
-        const float* a_at = ring + (t & 1) * (BM + BN) * TL_LD + ty * TL_LD;
-        const float* w_at = ring + ((t & 1) * (BM + BN) + BM + tx) * TL_LD;
 #pragma unroll
-        for (int kk = 0; kk < TL_BK; kk += 4) {
-            float4 a[TM];
+        for (int kk = 0; kk < TL_BK; ++kk) {
+            const float* a_at = As + (buf * TL_BK + kk) * BM;
+            const float* w_at = Ws + (buf * TL_BK + kk) * BN;
+            float2 w[4];
+            unsigned long long a[8];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(a_at + 16 * i * TL_LD + kk);
-#pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const float4 w = *reinterpret_cast<const float4*>(w_at + 8 * j * TL_LD + kk);
-#pragma unroll
-                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, w.x, acc[i][j]);
-#pragma unroll
-                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].y, w.y, acc[i][j]);
-#pragma unroll
-                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].z, w.z, acc[i][j]);
-#pragma unroll
-                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, w.w, acc[i][j]);
+            for (int c = 0; c < 2; ++c) {
+                const float4 v = *reinterpret_cast<const float4*>(w_at + ((64 * c + 4 * tx) ^ ((kk >> 2) << 3)));
+                w[2 * c] = make_float2(v.x, v.y);
+                w[2 * c + 1] = make_float2(v.z, v.w);
             }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float4 v = *reinterpret_cast<const float4*>(a_at + ((32 * r + 4 * ty) ^ ((kk >> 2) << 3)));
+                asm("mov.b64 %0, {%1, %1};" : "=l"(a[4 * r]) : "f"(v.x));
+                asm("mov.b64 %0, {%1, %1};" : "=l"(a[4 * r + 1]) : "f"(v.y));
+                asm("mov.b64 %0, {%1, %1};" : "=l"(a[4 * r + 2]) : "f"(v.z));
+                asm("mov.b64 %0, {%1, %1};" : "=l"(a[4 * r + 3]) : "f"(v.w));
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) fma_pair(acc[i][j], a[i], w[j]);
         }
+        if (t + 1 < nt) stash(buf ^ 1);          // the other buffer was last read before the barrier below, a tile ago
+        __syncthreads();
     }
     if (SPLIT) {
         cg::cluster_group cluster = cg::this_cluster();
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < TN; ++j) total[(ty + 16 * i) * BN + tx + 8 * j] = acc[i][j];
+            for (int c = 0; c < 2; ++c)
+                *reinterpret_cast<float4*>(total + (4 * ty + (i & 3) + 32 * (i >> 2)) * BN + 64 * c + 4 * tx) =
+                    make_float4(acc[i][2 * c].x, acc[i][2 * c].y, acc[i][2 * c + 1].x, acc[i][2 * c + 1].y);
         cluster.sync();
         const float4* mine = reinterpret_cast<const float4*>(total);
 #pragma unroll 2
@@ -306,13 +336,19 @@ __global__ void __launch_bounds__(TL_THREADS, 4) gemm_f32_tile_kernel(const floa
         return;
     }
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int m = m0 + ty + 16 * i;
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 4 * ty + (i & 3) + 32 * (i >> 2);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int n = n0 + tx + 8 * j;
-            if (m < M && n < N)
-                C[(int64_t)m * ldc + n] = folded ? total[(i * TN + j) * TL_THREADS + threadIdx.x] + acc[i][j] : acc[i][j];
+        for (int j = 0; j < 4; ++j) {
+            float2 v = acc[i][j];
+            if (folded) {
+                const float2 p = reinterpret_cast<const float2*>(total)[(i * 4 + j) * TL_THREADS + threadIdx.x];
+                v.x = p.x + v.x;
+                v.y = p.y + v.y;
+            }
+            const int n = n0 + 64 * (j >> 1) + 4 * tx + 2 * (j & 1);
+            if (m < M && n < N) C[(int64_t)m * ldc + n] = v.x;
+            if (m < M && n + 1 < N) C[(int64_t)m * ldc + n + 1] = v.y;
         }
     }
 }
@@ -378,11 +414,11 @@ extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64
         return wide ? launch_rows<8, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<8, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
     if (aligned) {
-        // A cluster to a tile where whole tiles would leave an SM fewer than four of them, which is what hides their loads'
-        // latency (777 rows, N = 1,024, K = 2,048, 208 tiles: 146 -> 98 us; N = 4,096, K = 1,024, 832 tiles: 203 against 199 us
-        // whole), and a range of K is worth its share of the exchange.
+        // A cluster to a tile where whole tiles would leave an SM fewer than two of them (777 rows, N = 1,024, K = 2,048, 104 tiles:
+        // 131 us whole, 97 us split; 2,048 rows of the same, 256 tiles: 316 and 216 us; 777 rows, N = 4,096, K = 1,024, 416
+        // tiles: 164 whole, 181 split), and a range of K is worth its share of the exchange.
         const int64_t tiles = (int64_t)((N + TL_BN - 1) / TL_BN) * ((M + TL_BM - 1) / TL_BM);
-        if (tiles < 4 * 148 && K >= 256) return launch_tile<true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+        if (tiles < 2 * 148 && K >= 256) return launch_tile<true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
         return launch_tile<false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
     dim3 grid((N + PL_BN - 1) / PL_BN, (M + PL_BM - 1) / PL_BM);
