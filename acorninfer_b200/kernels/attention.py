@@ -9,6 +9,8 @@ sizes and group sizes the fast kernels do not take.
 
 from __future__ import annotations
 
+from functools import lru_cache
+
 import numpy as np
 import torch
 
@@ -71,6 +73,7 @@ def merged_in_kernel(splits: int, limit: int) -> bool:
     return splits <= min(limit, 8) or (splits == 16 and limit >= 16)
 
 
+@lru_cache(maxsize=4096)        # asked by every layer of a step, with the same sizes
 def decode_splits(rows: int, num_kv_heads: int, key_bound: int, head_dim: int, num_sms: int = B200_SMS,
                   merge_free_upto: int = 1) -> int:
     """Splits of the key range.  ``key_bound`` bounds the keys any row reads; it changes only with

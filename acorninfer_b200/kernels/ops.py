@@ -9,8 +9,9 @@ to fall back to.  Tensors are passed as raw device pointers.
 from __future__ import annotations
 
 import ctypes
-from dataclasses import dataclass
 from ctypes import c_float, c_int, c_int64, c_void_p
+from dataclasses import dataclass
+from functools import lru_cache
 
 import torch
 
@@ -310,6 +311,8 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 def _check(t: torch.Tensor, name: str, dtype=None, dims: int | None = None) -> None:
+    if t.is_cuda and t.is_contiguous() and (dtype is None or t.dtype is dtype) and (dims is None or t.ndim == dims):
+        return
     if not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor")
     if not t.is_contiguous():
@@ -1019,6 +1022,7 @@ GEMM_PAIR_ALONE_MAX_ROWS = 8192
 GEMM_PAIR_ALONE_MIN_K = 2048      # ... whose K must be long enough for a tile's k-steps to hide its epilogue
 
 
+@lru_cache(maxsize=4096)
 def pair_fill(num_rows: int, width: int, num_sms: int = 148) -> float:
     """How full the paired kernel's rounds are for a product of ``num_rows`` rows and ``width`` output
     columns: its tiles of 256 x 256 are taken in rounds of one tile to a pair of SMs; the product's
