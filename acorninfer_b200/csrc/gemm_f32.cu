@@ -85,103 +85,121 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
 // ------------------------------------------------------------------ rows kernel
 
 #define RS_BK 32
-#define RS_STAGES 4
 #define RS_LD (RS_BK + 4)       // row stride in shared memory: 16-byte reads of 8 neighbouring rows hit 8 groups of banks
 #define RS_THREADS (32 * K_RANGES)
 
 // R rows and CPL columns a lane, 2 R rows and 16 CPL columns a block.
-template <int R, int CPL> constexpr int rs_smem() { return K_RANGES * RS_STAGES * (16 * CPL + 2 * R) * RS_LD * (int)sizeof(float); }
+template <int R, int CPL> constexpr int rs_stages() { return R == 8 && CPL == 2 ? 3 : 4; }     // what shared memory holds
+template <int R, int CPL> constexpr int rs_ring() { return K_RANGES * rs_stages<R, CPL>() * (16 * CPL + 2 * R) * RS_LD; }
+// the ranges' sums: with one column a lane in the place of the rings, with two behind them, for two tiles
+template <int R, int CPL> constexpr int rs_smem() {
+    return (rs_ring<R, CPL>() + (CPL == 2 ? 2 * K_RANGES * 2 * R * 16 * CPL : 0)) * (int)sizeof(float);
+}
 
-// Measured (B200): the 113 products of a decode step of 6 rows at Qwen3-1.7B sizes (6.9 GB), with one block for 32 columns and
-// 16 rows whose four warps walked K together 5.64 ms, this 2.09 ms.  At 6 rows the reads of A and W from shared memory that feed
-// the multiply-adds set the pace (3.6 TB/s at N = 12,288; 4.6 TB/s at one row).
 // With two columns a lane a row of A that was read serves two weights, but a block takes 32 columns: for wide matrices only.
+// A block then walks the tiles of its share one behind the other, and the next tile's weights are under way while the ranges'
+// sums of the one before are added: a block that ends with its tile spends a third of its time on filling and emptying its
+// rings (6 rows, N = 12,288, K = 2,048: 31 -> 25 us).
+// Measured (B200): the 113 products of a decode step of 6 rows at Qwen3-1.7B sizes (6.9 GB), with one block for 32 columns and
+// 16 rows whose four warps walked K together 5.64 ms, this 1.9 ms.  At 6 rows the reads of A and W from shared memory that feed
+// the multiply-adds set the pace (4.0 TB/s at N = 12,288, 4.9 at N = 151,936; at one row 4.9 and 6.2).
 template <int R, int CPL>
 __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* __restrict__ A, int64_t lda,
                                                                    const float* __restrict__ W, int64_t ldw,
                                                                    float* __restrict__ C, int64_t ldc, int M, int N, int K) {
     extern __shared__ __align__(16) float rs_buf[];
-    constexpr int BN = 16 * CPL, ROWS = BN + 2 * R, STAGE = ROWS * RS_LD;
-    const int n0 = blockIdx.x * BN;
+    constexpr int BN = 16 * CPL, ROWS = BN + 2 * R, STAGE = ROWS * RS_LD, STAGES = rs_stages<R, CPL>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int col = lane & 15, row0 = (lane >> 4) * R;
     const int range = k_range(K), kbeg = min(K, warp * range), kend = min(K, kbeg + range);
     const int nk = (kend - kbeg + RS_BK - 1) / RS_BK;
-    float* ring = rs_buf + warp * RS_STAGES * STAGE;
+    const int tiles = (N + BN - 1) / BN;
+    const int mine = CPL == 2 ? (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1;   // tiles of this block
+    float* ring = rs_buf + warp * STAGES * STAGE;
 
-    auto load = [&](int stage, int kb) {
-        float* dst = ring + stage * STAGE;
+    int ltile = 0, lkb = 0, fill = 0;            // the next stage to load: of which tile of this block, where in K, into which slot
+    auto load = [&]() {
+        if (ltile < mine && nk > 0) {
+            const int n0 = ((int)blockIdx.x + ltile * (int)gridDim.x) * BN;
+            float* dst = ring + fill * STAGE;
 #pragma unroll
-        for (int e = 0; e < ROWS / 4; ++e) {                     // rows of W, then of A; 8 lanes take 128 bytes of a row
-            const int row = e * 4 + (lane >> 3), seg = (lane & 7) * 4, k = kbeg + kb * RS_BK + seg;
-            const bool of_w = e < BN / 4;
-            const bool valid = k < kend && (of_w ? n0 + row < N : row - BN < M);
-            const float* src = of_w ? W + (int64_t)(n0 + row) * ldw + k : A + (int64_t)(row - BN) * lda + k;
-            cp_async_16(smem_addr(dst + row * RS_LD + seg), valid ? src : W, valid);
+            for (int e = 0; e < ROWS / 4; ++e) {                 // rows of W, then of A; 8 lanes take 128 bytes of a row
+                const int row = e * 4 + (lane >> 3), seg = (lane & 7) * 4, k = kbeg + lkb * RS_BK + seg;
+                const bool of_w = e < BN / 4;
+                const bool valid = k < kend && (of_w ? n0 + row < N : row - BN < M);
+                const float* src = of_w ? W + (int64_t)(n0 + row) * ldw + k : A + (int64_t)(row - BN) * lda + k;
+                cp_async_16(smem_addr(dst + row * RS_LD + seg), valid ? src : W, valid);
+            }
+            if (++lkb == nk) { lkb = 0; ++ltile; }
+            fill = fill + 1 == STAGES ? 0 : fill + 1;
         }
+        cp_async_commit();
     };
 
     // the first weights on their way to L2 while the kernel before this one ends (W may be its result: not read yet)
 #pragma unroll
-    for (int e = 0; e < CPL * (RS_STAGES - 1) / 2; ++e) {
-        const int row = (lane + 32 * e) % BN, k = kbeg + ((lane + 32 * e) / BN) * RS_BK;
-        if (k < kend && n0 + row < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (int64_t)(n0 + row) * ldw + k));
+    for (int e = 0; e < CPL * (STAGES - 1) / 2; ++e) {
+        const int n = (int)blockIdx.x * BN + (lane + 32 * e) % BN, k = kbeg + ((lane + 32 * e) / BN) * RS_BK;
+        if (k < kend && n < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (int64_t)n * ldw + k));
     }
     pdl_wait();
     pdl_trigger();
-    for (int s = 0; s < RS_STAGES - 1; ++s) {
-        if (s < nk) load(s, s);
-        cp_async_commit();
-    }
-    float acc[R][CPL];
+    for (int s = 0; s < STAGES - 1; ++s) load();
+    int stage = 0;
+    for (int it = 0; it < mine; ++it) {
+        const int n0 = ((int)blockIdx.x + it * (int)gridDim.x) * BN;
+        float acc[R][CPL];
 #pragma unroll
-    for (int i = 0; i < R; ++i)
+        for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int c = 0; c < CPL; ++c) acc[i][c] = 0.f;
-    int stage = 0, fill = RS_STAGES - 1;
-    for (int kb = 0; kb < nk; ++kb) {
-        cp_async_wait<RS_STAGES - 2>();          // this lane's copies of stage kb have landed
-        __syncwarp();                            // all lanes' have, and all are done with stage kb - 1
-        if (kb + RS_STAGES - 1 < nk) load(fill, kb + RS_STAGES - 1);
-        cp_async_commit();
-        const float* wrow = ring + stage * STAGE + col * RS_LD;
-        const float* arow = ring + stage * STAGE + (BN + row0) * RS_LD;
-        stage = stage + 1 == RS_STAGES ? 0 : stage + 1;
-        fill = fill + 1 == RS_STAGES ? 0 : fill + 1;
+            for (int c = 0; c < CPL; ++c) acc[i][c] = 0.f;
+        for (int kb = 0; kb < nk; ++kb) {
+            cp_async_wait<STAGES - 2>();         // this lane's copies of the stage have landed
+            __syncwarp();                        // all lanes' have, and all are done with the stage before
+            load();
+            const float* wrow = ring + stage * STAGE + col * RS_LD;
+            const float* arow = ring + stage * STAGE + (BN + row0) * RS_LD;
+            stage = stage + 1 == STAGES ? 0 : stage + 1;
 #pragma unroll
-        for (int kk = 0; kk < RS_BK; kk += 4) {
-            float4 w[CPL];
+            for (int kk = 0; kk < RS_BK; kk += 4) {
+                float4 w[CPL];
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) w[c] = *reinterpret_cast<const float4*>(wrow + 16 * c * RS_LD + kk);
+                for (int c = 0; c < CPL; ++c) w[c] = *reinterpret_cast<const float4*>(wrow + 16 * c * RS_LD + kk);
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const float4 a = *reinterpret_cast<const float4*>(arow + i * RS_LD + kk);
+                for (int i = 0; i < R; ++i) {
+                    const float4 a = *reinterpret_cast<const float4*>(arow + i * RS_LD + kk);
 #pragma unroll
-                for (int c = 0; c < CPL; ++c) {
-                    acc[i][c] = fmaf(a.x, w[c].x, acc[i][c]);
-                    acc[i][c] = fmaf(a.y, w[c].y, acc[i][c]);
-                    acc[i][c] = fmaf(a.z, w[c].z, acc[i][c]);
-                    acc[i][c] = fmaf(a.w, w[c].w, acc[i][c]);
+                    for (int c = 0; c < CPL; ++c) {
+                        acc[i][c] = fmaf(a.x, w[c].x, acc[i][c]);
+                        acc[i][c] = fmaf(a.y, w[c].y, acc[i][c]);
+                        acc[i][c] = fmaf(a.z, w[c].z, acc[i][c]);
+                        acc[i][c] = fmaf(a.w, w[c].w, acc[i][c]);
+                    }
                 }
             }
         }
+        float* parts = rs_buf;                   // [ranges][2 R][BN]
+        if (CPL == 2) {
+            parts += rs_ring<R, CPL>() + (it & 1) * K_RANGES * 2 * R * BN;
+        } else {
+            cp_async_wait<0>();
+            __syncthreads();                     // the rings are free
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int c = 0; c < CPL; ++c) parts[(warp * 2 * R + row0 + i) * BN + 16 * c + col] = acc[i][c];
+        __syncthreads();                         // the one barrier of a tile: its sums were read before the next tile's barrier
+        for (int o = threadIdx.x; o < 2 * R * BN; o += RS_THREADS) {
+            const int r = o / BN, c = o % BN;
+            if (r >= M || n0 + c >= N) continue;
+            float v = parts[o];
+#pragma unroll
+            for (int q = 1; q < K_RANGES; ++q) v += parts[q * 2 * R * BN + o];
+            C[(int64_t)r * ldc + n0 + c] = v;
+        }
     }
     cp_async_wait<0>();
-    __syncthreads();                             // the rings are free: the ranges' sums meet there
-    float* parts = rs_buf;                       // [ranges][2 R][BN]
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) parts[(warp * 2 * R + row0 + i) * BN + 16 * c + col] = acc[i][c];
-    __syncthreads();
-    for (int o = threadIdx.x; o < 2 * R * BN; o += RS_THREADS) {
-        const int r = o / BN, c = o % BN;
-        if (r >= M || n0 + c >= N) continue;
-        float v = parts[o];
-#pragma unroll
-        for (int q = 1; q < K_RANGES; ++q) v += parts[q * 2 * R * BN + o];
-        C[(int64_t)r * ldc + n0 + c] = v;
-    }
 }
 
 // ------------------------------------------------------------------ tile kernel
@@ -364,7 +382,8 @@ static int launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw,
         if (e != cudaSuccess) return (int)e;
         configured.mark();
     }
-    return acorn_launch(gemm_f32_rows_kernel<R, CPL>, dim3((N + 16 * CPL - 1) / (16 * CPL)), dim3(RS_THREADS), rs_smem<R, CPL>(), stream,
+    const int tiles = (N + 16 * CPL - 1) / (16 * CPL);
+    return acorn_launch(gemm_f32_rows_kernel<R, CPL>, dim3(CPL == 2 ? (tiles < 148 ? tiles : 148) : tiles), dim3(RS_THREADS), rs_smem<R, CPL>(), stream,
                         A, lda, W, ldw, C, ldc, M, N, K);
 }
 

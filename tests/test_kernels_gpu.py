@@ -129,6 +129,21 @@ def test_gemm_f32_gives_the_same_bits_from_each_of_its_kernels():
     assert torch.allclose(tile.double(), a.double() @ w.double().T, atol=1e-5 * math.sqrt(K), rtol=1e-5)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 8192, 2048), (3, 8193, 36), (8, 14208, 520), (6, 19001, 132), (16, 9500, 1028)])
+def test_gemm_f32_of_few_rows_and_many_columns(M, N, K):
+    """Blocks that walk several tiles of columns, ragged last ones, ranges of K shorter than a stage or empty: the bits of
+    the tile kernel, which adds in the same order."""
+    g = torch.Generator().manual_seed(N)
+    a = torch.randn(40, K, generator=g).to(DEV)
+    w = torch.randn(N, K, generator=g).to(DEV)
+    tile = ops().gemm_f32(a, w)
+    assert torch.equal(ops().gemm_f32(a[:M].contiguous(), w), tile[:M])
+    ref = a[:M].double() @ w.double().T
+    # chains of at most ceil(K / 128) * 16 products and seven sums: an error of 2^-24 a step on |a| |w|
+    bound = (a[:M].abs().double() @ w.abs().double().T) * (-(-K // 128) * 16 + 8) * 2.0 ** -24
+    assert ((tile[:M].double() - ref).abs() <= bound).all()
+
+
 def test_gemm_f32_shows_what_a_reduced_precision_mode_would_hide():
     # 1 + 2^-12 is lost by a product that rounds its inputs to 10 mantissa bits (TF32) or to bfloat16
     a = torch.full((4, 8), 1 + 2 ** -12, device=DEV)
