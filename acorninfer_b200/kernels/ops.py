@@ -53,7 +53,8 @@ def _load():
 
 
 _error_word: ctypes.c_int | None = None       # pinned host memory that kernels write when a bounded wait gives up
-_KERNEL_NAMES = {1: "gemm_tcgen05", 2: "attention_prefill_tc", 3: "attention_decode_tma", 4: "gemm_tcgen05_pair", 9: "error-word self-test"}
+_KERNEL_NAMES = {1: "gemm_tcgen05", 2: "attention_prefill_tc", 3: "attention_decode_tma", 4: "gemm_tcgen05_pair",
+                 5: "latent_prefill_tc", 9: "error-word self-test"}
 
 
 def _init_error_word(library) -> None:
@@ -64,7 +65,7 @@ def _init_error_word(library) -> None:
         raise KernelError(f"could not allocate the kernels' error word: CUDA error {code}")
     for setter in ("acorn_gemm_tc_set_error_word", "acorn_attention_tc_set_error_word",
                    "acorn_attention_decode_tma_set_error_word", "acorn_selftest_set_error_word",
-                   "acorn_gemm_tc_pair_set_error_word"):
+                   "acorn_gemm_tc_pair_set_error_word", "acorn_latent_prefill_tc_set_error_word"):
         code = getattr(library, setter)(dev)
         if code != 0:
             raise KernelError(f"{setter}: CUDA error {code}")
@@ -78,7 +79,7 @@ def raise_on_kernel_error() -> None:
         return
     word = _error_word.value
     _error_word.value = 0
-    for getter in (gemm_tc_error, attention_tc_error, attention_decode_tma_error, gemm_tc_pair_error):   # clear the kernels' own flags
+    for getter in (gemm_tc_error, attention_tc_error, attention_decode_tma_error, gemm_tc_pair_error, latent_prefill_tc_error):   # clear the kernels' own flags
         getter()
     raise KernelError(f"kernel {_KERNEL_NAMES.get(word // 100, word // 100)} gave up a bounded wait at point "
                       f"{word % 100}: the results of the step are not valid")
@@ -143,6 +144,11 @@ class _Sigs:
     acorn_latent_attention_tc = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
                                  c_void_p, c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
     acorn_latent_attention_tc_supported = [c_int, c_int, c_int, c_int]
+    acorn_latent_prefill_tc = [c_void_p, c_int, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
+                               c_int, c_void_p, c_float, c_int, c_int, c_int, c_int, c_int, c_void_p]
+    acorn_latent_prefill_tc_supported = [c_int, c_int, c_int, c_int]
+    acorn_latent_prefill_tc_error = []
+    acorn_latent_prefill_tc_set_error_word = [c_void_p]
     acorn_head_linear = [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_int,
                          c_int, c_void_p]
     acorn_delta_prep = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p,
@@ -1513,6 +1519,56 @@ def latent_attention_tc(q: torch.Tensor, pages: torch.Tensor, block_table: torch
                                         tiles.data_ptr(), n, _ptr(sink32), float(scale), int(window or 0), H, d,
                                         int(value_dim), pages.shape[2], int(splits), _ptr(part), _stream()), "latent_attention_tc")
     return out
+
+
+LATENT_PREFILL_ROWS = 128      # (token, head) pairs a block of the tcgen05 kernel takes
+
+
+def latent_prefill_tc_supported(dtype: torch.dtype, num_heads: int, head_dim: int, value_dim: int, page_size: int, scale: float) -> bool:
+    return (dtype == torch.bfloat16 and scale > 0 and
+            bool(lib().acorn_latent_prefill_tc_supported(num_heads, head_dim, value_dim, page_size)))
+
+
+def latent_prefill_tiles(row_lens: list[int], num_heads: int) -> int:
+    """Tiles of ``LATENT_PREFILL_ROWS // H`` tokens that the rows make."""
+    n = LATENT_PREFILL_ROWS // num_heads
+    return sum(-(-length // n) for length in row_lens)
+
+
+def latent_prefill_wins(num_tiles: int, general_tiles: int, key_bound: int) -> bool:
+    """Whether the tcgen05 kernel is the faster one, for so many tiles of 128 rows or of 64 (``latent_attention_tc``) and at
+    most so many keys a row.  It needs 1.6 to 2.3 us for 64 keys whatever the number of tiles (rows of 192 and of 448 entries),
+    the other 7.5 us an SM, but shares a tile's keys out while its tiles are few.  Measured (B200, us, general / tcgen05, rows
+    of 448): 64 requests decoding at 1,000 keys 84 / 42, 32 requests 43 / 41, 8 requests 26 / 41, at 250 keys 24 / 16; a prompt
+    of 300 tokens (16 heads) 40 / 22, of 2,000 under a window of 1,024 311 / 74; rows of 192, at 4,000 keys, 56 requests
+    107 / 102, 48 requests 84 / 101, at 60 keys 300 requests 14 / 21 (two waves with next to nothing to do)."""
+    if key_bound <= 128 and num_tiles > 148:
+        return False
+    return general_tiles >= 56 or key_bound <= 256
+
+
+def latent_prefill_tc(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tensor, page_base: torch.Tensor,
+                      row_start: torch.Tensor, row_pos: torch.Tensor, num_tiles: int, sink32: torch.Tensor | None,
+                      scale: float, window: int | None, value_dim: int) -> torch.Tensor:
+    """``latent_attention_tc`` on the 5th-generation tensor cores, for long rows; ``num_tiles``: ``latent_prefill_tiles``
+    of the rows' lengths."""
+    _check(q, "q", torch.bfloat16, 3)
+    _check(pages, "pages", torch.bfloat16, 4)
+    T, H, d = q.shape
+    if pages.shape[1] != 1 or pages.shape[3] != d:
+        raise KernelError(f"latent_prefill_tc: pages {tuple(pages.shape)} do not fit one row of {d} per token")
+    _check_sink(sink32, H)
+    out = torch.empty((T, H, value_dim), dtype=torch.bfloat16, device=q.device)
+    _ok(lib().acorn_latent_prefill_tc(q.data_ptr(), T, out.data_ptr(), pages.data_ptr(), pages.shape[0], block_table.data_ptr(),
+                                      page_base.data_ptr(), block_table.stride(0), row_start.data_ptr(), row_pos.data_ptr(),
+                                      row_pos.shape[0], int(num_tiles), _ptr(sink32), float(scale), int(window or 0), H, d,
+                                      int(value_dim), pages.shape[2], _stream()), "latent_prefill_tc")
+    return out
+
+
+def latent_prefill_tc_error() -> int:
+    """0, or where a bounded wait inside the tcgen05 kernel of latent attention gave up since the last call."""
+    return int(lib().acorn_latent_prefill_tc_error())
 
 
 def head_linear(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor) -> torch.Tensor:

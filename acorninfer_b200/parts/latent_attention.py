@@ -100,6 +100,18 @@ class LatentAttention(Mixer):
 
         return {f"latent.tiles{n}": tiles}
 
+    def _prefill_tiles(self, inputs, block_table, page_size, general_tiles):
+        """Tiles of the tcgen05 kernel, or 0 where it does not take the step or the general kernel is the faster one."""
+        if self.H > ops.LATENT_TILE_ROWS or not ops.latent_prefill_tc_supported(self.ctx.dtype, self.H, self.rank + self.rot, self.rank,
+                                                                                 page_size, self.scale):
+            return 0
+        n = ops.latent_prefill_tiles(inputs.plan.row_lens, self.H)
+        # by the table's width, not the lengths of this step: a captured step is replayed with others
+        bound = block_table.shape[1] * page_size
+        if self.window:
+            bound = min(bound, self.window + ops.LATENT_PREFILL_ROWS // self.H)
+        return n if ops.latent_prefill_wins(n, general_tiles, bound) else 0
+
     def forward(self, x, inputs, cache):
         if cache.write != self.own_cache:
             raise ValueError("latent attention: the schedule and the layer disagree on who writes the cache")
@@ -120,10 +132,15 @@ class LatentAttention(Mixer):
                         pos.rotary_dim if pos is not None else 0, self.eps, kv_rows=kv_rows)
         qu = proj[:, :H * (self.dim + self.rot)].view(T, H, self.dim + self.rot)[:, :, :self.dim]
         ops.head_linear(qu, self.w_uk_t, qcat[:, :, :self.rank])
-        if ops.latent_attention_tc_supported(dt, H, self.rank + self.rot, self.rank, cache.k_pages.shape[2]):
+        P = cache.k_pages.shape[2]
+        general = inputs.extra[f"latent.tiles{self._tile_tokens()}"]
+        tiles = self._prefill_tiles(inputs, g.block_table, P, general.shape[0])
+        if tiles:
+            o = ops.latent_prefill_tc(qcat, cache.k_pages, g.block_table, g.page_base, inputs.row_start, inputs.row_pos,
+                                      tiles, self.sink32, self.scale, self.window, self.rank)
+        elif ops.latent_attention_tc_supported(dt, H, self.rank + self.rot, self.rank, P):
             o = ops.latent_attention_tc(qcat, cache.k_pages, g.block_table, g.page_base, inputs.row_start, inputs.row_pos,
-                                        inputs.extra[f"latent.tiles{self._tile_tokens()}"], self.sink32, self.scale,
-                                        self.window, self.rank)
+                                        general, self.sink32, self.scale, self.window, self.rank)
         else:       # float32, or sizes the tensor-core kernel does not take
             o = ops.attention_plain(qcat, qcat.stride(0), cache.k_pages, cache.k_pages, g.block_table, g.page_base,
                                     inputs.token_row, inputs.positions, T, H, 1, self.rank + self.rot, self.scale,

@@ -432,6 +432,50 @@ def test_latent_layout_attention_window_edges_far_keys_and_sink(dtype, tol, kern
     assert (got - want).abs().max() < tol and got.abs().max() < 0.05
 
 
+@pytest.mark.parametrize("H,d,dv,P,window,sink", [(16, 448, 384, 16, 200, True), (8, 320, 192, 8, None, False), (5, 192, 128, 128, 70, True),
+                                                  (64, 64, 64, 32, None, True), (1, 128, 64, 16, 64, False)])
+def test_latent_attention_of_long_rows(H, d, dv, P, window, sink):
+    """The tcgen05 kernel against float64: rows that end anywhere in a tile and in a block of 64 keys, single tokens,
+    portions after cached keys, pages a window has given back, and pages that hold no numbers behind the last key."""
+    o = ops()
+    befores, qlens = [0, 130, 63, 300, 127], [333, 64, 1, 65, 193]
+    NP = sum(-(-(b + q) // P) for b, q in zip(befores, qlens)) + 3
+    lay = rows_layout(befores, qlens, P, NP, seed=H)
+    g = torch.Generator().manual_seed(d)
+    pages = torch.full((NP, 1, P, d), float("nan"), dtype=torch.bfloat16, device=DEV)
+    sinks = torch.randn(H, generator=g) if sink else None
+    scale, q_new, want = d ** -0.5, [], []
+    table, base = lay["block_table"].clone(), lay["page_base"].clone()
+    for r, (b, n) in enumerate(zip(befores, qlens)):
+        k = (torch.randn(b + n, d, generator=g) * 1.5).bfloat16()
+        q = (torch.randn(n, H, d, generator=g) * 1.5).bfloat16()
+        gone = max(0, b - window + 1) // P if window else 0              # pages no query sees any more
+        scatter_to_pages(pages, lay["tables"][r], k[:, None], P)
+        for page in lay["tables"][r][:gone]:
+            pages[page] = float("nan")
+        table[r] = torch.roll(lay["block_table"][r], -gone)
+        base[r] = gone
+        q_new.append(q)
+        i, j = torch.arange(b, b + n)[:, None], torch.arange(b + n)[None]
+        seen = (j <= i) & (i - j < window) if window else j <= i
+        s = torch.einsum("qhd,kd->hqk", q.double(), k.double()) * scale
+        s = s.masked_fill(~seen, float("-inf"))
+        if sink:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(H, n, 1)], 2)
+        w = torch.softmax(s, 2)[:, :, :b + n]
+        want.append(torch.einsum("hqk,kd->qhd", w, k[:, :dv].double()))
+    q_new, want = torch.cat(q_new).to(DEV), torch.cat(want)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    assert o.latent_prefill_tc_supported(torch.bfloat16, H, d, dv, P, scale)
+    got = o.latent_prefill_tc(q_new, pages, table, base, torch.tensor(np.cumsum([0] + qlens), **i32), torch.tensor(befores, **i32),
+                              o.latent_prefill_tiles(qlens, H), sinks.to(DEV) if sink else None, scale, window, dv).double().cpu()
+    o.raise_on_kernel_error()
+    # the weights and the result are rounded to 8 bits of mantissa (half a unit: 2^-9 each), a weighted mean of values up to
+    # `top`; float32 scores of a few units add less than 2^-13
+    top = 1.5 * 6
+    assert (got - want).abs().max() < top * (2 ** -9 + 2 ** -9 + 2 ** -13)
+
+
 def test_bigram_rows_carry_the_previous_token_between_steps():
     o = ops()
     buckets, mp, mc, H = 11, 7, 3, 8
