@@ -585,38 +585,54 @@ __global__ void gated_norm_kernel(const float* __restrict__ y, const T* __restri
     }
 }
 
-// The same for parts that are multiples of four up to 256: a warp a part, up to two vectors of four a lane.
-template <typename T>
-__global__ void gated_norm_vec_kernel(const float* __restrict__ y, const T* __restrict__ gate, int64_t ldg,
-                                      const float* __restrict__ weight, T* __restrict__ out, int64_t ldo, int W, int groups,
-                                      float eps, int mode, float out_scale, int64_t items) {
+// The same for parts that are multiples of four up to 4,096: WARPS warps a part, N vectors of four a lane, all on their way
+// before the first is used.  Bound by memory.  Measured (B200, 2,000 tokens of 8 parts of 512, gate first): a block a part,
+// 4 and 2 bytes a load, 34 us; this 17 us.
+template <typename T, int N, int WARPS>
+__global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* __restrict__ y, const T* __restrict__ gate, int64_t ldg,
+                                                             const float* __restrict__ weight, T* __restrict__ out, int64_t ldo,
+                                                             int W, int groups, float eps, int mode, float out_scale, int64_t items) {
+    __shared__ float sums[8];
     pdl_wait();
     pdl_trigger();
-    const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (item >= items) return;
-    const int lane = threadIdx.x & 31, part = W / groups;
-    const int64_t t = item / groups;
-    const int i0 = (int)(item - t * groups) * part;
-    float4 u[2], z[2];
-    float ss = 0.f;
+    const int warp = threadIdx.x >> 5;
+    const int64_t item = (int64_t)blockIdx.x * (8 / WARPS) + warp / WARPS;
+    const bool live = item < items;
+    const int lane = (threadIdx.x & 31) + 32 * (warp % WARPS), part = W / groups;
+    const int64_t t = live ? item / groups : 0;
+    const int i0 = live ? (int)(item - t * groups) * part : 0;
+    float4 u[N], z[N];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int i = 4 * (lane + 32 * k);
+    for (int k = 0; k < N; ++k) {
+        const int i = 4 * (lane + 32 * WARPS * k);
         u[k] = z[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < part) {
+        if (live && i < part) {
             u[k] = *reinterpret_cast<const float4*>(y + t * W + i0 + i);
             z[k] = Vec4<T>::load(gate + t * ldg + i0 + i);
-            if (mode == 0) {
-                u[k].x *= lr_gate(z[k].x, 2); u[k].y *= lr_gate(z[k].y, 2);
-                u[k].z *= lr_gate(z[k].z, 2); u[k].w *= lr_gate(z[k].w, 2);
-            }
-            ss += u[k].x * u[k].x + u[k].y * u[k].y + u[k].z * u[k].z + u[k].w * u[k].w;
         }
     }
-    const float inv = rsqrtf(warp_sum(ss) / (float)part + eps);
+    float ss = 0.f;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int i = 4 * (lane + 32 * k);
+    for (int k = 0; k < N; ++k) {
+        if (mode == 0) {
+            u[k].x *= lr_gate(z[k].x, 2); u[k].y *= lr_gate(z[k].y, 2);
+            u[k].z *= lr_gate(z[k].z, 2); u[k].w *= lr_gate(z[k].w, 2);
+        }
+        ss += u[k].x * u[k].x + u[k].y * u[k].y + u[k].z * u[k].z + u[k].w * u[k].w;
+    }
+    ss = warp_sum(ss);
+    if (WARPS > 1) {
+        if ((threadIdx.x & 31) == 0) sums[warp] = ss;
+        __syncthreads();
+        ss = 0.f;
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) ss += sums[warp / WARPS * WARPS + q];
+    }
+    if (!live) return;
+    const float inv = rsqrtf(ss / (float)part + eps);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int i = 4 * (lane + 32 * WARPS * k);
         if (i >= part) break;
         const float4 w = *reinterpret_cast<const float4*>(weight + i0 + i);
         float4 o = make_float4(u[k].x * inv * w.x, u[k].y * inv * w.y, u[k].z * inv * w.z, u[k].w * inv * w.w);
@@ -634,15 +650,23 @@ extern "C" int acorn_gated_norm(const float* y, const void* gate, int64_t ldg, c
     if (tokens <= 0) return 0;
     if (groups < 1 || W % groups || groups > 65535 || mode < 0 || mode > 2) return ACORN_ERR_UNSUPPORTED;
     const int part = W / groups;
-    if (part % 4 == 0 && part <= 256 && ldg % 4 == 0 && ldo % 4 == 0 &&
+    if (part % 4 == 0 && part <= 4096 && ldg % 4 == 0 && ldo % 4 == 0 &&
         (((uintptr_t)y | (uintptr_t)weight) & 15) == 0 &&
         (((uintptr_t)gate | (uintptr_t)out) & (dtype == ACORN_DTYPE_BF16 ? 7 : 15)) == 0) {
         const int64_t items = (int64_t)tokens * groups;
-        const int64_t blocks = (items + 7) / 8;
+        const int warps = part <= 512 ? 1 : part <= 1024 ? 2 : part <= 2048 ? 4 : 8;
+        const int64_t blocks = (items + 8 / warps - 1) / (8 / warps);
         if (blocks > 0x7fffffff) return ACORN_ERR_UNSUPPORTED;
-        ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(gated_norm_vec_kernel<T>, dim3((unsigned)blocks), dim3(256), 0, stream, y,
-                                                           (const T*)gate, ldg, weight, (T*)out, ldo, W, groups, eps, mode,
-                                                           out_scale, items));
+#define GN_LAUNCH(N, WARPS)                                                                                                     \
+    ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(gated_norm_vec_kernel<T, N, WARPS>, dim3((unsigned)blocks), dim3(256), 0, \
+                                                       stream, y, (const T*)gate, ldg, weight, (T*)out, ldo, W, groups, eps,    \
+                                                       mode, out_scale, items))
+        if (part <= 256) GN_LAUNCH(2, 1);
+        if (warps == 1) GN_LAUNCH(4, 1);
+        if (warps == 2) GN_LAUNCH(4, 2);
+        if (warps == 4) GN_LAUNCH(4, 4);
+        GN_LAUNCH(4, 8);
+#undef GN_LAUNCH
     }
     const int threads = part >= 1024 ? 256 : 128;
     ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(gated_norm_kernel<T>, dim3(tokens, groups), dim3(threads), 0, stream,

@@ -483,6 +483,27 @@ def test_linear_scan_with_one_decay_per_head_and_no_step_sizes():
     assert (y - want).abs().max() < 1e-4 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("part,groups", [(260, 3), (512, 2), (516, 1), (1024, 3), (1028, 2), (2048, 1), (2052, 1), (4096, 1), (4100, 1), (514, 2)])
+def test_gated_norm_of_wide_parts(part, groups, dtype):
+    """One to eight warps a part and the general kernel behind them, ragged last blocks of parts, all gates."""
+    o = ops()
+    T, W = 5, part * groups
+    g = torch.Generator().manual_seed(part)
+    y, z = torch.randn(T, W, generator=g), torch.randn(T, W + 4, generator=g).to(dtype)
+    w = torch.rand(W, generator=g) + 0.5
+    zz = z[:, 4:].double()
+    for gate_first, silu in ((True, False), (False, False), (False, True)):
+        out = torch.zeros(T, W + 8, dtype=dtype, device=DEV)
+        o.gated_norm(y.to(DEV), z.to(DEV)[:, 4:], w.to(DEV), 1e-5, groups, gate_first, out[:, 8:], 0.75, silu=silu)
+        u = y.double() * plain.silu(zz) if gate_first else y.double()
+        u = plain.rms_norm(u.view(T, groups, part), 1e-5).reshape(T, W) * w.double()
+        want = 0.75 * (u if gate_first else u * (plain.silu(zz) if silu else torch.sigmoid(zz)))
+        # a dozen float32 operations on a value (the root's argument is a sum of positive terms), then one rounding to dtype
+        bound = want.abs() * ((2.0 ** -8 if dtype == torch.bfloat16 else 0.0) + 24 * 2.0 ** -23) + 1e-6
+        assert ((out[:, 8:].double().cpu() - want).abs() <= bound).all() and float(out[:, :8].abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
 def test_gated_norm_layernorm_glu_and_head_gate(dtype, tol):
     o = ops()
