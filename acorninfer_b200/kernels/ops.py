@@ -1727,13 +1727,18 @@ def mix_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bonus32: torch.
     _check(state, "state", torch.float32, 2)
     if log2_g.shape != (T, H, dim) or bonus32.shape != (H, dim) or state.shape[1] < state_off + H * dim * vdim:
         raise KernelError(f"mix_chunk: log2_g {tuple(log2_g.shape)}, bonus {tuple(bonus32.shape)}, state {tuple(state.shape)} do not fit")
-    f = lambda *shape: torch.empty(shape, dtype=torch.float32, device=v.device)
     ids = lib().acorn_delta_chunk_ids(T, num_rows)
-    p, qs, out = f(T, H, 64), f(T, H, dim), f(T, H, vdim)
-    s0, decay = f(ids, H, dim, vdim), f(ids, H, dim)
+    out = torch.empty((T, H, vdim), dtype=torch.float32, device=v.device)
+    # the kernels' own arrays, one behind the other: p [T, H, 64], q at the chunk's start [T, H, dim], the chunks' decays and states
+    sizes = (T * H * 64, T * H * dim, ids * H * dim, ids * H * dim * vdim)
+    scratch = torch.empty(sum(sizes), dtype=torch.float32, device=v.device)
+    p = scratch.data_ptr()
+    qs = p + 4 * sizes[0]
+    decay = qs + 4 * sizes[1]
+    s0 = decay + 4 * sizes[2]
     _ok(lib().acorn_mix_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), bonus32.data_ptr(), log2_g.data_ptr(),
                               state.data_ptr() + 4 * int(state_off), state.stride(0), row_start.data_ptr(), row_slot.data_ptr(),
-                              p.data_ptr(), qs.data_ptr(), decay.data_ptr(), s0.data_ptr(), out.data_ptr(), T, num_rows, H, KH, dim,
+                              p, qs, decay, s0, out.data_ptr(), T, num_rows, H, KH, dim,
                               vdim, _stream()), "delta_rule")
     return out
 
