@@ -596,11 +596,78 @@ __global__ void add_layernorm_kernel(float* __restrict__ resid32, const T* __res
         o[i] = from_float<T>((rowv[i] - mean) * inv * w[i] + (b ? b[i] : 0.f));
 }
 
+// The same for rows that are a multiple of four up to 4,096: vectors of four, the row in registers from its one read on.
+// Bound by memory and two sums over the block.  Measured (B200, 2,048 rows of 2,048 with two results to add): 15 us with the
+// row in shared memory an element at a time, 7.4 us so.
+template <typename T, int N>
+__global__ void __launch_bounds__(256) add_layernorm_vec_kernel(float* __restrict__ resid32, const T* __restrict__ delta,
+                                                                const T* __restrict__ delta2, const float* __restrict__ w,
+                                                                const float* __restrict__ b, T* __restrict__ out,
+                                                                const int* __restrict__ row_idx, int H, float eps) {
+    __shared__ float scratch[32];
+    pdl_wait();
+    pdl_trigger();
+    const int r = blockIdx.x;
+    const int64_t row = row_idx ? row_idx[r] : r;
+    const bool write_resid = (row_idx == nullptr) && (delta != nullptr || delta2 != nullptr);
+    float* x = resid32 + row * H;
+    float4 v[N], d1[N], d2[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int i = 4 * (threadIdx.x + 256 * k);
+        v[k] = d1[k] = d2[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < H) {
+            v[k] = *reinterpret_cast<const float4*>(x + i);
+            if (delta) d1[k] = Vec4<T>::load(delta + row * H + i);
+            if (delta2) d2[k] = Vec4<T>::load(delta2 + row * H + i);
+        }
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int i = 4 * (threadIdx.x + 256 * k);
+        v[k].x = v[k].x + d1[k].x + d2[k].x; v[k].y = v[k].y + d1[k].y + d2[k].y;
+        v[k].z = v[k].z + d1[k].z + d2[k].z; v[k].w = v[k].w + d1[k].w + d2[k].w;
+        if (write_resid && i < H) *reinterpret_cast<float4*>(x + i) = v[k];
+        s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+    }
+    const float mean = block_sum(s, scratch) / (float)H;
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        if (4 * (threadIdx.x + 256 * k) >= H) break;
+        v[k].x -= mean; v[k].y -= mean; v[k].z -= mean; v[k].w -= mean;
+        ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+    }
+    const float inv = rsqrtf(block_sum(ss, scratch) / (float)H + eps);
+    T* o = out + (int64_t)r * H;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int i = 4 * (threadIdx.x + 256 * k);
+        if (i >= H) break;
+        const float4 ww = *reinterpret_cast<const float4*>(w + i);
+        const float4 bb = b ? *reinterpret_cast<const float4*>(b + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        Vec4<T>::store(o + i, make_float4(v[k].x * inv * ww.x + bb.x, v[k].y * inv * ww.y + bb.y, v[k].z * inv * ww.z + bb.z,
+                                          v[k].w * inv * ww.w + bb.w));
+    }
+}
+
 extern "C" int acorn_add_layernorm(float* resid32, const void* delta, const void* delta2, const float* w,
                                    const float* b, void* out, const int* row_idx, int rows, int H, float eps,
                                    int dtype, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if ((size_t)H * sizeof(float) > 48 * 1024) return ACORN_ERR_UNSUPPORTED;
+    const uintptr_t narrow = (uintptr_t)delta | (uintptr_t)delta2 | (uintptr_t)out;
+    if (H % 4 == 0 && H >= 512 && H <= 4096 && (((uintptr_t)resid32 | (uintptr_t)w | (uintptr_t)b) & 15) == 0 &&
+        (narrow & (dtype == ACORN_DTYPE_BF16 ? 7 : 15)) == 0) {
+#define LN_LAUNCH(N)                                                                                                              \
+    ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(add_layernorm_vec_kernel<T, N>, dim3(rows), dim3(256), 0, stream, resid32, \
+                                                       (const T*)delta, (const T*)delta2, w, b, (T*)out, row_idx, H, eps))
+        if (H <= 1024) LN_LAUNCH(1);
+        if (H <= 2048) LN_LAUNCH(2);
+        LN_LAUNCH(4);
+#undef LN_LAUNCH
+    }
     const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
     ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(add_layernorm_kernel<T>, dim3(rows), dim3(threads),
                                                        (size_t)H * sizeof(float), stream, resid32, (const T*)delta,

@@ -504,6 +504,46 @@ def test_gated_norm_of_wide_parts(part, groups, dtype):
         assert ((out[:, 8:].double().cpu() - want).abs() <= bound).all() and float(out[:, :8].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,W,skip", [(1, 4, 0), (5, 1028, 4), (4, 6144, 8), (7, 1022, 4), (3, 60, 2)])
+def test_silu_of_rows(T, W, skip, dtype):
+    """Four columns a thread and four tokens at once (ragged last ones of both), and rows that are not aligned for it."""
+    z = torch.randn(T, W + skip, generator=torch.Generator().manual_seed(W)).to(dtype)
+    want = plain.silu(z[:, skip:].double())
+    got = ops().silu_rows(z.to(DEV)[:, skip:]).double().cpu()
+    # an exponential, a sum, a quotient and a product in float32
+    assert ((got - want).abs() <= want.abs() * 16 * 2.0 ** -23 + 1e-30).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H", [512, 516, 1024, 1028, 2048, 2052, 4096, 4100, 1026])
+def test_layernorm_with_the_row_in_registers(H, dtype):
+    """One to four vectors a thread and the general kernel on either side, with no, one and two results to add, with chosen
+    rows and without a bias."""
+    o = ops()
+    g = torch.Generator().manual_seed(H)
+    T = 3
+    x = torch.randn(T, H, generator=g) * 3 + 1
+    a, b = torch.randn(T, H, generator=g).to(dtype), torch.randn(T, H, generator=g).to(dtype)
+    w, bias = torch.rand(H, generator=g) + 0.5, torch.randn(H, generator=g)
+    s = x.double()
+    for delta, add, bb in ((None, 0, bias), (a, a.double(), bias), ((a, b), a.double() + b.double(), None)):
+        resid = x.clone().to(DEV)
+        d = None if delta is None else (o.DeltaPair(a.to(DEV), b.to(DEV)) if isinstance(delta, tuple) else delta.to(DEV))
+        out = o.add_layernorm(resid, d, w.to(DEV), None if bb is None else bb.to(DEV), 1e-5, dtype).double().cpu()
+        sums = s + add
+        # two float32 sums of values up to 20, then one rounding to dtype of values up to 10; the mean's and the root's errors are
+        # below 2^-20 of them
+        assert (resid.cpu().double() - sums).abs().max() < 20 * 2.0 ** -22
+        want = plain.layer_norm(sums, w.double(), torch.zeros(H, dtype=torch.float64) if bb is None else bias.double(), 1e-5)
+        bound = want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) + 10 * 2.0 ** -19
+        assert ((out - want).abs() <= bound).all()
+    rows = torch.tensor([2, 0, 2], dtype=torch.int32, device=DEV)
+    part = o.add_layernorm(x.clone().to(DEV), None, w.to(DEV), bias.to(DEV), 1e-5, dtype, row_idx=rows).double().cpu()
+    want = plain.layer_norm(s[[2, 0, 2]], w.double(), bias.double(), 1e-5)
+    assert ((part - want).abs() <= want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) + 10 * 2.0 ** -19).all()
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
 def test_gated_norm_layernorm_glu_and_head_gate(dtype, tol):
     o = ops()
