@@ -193,7 +193,8 @@ __device__ __forceinline__ float4 at4(const float* q) { return *reinterpret_cast
 __device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float4 sub4(const float4& a, const float4& b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
 __device__ __forceinline__ float4 mul4(const float4& a, const float4& b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
-// 2^x for x <= 0 by the instruction that exp2f is made of, without its care for results below 2^-126 (they are 0 here)
+// 2^x for x <= 0 by the PTX instruction ex2.approx.ftz.f32: an approximation (relative error up to 2^-22), results below 2^-126
+// are 0
 __device__ __forceinline__ float exp2_neg(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
