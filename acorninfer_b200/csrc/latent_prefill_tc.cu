@@ -33,7 +33,7 @@
 #define LT_K_PIECE (LT_KB * 128)
 #define LT_GROUPS 4                      // groups of 128 columns a block's keys come in, at most
 #define LT_MAX_PIECES 7                  // queries and two blocks of keys within 227 KB
-#define LT_BARS (1 + 2 * 2 * LT_GROUPS + 2 + 2 + 1)
+#define LT_BARS (1 + 2 * 2 * LT_GROUPS + 2 + 2 + 2)
 
 __device__ int g_latent_tc_error = 0;
 
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
     uint64_t* bars = reinterpret_cast<uint64_t*>(sK + 2 * slot_bytes);
     const uint32_t q_full = tc_smem(bars);
     const uint32_t full0 = q_full + 8, empty0 = full0 + 8 * 2 * LT_GROUPS;     // [slot][group]
-    const uint32_t s_full0 = empty0 + 8 * 2 * LT_GROUPS, p_full0 = s_full0 + 16, o_done = p_full0 + 16;
+    const uint32_t s_full0 = empty0 + 8 * 2 * LT_GROUPS, p_full0 = s_full0 + 16, o_done = p_full0 + 16, o_last = o_done + 8;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + LT_BARS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
         for (int s = 0; s < 2 * LT_GROUPS; ++s) { mbar_init(full0 + 8 * s, LT_PRODUCERS); mbar_init(empty0 + 8 * s, 1); }
         for (int u = 0; u < 2; ++u) { mbar_init(s_full0 + 8 * u, 1); mbar_init(p_full0 + 8 * u, 4); }
         mbar_init(o_done, 1);
+        mbar_init(o_last, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 5) {
@@ -223,6 +224,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
                 umma_commit_elect(empty0 + 8 * (slot * LT_GROUPS + g));
             }
             umma_commit_elect(o_done);
+            if (j == nb - 1) umma_commit_elect(o_last);
             return true;
         };
         bool good = wait_all(q_full, 0, 2) && scores(0) && (nb < 2 || scores(1));
@@ -265,7 +267,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
                     m_ref = mx;
                 }
                 if (j > 0) {
-                    // O holds the blocks before this one when the last of their products is done
+                    // O holds the blocks before this one when the last of their products is done.  o_done completes a phase a
+                    // block, and a wait by parity tells phase j - 1 from phase j - 2 only if j - 2 is over: the scores of block j
+                    // have come, and they are issued behind the values of block j - 1 (j even) or j - 2 (j odd)
                     if (!mbar_wait(o_done, (j - 1) & 1)) { tc_fail(&g_latent_tc_error, 7, ACORN_KERNEL_LATENT_PREFILL_TC); good = false; }
                     good = __all_sync(0xffffffffu, good);
                     if (!good) break;
@@ -297,7 +301,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
             if (lane == 0) mbar_arrive(p_full0 + 8 * (j & 1));
         }
         if (good) {
-            if (!mbar_wait(o_done, (nb - 1) & 1)) { tc_fail(&g_latent_tc_error, 8, ACORN_KERNEL_LATENT_PREFILL_TC); good = false; }
+            // a barrier of its own, of one phase: of the last two blocks' values neither need be done here (their scores are
+            // issued together), and o_done's parity could not tell its state two phases ago from its last
+            if (!mbar_wait(o_last, 0)) { tc_fail(&g_latent_tc_error, 8, ACORN_KERNEL_LATENT_PREFILL_TC); good = false; }
             good = __all_sync(0xffffffffu, good);
         }
         if (good) {

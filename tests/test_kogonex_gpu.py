@@ -476,6 +476,41 @@ def test_latent_attention_of_long_rows(H, d, dv, P, window, sink):
     assert (got - want).abs().max() < top * (2 ** -9 + 2 ** -9 + 2 ** -13)
 
 
+@pytest.mark.parametrize("H,d,dv", [(32, 192, 128), (64, 448, 384), (128, 64, 64)])
+def test_latent_attention_scores_that_outgrow_late(H, d, dv):
+    """Rows of one tile and of one to seven blocks of 64 keys, the scores of one warp's rows (32 of the tile's 128) raised far
+    beyond all before by a key of the second-to-last or of the last block: its rows rescale while the others run ahead."""
+    o = ops()
+    P, TQ = 16, 128 // H
+    cases = [(nb, nb - 1 - back, warp) for nb in range(1, 8) for back in (0, 1) if back < nb for warp in range(4)]
+    befores = [64 * nb - TQ - 3 * (i % 3) for i, (nb, _, _) in enumerate(cases)]
+    NP = sum(-(-(b + TQ) // P) for b in befores) + 3
+    lay = rows_layout(befores, [TQ] * len(cases), P, NP, seed=H)
+    g = torch.Generator().manual_seed(d)
+    pages = torch.full((NP, 1, P, d), float("nan"), dtype=torch.bfloat16, device=DEV)
+    scale, q_new, want = d ** -0.5, [], []
+    for r, (b, (nb, block, warp)) in enumerate(zip(befores, cases)):
+        k = torch.randn(b + TQ, d, generator=g).bfloat16()
+        q = torch.randn(TQ * H, d, generator=g).bfloat16()
+        k[:, 0], q[:, 0] = 0, 0
+        k[64 * block + 5, 0], q[32 * warp:32 * warp + 32, 0] = 8, 4 * math.sqrt(d)   # 32 in the score's units, 46 to base 2
+        q = q.view(TQ, H, d)
+        scatter_to_pages(pages, lay["tables"][r], k[:, None], P)
+        q_new.append(q)
+        seen = torch.arange(b + TQ)[None] <= torch.arange(b, b + TQ)[:, None]
+        s = (torch.einsum("qhd,kd->hqk", q.double(), k.double()) * scale).masked_fill(~seen, float("-inf"))
+        want.append(torch.einsum("hqk,kd->qhd", torch.softmax(s, 2), k[:, :dv].double()))
+    i32 = dict(dtype=torch.int32, device=DEV)
+    lens = [TQ] * len(cases)
+    for _ in range(20):                 # a hand-over that comes too early need not show every time
+        got = o.latent_prefill_tc(torch.cat(q_new).to(DEV), pages, lay["block_table"], lay["page_base"],
+                                  torch.tensor(np.cumsum([0] + lens), **i32), torch.tensor(befores, **i32),
+                                  o.latent_prefill_tiles(lens, H), None, scale, None, dv).double().cpu()
+        o.raise_on_kernel_error()
+        # weights and results rounded to 8 bits of mantissa as above; values up to 8; float32 scores up to 40, 2^-18 of error
+        assert (got - torch.cat(want)).abs().max() < 8 * (2 ** -9 + 2 ** -9 + 2 ** -13)
+
+
 def test_bigram_rows_carry_the_previous_token_between_steps():
     o = ops()
     buckets, mp, mc, H = 11, 7, 3, 8
