@@ -202,7 +202,9 @@ __device__ __forceinline__ float exp2_neg(float x) {
 }
 __device__ __forceinline__ float4 exp2_4(const float4& a) { return make_float4(exp2_neg(a.x), exp2_neg(a.y), exp2_neg(a.z), exp2_neg(a.w)); }
 
-// Sums of a chunk's logarithms within blocks of 16 tokens, in place, and what they lack of the exact sums.
+// Sums of a chunk's logarithms within blocks of 16 tokens, in place, and what they lack of the exact sums.  A logarithm below
+// -1,000, minus infinity among them, counts as -1,000: its factor is 0 in float32 as well, and the sums stay small (infinite
+// ones have no differences).
 template <int DP> __device__ __forceinline__ void block_sums(float* sB, float* sB2) {
     constexpr int LD = DP + DC_PAD;
     for (int e = threadIdx.x; e < 4 * DP; e += blockDim.x) {
@@ -210,7 +212,8 @@ template <int DP> __device__ __forceinline__ void block_sums(float* sB, float* s
         const int at = (e / DP) * 16 * LD + e % DP;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            const float x = sB[at + i * LD], sum = run + x, back = sum - run;
+            const float given = sB[at + i * LD], x = given < -1000.f ? -1000.f : given;     // no number stays none
+            const float sum = run + x, back = sum - run;
             rest += (run - (sum - back)) + (x - back);
             run = sum;
             sB[at + i * LD] = run;

@@ -582,3 +582,37 @@ def test_delta_rule_with_channel_decays_over_chunks(H, KH, dim, vdim):
             assert err["chunks"] < max(3 * err["walk"], 1e-6) and end["chunks"] < max(3 * end["walk"], 1e-6), (lens, r, err, end)
         untouched = [s for s in range(10) if s not in slots]
         assert torch.equal(ends["chunks"][untouched], state[untouched].double()) and torch.equal(ends["chunks"][:, :4], state[:, :4].double())
+
+
+@pytest.mark.parametrize("dim,vdim,dtype", [(32, 20, torch.float32), (64, 64, torch.bfloat16), (128, 128, torch.float32), (9 * 4, 12, torch.bfloat16)])
+def test_delta_rule_over_chunks_with_decays_that_leave_nothing(dim, vdim, dtype):
+    """Logarithms of minus infinity and of numbers whose sums leave float32, as they are and as the prep kernel makes them of
+    large weights: zeros as decays in the walk over tokens, and the same outputs and states over chunks."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim)
+    H, KH, taps = 4, 2, 3
+    lens = [130, 64, 200]
+    T, C = sum(lens), 2 * KH * dim + H * vdim
+    starts = torch.tensor(np.cumsum([0] + lens), dtype=torch.int32, device=DEV)
+    token_row = torch.repeat_interleave(torch.arange(3), torch.tensor(lens)).int().to(DEV)
+    slots = torch.tensor([2, 0, 3], dtype=torch.int32, device=DEV)
+    state = torch.randn(4, H * dim * vdim, generator=g)
+    main = torch.randn(T, C + H, generator=g).to(dtype).to(DEV)
+    conv, conv_state = torch.randn(C, taps, generator=g).to(DEV), torch.zeros(4, (taps - 1) * C, device=DEV)
+    for a_log, bias in (([90.0, 0.5, 200.0, -3.0], 0.0), ([0.0, 80.0, 1.0, 85.0], 200.0)):
+        up = (torch.randn(T, H * (dim + vdim), generator=g) + 1).to(DEV)
+        a32, b32 = torch.tensor(a_log, device=DEV), torch.full((H * dim,), bias, device=DEV)
+        prep = lambda logs: o.delta_prep(main, up, conv, conv_state, 0, a32, b32, token_row, starts, slots, H, KH, dim, vdim, taps, log2_decays=logs)
+        q, k, v, beta, decays, _ = prep(False)
+        logs = prep(True)[4]
+        assert bool((logs < -1e30).any())
+        logs[40:44, 1, :5], decays[40:44, 1, :5] = float("-inf"), 0.0
+        logs[45:61, 3, 1:3], decays[45:61, 3, 1:3] = -1e38, 0.0
+        ends = {how: state.to(DEV) for how in ("chunks", "walk")}
+        got = o.channel_chunk(q, k, v, beta, logs, ends["chunks"], starts, slots, 3)
+        want = o.delta_rule(q, k, v, beta, decays, ends["walk"], starts, slots, 3)
+        assert bool(torch.isfinite(want).all())
+        # both are float32 sums of the same recurrence: as far apart as either is from 64 bits (1e-6, see the test above) but for
+        # the decays, rounded once as numbers and once as logarithms
+        assert float((got - want).norm() / want.norm()) < 1e-5
+        assert float((ends["chunks"] - ends["walk"]).norm() / ends["walk"].norm()) < 1e-5

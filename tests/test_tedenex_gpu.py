@@ -471,6 +471,32 @@ def test_recurrence_that_reads_the_state_first_over_chunks(H, dim, vdim):
         assert torch.equal(ends["chunks"][:, :4], state[:, :4].double())
 
 
+@pytest.mark.parametrize("dim,dtype", [(12, torch.float32), (64, torch.bfloat16), (128, torch.float32)])
+def test_time_mixing_over_chunks_with_decays_that_leave_nothing(dim, dtype):
+    """Pre-activations of 90 and 200, whose logarithms are minus infinity or have sums that leave float32: a decay of 0 in the
+    walk over tokens, and the same outputs and states over chunks."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim)
+    H, lens = 3, [130, 64, 200]
+    T = sum(lens)
+    starts, slots = torch.tensor(np.cumsum([0] + lens), dtype=torch.int32, device=DEV), torch.tensor([2, 0, 3], dtype=torch.int32, device=DEV)
+    r, k, v, gate = (torch.randn(T, H * dim, generator=g).to(dtype).to(DEV) for _ in range(4))
+    u, w0 = torch.randn(H, dim, generator=g).to(DEV), torch.full((H * dim,), -1.0, device=DEV)
+    z = torch.randn(T, H * dim, generator=g)
+    z[20:24, 1::3], z[100:140, ::5], z[150, :], z[300:, 2] = 200.0, 90.0, 87.0, 86.0
+    state = torch.randn(4, H * dim * dim, generator=g)
+    r32, k32, v32, decays, _ = o.wkv_prep(r, k, v, gate, z.to(DEV), w0, H)
+    logs = o.wkv_prep(r, k, v, gate, z.to(DEV), w0, H, log2_decays=True)[3]
+    assert bool(torch.isinf(logs).any())
+    ends = {how: state.to(DEV) for how in ("chunks", "walk")}
+    got = o.mix_chunk(r32, k32, v32, u, logs, ends["chunks"], starts, slots, 3)
+    want = o.delta_rule(r32, k32, v32, None, decays, ends["walk"], starts, slots, 3, bonus32=u)
+    assert bool(torch.isfinite(want).all())
+    # float32 sums of the same recurrence (1e-6 from 64 bits each, see above), its decays rounded as numbers and as logarithms
+    assert float((got - want).norm() / want.norm()) < 1e-5
+    assert float((ends["chunks"] - ends["walk"]).norm() / ends["walk"].norm()) < 1e-5
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
 @pytest.mark.parametrize("W,off,tail,single", [(20, 7, 3, False), (20, 8, 4, False), (20, 8, 4, True), (520, 4, 0, True),
                                                (22, 8, 2, True)])
