@@ -127,7 +127,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
     const int pos0 = p.row_pos[r] + q0;
     const int hi = pos0 + ntok;                                          // keys < hi are read by the tile
     const int kept = p.row_pos[r] + row_tokens;                          // keys < kept are in the cache
-    const int lo = (p.window > 0 ? max(0, pos0 - p.window + 1) : 0) & ~(LT_KB - 1);
+    const int seen = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;      // keys >= seen are read by the tile
+    const int lo = seen & ~(LT_KB - 1);
     const int nb = (hi - lo + LT_KB - 1) / LT_KB;
 
     if (!live) {
@@ -187,15 +188,19 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
         };
         const uint32_t qlo = umma_lo(tc_smem(sQ)), klo0 = umma_lo(tc_smem(sK)), vlo0 = umma_lo_mn(tc_smem(sK), LT_K_PIECE);
         auto scores = [&](int j) -> bool {                               // S[j & 1] = Q K_j^T
-            const int slot = j & 1, tail = kept - (lo + j * LT_KB);      // rows of the block from `tail` on are in no request's cache
+            // rows of the block that no query of the tile reads: in front of the first one's window (where pages were given back
+            // others stand in for them), and from the last one's key on (where a page may hold no request's tokens)
+            const int slot = j & 1, key0 = lo + j * LT_KB, front = min(LT_KB, seen - key0), tail = min(LT_KB, hi - key0);
             for (int i = 0; i < groups; ++i) {
                 const int g = i == 0 ? groups - 1 : i - 1;
                 const int n = min(2, pieces - 2 * g);
                 if (!wait_all(full0 + 8 * (slot * LT_GROUPS + g), (j >> 1) & 1, 3)) return false;
-                if (tail < LT_KB) {                                      // zeros there: what lies in a page may be no number
-                    for (int c = 0; c < n; ++c)
-                        for (int at = tail * 128 + lane * 16; at < LT_K_PIECE; at += 32 * 16)
-                            *reinterpret_cast<uint4*>(sK + slot * slot_bytes + (2 * g + c) * LT_K_PIECE + at) = make_uint4(0, 0, 0, 0);
+                if (front > 0 || tail < LT_KB) {                         // values of zero there: their weights are, and 0 times no number is none
+                    for (int c = 2 * g; c < min(2 * g + n, vpieces); ++c) {
+                        uint8_t* piece = sK + slot * slot_bytes + c * LT_K_PIECE;
+                        for (int at = lane * 16; at < front * 128; at += 32 * 16) *reinterpret_cast<uint4*>(piece + at) = make_uint4(0, 0, 0, 0);
+                        for (int at = tail * 128 + lane * 16; at < LT_K_PIECE; at += 32 * 16) *reinterpret_cast<uint4*>(piece + at) = make_uint4(0, 0, 0, 0);
+                    }
                     fence_proxy_async();
                     __syncwarp();
                 }

@@ -511,6 +511,36 @@ def test_latent_attention_scores_that_outgrow_late(H, d, dv):
         assert (got - torch.cat(want)).abs().max() < 8 * (2 ** -9 + 2 ** -9 + 2 ** -13)
 
 
+@pytest.mark.parametrize("P,window", [(16, 4), (8, 1), (32, 9), (64, 20), (128, 70)])
+def test_latent_attention_reads_no_rows_but_its_own(P, window):
+    """Windows smaller than a page and than a block of 64 keys: what lies in the pages behind the request's last token, in
+    those given back, and in the request's own rows in front of a window, is NaN and stays out."""
+    o = ops()
+    H, d, dv = 16, 192, 128
+    befores, qlens = [100, 3, 70, 97, 250, 0, 120], [1, 2, 3, 1, 5, 40, 30]
+    NP = sum(-(-(b + q) // P) for b, q in zip(befores, qlens)) + 3
+    lay = rows_layout(befores, qlens, P, NP, seed=P)
+    g = torch.Generator().manual_seed(P)
+    pages = torch.full((NP, 1, P, d), float("nan"), dtype=torch.bfloat16, device=DEV)
+    table, base = lay["block_table"].clone(), lay["page_base"].clone()
+    scale, q_new, want = d ** -0.5, [], []
+    for r, (b, n) in enumerate(zip(befores, qlens)):
+        k, q = torch.randn(b + n, d, generator=g).bfloat16(), torch.randn(n, H, d, generator=g).bfloat16()
+        k[:max(0, b - window + 1)] = float("nan")                        # rows that no query of the step reads
+        scatter_to_pages(pages, lay["tables"][r], k[:, None], P)
+        gone = max(0, b - window + 1) // P
+        table[r], base[r] = torch.roll(lay["block_table"][r], -gone), gone
+        q_new.append(q)
+        for i in range(n):
+            kd = k[max(0, b + i - window + 1):b + i + 1].double()
+            want.append(torch.softmax(q[i].double() @ kd.T * scale, 1) @ kd[:, :dv])
+    i32 = dict(dtype=torch.int32, device=DEV)
+    got = o.latent_prefill_tc(torch.cat(q_new).to(DEV), pages, table, base, torch.tensor(np.cumsum([0] + qlens), **i32),
+                              torch.tensor(befores, **i32), o.latent_prefill_tiles(qlens, H), None, scale, window, dv).double().cpu()
+    o.raise_on_kernel_error()
+    assert (got - torch.stack(want)).abs().max() < 6 * (2 ** -9 + 2 ** -9 + 2 ** -13)       # as for long rows; values up to 6
+
+
 def test_bigram_rows_carry_the_previous_token_between_steps():
     o = ops()
     buckets, mp, mc, H = 11, 7, 3, 8
