@@ -21,6 +21,8 @@
 // block's own chain, its keys' way from L2, scores, softmax, values, is what bounds it, not the rates.
 // Measured (B200, rows of 448 with 384 values, 16 heads), the general kernel and this: 2,000 tokens under a window of 1,024
 // 311 -> 74 us, 3 x 601 tokens 131 -> 44 us, 2,048 tokens behind 6,000 2,920 -> 432 us.
+// A tile in which a value row that only some of its queries read holds an infinity or no number is computed again at the end,
+// a row at a time: in a product, 0 times such a value would reach the queries that do not read it.
 // Every mbarrier wait is bounded; a wait that gives up records g_latent_tc_error and the CTA drains.
 #include "tcgen05_helpers.cuh"
 
@@ -39,6 +41,8 @@ __device__ int g_latent_tc_error = 0;
 
 struct LatentTcParams {
     bf16* out;               // [tokens * H, dv]
+    const bf16* q;           // [tokens * H, d]
+    const bf16* pages;       // [pages, P, d]
     const int* block_table;
     const int* page_base;
     const int* row_start;
@@ -56,6 +60,44 @@ __device__ __forceinline__ float lt_max(const float (&s)[64]) {
         m[2] = fmaxf(m[2], s[c + 2]); m[3] = fmaxf(m[3], s[c + 3]);
     }
     return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+}
+
+// Whether one of eight bfloat16 entries is infinite or no number.
+__device__ __forceinline__ bool lt_not_finite(const uint4& v) {
+    auto full = [](uint32_t w) { return ((w & 0x7f807f80u) + 0x00800080u) & 0x80008000u; };       // an exponent of all ones
+    return (full(v.x) | full(v.y) | full(v.z) | full(v.w)) != 0;
+}
+
+// One (token, head) row by one warp, key by key, float32 throughout.
+__device__ __noinline__ void latent_row_alone(const LatentTcParams& p, const int* table, int64_t row, int head, int qpos) {
+    const int lane = threadIdx.x & 31, P = 1 << p.logP;
+    float q[2 * LT_MAX_PIECES], o[2 * LT_MAX_PIECES], m = -INFINITY, l = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2 * LT_MAX_PIECES; ++i) {
+        const int e = lane + 32 * i;
+        q[i] = e < p.d ? to_float(p.q[row * p.d + e]) : 0.f;
+        o[i] = 0.f;
+    }
+    for (int key = p.window > 0 ? max(0, qpos - p.window + 1) : 0; key <= qpos; ++key) {
+        const bf16* k = p.pages + (((int64_t)table[key >> p.logP] << p.logP) + (key & (P - 1))) * p.d;
+        float kv[2 * LT_MAX_PIECES], s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 2 * LT_MAX_PIECES; ++i) {
+            const int e = lane + 32 * i;
+            kv[i] = e < p.d ? to_float(k[e]) : 0.f;
+            s = fmaf(q[i], kv[i], s);
+        }
+        s = warp_sum(s) * p.scale_log2;
+        const float top = fmaxf(m, s), corr = m == -INFINITY ? 0.f : exp2f(m - top), w = s == -INFINITY ? 0.f : exp2f(s - top);
+        m = top;
+        l = l * corr + w;
+#pragma unroll
+        for (int i = 0; i < 2 * LT_MAX_PIECES; ++i) o[i] = o[i] * corr + w * kv[i];
+    }
+    if (p.sink) l += exp2f(p.sink[head] * 1.4426950408889634f - m);
+#pragma unroll
+    for (int i = 0; i < 2 * LT_MAX_PIECES; ++i)
+        if (lane + 32 * i < p.dv) p.out[row * p.dv + lane + 32 * i] = from_float<bf16>(o[i] / l);
 }
 
 __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -84,6 +126,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
         for (int u = 0; u < 2; ++u) { mbar_init(s_full0 + 8 * u, 1); mbar_init(p_full0 + 8 * u, 4); }
         mbar_init(o_done, 1);
         mbar_init(o_last, 1);
+        tmem_slot[1] = 0;                   // whether the rows are computed one by one at the end
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 5) {
@@ -187,10 +230,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
             return __all_sync(0xffffffffu, ok);
         };
         const uint32_t qlo = umma_lo(tc_smem(sQ)), klo0 = umma_lo(tc_smem(sK)), vlo0 = umma_lo_mn(tc_smem(sK), LT_K_PIECE);
+        bool odd = false;
         auto scores = [&](int j) -> bool {                               // S[j & 1] = Q K_j^T
             // rows of the block that no query of the tile reads: in front of the first one's window (where pages were given back
             // others stand in for them), and from the last one's key on (where a page may hold no request's tokens)
             const int slot = j & 1, key0 = lo + j * LT_KB, front = min(LT_KB, seen - key0), tail = min(LT_KB, hi - key0);
+            const int part_front = p.window > 0 ? min(tail, hi - p.window - key0) : 0, part_tail = max(max(part_front, 0), pos0 + 1 - key0);
             for (int i = 0; i < groups; ++i) {
                 const int g = i == 0 ? groups - 1 : i - 1;
                 const int n = min(2, pieces - 2 * g);
@@ -203,6 +248,14 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
                     }
                     fence_proxy_async();
                     __syncwarp();
+                }
+                // rows that some queries of the tile read and some do not: a value that is no number would reach all of them
+                for (int c = 2 * g; c < min(2 * g + n, vpieces); ++c) {
+                    const uint8_t* piece = sK + slot * slot_bytes + c * LT_K_PIECE;
+                    for (int at = max(0, front) * 128 + lane * 16; at < part_front * 128; at += 32 * 16)
+                        odd |= lt_not_finite(*reinterpret_cast<const uint4*>(piece + at));
+                    for (int at = part_tail * 128 + lane * 16; at < tail * 128; at += 32 * 16)
+                        odd |= lt_not_finite(*reinterpret_cast<const uint4*>(piece + at));
                 }
                 for (int c = 2 * g; c < 2 * g + n; ++c)
 #pragma unroll
@@ -235,6 +288,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
         bool good = wait_all(q_full, 0, 2) && scores(0) && (nb < 2 || scores(1));
         for (int j = 0; j < nb && good; j += 2)
             good = values(j) && (j + 1 >= nb || values(j + 1)) && (j + 2 >= nb || scores(j + 2)) && (j + 3 >= nb || scores(j + 3));
+        if (good && __any_sync(0xffffffffu, odd) && lane == 0) tmem_slot[1] = 1;
     } else {
         // ---------------------------------------------------------------- softmax and output
         const int row = warp * 32 + lane;                                // TMEM lane
@@ -336,6 +390,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
     }
     tc_fence_before();
     __syncthreads();
+    if (live && tmem_slot[1] != 0)          // (after the barrier: in the place of what the products gave)
+        for (int row = warp; row < rows_valid; row += LT_THREADS / 32)
+            latent_row_alone(p, p.block_table + (int64_t)r * p.table_stride - p.page_base[r], qrow0 + row, row % p.H, pos0 + row / p.H);
     if (warp == 5)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_s), "r"(512u) : "memory");
 }
@@ -359,7 +416,7 @@ extern "C" int acorn_latent_prefill_tc(const void* q, int tokens, void* out, con
         ((uintptr_t)out & 15) || (int64_t)tokens * H > 0x7fffffff || num_pages * P > 0x7fffffff)
         return ACORN_ERR_UNSUPPORTED;
     LatentTcParams p;
-    p.out = (bf16*)out; p.block_table = block_table; p.page_base = page_base;
+    p.out = (bf16*)out; p.q = (const bf16*)q; p.pages = (const bf16*)pages; p.block_table = block_table; p.page_base = page_base;
     p.row_start = row_start; p.row_pos = row_pos; p.num_rows = num_rows; p.sink = sink; p.table_stride = table_stride;
     p.H = H; p.d = d; p.dv = dv; p.logP = acorn_log2_exact_tc(P); p.window = window; p.scale_log2 = scale * 1.4426950408889634f;
     CUtensorMap mq, mk;

@@ -541,6 +541,36 @@ def test_latent_attention_reads_no_rows_but_its_own(P, window):
     assert (got - torch.stack(want)).abs().max() < 6 * (2 ** -9 + 2 ** -9 + 2 ** -13)       # as for long rows; values up to 6
 
 
+@pytest.mark.parametrize("H,d,dv,P,window", [(16, 192, 128, 16, None), (16, 448, 384, 16, 70), (1, 128, 64, 8, 100), (5, 192, 128, 64, 3), (128, 64, 64, 16, None)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_latent_attention_keeps_what_is_no_number_to_the_queries_that_read_it(H, d, dv, P, window, value):
+    """An infinite value or one that is no number, at tokens anywhere in a tile and a block of 64 keys: queries that read the
+    token are what float64 makes of it, the others untouched."""
+    o = ops()
+    befores, qlens, bad = [0, 130, 61, 10, 200], [150, 64, 9, 1, 70], [[37, 101], [131], [62, 66], [10], [150, 203]]
+    NP = sum(-(-(b + q) // P) for b, q in zip(befores, qlens)) + 3
+    lay = rows_layout(befores, qlens, P, NP, seed=P)
+    g = torch.Generator().manual_seed(P)
+    pages = torch.full((NP, 1, P, d), float("nan"), dtype=torch.bfloat16, device=DEV)
+    scale, q_new, want = d ** -0.5, [], []
+    for r, (b, n) in enumerate(zip(befores, qlens)):
+        k, q = torch.randn(b + n, d, generator=g).bfloat16(), torch.randn(n, H, d, generator=g).bfloat16()
+        k[bad[r], 7 % dv] = value
+        scatter_to_pages(pages, lay["tables"][r], k[:, None], P)
+        q_new.append(q)
+        for i in range(n):
+            kd = k[max(0, b + i - window + 1) if window else 0:b + i + 1].double()
+            want.append(torch.softmax(q[i].double() @ kd.T * scale, 1) @ kd[:, :dv])
+    i32, want = dict(dtype=torch.int32, device=DEV), torch.stack(want)
+    got = o.latent_prefill_tc(torch.cat(q_new).to(DEV), pages, lay["block_table"], lay["page_base"],
+                              torch.tensor(np.cumsum([0] + qlens), **i32), torch.tensor(befores, **i32),
+                              o.latent_prefill_tiles(qlens, H), None, scale, window, dv).double().cpu()
+    o.raise_on_kernel_error()
+    assert torch.equal(torch.isfinite(got), torch.isfinite(want)) and bool(torch.isfinite(want).any()) and not bool(torch.isfinite(want).all())
+    fine = torch.isfinite(want)
+    assert (got - want)[fine].abs().max() < 6 * (2 ** -9 + 2 ** -9 + 2 ** -13)              # as for long rows; values up to 6
+
+
 def test_bigram_rows_carry_the_previous_token_between_steps():
     o = ops()
     buckets, mp, mc, H = 11, 7, 3, 8
