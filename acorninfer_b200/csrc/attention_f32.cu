@@ -8,13 +8,16 @@
 //   decode    rows of one token: a block takes 128 keys of one kv head for all of its query heads, a second kernel
 //             puts a row's blocks together.
 //
-// Key blocks and the runs of 512 (128) keys that a block takes start at multiples of their size, and a key that a query does not read adds exact zeros, so a
-// query's bits do not depend on the other queries of its tile, on the step's other rows or on padding.
+// Key blocks and the runs of 512 (128) keys that a block takes start at multiples of their size, and a key that a query does
+// not read adds exact zeros (nothing at all where its values are not finite), so a query's bits do not depend on the other
+// queries of its tile, on the step's other rows or on padding.
 //
 // What bounded the plain kernel: a block a token read every key row again from L2 and made one chain of adds per thread.
 // Measured (B200): 777 tokens, 16 heads of 128: 1,596 -> 153 us a layer; 6 rows of 1,500 keys, 8 kv heads:
 // 128 -> 27 us a layer (74 MB).
 #include "mma_helpers.cuh"
+
+#include <cfloat>
 
 typedef unsigned long long f32x2_t;
 
@@ -172,28 +175,59 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
             for (int j = 0; j < 2 * DC; ++j) mul_pair(acc[i][j], c2);
         }
         cp_async_wait<0>();                         // the values
-        __syncthreads();                            // and the probabilities; the keys' room is free
+        // a block that some queries see in part: in a sum over all of it 0 times a value that is no number would reach them
+        bool odd = false;
+        if (kb + FP_K - 1 > p0 || (window > 0 && kb < p0 + n - window)) {
+#pragma unroll
+            for (int e = 0; e < FP_K * CHUNKS / FP_THREADS; ++e) {
+                const int c = e * FP_THREADS + threadIdx.x;             // what this thread has brought
+                const float4 v = *reinterpret_cast<const float4*>(Vs + c * 4);
+                odd |= !(fabsf(v.x) <= FLT_MAX && fabsf(v.y) <= FLT_MAX && fabsf(v.z) <= FLT_MAX && fabsf(v.w) <= FLT_MAX);
+            }
+        }
+        odd = __syncthreads_or(odd);                // and the probabilities; the keys' room is free
         if (kb + FP_K <= last) load(Ks, D + 4, k_pages, kb + FP_K);
-#pragma unroll 2
-        for (int k = 0; k < FP_K; k += 4) {
-            float4 p[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (ty * 4 + i) * FP_K + k);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
+        if (odd) {
+            for (int k = 0; k < FP_K; ++k) {
                 f32x2_t v[2 * DC];
 #pragma unroll
                 for (int c = 0; c < DC; ++c) {
-                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(Vs + (k + u) * D + c * 64 + tx * 4);
+                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(Vs + k * D + c * 64 + tx * 4);
                     v[2 * c] = w.x;
                     v[2 * c + 1] = w.y;
                 }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float pv = u == 0 ? p[i].x : u == 1 ? p[i].y : u == 2 ? p[i].z : p[i].w;
+                    const int pos = p0 + ty * 4 + i, key = kb + k;
+                    const float pv = Ps[(ty * 4 + i) * FP_K + k];
                     const f32x2_t pp = pair_of(pv, pv);
+                    if (key <= pos && (window <= 0 || key > pos - window))
 #pragma unroll
-                    for (int j = 0; j < 2 * DC; ++j) fma_pair(acc[i][j], pp, v[j]);
+                        for (int j = 0; j < 2 * DC; ++j) fma_pair(acc[i][j], pp, v[j]);
+                }
+            }
+        } else {
+#pragma unroll 2
+            for (int k = 0; k < FP_K; k += 4) {
+                float4 p[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (ty * 4 + i) * FP_K + k);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    f32x2_t v[2 * DC];
+#pragma unroll
+                    for (int c = 0; c < DC; ++c) {
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(Vs + (k + u) * D + c * 64 + tx * 4);
+                        v[2 * c] = w.x;
+                        v[2 * c + 1] = w.y;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float pv = u == 0 ? p[i].x : u == 1 ? p[i].y : u == 2 ? p[i].z : p[i].w;
+                        const f32x2_t pp = pair_of(pv, pv);
+#pragma unroll
+                        for (int j = 0; j < 2 * DC; ++j) fma_pair(acc[i][j], pp, v[j]);
+                    }
                 }
             }
         }
@@ -335,7 +369,8 @@ __global__ void __launch_bounds__(FD_THREADS) attention_f32_decode_kernel(
     for (int e = 0; e < 32 / VK; ++e) {
         const int key = warp * 32 + e * VK + vk;
         const int64_t at = row_at[key];
-        const float4 v = *reinterpret_cast<const float4*>(v_pages + at + vd);
+        const bool read = kb + key >= lo && kb + key <= pos;
+        const float4 v = read ? *reinterpret_cast<const float4*>(v_pages + at + vd) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const float p = sc[g][key];

@@ -253,6 +253,47 @@ def test_attention_decode_token_list_leaves_other_rows():
     assert bool((out[[0, 2]] == 7.0).all())
 
 
+@pytest.mark.parametrize("nq,nkv,d,P,window", [(4, 2, 128, 16, None), (3, 1, 64, 8, 70), (8, 1, 64, 64, None), (2, 2, 128, 4, 300)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_float32_attention_keeps_what_is_no_number_to_the_queries_that_read_it(nq, nkv, d, P, window, value):
+    """A value that is no number, at keys around the edges of a block of 64 keys and of a run of 512 and in a decoded row's
+    last key: the queries that read it get what a loop over their keys gives, the others are untouched."""
+    before, qlens, bad = [0, 130, 500, 700, 40], [150, 64, 90, 1, 1], [[63, 100], [131, 193], [511, 520], [650, 700], [20]]
+    T, starts = sum(qlens), [0]
+    g = torch.Generator().manual_seed(d + P)
+    NP = sum(-(-(b + n) // P) for b, n in zip(before, qlens)) + 3
+    lay = rows_layout(before, qlens, P, NP, seed=nq)
+    k_pages = torch.zeros(NP, nkv, P, d, device=DEV)
+    v_pages = torch.full((NP, nkv, P, d), float("nan"), device=DEV)
+    q, want = torch.randn(T, nq * d, generator=g), []
+    for r, (b, n) in enumerate(zip(before, qlens)):
+        k, v = torch.randn(b + n, nkv, d, generator=g), torch.randn(b + n, nkv, d, generator=g)
+        v[bad[r], :, 3] = value
+        scatter_to_pages(k_pages, lay["tables"][r], k, P)
+        scatter_to_pages(v_pages, lay["tables"][r], v, P)
+        for i in range(n):
+            keys = slice(max(0, b + i - window + 1) if window else 0, b + i + 1)
+            kh, vh = (t[keys].double().repeat_interleave(nq // nkv, 1) for t in (k, v))
+            w = torch.softmax(torch.einsum("hd,khd->hk", q[starts[r] + i].view(nq, d).double(), kh) * d ** -0.5, 1)
+            want.append(torch.einsum("hk,khd->hd", w, vh).reshape(-1))
+        starts.append(starts[-1] + n)
+    want, qd = torch.stack(want), q.to(DEV)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)
+    tiles = [(r, q0) for r, n in enumerate(qlens) if n > 1 for q0 in range(0, n, ops().F32_Q_TILE)]
+    single = [starts[r] for r, n in enumerate(qlens) if n == 1]
+    common = (k_pages, v_pages, lay["block_table"], lay["page_base"])
+    keys = lay["block_table"].shape[1] * P
+    out = torch.full((T, nq * d), 7.0, device=DEV)
+    ops().attention_f32_prefill(qd, qd.stride(0), *common, i32(starts), i32(before), i32(tiles).view(-1, 2), nq, nkv, d, d ** -0.5,
+                                window, ops().f32_prefill_chunks(keys, window), out)
+    ops().attention_f32_decode(qd, qd.stride(0), *common, lay["token_row"], lay["positions"], i32(single), len(single), nq, nkv, d,
+                               d ** -0.5, window, ops().f32_decode_chunks(min(window or 1 << 20, keys), window), out)
+    got, fine = out.double().cpu(), torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), fine) and bool(fine.any()) and not bool(fine.all())
+    assert torch.equal(torch.isposinf(got), torch.isposinf(want))
+    assert (got - want)[fine].abs().max() < 2e-6 * 5          # float32 sums of a few hundred weights of values up to 5
+
+
 def test_attention_decode_refuses_what_it_cannot_compute():
     from acorninfer_b200.kernels.ops import KernelError
     assert not ops().attention_decode_supported(34, 2, 64)       # 17 query heads a group
