@@ -1,6 +1,7 @@
 // The linear recurrence of linear_recurrence.cu over chunks of 64 tokens (float32 throughout):
 //     S_i = a_i S_(i-1) + b_i (w_i x_i)^T,   y_i = S_i^T c_i + skip x_i,   a number a_i per token and head.
-// With L_i the sum of log a up to i within the chunk (in double: differences of sums lose nothing that float32 would show),
+// With L_i the sum of log |a| up to i within the chunk (in double: differences of sums lose nothing that float32 would show),
+// and the product of the decays' signs up to i beside it,
 //     y = diag(exp(L)) C S_0 + P X + skip X,   P_ij = exp(L_i - L_j) w_j (c_i . b_j) for j <= i
 //     S_end = exp(L_n) S_0 + sum_j exp(L_n - L_j) w_j b_j x_j^T
 // (the block form of state space duality: Dao, Gu, "Transformers are SSMs").  Three kernels:
@@ -33,17 +34,23 @@ struct ScanChunkParams {
     int rows, H, G, N, V;
 };
 
-// Sums of the decays' logarithms of a chunk and its step sizes, by one warp (two tokens a lane).  A decay of zero counts as
-// exp(-1000): its products vanish as well.
-__device__ __forceinline__ void chunk_decays(const ScanChunkParams& p, int h, int first, int n, double* L, float* w) {
+// Sums of the logarithms of a chunk's decays, the products of their signs (1 or -1), and its step sizes times those, by one
+// warp (two tokens a lane).  A decay of zero counts as exp(-1000): its products vanish as well.  What is no number stays none
+// from its token on, and the tokens before do without it.
+__device__ __forceinline__ void chunk_decays(const ScanChunkParams& p, int h, int first, int n, double* L, float* sign, float* w) {
     const int lane = threadIdx.x & 31;
     double v[2];
+    bool neg[2];
+    float step[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         const int i = 2 * lane + q;
         const int64_t t = first + i;
-        v[q] = i < n ? fmax(log((double)(p.lda ? p.decay[t * p.lda + h] : p.decay[h])), -1000.0) : 0.0;
-        w[i] = i < n ? (p.w ? p.w[t * p.ldw + h] : 1.f) : 0.f;
+        const float a = i < n ? (p.lda ? p.decay[t * p.lda + h] : p.decay[h]) : 1.f;
+        const double lg = log(fabs((double)a));
+        v[q] = lg < -1000.0 ? -1000.0 : lg;
+        neg[q] = a < 0.f;
+        step[q] = i < n ? (p.w ? p.w[t * p.ldw + h] : 1.f) : 0.f;
     }
     double run = v[0] + v[1];
 #pragma unroll
@@ -51,8 +58,16 @@ __device__ __forceinline__ void chunk_decays(const ScanChunkParams& p, int h, in
         const double before = __shfl_up_sync(0xffffffffu, run, o);
         if (lane >= o) run += before;
     }
-    L[2 * lane] = run - v[1];
+    const double before = __shfl_up_sync(0xffffffffu, run, 1);
+    L[2 * lane] = lane ? before + v[0] : v[0];
     L[2 * lane + 1] = run;
+    const unsigned int below = (1u << lane) - 1, even = __ballot_sync(0xffffffffu, neg[0]), odd = __ballot_sync(0xffffffffu, neg[1]);
+    const int count = __popc(even & below) + __popc(odd & below) + (neg[0] ? 1 : 0);
+    const float s0 = count & 1 ? -1.f : 1.f, s1 = neg[1] ? -s0 : s0;
+    sign[2 * lane] = s0;
+    sign[2 * lane + 1] = s1;
+    w[2 * lane] = step[0] * s0;
+    w[2 * lane + 1] = step[1] * s1;
 }
 
 __device__ __forceinline__ void axpy4(float a, const float4& x, float4& y) {
@@ -66,7 +81,7 @@ __global__ void __launch_bounds__(256) scan_chunk_sum_kernel(const ScanChunkPara
     float* sB = sm;                                     // [DC][LN]
     float* sX = sB + DC * LN;                           // [DC][SCO_LV], times exp(L_n - L_j) w_j
     __shared__ double L[DC];
-    __shared__ float w[DC];
+    __shared__ float sign[DC], w[DC];
     pdl_wait();
     pdl_trigger();
     const int h = blockIdx.y, g = h / (p.H / p.G), v0 = blockIdx.z * SCO_VT, tid = threadIdx.x;
@@ -74,20 +89,21 @@ __global__ void __launch_bounds__(256) scan_chunk_sum_kernel(const ScanChunkPara
     if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
     load_rows<NP>(sB, p.b + (int64_t)first * p.ldb + (int64_t)g * p.N, p.ldb, n, p.N);
     asm volatile("cp.async.commit_group;\n" ::);
-    if (tid < 32) chunk_decays(p, h, first, n, L, w);
+    if (tid < 32) chunk_decays(p, h, first, n, L, sign, w);
     __syncthreads();
     const double Ln = L[DC - 1];
+    const float sign_n = sign[DC - 1];
     for (int e = tid; e < DC * (SCO_VT / 4); e += 256) {
         const int j = e / (SCO_VT / 4), c = (e % (SCO_VT / 4)) * 4;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (j < n && v0 + c < p.V) {
             x = *reinterpret_cast<const float4*>(p.x + (int64_t)(first + j) * p.ldx + (int64_t)h * p.V + v0 + c);
-            const float f = expf((float)(Ln - L[j])) * w[j];
+            const float f = expf((float)(Ln - L[j])) * (w[j] * sign_n);
             x = make_float4(x.x * f, x.y * f, x.z * f, x.w * f);
         }
         *reinterpret_cast<float4*>(sX + j * SCO_LV + c) = x;
     }
-    if (tid == 0 && blockIdx.z == 0) p.dec[(int64_t)blockIdx.x * p.H + h] = expf((float)Ln);
+    if (tid == 0 && blockIdx.z == 0) p.dec[(int64_t)blockIdx.x * p.H + h] = expf((float)Ln) * sign_n;
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
     const int tx = tid & 15, ty = tid >> 4;
@@ -163,7 +179,7 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
     float* sP = sX + DC * SCO_LV;                       // [DC][DC + DC_PAD]
     constexpr int LP = DC + DC_PAD;
     __shared__ double L[SCO_HEADS][DC];
-    __shared__ float w[SCO_HEADS][DC];
+    __shared__ float sign[SCO_HEADS][DC], w[SCO_HEADS][DC];
     pdl_wait();
     pdl_trigger();
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -175,7 +191,7 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
     load_rows<NP>(sC, p.c + (int64_t)first * p.ldc + (int64_t)g * p.N, p.ldc, n, p.N);
     load_rows<NP>(sB, p.b + (int64_t)first * p.ldb + (int64_t)g * p.N, p.ldb, n, p.N);
     asm volatile("cp.async.commit_group;\n" ::);
-    for (int q = tid >> 5; q < heads; q += 8) chunk_decays(p, h0 + q, first, n, L[q], w[q]);
+    for (int q = tid >> 5; q < heads; q += 8) chunk_decays(p, h0 + q, first, n, L[q], sign[q], w[q]);
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
     float M[4][4];                                      // c . b of rows ty + 16 ii and columns tx + 16 jj, jj <= ii
@@ -215,10 +231,11 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
         for (int ii = 0; ii < 4; ++ii) {
             const int i = ty + 16 * ii;
             const double Li = L[q][i];
+            const float sign_i = sign[q][i];
 #pragma unroll
             for (int jj = 0; jj <= ii; ++jj) {
                 const int j = tx + 16 * jj;
-                sP[i * LP + j] = j <= i ? expf((float)(Li - L[q][j])) * w[q][j] * M[ii][jj] : 0.f;
+                sP[i * LP + j] = j <= i ? expf((float)(Li - L[q][j])) * (w[q][j] * sign_i) * M[ii][jj] : 0.f;
             }
         }
         asm volatile("cp.async.wait_group 0;\n" ::);
@@ -239,7 +256,7 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
         }
 #pragma unroll
         for (int ii = 0; ii < 4; ++ii) {
-            const float e = expf((float)L[q][ty + 16 * ii]);
+            const float e = expf((float)L[q][ty + 16 * ii]) * sign[q][ty + 16 * ii];
             acc[ii] = make_float4(acc[ii].x * e, acc[ii].y * e, acc[ii].z * e, acc[ii].w * e);
         }
 #pragma unroll

@@ -468,6 +468,43 @@ def test_linear_scan_over_chunks(H, G, N, V, fixed):
     assert torch.equal(after[[4, 7]], before[[4, 7]]) and torch.equal(after[:, :5], before[:, :5])
 
 
+@pytest.mark.parametrize("H,G,N,V,fixed", [(4, 2, 64, 64, False), (3, 1, 12, 20, False), (8, 1, 128, 64, True)])
+def test_linear_scan_over_chunks_takes_decays_of_any_sign(H, G, N, V, fixed):
+    """Negative decays, zeros of either sign and very small ones, one NaN: the loop in 64 bits; from the NaN's token on no
+    output of its head and row is a number, and all before are."""
+    o = ops()
+    g = torch.Generator().manual_seed(N)
+    lens, slots = [200, 64, 70], [2, 0, 3]
+    T = sum(lens)
+    starts = np.cumsum([0] + lens)
+    b, c = torch.randn(T, G * N, generator=g), torch.randn(T, G * N, generator=g)
+    x, dt = torch.randn(T, H * V, generator=g), torch.rand(T, H, generator=g)
+    a = 1.2 * torch.rand(T, H, generator=g) - 0.6 if not fixed else (torch.rand(H, generator=g) - 0.8).expand(T, H).clone()
+    if not fixed:
+        a[10, 0], a[30:33, 1], a[77, :], a[130, 0], a[150, 2] = 0.0, -0.0, 1e-40, -1e-40, -1.0
+        a[starts[1] + 21, 1] = float("nan")
+    state = torch.randn(4, H * V * N + 5, generator=g)
+    f = lambda t: t.float().contiguous().to(DEV)
+    sd, i32 = state.to(DEV), dict(dtype=torch.int32, device=DEV)
+    assert o.scan_chunk_ok(max(lens), 3, f(b), f(c), f(x), H, N, V)
+    y = o.linear_scan(f(b), f(c), f(x), f(a[0] if fixed else a), f(dt), None, sd, 5, torch.tensor(starts, **i32), torch.tensor(slots, **i32),
+                      3, H, G, N, V, longest_row=max(lens)).double().cpu().view(T, H, V)
+    group = torch.arange(H) // (H // G)
+    for r, (n, slot) in enumerate(zip(lens, slots)):
+        S, want = state[slot, 5:].double().view(H, V, N), []
+        for t in range(starts[r], starts[r] + n):
+            bt, ct = b[t].double().view(G, N)[group], c[t].double().view(G, N)[group]
+            S = a[t].double()[:, None, None] * S + (dt[t].double()[:, None] * x[t].double().view(H, V))[:, :, None] * bt[:, None]
+            want.append(torch.einsum("hvn,hn->hv", S, ct))
+        want, got, end = torch.stack(want), y[starts[r]:starts[r] + n], sd[slot, 5:].double().cpu().view(H, V, N)
+        assert torch.equal(torch.isfinite(got), torch.isfinite(want)) and torch.equal(torch.isfinite(end), torch.isfinite(S))
+        fine = torch.isfinite(want)
+        assert float((got - want)[fine].norm() / want[fine].norm()) < 1e-6 and (fine.all() or r == 1)
+        fine = torch.isfinite(S)
+        assert float((end - S)[fine].norm() / S[fine].norm()) < 1e-6
+    assert torch.equal(sd[:, :5].cpu(), state[:, :5])
+
+
 def test_linear_scan_with_one_decay_per_head_and_no_step_sizes():
     o = ops()
     g = torch.Generator().manual_seed(1)
