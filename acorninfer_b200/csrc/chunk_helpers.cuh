@@ -6,6 +6,8 @@
 
 #include "common.cuh"
 
+#include <cfloat>
+
 #define DC 64                       // tokens a chunk
 #define DC_PAD 4                    // floats between rows in shared memory (16-byte reads of neighbouring rows hit distinct banks)
 
@@ -40,4 +42,8 @@ template <int DP> __device__ __forceinline__ void load_rows(float* dst, const fl
 
 __device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
     return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
+}
+
+__device__ __forceinline__ bool not_finite(const float4& v) {
+    return !(fabsf(v.x) <= FLT_MAX && fabsf(v.y) <= FLT_MAX && fabsf(v.z) <= FLT_MAX && fabsf(v.w) <= FLT_MAX);
 }

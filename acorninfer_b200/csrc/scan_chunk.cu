@@ -239,7 +239,10 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
             }
         }
         asm volatile("cp.async.wait_group 0;\n" ::);
-        __syncthreads();
+        bool odd = false;                               // an input that is no number: 0 times it would reach the tokens before
+        for (int e = tid; e < DC * (SCO_VT / 4); e += 256)      // what this thread has brought
+            odd |= not_finite(*reinterpret_cast<const float4*>(sX + (e / (SCO_VT / 4)) * SCO_LV + (e % (SCO_VT / 4)) * 4));
+        odd = __syncthreads_or(odd);
         float4 acc[4];
 #pragma unroll
         for (int ii = 0; ii < 4; ++ii) acc[ii] = zero;
@@ -259,8 +262,17 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
             const float e = expf((float)L[q][ty + 16 * ii]) * sign[q][ty + 16 * ii];
             acc[ii] = make_float4(acc[ii].x * e, acc[ii].y * e, acc[ii].z * e, acc[ii].w * e);
         }
+        if (odd) {
+            for (int j = 0; j < DC; ++j) {
+                const float4 x = *reinterpret_cast<const float4*>(sX + j * SCO_LV + 4 * tx);
+#pragma unroll
+                for (int ii = 0; ii < 4; ++ii)
+                    if (j <= ty + 16 * ii) axpy4(sP[(ty + 16 * ii) * LP + j], x, acc[ii]);
+            }
+        }
 #pragma unroll
         for (int jb = 0; jb < 4; ++jb) {                // blocks of 16 tokens; rows before the block see none of it
+            if (odd) break;
 #pragma unroll
             for (int j = 16 * jb; j < 16 * jb + 16; j += 4) {
                 float4 x[4];

@@ -505,6 +505,37 @@ def test_linear_scan_over_chunks_takes_decays_of_any_sign(H, G, N, V, fixed):
     assert torch.equal(sd[:, :5].cpu(), state[:, :5])
 
 
+@pytest.mark.parametrize("H,G,N,V", [(9, 1, 36, 100), (4, 2, 128, 64)])
+@pytest.mark.parametrize("where", ["x", "b", "c", "w", "decay"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_linear_scan_over_chunks_leaves_earlier_tokens_alone(H, G, N, V, where, value):
+    """One input of a token is no number: the outputs of its row's earlier tokens and of the other rows keep every bit, and the
+    later ones are finite where the kernel that walks the tokens has finite ones."""
+    o = ops()
+    g = torch.Generator().manual_seed(N)
+    lens, slots, bad = [200, 64, 70], [2, 0, 3], 133
+    T, starts = sum(lens), [0, 200, 264, 334]
+    ins = {"b": torch.randn(T, G * N, generator=g), "c": torch.randn(T, G * N, generator=g), "x": torch.randn(T, H * V, generator=g),
+           "decay": torch.rand(T, H, generator=g) * 0.3 + 0.7, "w": torch.rand(T, H, generator=g)}
+    state = torch.randn(4, H * V * N, generator=g)
+    i32 = dict(dtype=torch.int32, device=DEV)
+
+    def run(longest):
+        d, sd = {k: t.to(DEV) for k, t in ins.items()}, state.to(DEV)
+        y = o.linear_scan(d["b"], d["c"], d["x"], d["decay"], d["w"], None, sd, 0, torch.tensor(starts, **i32), torch.tensor(slots, **i32),
+                          3, H, G, N, V, longest_row=longest)
+        return y.cpu(), sd.cpu()
+
+    clean, _ = run(200)
+    ins[where][bad, 2 % ins[where].shape[1]] = value
+    got, end = run(200)
+    walk, walk_end = run(1)
+    assert torch.equal(got[:bad], clean[:bad]) and torch.equal(got[200:], clean[200:])
+    assert not bool(torch.isfinite(got[bad:200]).all())
+    if not (where == "decay" and value == float("inf")):        # (an infinite decay: the logarithms' differences are no numbers at once)
+        assert torch.equal(torch.isfinite(got), torch.isfinite(walk)) and torch.equal(torch.isfinite(end), torch.isfinite(walk_end))
+
+
 def test_linear_scan_with_one_decay_per_head_and_no_step_sizes():
     o = ops()
     g = torch.Generator().manual_seed(1)
