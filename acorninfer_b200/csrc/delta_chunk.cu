@@ -556,7 +556,10 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_out_kernel(const DeltaChun
     asm volatile("cp.async.commit_group;\n" ::);
     if (!SCALED && tid < DC) sb[tid] = p.b[(int64_t)(first + min(tid, n - 1)) * p.H + h];
     asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncthreads();
+    bool odd = false;                                   // a value that is no number: 0 times it would reach the tokens before
+    for (int e = tid; e < DC * (DC_OT / 4); e += 256)   // what this thread has brought
+        odd |= not_finite(*reinterpret_cast<const float4*>(sU + (e / (DC_OT / 4)) * LO + (e % (DC_OT / 4)) * 4));
+    odd = __syncthreads_or(odd);
     const int tx = tid & 15, ty = tid >> 4;             // rows ty + 16 ii, columns 4 tx .. 4 tx + 3
     float4 acc[4];
 #pragma unroll
@@ -582,8 +585,17 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_out_kernel(const DeltaChun
             acc[ii] = make_float4(acc[ii].x * g, acc[ii].y * g, acc[ii].z * g, acc[ii].w * g);
         }
     }
+    if (odd) {
+        for (int j = 0; j < DC; ++j) {
+            const float4 u = *reinterpret_cast<const float4*>(sU + j * LO + 4 * tx);
+#pragma unroll
+            for (int ii = 0; ii < 4; ++ii)
+                if (j <= ty + 16 * ii) axpy(sP[(ty + 16 * ii) * LA + j], u, acc[ii]);
+        }
+    }
 #pragma unroll
     for (int jb = 0; jb < 4; ++jb) {                    // blocks of 16 keys; rows before the block see none of it
+        if (odd) break;
 #pragma unroll
         for (int j = 16 * jb; j < 16 * jb + 16; j += 4) {
             float4 u[4];

@@ -497,6 +497,41 @@ def test_time_mixing_over_chunks_with_decays_that_leave_nothing(dim, dtype):
     assert float((ends["chunks"] - ends["walk"]).norm() / ends["walk"].norm()) < 1e-5
 
 
+@pytest.mark.parametrize("form", ["mix", "channel"])
+@pytest.mark.parametrize("dim,vdim", [(32, 20), (100, 68), (128, 128)])
+@pytest.mark.parametrize("where", ["q", "k", "v", "log2_g", "beta"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_recurrences_over_chunks_leave_earlier_tokens_alone(form, dim, vdim, where, value):
+    """One input of a token is no number: the outputs of its row's earlier tokens and of the other rows keep every bit, and the
+    later ones are finite where the kernel that walks the tokens has finite ones."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim)
+    H, lens, bad = 2, [200, 64, 70], 133
+    if (where == "log2_g" and value > 0) or (where == "beta" and form == "mix"):
+        return                                          # a logarithm of a decay is not positive; time mixing has no beta
+    T = sum(lens)
+    starts, slots = torch.tensor([0, 200, 264, 334], dtype=torch.int32, device=DEV), torch.tensor([2, 0, 3], dtype=torch.int32, device=DEV)
+    ins = {"q": torch.randn(T, H, dim, generator=g), "k": torch.randn(T, H, dim, generator=g) * dim ** -0.5, "v": torch.randn(T, H, vdim, generator=g),
+           "beta": torch.rand(T, H, generator=g), "log2_g": -torch.rand(T, H, dim, generator=g)}
+    u, state = torch.randn(H, dim, generator=g).to(DEV), torch.randn(4, H * dim * vdim, generator=g)
+
+    def run(chunks):
+        d, sd = {k: t.to(DEV) for k, t in ins.items()}, state.to(DEV)
+        args = (d["log2_g"] if chunks else torch.exp2(d["log2_g"]), sd, starts, slots, 3)
+        if form == "mix":
+            y = (o.mix_chunk(d["q"], d["k"], d["v"], u, *args) if chunks else o.delta_rule(d["q"], d["k"], d["v"], None, *args, bonus32=u))
+        else:
+            y = (o.channel_chunk if chunks else o.delta_rule)(d["q"], d["k"], d["v"], d["beta"], *args)
+        return y.cpu(), sd.cpu()
+
+    clean, _ = run(True)
+    ins[where].view(T, -1)[bad, 1] = value
+    (got, end), (walk, walk_end) = run(True), run(False)
+    assert torch.equal(got[:bad], clean[:bad]) and torch.equal(got[200:], clean[200:])
+    assert torch.equal(torch.isfinite(got), torch.isfinite(walk)) and torch.equal(torch.isfinite(end), torch.isfinite(walk_end))
+    assert not bool(torch.isfinite(got[bad:200]).all())
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
 @pytest.mark.parametrize("W,off,tail,single", [(20, 7, 3, False), (20, 8, 4, False), (20, 8, 4, True), (520, 4, 0, True),
                                                (22, 8, 2, True)])
