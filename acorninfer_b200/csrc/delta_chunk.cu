@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(const DeltaCh
     pdl_trigger();
     const int h = blockIdx.y, kh = h / (p.H / p.KH), tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, 0, r, first, n)) return;
     load_rows<DP>(sK, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
     load_rows<DP>(sQ, p.q + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
     asm volatile("cp.async.commit_group;\n" ::);
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(CC_THREADS) channel_chunk_solve_kernel(const D
     pdl_trigger();
     const int h = blockIdx.y, kh = h / (p.H / p.KH), tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, 0, r, first, n)) return;
     load_rows<DP>(sB, p.log_g + ((int64_t)first * p.H + h) * p.dim, (int64_t)p.H * p.dim, n, p.dim);
     asm volatile("cp.async.commit_group;\n" ::);
     load_rows<DP>(sK, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_out_kernel(const DeltaChun
     pdl_trigger();
     const int h = blockIdx.y, kh = h / (p.H / p.KH), v0 = blockIdx.z * DC_OT, tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, 0, r, first, n)) return;
     load_rows<DP>(sQ, p.q + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
     const float* S = p.s0 + ((int64_t)blockIdx.x * p.H + h) * p.dim * p.vdim + v0;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(256) linear_chunk_local_kernel(const LinearChu
     pdl_trigger();
     const int h = blockIdx.y, tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, 0, r, first, n)) return;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const int Hd = p.H * p.dim;
     const float to_log2 = -1.4426950408889634f * p.inv_tau;
@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(256) mix_chunk_local_kernel(const DeltaChunkPa
     pdl_trigger();
     const int h = blockIdx.y, kh = h / (p.H / p.KH), tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, 0, r, first, n)) return;
     load_rows<DP>(sB, p.log_g + ((int64_t)first * p.H + h) * p.dim, (int64_t)p.H * p.dim, n, p.dim);
     asm volatile("cp.async.commit_group;\n" ::);
     load_rows<DP>(sK, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);

@@ -251,6 +251,7 @@ struct ScanParams {
     float* seg_state;
     float* seg_decay;
     int seg, nseg;
+    int max_row;                        // > 0: longer rows are left alone (SCAN_WHOLE)
 };
 
 #define SCAN_WHOLE 0        // a row from its slot's state to the end, the state back into the slot
@@ -309,6 +310,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, CPT == 4 ? 3 : 4) linear_scan_ke
     const int col = threadIdx.x / p.LN, l = threadIdx.x % p.LN;
     const int v0 = blockIdx.x * cpb;
     int first = p.row_start[r], L = p.row_start[r + 1] - first;
+    if (MODE == SCAN_WHOLE && p.max_row > 0 && L > p.max_row) return;
     int nseg_r = 1;
     if (MODE != SCAN_WHOLE) {
         nseg_r = (L + p.seg - 1) / p.seg;
@@ -529,11 +531,11 @@ extern "C" int acorn_linear_scan_columns(int N, int V) {
 
 // seg_tokens = 0: every row in one piece (seg_state, seg_decay unused).  Otherwise rows are cut into segments of
 // seg_tokens tokens, at most nseg a row (the caller sees to nseg * seg_tokens >= the longest row); seg_state holds
-// rows * (nseg + 1) * H * V * N floats, seg_decay rows * nseg * H.
+// rows * (nseg + 1) * H * V * N floats, seg_decay rows * nseg * H.  max_row > 0 (rows in one piece): longer rows are left alone.
 extern "C" int acorn_linear_scan(const float* b, int64_t ldb, const float* c, int64_t ldc, const float* x, int64_t ldx,
                                  const float* decay, int64_t lda, const float* w, int64_t ldw, const float* skip,
                                  float* state, int64_t slot_stride, int64_t state_off, float* y, const int* row_start,
-                                 const int* row_slot, int rows, int H, int G, int N, int V, int seg_tokens, int nseg,
+                                 const int* row_slot, int rows, int H, int G, int N, int V, int seg_tokens, int nseg, int max_row,
                                  float* seg_state, float* seg_decay, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (H < 1 || G < 1 || H % G || N < 1 || N > 32 * SCAN_STRIP || V < 1 || H > 65535) return ACORN_ERR_UNSUPPORTED;
@@ -543,7 +545,7 @@ extern "C" int acorn_linear_scan(const float* b, int64_t ldb, const float* c, in
     int LN = 1;
     while (LN * SCAN_STRIP < N) LN *= 2;
     ScanParams p = {b, ldb, c, ldc, x, ldx, decay, lda, w, ldw, skip, state, slot_stride, state_off, y, row_start, row_slot,
-                    H, G, N, V, LN, seg_state, seg_decay, seg_tokens, cut ? nseg : 1};
+                    H, G, N, V, LN, seg_state, seg_decay, seg_tokens, cut ? nseg : 1, max_row};
     switch (acorn_linear_scan_columns(N, V)) {
         case 4: return launch_scan<4>(p, rows, cut, stream);
         case 2: return launch_scan<2>(p, rows, cut, stream);

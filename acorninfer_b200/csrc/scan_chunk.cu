@@ -32,6 +32,7 @@ struct ScanChunkParams {
     float* s0;                          // [chunk numbers, H, N, V]: the chunk's own sum, then the state it starts from
     float* dec;                         // [chunk numbers, H]: exp(L_n)
     int rows, H, G, N, V;
+    int min_row;                        // rows of fewer tokens are left alone
 };
 
 // Sums of the logarithms of a chunk's decays, the products of their signs (1 or -1), and its step sizes times those, by one
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(256) scan_chunk_sum_kernel(const ScanChunkPara
     pdl_trigger();
     const int h = blockIdx.y, g = h / (p.H / p.G), v0 = blockIdx.z * SCO_VT, tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, p.min_row, r, first, n)) return;
     load_rows<NP>(sB, p.b + (int64_t)first * p.ldb + (int64_t)g * p.N, p.ldb, n, p.N);
     asm volatile("cp.async.commit_group;\n" ::);
     if (tid < 32) chunk_decays(p, h, first, n, L, sign, w);
@@ -135,11 +136,12 @@ __global__ void __launch_bounds__(256) scan_chunk_sum_kernel(const ScanChunkPara
 __global__ void scan_chunk_fold_kernel(const ScanChunkParams p) {
     pdl_wait();
     pdl_trigger();
-    const int r = blockIdx.z, h = blockIdx.y, V4 = p.V / 4;
+    const int h = blockIdx.y, V4 = p.V / 4;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= p.N * V4) return;
+    int r, id0;
+    if (!row_of_block(blockIdx.z, p.row_start, p.rows, p.min_row, r, id0) || e >= p.N * V4) return;
     const int d = e / V4, v = (e % V4) * 4;
-    const int start = p.row_start[r], chunks = (p.row_start[r + 1] - start + DC - 1) / DC, id0 = start / DC + r;
+    const int chunks = (p.row_start[r + 1] - p.row_start[r] + DC - 1) / DC;
     float* slot = p.state + (int64_t)p.row_slot[r] * p.slot_stride + ((int64_t)h * p.V + v) * p.N + d;
     float4* E = reinterpret_cast<float4*>(p.s0 + ((int64_t)id0 * p.H + h) * p.N * p.V) + e;
     const float* a = p.dec + (int64_t)id0 * p.H + h;
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
     const int g = blockIdx.y, v0 = (blockIdx.z % tiles) * SCO_VT;
     const int h0 = g * rep + (blockIdx.z / tiles) * per_block, heads = min(per_block, (g + 1) * rep - h0);
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, p.min_row, r, first, n)) return;
     load_rows<NP>(sC, p.c + (int64_t)first * p.ldc + (int64_t)g * p.N, p.ldc, n, p.N);
     load_rows<NP>(sB, p.b + (int64_t)first * p.ldb + (int64_t)g * p.N, p.ldb, n, p.N);
     asm volatile("cp.async.commit_group;\n" ::);
@@ -297,7 +299,7 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
     }
 }
 
-template <int NP> static int launch_scan_chunk(const ScanChunkParams& p, int ids, cudaStream_t stream) {
+template <int NP> static int launch_scan_chunk(const ScanChunkParams& p, int ids, int walks, cudaStream_t stream) {
     constexpr int LN = NP + DC_PAD;
     constexpr int BS = DC * LN > NP * SCO_LV ? DC * LN : NP * SCO_LV;
     const size_t sum = (size_t)(DC * LN + DC * SCO_LV) * sizeof(float);
@@ -312,7 +314,7 @@ template <int NP> static int launch_scan_chunk(const ScanChunkParams& p, int ids
     const int tiles = (p.V + SCO_VT - 1) / SCO_VT, rep = p.H / p.G;
     int rc = acorn_launch(scan_chunk_sum_kernel<NP>, dim3(ids, p.H, tiles), dim3(256), sum, stream, p);
     if (rc) return rc;
-    rc = acorn_launch(scan_chunk_fold_kernel, dim3((p.N * (p.V / 4) + 255) / 256, p.H, p.rows), dim3(256), 0, stream, p);
+    rc = acorn_launch(scan_chunk_fold_kernel, dim3((p.N * (p.V / 4) + 255) / 256, p.H, walks), dim3(256), 0, stream, p);
     if (rc) return rc;
     // The heads of a group share C B^T, about 0.4 of a head's own work, so a block wants many of them, and the 296 blocks
     // that run at a time want to be filled: the share with the least estimated time.
@@ -328,20 +330,21 @@ template <int NP> static int launch_scan_chunk(const ScanChunkParams& p, int ids
 
 extern "C" int acorn_scan_chunk_supported(int N, int V) { return N >= 4 && N <= 128 && N % 4 == 0 && V >= 4 && V % 4 == 0; }
 
-// Arguments as acorn_linear_scan (state at the first float of S in slot 0); s0 holds tokens / 64 + rows chunks of
-// [H, N, V] floats, dec as many of [H].
+// Arguments as acorn_linear_scan (state at the first float of S in slot 0), for the rows of min_row tokens or more; s0 holds
+// chunk_ids(tokens, rows, min_row) chunks of [H, N, V] floats, dec as many of [H].
 extern "C" int acorn_scan_chunk(const float* b, int64_t ldb, const float* c, int64_t ldc, const float* x, int64_t ldx,
                                 const float* decay, int64_t lda, const float* w, int64_t ldw, const float* skip, float* state,
                                 int64_t slot_stride, float* y, const int* row_start, const int* row_slot, int tokens, int rows,
-                                int H, int G, int N, int V, float* s0, float* dec, cudaStream_t stream) {
+                                int H, int G, int N, int V, int min_row, float* s0, float* dec, cudaStream_t stream) {
     if (tokens <= 0 || rows <= 0) return 0;
     const uintptr_t all = (uintptr_t)b | (uintptr_t)c | (uintptr_t)x | (uintptr_t)y | (uintptr_t)s0;
     if (!acorn_scan_chunk_supported(N, V) || G < 1 || H < 1 || H % G || H > 65535 || rows > 65535 || (all & 15) || ldb % 4 ||
         ldc % 4 || ldx % 4)
         return ACORN_ERR_UNSUPPORTED;
-    const int ids = tokens / DC + rows;
+    const int ids = chunk_ids(tokens, rows, min_row), walks = chunk_rows(tokens, rows, min_row);
+    if (walks == 0) return 0;
     if ((int64_t)((V + SCO_VT - 1) / SCO_VT) * (H / G) > 65535) return ACORN_ERR_UNSUPPORTED;
     const ScanChunkParams p = {b, ldb, c, ldc, x, ldx, decay, lda, w, ldw, skip, state, slot_stride, y, row_start, row_slot, s0, dec,
-                               rows, H, G, N, V};
-    return N <= 64 ? launch_scan_chunk<64>(p, ids, stream) : launch_scan_chunk<128>(p, ids, stream);
+                               rows, H, G, N, V, min_row};
+    return N <= 64 ? launch_scan_chunk<64>(p, ids, walks, stream) : launch_scan_chunk<128>(p, ids, walks, stream);
 }

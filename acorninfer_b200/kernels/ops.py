@@ -105,7 +105,7 @@ class _Sigs:
     acorn_silu_rows = [c_void_p, c_int64, c_void_p, c_int, c_int, c_int, c_void_p]
     acorn_linear_scan = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                          c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                         c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]
+                         c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]
     acorn_gated_norm = [c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_float, c_int,
                         c_float, c_int, c_void_p]
     acorn_cast = [c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]
@@ -117,7 +117,7 @@ class _Sigs:
                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
                              c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_int, c_void_p]
     acorn_scan_chunk = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
-                        c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                        c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                         c_void_p]
     acorn_scan_chunk_supported = [c_int, c_int]
     acorn_attention_f32_supported = [c_int, c_int, c_int]
@@ -2373,26 +2373,47 @@ def scan_segments(longest_row: int, num_rows: int, heads: int, n: int, v: int) -
 
 
 SCAN_CHUNK = 64                   # tokens a chunk of the chunked scan
+# Tokens: shorter rows are walked.  Measured (B200, us, walk / chunks; 64 heads of 64 columns, 8 groups of keys of 128): 1 row of
+# 64 tokens 30 / 40, of 128 65 / 44; 4 rows of 64 50 / 67, of 96 73 / 89, of 128 121 / 89; 16 rows of 64 166 / 217, of 128 320 / 306.
+SCAN_CHUNK_MIN_ROW = 128
+
+
+def scan_chunk_ids(tokens: int, num_rows: int) -> int:
+    """Chunks that the rows of ``SCAN_CHUNK_MIN_ROW`` tokens or more of a step can hold together."""
+    return tokens // SCAN_CHUNK + min(num_rows, tokens // SCAN_CHUNK_MIN_ROW)
 
 
 def scan_chunk_ok(longest_row: int, num_rows: int, b: torch.Tensor, c: torch.Tensor, x: torch.Tensor, heads: int, n: int, v: int) -> bool:
-    """Whether the scan of these rows runs over chunks of tokens: a row of a chunk or more, sizes and alignments the kernels
+    """Whether the scan of these rows runs over chunks of tokens: a row long enough to gain by it, sizes and alignments the kernels
     know (16-byte reads of b, c and x), and room for the chunks' states."""
-    return (longest_row >= SCAN_CHUNK and bool(lib().acorn_scan_chunk_supported(n, v)) and num_rows <= 65535 and heads <= 65535
+    return (longest_row >= SCAN_CHUNK_MIN_ROW and bool(lib().acorn_scan_chunk_supported(n, v)) and num_rows <= 65535 and heads <= 65535
             and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in (b, c, x))
-            and 4 * (x.shape[0] // SCAN_CHUNK + num_rows) * heads * n * v <= DELTA_CHUNK_SCRATCH_BYTES)
+            and 4 * scan_chunk_ids(x.shape[0], num_rows) * heads * n * v <= DELTA_CHUNK_SCRATCH_BYTES)
+
+
+def chunk_min_row(row_lens: list[int], rules: tuple[tuple[int, int], ...]) -> int:
+    """The least tokens of the rows that run over chunks in a step of these rows, 0: none do.  ``rules``: (least, enough) pairs, of
+    which the first holds whose rows bring ``enough`` tokens together, and half of the step's: the kernels that walk tokens run
+    all rows side by side, so a few long rows among many others hardly add to their time."""
+    total = sum(row_lens)
+    for least, enough in rules:
+        long = sum(n for n in row_lens if n >= least)
+        if long >= enough and 2 * long >= total:
+            return least
+    return 0
 
 
 def linear_scan(b: torch.Tensor, c: torch.Tensor, x: torch.Tensor, decay: torch.Tensor, w: torch.Tensor | None,
                 skip32: torch.Tensor | None, state: torch.Tensor, state_off: int, row_start: torch.Tensor,
                 row_slot: torch.Tensor, num_rows: int, heads: int, groups: int, n: int, v: int,
-                longest_row: int = 1) -> torch.Tensor:
+                longest_row: int = 1, row_lens: list[int] | None = None) -> torch.Tensor:
     """Per head ``S <- a S + b (w x)^T; y = S^T c + skip x`` over every row's tokens, from the state in the
     row's slot (``[heads, v, n]`` float32 at ``state_off``, updated in place).  ``b``, ``c`` [T, groups * n],
     ``x`` [T, heads * v] float32 (column slices allowed); ``decay`` [T, heads] per token or [heads] for all;
-    ``w`` [T, heads] or None.  Returns float32 y [T, heads * v].  ``longest_row``: a bound on the tokens of a row
-    (a host number); steps with a long row run over chunks of tokens (``scan_chunk_ok``) or, at sizes those kernels do not
-    take, with their rows in segments side by side (``scan_segments``)."""
+    ``w`` [T, heads] or None.  Returns float32 y [T, heads * v].  ``longest_row``: a bound on the tokens of a row (a host
+    number); ``row_lens``: every row's, where they are known.  Rows of ``SCAN_CHUNK_MIN_ROW`` tokens or more run over chunks of
+    tokens (``scan_chunk_ok``; not where other rows bring most of the step's tokens), and the others token by token, as they
+    would without the long ones beside them.  Elsewhere long rows run in segments side by side (``scan_segments``)."""
     for t, name in ((b, "b"), (c, "c"), (x, "x")):
         _rows2(t, name, torch.float32)
     _check(state, "state", torch.float32, 2)
@@ -2410,17 +2431,20 @@ def linear_scan(b: torch.Tensor, c: torch.Tensor, x: torch.Tensor, decay: torch.
     if skip32 is not None:
         _check(skip32, "skip", torch.float32, 1)
     y = torch.empty((T, heads * v), dtype=torch.float32, device=x.device)
-    if scan_chunk_ok(int(longest_row), num_rows, b, c, x, heads, n, v):
-        ids = T // SCAN_CHUNK + num_rows
+    chunks = scan_chunk_ok(int(longest_row), num_rows, b, c, x, heads, n, v) and (
+        row_lens is None or chunk_min_row(row_lens, ((SCAN_CHUNK_MIN_ROW, 1),)) > 0)
+    if chunks:
+        ids = scan_chunk_ids(T, num_rows)
         s0 = torch.empty((ids, heads, n, v), dtype=torch.float32, device=x.device)
         dec = torch.empty((ids, heads), dtype=torch.float32, device=x.device)
         _ok(lib().acorn_scan_chunk(b.data_ptr(), b.stride(0), c.data_ptr(), c.stride(0), x.data_ptr(), x.stride(0), decay.data_ptr(),
                                    decay.stride(0) if decay.dim() == 2 else 0, _ptr(w), w.stride(0) if w is not None else 0,
                                    _ptr(skip32), state.data_ptr() + 4 * int(state_off), state.stride(0), y.data_ptr(),
-                                   row_start.data_ptr(), row_slot.data_ptr(), T, num_rows, heads, groups, n, v, s0.data_ptr(),
-                                   dec.data_ptr(), _stream()), "linear_scan")
-        return y
-    seg, nseg = scan_segments(int(longest_row), num_rows, heads, n, v)
+                                   row_start.data_ptr(), row_slot.data_ptr(), T, num_rows, heads, groups, n, v, SCAN_CHUNK_MIN_ROW,
+                                   s0.data_ptr(), dec.data_ptr(), _stream()), "linear_scan")
+        if row_lens is not None and min(row_lens) >= SCAN_CHUNK_MIN_ROW:
+            return y
+    seg, nseg = (0, 1) if chunks else scan_segments(int(longest_row), num_rows, heads, n, v)
     seg_state = seg_decay = None
     if seg:
         seg_state = torch.empty((num_rows, nseg + 1, heads * n * v), dtype=torch.float32, device=x.device)
@@ -2429,7 +2453,8 @@ def linear_scan(b: torch.Tensor, c: torch.Tensor, x: torch.Tensor, decay: torch.
                                 decay.data_ptr(), decay.stride(0) if decay.dim() == 2 else 0, _ptr(w),
                                 w.stride(0) if w is not None else 0, _ptr(skip32), state.data_ptr(), state.stride(0),
                                 int(state_off), y.data_ptr(), row_start.data_ptr(), row_slot.data_ptr(), num_rows, heads,
-                                groups, n, v, seg, nseg, _ptr(seg_state), _ptr(seg_decay), _stream()), "linear_scan")
+                                groups, n, v, seg, nseg, SCAN_CHUNK_MIN_ROW - 1 if chunks else 0, _ptr(seg_state), _ptr(seg_decay),
+                                _stream()), "linear_scan")
     return y
 
 

@@ -94,7 +94,7 @@ class StateSpace(_RecurrentMixer):
                                   inputs.num_rows, C, self.taps, skip_single=True)
         y = ops.linear_scan(act[:, I:I + GN], act[:, I + GN:], act[:, :I], decay, dt, self.d32, cache.state,
                             self.state_base, inputs.row_start, inputs.row_slot, inputs.num_rows, self.H, self.G,
-                            self.N, self.V, longest_row=inputs.plan.max_q_len)
+                            self.N, self.V, longest_row=inputs.plan.max_q_len, row_lens=inputs.plan.row_lens)
         if out is None:
             out = torch.empty((proj.shape[0], I), dtype=self.ctx.dtype, device=proj.device)
         return ops.gated_norm(y, proj[:, :I], self.norm32, self.eps, self.norm_groups, True, out, out_scale)
@@ -140,7 +140,7 @@ class DecayLinearAttention(_RecurrentMixer):
         act = ops.silu_rows(proj[:, :2 * Hd + Hv])
         y = ops.linear_scan(act[:, Hd:2 * Hd], act[:, :Hd], act[:, 2 * Hd:], self._decay32, None, None, cache.state,
                             self.state_base, inputs.row_start, inputs.row_slot, inputs.num_rows, self.H, self.H,
-                            self.dim, self.V, longest_row=inputs.plan.max_q_len)
+                            self.dim, self.V, longest_row=inputs.plan.max_q_len, row_lens=inputs.plan.row_lens)
         if out is None:
             out = torch.empty((proj.shape[0], Hv), dtype=self.ctx.dtype, device=proj.device)
         return ops.gated_norm(y, proj[:, 2 * Hd + Hv:], self.norm32, self.eps, 1, False, out, out_scale)

@@ -213,3 +213,16 @@ def test_a_prompt_portion_alone_is_padded_with_tokens_that_touch_only_its_own_sl
     m.extend(rc3, 3)
     two = plan_step([StepEntry(rc2, [1] * 32, []), StepEntry(rc3, [1, 2, 3], [2])], m, STEP_ARRAYS)
     assert pad_prefill_plan(two, m.pad_pages, P, STEP_ARRAYS) is two
+
+
+def test_which_rows_of_a_step_run_over_chunks():
+    from acorninfer_b200.kernels.ops import chunk_min_row
+
+    rules = ((64, 256), (160, 160))
+    assert chunk_min_row([63] * 10, rules) == 0
+    assert chunk_min_row([64], rules) == 0 and chunk_min_row([159], rules) == 0 and chunk_min_row([160], rules) == 160
+    assert chunk_min_row([64] * 4, rules) == 64 and chunk_min_row([256], rules) == 64
+    assert chunk_min_row([1] * 47 + [160], rules) == 160 and chunk_min_row([64, 160], rules) == 160
+    # rows that other ones outnumber by far stay with them
+    assert chunk_min_row([30] * 40 + [200], rules) == 0 and chunk_min_row([30] * 40 + [1200], rules) == 64
+    assert chunk_min_row([1, 5], ((128, 1),)) == 0 and chunk_min_row([127, 128], ((128, 1),)) == 128

@@ -536,6 +536,40 @@ def test_linear_scan_over_chunks_leaves_earlier_tokens_alone(H, G, N, V, where, 
         assert torch.equal(torch.isfinite(got), torch.isfinite(walk)) and torch.equal(torch.isfinite(end), torch.isfinite(walk_end))
 
 
+@pytest.mark.parametrize("H,G,N,V,fixed", [(4, 2, 64, 64, False), (3, 3, 12, 8, True), (16, 8, 128, 64, False)])
+def test_linear_scan_of_short_rows_beside_long_ones(H, G, N, V, fixed):
+    """Rows too short for chunks of tokens, single ones among them, keep every bit of their outputs and states whatever long
+    rows share their step."""
+    o = ops()
+    g = torch.Generator().manual_seed(N)
+    least = o.SCAN_CHUNK_MIN_ROW
+    lens, long = [1, least, least - 1, 1, 200, 17, 2] + [1] * 140 + [least + 1, 64, 3], (1, 4, 147)    # (more than 128 rows)
+    T, starts = sum(lens), np.cumsum([0] + lens)
+    ins = [torch.randn(T, G * N, generator=g), torch.randn(T, G * N, generator=g), torch.randn(T, H * V, generator=g),
+           torch.rand(H, generator=g) if fixed else torch.rand(T, H, generator=g), torch.rand(T, H, generator=g)]
+    slots = torch.randperm(len(lens) + 2, generator=g)[:len(lens)].tolist()
+    state = torch.randn(len(lens) + 2, H * V * N, generator=g)
+    i32 = dict(dtype=torch.int32, device=DEV)
+
+    def run(rows, ahead=True):
+        at = torch.cat([torch.arange(starts[r], starts[r + 1]) for r in rows])
+        b, c, x, a, w = (t.to(DEV) if t.dim() == 1 else t[at].to(DEV) for t in ins)
+        n, sd = [lens[r] for r in rows], state.to(DEV)
+        y = o.linear_scan(b, c, x, a, w, None, sd, 0, torch.tensor(np.cumsum([0] + n), **i32), torch.tensor([slots[r] for r in rows], **i32),
+                          len(rows), H, G, N, V, longest_row=max(n), row_lens=n if ahead else None)
+        return dict(zip(rows, y.cpu().split(n))), sd.cpu()
+
+    every, states = run(range(len(lens)), ahead=False)
+    known, known_states = run(range(len(lens)))
+    assert all(torch.equal(every[r], known[r]) for r in every) and torch.equal(states, known_states)
+    short, short_states = run([r for r in range(len(lens)) if r not in long])
+    lone, lone_states = run(long)
+    for r, alone, alone_states in [(r, short, short_states) for r in short] + [(r, lone, lone_states) for r in long]:
+        assert torch.equal(every[r], alone[r]) and torch.equal(states[slots[r]], alone_states[slots[r]]), r
+    spare = [s for s in range(len(lens) + 2) if s not in slots]
+    assert torch.equal(states[spare], state[spare])
+
+
 def test_linear_scan_with_one_decay_per_head_and_no_step_sizes():
     o = ops()
     g = torch.Generator().manual_seed(1)
