@@ -57,6 +57,7 @@ struct DeltaChunkParams {
     float* qs;                      // [T, H, dim]: q exp(b)
     float* kend;                    // [T, H, dim]: k exp(b_n - b)
     float* decay;                   // [chunk numbers, H, dim]: exp(b_n)
+    int min_row;                    // rows of fewer tokens are left alone
 };
 
 template <typename T> struct LinearChunkParams {
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(CC_THREADS) channel_chunk_solve_kernel(const D
     pdl_trigger();
     const int h = blockIdx.y, kh = h / (p.H / p.KH), tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, 0, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, p.min_row, r, first, n)) return;
     load_rows<DP>(sB, p.log_g + ((int64_t)first * p.H + h) * p.dim, (int64_t)p.H * p.dim, n, p.dim);
     asm volatile("cp.async.commit_group;\n" ::);
     load_rows<DP>(sK, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
@@ -384,10 +385,12 @@ __global__ void __launch_bounds__(256) delta_chunk_state_kernel(const DeltaChunk
     float* part = sU + DC * LV;                         // [PARTS][LV] slices of the sums
     pdl_wait();
     pdl_trigger();
-    const int h = blockIdx.y, r = blockIdx.z, kh = h / (p.H / p.KH), v0 = blockIdx.x * DC_VT, tid = threadIdx.x;
+    const int h = blockIdx.y, kh = h / (p.H / p.KH), v0 = blockIdx.x * DC_VT, tid = threadIdx.x;
+    int r, id0;
+    if (!row_of_block(blockIdx.z, p.row_start, p.rows, p.min_row, r, id0)) return;
     const int lane = tid & 31, warp = tid >> 5, rg = lane >> 2, cg = lane & 3;
     const int start = p.row_start[r], L = p.row_start[r + 1] - start;
-    const int chunks = (L + DC - 1) / DC, id0 = start / DC + r;
+    const int chunks = (L + DC - 1) / DC;
     const int c4 = v0 + 4 * (tid & 3);                  // this thread's four columns when sums are collected
     const bool on = c4 < p.vdim;
     float* slot = p.state + (int64_t)p.row_slot[r] * p.slot_stride + (int64_t)h * p.dim * p.vdim;
@@ -534,7 +537,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_out_kernel(const DeltaChun
     pdl_trigger();
     const int h = blockIdx.y, kh = h / (p.H / p.KH), v0 = blockIdx.z * DC_OT, tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, 0, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, p.min_row, r, first, n)) return;
     load_rows<DP>(sQ, p.q + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
     const float* S = p.s0 + ((int64_t)blockIdx.x * p.H + h) * p.dim * p.vdim + v0;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -637,7 +640,7 @@ template <int DP> static int launch_delta_chunk(const DeltaChunkParams& p, int i
     return acorn_launch(delta_chunk_out_kernel<DP, false>, dim3(ids, p.H, (p.vdim + DC_OT - 1) / DC_OT), dim3(256), out, stream, p);
 }
 
-template <int DP> static int launch_channel_chunk(const DeltaChunkParams& p, int ids, cudaStream_t stream) {
+template <int DP> static int launch_channel_chunk(const DeltaChunkParams& p, int ids, int walks, cudaStream_t stream) {
     constexpr int LD = DP + DC_PAD, LV = DC_VT + DC_PAD, PARTS = 8 * DC > 4 * DP ? 8 * DC : 4 * DP;
     const size_t solve = (size_t)((4 * DC + 64) * LD + DC * (DC + DC_PAD)) * sizeof(float);
     const size_t walk = (size_t)(4 * DC * LD + (DP + DC + PARTS) * LV) * sizeof(float);
@@ -652,7 +655,7 @@ template <int DP> static int launch_channel_chunk(const DeltaChunkParams& p, int
     }
     int rc = acorn_launch(channel_chunk_solve_kernel<DP>, dim3(ids, p.H), dim3(CC_THREADS), solve, stream, p);
     if (rc) return rc;
-    rc = acorn_launch(delta_chunk_state_kernel<DP, true>, dim3((p.vdim + DC_VT - 1) / DC_VT, p.H, p.rows), dim3(256), walk, stream, p);
+    rc = acorn_launch(delta_chunk_state_kernel<DP, true>, dim3((p.vdim + DC_VT - 1) / DC_VT, p.H, walks), dim3(256), walk, stream, p);
     if (rc) return rc;
     DeltaChunkParams o = p;                             // the scaled queries are per head
     o.q = p.qs;
@@ -836,14 +839,15 @@ __global__ void __launch_bounds__(256) linear_chunk_local_kernel(const LinearChu
 // A thread four value columns of a key channel's state, along a row's chunks; the chunks' sums are fetched a few ahead.
 __global__ void linear_chunk_fold_kernel(float* __restrict__ state, int64_t slot_stride, const int* __restrict__ row_start,
                                          const int* __restrict__ row_slot, float* __restrict__ s0, const float* __restrict__ decay,
-                                         int H, int dim, int vdim) {
+                                         int H, int dim, int vdim, int rows, int min_row) {
     pdl_wait();
     pdl_trigger();
-    const int r = blockIdx.z, h = blockIdx.y;
+    const int h = blockIdx.y;
     const int per = dim * (vdim / 4), e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= per) return;
+    int r, id0;
+    if (!row_of_block(blockIdx.z, row_start, rows, min_row, r, id0) || e >= per) return;
     const int d = e / (vdim / 4);
-    const int start = row_start[r], chunks = (row_start[r + 1] - start + DC - 1) / DC, id0 = start / DC + r;
+    const int chunks = (row_start[r + 1] - row_start[r] + DC - 1) / DC;
     float4* slot = reinterpret_cast<float4*>(state + (int64_t)row_slot[r] * slot_stride + (int64_t)h * dim * vdim) + e;
     float4* E = reinterpret_cast<float4*>(s0 + ((int64_t)id0 * H + h) * dim * vdim) + e;
     const float* a = decay + ((int64_t)id0 * H + h) * dim + d;
@@ -883,7 +887,7 @@ template <typename T, int DP> static int launch_linear_chunk(const LinearChunkPa
     int rc = acorn_launch(linear_chunk_local_kernel<T, DP>, dim3(ids, p.H), dim3(256), local, stream, p);
     if (rc) return rc;
     rc = acorn_launch(linear_chunk_fold_kernel, dim3((p.dim * (p.vdim / 4) + 255) / 256, p.H, p.rows), dim3(256), 0, stream, o.state,
-                      o.slot_stride, o.row_start, o.row_slot, p.s0, (const float*)p.decay, p.H, p.dim, p.vdim);
+                      o.slot_stride, o.row_start, o.row_slot, p.s0, (const float*)p.decay, p.H, p.dim, p.vdim, p.rows, 0);
     if (rc) return rc;
     return acorn_launch(delta_chunk_out_kernel<DP, true>, dim3(ids, p.H, (p.vdim + DC_OT - 1) / DC_OT), dim3(256), out, stream, o);
 }
@@ -898,7 +902,7 @@ extern "C" int acorn_linear_chunk(const void* in, int64_t ld, const float* z, in
         return ACORN_ERR_UNSUPPORTED;
     const DeltaChunkParams o = {q, nullptr, nullptr, nullptr, nullptr, state, slot_stride, row_start, row_slot, nullptr, v, pp, nullptr, s0, out,
                                 rows, H, H, dim, vdim};
-    const int ids = tokens / DC + rows;
+    const int ids = chunk_ids(tokens, rows, 0);
     ACORN_DISPATCH_DTYPE(dtype, T, {
         LinearChunkParams<T> p;
         p.in = (const T*)in; p.ld = ld; p.z = z; p.ldz = ldz; p.bias = bias; p.inv_tau = inv_tau; p.q_scale = (float)(1.0 / sqrt((double)dim));
@@ -932,7 +936,7 @@ __global__ void __launch_bounds__(256) mix_chunk_local_kernel(const DeltaChunkPa
     pdl_trigger();
     const int h = blockIdx.y, kh = h / (p.H / p.KH), tid = threadIdx.x;
     int r, first, n;
-    if (!chunk_of(blockIdx.x, p.row_start, p.rows, 0, r, first, n)) return;
+    if (!chunk_of(blockIdx.x, p.row_start, p.rows, p.min_row, r, first, n)) return;
     load_rows<DP>(sB, p.log_g + ((int64_t)first * p.H + h) * p.dim, (int64_t)p.H * p.dim, n, p.dim);
     asm volatile("cp.async.commit_group;\n" ::);
     load_rows<DP>(sK, p.k + ((int64_t)first * p.KH + kh) * p.dim, (int64_t)p.KH * p.dim, n, p.dim);
@@ -1047,7 +1051,7 @@ __global__ void __launch_bounds__(256) mix_chunk_local_kernel(const DeltaChunkPa
     }
 }
 
-template <int DP> static int launch_mix_chunk(const DeltaChunkParams& p, const float* bonus, int ids, cudaStream_t stream) {
+template <int DP> static int launch_mix_chunk(const DeltaChunkParams& p, const float* bonus, int ids, int walks, cudaStream_t stream) {
     constexpr int LD = DP + DC_PAD, LO = DC_OT + DC_PAD;
     const size_t local = (size_t)((4 * DC + 48) * LD + DC * LO) * sizeof(float);
     const size_t out = (size_t)(DC * LD + DP * LO + DC * LO + DC * (DC + DC_PAD)) * sizeof(float);
@@ -1060,8 +1064,8 @@ template <int DP> static int launch_mix_chunk(const DeltaChunkParams& p, const f
     }
     int rc = acorn_launch(mix_chunk_local_kernel<DP>, dim3(ids, p.H), dim3(256), local, stream, p, bonus);
     if (rc) return rc;
-    rc = acorn_launch(linear_chunk_fold_kernel, dim3((p.dim * (p.vdim / 4) + 255) / 256, p.H, p.rows), dim3(256), 0, stream, p.state,
-                      p.slot_stride, p.row_start, p.row_slot, p.s0, (const float*)p.decay, p.H, p.dim, p.vdim);
+    rc = acorn_launch(linear_chunk_fold_kernel, dim3((p.dim * (p.vdim / 4) + 255) / 256, p.H, walks), dim3(256), 0, stream, p.state,
+                      p.slot_stride, p.row_start, p.row_slot, p.s0, (const float*)p.decay, p.H, p.dim, p.vdim, p.rows, p.min_row);
     if (rc) return rc;
     DeltaChunkParams o = p;                             // the scaled queries are per head
     o.q = p.qs;
@@ -1072,7 +1076,7 @@ template <int DP> static int launch_mix_chunk(const DeltaChunkParams& p, const f
 extern "C" int acorn_delta_chunk_supported(int dim, int vdim) { return dim >= 4 && dim <= 128 && dim % 4 == 0 && vdim >= 4 && vdim % 4 == 0; }
 
 // chunk numbers of a step (what s0 must have room for)
-extern "C" int acorn_delta_chunk_ids(int tokens, int rows) { return tokens / DC + rows; }
+extern "C" int acorn_delta_chunk_ids(int tokens, int rows, int min_row) { return chunk_ids(tokens, rows, min_row); }
 
 extern "C" int acorn_delta_chunk(const float* q, const float* k, const float* v, const float* beta, const float* log_g, float* state,
                                  int64_t slot_stride, const int* row_start, const int* row_slot, float* w, float* u, float* pp, float* b,
@@ -1081,42 +1085,45 @@ extern "C" int acorn_delta_chunk(const float* q, const float* k, const float* v,
     const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)w | (uintptr_t)u | (uintptr_t)pp | (uintptr_t)s0 | (uintptr_t)out;
     if (!acorn_delta_chunk_supported(dim, vdim) || KH < 1 || H < 1 || H % KH || H > 65535 || rows > 65535 || (all & 15)) return ACORN_ERR_UNSUPPORTED;
     DeltaChunkParams p = {q, k, v, beta, log_g, state, slot_stride, row_start, row_slot, w, u, pp, b, s0, out, rows, H, KH, dim, vdim};
-    const int ids = acorn_delta_chunk_ids(tokens, rows);
+    const int ids = chunk_ids(tokens, rows, 0);
     if (dim <= 32) return launch_delta_chunk<32>(p, ids, stream);
     if (dim <= 64) return launch_delta_chunk<64>(p, ids, stream);
     return launch_delta_chunk<128>(p, ids, stream);
 }
 
-// log2_g [T, H, dim]: the decays' logarithms to base 2, none positive
+// log2_g [T, H, dim]: the decays' logarithms to base 2, none positive; the rows of min_row tokens or more
 extern "C" int acorn_channel_chunk(const float* q, const float* k, const float* v, const float* beta, const float* log2_g, float* state,
                                    int64_t slot_stride, const int* row_start, const int* row_slot, float* w, float* u, float* pp,
                                    float* qs, float* kend, float* decay, float* s0, float* out, int tokens, int rows, int H, int KH,
-                                   int dim, int vdim, cudaStream_t stream) {
+                                   int dim, int vdim, int min_row, cudaStream_t stream) {
     if (tokens <= 0 || rows <= 0) return 0;
     const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)log2_g | (uintptr_t)w | (uintptr_t)u | (uintptr_t)pp | (uintptr_t)qs |
                           (uintptr_t)kend | (uintptr_t)decay | (uintptr_t)s0 | (uintptr_t)out;
     if (!acorn_delta_chunk_supported(dim, vdim) || KH < 1 || H < 1 || H % KH || H > 65535 || rows > 65535 || (all & 15)) return ACORN_ERR_UNSUPPORTED;
     DeltaChunkParams p = {q, k, v, beta, log2_g, state, slot_stride, row_start, row_slot, w, u, pp, nullptr, s0, out, rows, H, KH, dim, vdim,
-                          qs, kend, decay};
-    const int ids = acorn_delta_chunk_ids(tokens, rows);
-    if (dim <= 32) return launch_channel_chunk<32>(p, ids, stream);
-    if (dim <= 64) return launch_channel_chunk<64>(p, ids, stream);
-    return launch_channel_chunk<128>(p, ids, stream);
+                          qs, kend, decay, min_row};
+    const int ids = chunk_ids(tokens, rows, min_row), walks = chunk_rows(tokens, rows, min_row);
+    if (walks == 0) return 0;
+    if (dim <= 32) return launch_channel_chunk<32>(p, ids, walks, stream);
+    if (dim <= 64) return launch_channel_chunk<64>(p, ids, walks, stream);
+    return launch_channel_chunk<128>(p, ids, walks, stream);
 }
 
 // v as it is; bonus [H, dim]; log2_g as above
 extern "C" int acorn_mix_chunk(const float* q, const float* k, const float* v, const float* bonus, const float* log2_g, float* state,
                                int64_t slot_stride, const int* row_start, const int* row_slot, float* pp, float* qs, float* decay,
-                               float* s0, float* out, int tokens, int rows, int H, int KH, int dim, int vdim, cudaStream_t stream) {
+                               float* s0, float* out, int tokens, int rows, int H, int KH, int dim, int vdim, int min_row,
+                               cudaStream_t stream) {
     if (tokens <= 0 || rows <= 0) return 0;
     const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)log2_g | (uintptr_t)pp | (uintptr_t)qs | (uintptr_t)decay |
                           (uintptr_t)s0 | (uintptr_t)out | (uintptr_t)state;
     if (!acorn_delta_chunk_supported(dim, vdim) || KH < 1 || H < 1 || H % KH || H > 65535 || rows > 65535 || (all & 15) || slot_stride % 4)
         return ACORN_ERR_UNSUPPORTED;
     DeltaChunkParams p = {q, k, v, nullptr, log2_g, state, slot_stride, row_start, row_slot, nullptr, const_cast<float*>(v), pp, nullptr, s0, out,
-                          rows, H, KH, dim, vdim, qs, nullptr, decay};
-    const int ids = acorn_delta_chunk_ids(tokens, rows);
-    if (dim <= 32) return launch_mix_chunk<32>(p, bonus, ids, stream);
-    if (dim <= 64) return launch_mix_chunk<64>(p, bonus, ids, stream);
-    return launch_mix_chunk<128>(p, bonus, ids, stream);
+                          rows, H, KH, dim, vdim, qs, nullptr, decay, min_row};
+    const int ids = chunk_ids(tokens, rows, min_row), walks = chunk_rows(tokens, rows, min_row);
+    if (walks == 0) return 0;
+    if (dim <= 32) return launch_mix_chunk<32>(p, bonus, ids, walks, stream);
+    if (dim <= 64) return launch_mix_chunk<64>(p, bonus, ids, walks, stream);
+    return launch_mix_chunk<128>(p, bonus, ids, walks, stream);
 }

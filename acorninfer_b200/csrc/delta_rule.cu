@@ -9,7 +9,8 @@
 //   delta_prep          per token: the short causal convolution over time of the q, k, v channels
 //                       (inputs before the step's first token come from the request's state), silu,
 //                       unit norms, beta = sigmoid(.), g = exp(-exp(A_log) softplus(. + dt_bias)),
-//                       (or its logarithm to base 2), the output gate sigmoid(.); float32 outputs
+//                       (or its logarithm to base 2, for the tokens of rows of `logs` tokens or more), the output gate
+//                       sigmoid(.); float32 outputs
 //   conv_state_update   per row: the last taps - 1 convolution inputs into the request's state
 //   delta_rule          the recurrence over a row's tokens, state in registers
 //   delta_out           per token and head: o / rms(o) * w * gate
@@ -70,9 +71,10 @@ __global__ void delta_prep_kernel(const T* __restrict__ main_, int64_t ld, const
         vv[(int64_t)t * H * vdim + c] = act[2 * KH * dim + c];
         gate[(int64_t)t * H * vdim + c] = sigmoidf_(up[(int64_t)t * ld_up + H * dim + c]);
     }
+    const bool as_log = logs > 0 && row_start[r + 1] - row_start[r] >= logs;
     for (int c = threadIdx.x; c < H * dim; c += blockDim.x) {
         const float lg = -expf(A_log[c / dim]) * softplusf_(up[(int64_t)t * ld_up + c] + dt_bias[c]);
-        g[(int64_t)t * H * dim + c] = logs ? lg * 1.4426950408889634f : expf(lg);
+        g[(int64_t)t * H * dim + c] = as_log ? lg * 1.4426950408889634f : expf(lg);
     }
     for (int h = threadIdx.x; h < H; h += blockDim.x) beta[(int64_t)t * H + h] = sigmoidf_(to_float(main_[(int64_t)t * ld + C + h]));
 }
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(256) delta_prep_vec_kernel(const T* __restrict
     if (!on) return;
     const bool is_gate = h - conv_heads >= H;
     const int hh = (h - conv_heads) % H, col = hh * width + 4 * l;
-    const float A = is_gate ? 0.f : -expf(A_log[hh]) * (logs ? 1.4426950408889634f : 1.f);
+    const float A = is_gate ? 0.f : -expf(A_log[hh]);
     const float4 bias = is_gate ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(dt_bias + col);
     float4 z[TPT];
 #pragma unroll
@@ -165,7 +167,13 @@ __global__ void __launch_bounds__(256) delta_prep_vec_kernel(const T* __restrict
         } else {
             o = make_float4(A * softplusf_(z[q].x + bias.x), A * softplusf_(z[q].y + bias.y), A * softplusf_(z[q].z + bias.z),
                             A * softplusf_(z[q].w + bias.w));
-            if (!logs) o = make_float4(expf(o.x), expf(o.y), expf(o.z), expf(o.w));
+            bool as_log = logs == 1;                        // (every row has a token)
+            if (logs > 1) {
+                const int r = token_row[t0 + q];
+                as_log = row_start[r + 1] - row_start[r] >= logs;
+            }
+            const float f = 1.4426950408889634f;
+            o = as_log ? make_float4(o.x * f, o.y * f, o.z * f, o.w * f) : make_float4(expf(o.x), expf(o.y), expf(o.z), expf(o.w));
         }
         *reinterpret_cast<float4*>((is_gate ? gate + (int64_t)(t0 + q) * H * vdim : g + (int64_t)(t0 + q) * H * dim) + col) = o;
     }
@@ -304,6 +312,7 @@ struct DeltaSegments {
     int nseg, seg_len;        // segments a row, tokens a segment
     float* seg_state;         // [rows * nseg, H, dim, vdim]
     float* seg_decay;         // [rows * nseg, H, dim]
+    int max_row;              // > 0: longer rows are left alone (pass 0)
 };
 // CPT: columns a thread holds (an entry read from shared memory then serves them all); NT: threads a block.
 #define DELTA_FORM_RULE 0
@@ -330,6 +339,7 @@ __global__ void __launch_bounds__(NT) delta_rule_kernel(
     pdl_trigger();
     const int r = sg.pass ? blockIdx.x / sg.nseg : blockIdx.x, seg = sg.pass ? blockIdx.x % sg.nseg : 0;
     const int h = blockIdx.y, c0 = blockIdx.z * DELTA_COLS;
+    if (sg.max_row > 0 && row_start[r + 1] - row_start[r] > sg.max_row) return;
     const int kh = h / (H / KH);
     const int slice = threadIdx.x & (DELTA_SLICES - 1), col = threadIdx.x / DELTA_SLICES;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -482,12 +492,12 @@ __global__ void delta_fold_kernel(float* __restrict__ state, int64_t slot_stride
 extern "C" int acorn_delta_rule(const float* qn, const float* kn, const float* vv, const float* beta, const float* g,
                                 float* state, int64_t slot_stride, const int* row_start, const int* row_slot, float* out,
                                 int rows, int H, int KH, int dim, int vdim, const float* bonus, int form, int g_heads, int pass, int nseg,
-                                int seg_len, float* seg_state, float* seg_decay, cudaStream_t stream) {
+                                int seg_len, int max_row, float* seg_state, float* seg_decay, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (H > 65535 || vdim > 65535 || dim > 256 || H % KH) return ACORN_ERR_UNSUPPORTED;
     if (form < 0 || form > 2 || (form == DELTA_FORM_RULE && beta == nullptr) || (form == DELTA_FORM_PRE && bonus == nullptr))
         return ACORN_ERR_UNSUPPORTED;
-    DeltaSegments sg = {pass, nseg, seg_len, seg_state, seg_decay};
+    DeltaSegments sg = {pass, nseg, seg_len, seg_state, seg_decay, pass ? 0 : max_row};
     if (pass != 0 && (form == DELTA_FORM_RULE || pass < 0 || pass > 2 || nseg < 1 || seg_len < 1 || seg_state == nullptr ||
                       seg_decay == nullptr || (int64_t)rows * nseg > 0x7fffffff))
         return ACORN_ERR_UNSUPPORTED;                   // segments fold only in the forms without the delta correction

@@ -95,12 +95,14 @@ extern "C" int acorn_token_shift(const void* h, int64_t ld, const float* mu, flo
 }
 
 // r, k, v, g: [T, C] of the activation type (row strides in elements); z: [T, C] float32, the decay's
-// pre-activation without its constant part w0 [C].
+// pre-activation without its constant part w0 [C].  logs > 0: the decays' logarithms to base 2 for the tokens of rows of
+// `logs` tokens or more (token_row, row_start: read for logs > 1).
 template <typename T>
 __global__ void wkv_prep_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v,
                                 const T* __restrict__ g, int64_t ld, const float* __restrict__ z, int64_t ld_z,
                                 const float* __restrict__ w0, float* __restrict__ r32, float* __restrict__ k32,
-                                float* __restrict__ v32, float* __restrict__ decay, float* __restrict__ gate, int C, int logs) {
+                                float* __restrict__ v32, float* __restrict__ decay, float* __restrict__ gate, int C, int logs,
+                                const int* __restrict__ token_row, const int* __restrict__ row_start) {
     pdl_wait();
     pdl_trigger();
     const int64_t t = blockIdx.x;
@@ -113,17 +115,21 @@ __global__ void wkv_prep_kernel(const T* __restrict__ r, const T* __restrict__ k
     const float gv = to_float(g[in]);
     gate[o] = gv / (1.f + expf(-gv));
     const float lg = -expf(z[t * ld_z + c] + w0[c]);
-    decay[o] = logs ? lg * 1.4426950408889634f : expf(lg);
+    bool as_log = logs == 1;                                // (every row has a token)
+    if (logs > 1) as_log = row_start[token_row[t] + 1] - row_start[token_row[t]] >= logs;
+    decay[o] = as_log ? lg * 1.4426950408889634f : expf(lg);
 }
 
 extern "C" int acorn_wkv_prep(const void* r, const void* k, const void* v, const void* g, int64_t ld, const float* z,
                               int64_t ld_z, const float* w0, float* r32, float* k32, float* v32, float* decay,
-                              float* gate, int tokens, int C, int dtype, int logs, cudaStream_t stream) {
+                              float* gate, int tokens, int C, int dtype, int logs, const int* token_row, const int* row_start,
+                              cudaStream_t stream) {
+    if (logs > 1 && (token_row == nullptr || row_start == nullptr)) return ACORN_ERR_UNSUPPORTED;
     if (tokens <= 0) return 0;
     if ((C + 127) / 128 > 65535) return ACORN_ERR_UNSUPPORTED;
     dim3 grid(tokens, (C + 127) / 128);
     ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(wkv_prep_kernel<T>, grid, dim3(128), 0, stream, (const T*)r,
                                                        (const T*)k, (const T*)v, (const T*)g, ld, z, ld_z, w0, r32, k32,
-                                                       v32, decay, gate, C, logs));
+                                                       v32, decay, gate, C, logs, token_row, row_start));
     return ACORN_ERR_UNSUPPORTED;
 }

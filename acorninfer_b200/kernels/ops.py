@@ -135,9 +135,9 @@ class _Sigs:
     acorn_token_shift = [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
                          c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_wkv_prep = [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
-                      c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
+                      c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]
     acorn_mix_chunk = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
-                       c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+                       c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_latent_prep = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
                          c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
                          c_int, c_void_p, c_int64, c_void_p]
@@ -155,11 +155,11 @@ class _Sigs:
                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                         c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_channel_chunk = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
-                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_conv_state_update = [c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int, c_int, c_int,
                                c_int, c_int, c_void_p, c_void_p]
     acorn_delta_rule = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
-                        c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                        c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                         c_void_p, c_void_p]
     acorn_delta_fold = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_delta_out = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p]
@@ -196,7 +196,7 @@ class _Sigs:
     acorn_delta_chunk_supported = [c_int, c_int]
     acorn_linear_chunk = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_float, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
-    acorn_delta_chunk_ids = [c_int, c_int]
+    acorn_delta_chunk_ids = [c_int, c_int, c_int]
     acorn_linear_heads_prep = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_int, c_int, c_int, c_int, c_int, c_void_p]
     acorn_recurrent_step = [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int64,
@@ -1598,10 +1598,11 @@ def head_linear(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor) -> torch.Tens
 
 def delta_prep(main: torch.Tensor, up32: torch.Tensor, conv_w32: torch.Tensor, state: torch.Tensor, conv_off: int,
                a_log32: torch.Tensor, dt_bias32: torch.Tensor, token_row: torch.Tensor, row_start: torch.Tensor,
-               row_slot: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, taps: int, log2_decays: bool = False):
+               row_slot: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, taps: int, log2_decays: int = 0):
     """Convolution + silu of the q, k, v channels, unit norms, write strength, decays and output gate of
     every token: returns float32 (q [T, KH, dim], k [T, KH, dim], v [T, H, vdim], beta [T, H],
-    g [T, H, dim], gate [T, H, vdim]).  ``log2_decays``: g holds the decays' logarithms to base 2."""
+    g [T, H, dim], gate [T, H, vdim]).  ``log2_decays`` n > 0: g holds the decays' logarithms to base 2 for the tokens of rows
+    of n tokens or more (1: all)."""
     _check(main, "main", None, 2)
     _check(up32, "up", torch.float32, 2)
     _check(state, "state", torch.float32, 2)
@@ -1678,7 +1679,7 @@ def delta_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.T
         raise KernelError(f"delta_chunk: log_g {tuple(log_g.shape)}, state {tuple(state.shape)} do not fit")
     f = lambda *shape: torch.empty(shape, dtype=torch.float32, device=v.device)
     w, u, p, b, out = f(T, H, dim), f(T, H, vdim), f(T, H, 64), f(T, H), f(T, H, vdim)
-    s0 = f(lib().acorn_delta_chunk_ids(T, num_rows), H, dim, vdim)
+    s0 = f(lib().acorn_delta_chunk_ids(T, num_rows, 0), H, dim, vdim)
     _ok(lib().acorn_delta_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), log_g.data_ptr(),
                                 state.data_ptr() + 4 * int(state_off), state.stride(0), row_start.data_ptr(), row_slot.data_ptr(),
                                 w.data_ptr(), u.data_ptr(), p.data_ptr(), b.data_ptr(), s0.data_ptr(), out.data_ptr(), T, num_rows, H,
@@ -1686,16 +1687,24 @@ def delta_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.T
     return out
 
 
+# (Least tokens of a row that runs over chunks, tokens of such rows together: ``chunk_min_row``.)  Measured (B200, us, walk /
+# chunks), the delta rule of 16 heads of 128 x 128: 1 row of 64 tokens 30 / 61, of 160 69 / 69, of 256 109 / 74; 4 rows of 64 80 / 78,
+# of 128 151 / 94; time mixing of 32 heads of 64 x 64: 1 row of 64 tokens 22 / 29, of 96 32 / 25; 4 rows of 64 58 / 39.
+CHANNEL_CHUNK_ROWS = ((64, 256), (160, 160))
+MIX_CHUNK_ROWS = ((64, 128), (96, 96))
+
+
 def channel_chunk_ok(longest_row: int, tokens: int, num_rows: int, heads: int, dim: int, vdim: int) -> bool:
     """Whether the delta rule with decays per key channel runs over chunks (``channel_chunk``) in a step of these rows."""
     return (longest_row >= DELTA_CHUNK_MIN_ROW and bool(lib().acorn_delta_chunk_supported(dim, vdim)) and heads <= 65535
-            and num_rows <= 65535 and 4 * lib().acorn_delta_chunk_ids(tokens, num_rows) * heads * dim * vdim <= DELTA_CHUNK_SCRATCH_BYTES)
+            and num_rows <= 65535 and 4 * lib().acorn_delta_chunk_ids(tokens, num_rows, 0) * heads * dim * vdim <= DELTA_CHUNK_SCRATCH_BYTES)
 
 
 def channel_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, log2_g: torch.Tensor, state: torch.Tensor,
-                  row_start: torch.Tensor, row_slot: torch.Tensor, num_rows: int, state_off: int = 0) -> torch.Tensor:
+                  row_start: torch.Tensor, row_slot: torch.Tensor, num_rows: int, state_off: int = 0, min_row: int = 0) -> torch.Tensor:
     """The gated delta rule with a decay per key channel (``log2_g`` [T, H, dim], logarithms to base 2) over chunks of 64
-    tokens, as ``delta_chunk`` does with one per head.  Other arguments and result as for ``delta_rule``."""
+    tokens, as ``delta_chunk`` does with one per head.  Other arguments and result as for ``delta_rule``.  Rows of fewer than
+    ``min_row`` tokens are left alone, their places in the result unset."""
     T, H, vdim = v.shape
     KH, dim = q.shape[1], q.shape[2]
     for t, n in ((q, "q"), (k, "k"), (v, "v"), (beta, "beta"), (log2_g, "log2_g")):
@@ -1704,21 +1713,21 @@ def channel_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch
     if log2_g.shape != (T, H, dim) or beta.shape != (T, H) or state.shape[1] < state_off + H * dim * vdim:
         raise KernelError(f"channel_chunk: log2_g {tuple(log2_g.shape)}, state {tuple(state.shape)} do not fit")
     f = lambda *shape: torch.empty(shape, dtype=torch.float32, device=v.device)
-    ids = lib().acorn_delta_chunk_ids(T, num_rows)
+    ids = lib().acorn_delta_chunk_ids(T, num_rows, int(min_row))
     w, u, p, qs, kend, out = f(T, H, dim), f(T, H, vdim), f(T, H, 64), f(T, H, dim), f(T, H, dim), f(T, H, vdim)
     s0, decay = f(ids, H, dim, vdim), f(ids, H, dim)
     _ok(lib().acorn_channel_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), log2_g.data_ptr(),
                                   state.data_ptr() + 4 * int(state_off), state.stride(0), row_start.data_ptr(), row_slot.data_ptr(),
                                   w.data_ptr(), u.data_ptr(), p.data_ptr(), qs.data_ptr(), kend.data_ptr(), decay.data_ptr(),
-                                  s0.data_ptr(), out.data_ptr(), T, num_rows, H, KH, dim, vdim, _stream()), "delta_rule")
+                                  s0.data_ptr(), out.data_ptr(), T, num_rows, H, KH, dim, vdim, int(min_row), _stream()), "delta_rule")
     return out
 
 
 def mix_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bonus32: torch.Tensor, log2_g: torch.Tensor, state: torch.Tensor,
-              row_start: torch.Tensor, row_slot: torch.Tensor, num_rows: int, state_off: int = 0) -> torch.Tensor:
+              row_start: torch.Tensor, row_slot: torch.Tensor, num_rows: int, state_off: int = 0, min_row: int = 0) -> torch.Tensor:
     """The form of ``delta_rule`` that reads the state first (``bonus32``) over chunks of 64 tokens; ``log2_g`` [T, H, dim]:
     logarithms to base 2 of the decays.  Taken where ``channel_chunk_ok`` says so and the slots are aligned
-    (``state_off`` and the slots' stride multiples of four)."""
+    (``state_off`` and the slots' stride multiples of four).  ``min_row`` as for ``channel_chunk``."""
     T, H, vdim = v.shape
     KH, dim = q.shape[1], q.shape[2]
     for t, n in ((q, "q"), (k, "k"), (v, "v"), (log2_g, "log2_g")):
@@ -1727,7 +1736,7 @@ def mix_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bonus32: torch.
     _check(state, "state", torch.float32, 2)
     if log2_g.shape != (T, H, dim) or bonus32.shape != (H, dim) or state.shape[1] < state_off + H * dim * vdim:
         raise KernelError(f"mix_chunk: log2_g {tuple(log2_g.shape)}, bonus {tuple(bonus32.shape)}, state {tuple(state.shape)} do not fit")
-    ids = lib().acorn_delta_chunk_ids(T, num_rows)
+    ids = lib().acorn_delta_chunk_ids(T, num_rows, int(min_row))
     out = torch.empty((T, H, vdim), dtype=torch.float32, device=v.device)
     # the kernels' own arrays, one behind the other: p [T, H, 64], q at the chunk's start [T, H, dim], the chunks' decays and states
     sizes = (T * H * 64, T * H * dim, ids * H * dim, ids * H * dim * vdim)
@@ -1739,7 +1748,7 @@ def mix_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bonus32: torch.
     _ok(lib().acorn_mix_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), bonus32.data_ptr(), log2_g.data_ptr(),
                               state.data_ptr() + 4 * int(state_off), state.stride(0), row_start.data_ptr(), row_slot.data_ptr(),
                               p, qs, decay, s0, out.data_ptr(), T, num_rows, H, KH, dim,
-                              vdim, _stream()), "delta_rule")
+                              vdim, int(min_row), _stream()), "delta_rule")
     return out
 
 
@@ -1749,7 +1758,7 @@ def linear_chunk_ok(longest_row: int, proj: torch.Tensor, z32: torch.Tensor, sta
     return (longest_row >= DELTA_CHUNK_MIN_ROW and bool(lib().acorn_delta_chunk_supported(dim, vdim)) and state_off % 4 == 0
             and state.stride(0) % 4 == 0 and proj.stride(0) % 4 == 0 and proj.data_ptr() % (8 if proj.dtype == torch.bfloat16 else 16) == 0
             and z32.stride(0) % 4 == 0
-            and 4 * lib().acorn_delta_chunk_ids(proj.shape[0], num_rows) * heads * dim * vdim <= DELTA_CHUNK_SCRATCH_BYTES)
+            and 4 * lib().acorn_delta_chunk_ids(proj.shape[0], num_rows, 0) * heads * dim * vdim <= DELTA_CHUNK_SCRATCH_BYTES)
 
 
 def linear_chunk(proj: torch.Tensor, z32: torch.Tensor, bias32: torch.Tensor, tau: float, state: torch.Tensor, row_start: torch.Tensor,
@@ -1763,7 +1772,7 @@ def linear_chunk(proj: torch.Tensor, z32: torch.Tensor, bias32: torch.Tensor, ta
     T = proj.shape[0]
     if proj.shape[1] < heads * (2 * dim + vdim) or z32.shape != (T, heads * dim) or state.shape[1] < state_off + heads * dim * vdim:
         raise KernelError(f"linear_chunk: proj {tuple(proj.shape)}, z {tuple(z32.shape)}, state {tuple(state.shape)} do not fit")
-    ids = lib().acorn_delta_chunk_ids(T, num_rows)
+    ids = lib().acorn_delta_chunk_ids(T, num_rows, 0)
     f = lambda *shape: torch.empty(shape, dtype=torch.float32, device=proj.device)
     q, v, p, out = f(T, heads, dim), f(T, heads, vdim), f(T, heads, 64), f(T, heads, vdim)
     s0, decay = f(ids, heads, dim, vdim), f(ids, heads, dim)
@@ -1780,7 +1789,7 @@ DELTA_FORMS = {"rule": 0, "pre": 1, "linear": 2}
 def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor | None, g: torch.Tensor,
                state: torch.Tensor, row_start: torch.Tensor, row_slot: torch.Tensor, num_rows: int,
                bonus32: torch.Tensor | None = None, longest_row: int | None = None, state_off: int = 0,
-               log_g: torch.Tensor | None = None) -> torch.Tensor:
+               log_g: torch.Tensor | None = None, max_row: int = 0, out: torch.Tensor | None = None) -> torch.Tensor:
     """The recurrence over every row's tokens from the state in its slot (at ``state_off``, updated in place): float32
     o [T, H, vdim].  Three forms: with ``beta`` the delta rule; with ``bonus32`` (float32 [H, dim]) and no ``beta`` the form
     without the correction whose output reads the state before the token's decay and write and sees the token itself
@@ -1789,7 +1798,8 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     without correction, with ``longest_row`` (the most tokens a row of the step brings, a host value), long rows of a
     step with few rows run in segments side by side (``delta_segments``).  The delta rule with decays per head runs over
     chunks of tokens (``delta_chunk``) where a step has a row of ``DELTA_CHUNK_MIN_ROW`` tokens and the decays' logarithms
-    ``log_g`` [T, H] are given."""
+    ``log_g`` [T, H] are given.  ``max_row`` > 0: only rows of so many tokens at most, in one piece each, into their places of
+    ``out``."""
     T, H, vdim = v.shape
     KH, dim = q.shape[1], q.shape[2]
     if beta is not None and bonus32 is not None:
@@ -1805,19 +1815,23 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     per_head = g.dim() == 2
     if state.shape[1] < state_off + H * dim * vdim or g.shape != ((T, H) if per_head else (T, H, dim)) or dim > 256:
         raise KernelError(f"delta_rule: sizes do not fit (state {tuple(state.shape)}, g {tuple(g.shape)}, H={H}, dim={dim}, vdim={vdim})")
-    if (beta is not None and log_g is not None and (longest_row or 0) >= DELTA_CHUNK_MIN_ROW
+    if (beta is not None and log_g is not None and not max_row and (longest_row or 0) >= DELTA_CHUNK_MIN_ROW
             and lib().acorn_delta_chunk_supported(dim, vdim)
-            and 4 * lib().acorn_delta_chunk_ids(T, num_rows) * H * dim * vdim <= DELTA_CHUNK_SCRATCH_BYTES):
+            and 4 * lib().acorn_delta_chunk_ids(T, num_rows, 0) * H * dim * vdim <= DELTA_CHUNK_SCRATCH_BYTES):
         return delta_chunk(q, k, v, beta, log_g, state, row_start, row_slot, num_rows, state_off)
-    out = torch.empty((T, H, vdim), dtype=torch.float32, device=v.device)
-    seg_len, nseg = delta_segments(longest_row, num_rows, H, dim, vdim) if (beta is None and longest_row) else (0, 1)
+    if out is None:
+        out = torch.empty((T, H, vdim), dtype=torch.float32, device=v.device)
+    _check(out, "out", torch.float32, 3)
+    if out.shape != v.shape:
+        raise KernelError(f"delta_rule: out {tuple(out.shape)} does not fit v {tuple(v.shape)}")
+    seg_len, nseg = delta_segments(longest_row, num_rows, H, dim, vdim) if (beta is None and longest_row and not max_row) else (0, 1)
     s_ptr = state.data_ptr() + 4 * int(state_off)
 
     def run(pass_, seg_state=None, seg_decay=None):
         _ok(lib().acorn_delta_rule(q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(beta), g.data_ptr(), s_ptr,
                                    state.stride(0), row_start.data_ptr(), row_slot.data_ptr(), out.data_ptr(), num_rows, H,
                                    KH, dim, vdim, _ptr(bonus32), form, 1 if per_head else 0, pass_, nseg, max(seg_len, 1),
-                                   _ptr(seg_state), _ptr(seg_decay), _stream()), "delta_rule", f"pass {pass_}")
+                                   int(max_row), _ptr(seg_state), _ptr(seg_decay), _stream()), "delta_rule", f"pass {pass_}")
 
     if nseg == 1:
         run(0)
@@ -1965,9 +1979,10 @@ def token_shift(h: torch.Tensor, mu32: torch.Tensor, state: torch.Tensor, prev_o
 
 
 def wkv_prep(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, z32: torch.Tensor, w0_32: torch.Tensor,
-             heads: int, log2_decays: bool = False):
-    """For the recurrence, float32 [T, H, dim] each: r, k, v as they are, the decay ``exp(-exp(z + w0))`` (``log2_decays``: its
-    logarithm to base 2) and the gate ``silu(g)``.  r, k, v, g: [T, H dim] of the activation dtype with one row stride; z32 [T, H dim] float32."""
+             heads: int, log2_decays: int = 0, token_row: torch.Tensor | None = None, row_start: torch.Tensor | None = None):
+    """For the recurrence, float32 [T, H, dim] each: r, k, v as they are, the decay ``exp(-exp(z + w0))`` (``log2_decays``
+    n > 0: its logarithm to base 2 for the tokens of rows of n tokens or more, all with 1; ``token_row`` and ``row_start`` say which)
+    and the gate ``silu(g)``.  r, k, v, g: [T, H dim] of the activation dtype with one row stride; z32 [T, H dim] float32."""
     T, C = r.shape
     for t, n in ((r, "r"), (k, "k"), (v, "v"), (g, "g")):
         if not t.is_cuda or t.dtype != r.dtype or t.dim() != 2:
@@ -1981,7 +1996,8 @@ def wkv_prep(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor,
     outs = torch.empty((5, T, heads, C // heads), dtype=torch.float32, device=r.device)
     _ok(lib().acorn_wkv_prep(r.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), r.stride(0), z32.data_ptr(),
                              z32.stride(0), w0_32.data_ptr(), outs[0].data_ptr(), outs[1].data_ptr(), outs[2].data_ptr(),
-                             outs[3].data_ptr(), outs[4].data_ptr(), T, C, dtype_code(r.dtype), int(log2_decays), _stream()), "wkv_prep")
+                             outs[3].data_ptr(), outs[4].data_ptr(), T, C, dtype_code(r.dtype), int(log2_decays), _ptr(token_row), _ptr(row_start),
+                             _stream()), "wkv_prep")
     return outs[0], outs[1], outs[2], outs[3], outs[4]
 
 

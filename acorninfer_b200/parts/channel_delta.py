@@ -81,13 +81,19 @@ class ChannelDelta(Mixer):
         dt = self.ctx.dtype
         main = ops.linear(x, self.w_main, out_dtype=dt)
         up = ops.linear(ops.linear(x, self.w_low, out_dtype=dt), self.w_up, out_dtype=torch.float32)
-        # long rows over chunks of tokens, whose kernels want the decays' logarithms; other steps token by token
-        chunks = ops.channel_chunk_ok(inputs.plan.max_q_len, main.shape[0], inputs.num_rows, self.H, self.dim, self.vdim)
+        # long rows over chunks of tokens, whose kernels want the decays' logarithms; the others token by token
+        lens, min_row = inputs.plan.row_lens, 0
+        if ops.channel_chunk_ok(inputs.plan.max_q_len, main.shape[0], inputs.num_rows, self.H, self.dim, self.vdim):
+            min_row = ops.chunk_min_row(lens, ops.CHANNEL_CHUNK_ROWS)
         q, k, v, beta, g, gate = ops.delta_prep(main, up, self.conv32, cache.state, self.state_s, self.a_log32,
                                                 self.dt_bias32, inputs.token_row, inputs.row_start, inputs.row_slot,
-                                                self.H, self.KH, self.dim, self.vdim, self.taps, log2_decays=chunks)
+                                                self.H, self.KH, self.dim, self.vdim, self.taps, log2_decays=min_row)
         ops.conv_state_update(main, cache.state, self.state_s, inputs.row_start, inputs.row_slot, inputs.num_rows,
                               self.channels, self.taps)
-        o = (ops.channel_chunk if chunks else ops.delta_rule)(q, k, v, beta, g, cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)
+        o, rows = None, (cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)
+        if min_row:
+            o = ops.channel_chunk(q, k, v, beta, g, *rows, min_row=min_row)
+        if not min_row or min(lens) < min_row:
+            o = ops.delta_rule(q, k, v, beta, g, *rows, max_row=min_row - 1 if min_row else 0, out=o)
         y = ops.delta_out(o, gate, self.norm32, self.eps, dt)
         return ops.linear(y, self.w_o, out_dtype=dt)

@@ -77,14 +77,17 @@ class TimeMix(Mixer):
         r, k, v, g = ops.grouped_gemm(mixes[:4].view(4 * T, self.hidden_size), None, self.w_rkvg,
                                       inputs.extra["time_mix.blend_rows"], 4 * T).view(4, T, -1).unbind(0)
         z = ops.linear(ops.linear(mixes[4], w["w1"], out_dtype=dt, act="tanh"), w["w2"], out_dtype=torch.float32)
-        # long rows over chunks of tokens, whose kernels want the decays' logarithms; other steps token by token
-        d = r.shape[1] // self.H
-        chunks = cache.state.stride(0) % 4 == 0 and ops.channel_chunk_ok(inputs.plan.max_q_len, T, inputs.num_rows, self.H, d, d)
-        r32, k32, v32, decay, gate = ops.wkv_prep(r, k, v, g, z, self.w0_32, self.H, log2_decays=chunks)
-        if chunks:
-            o = ops.mix_chunk(r32, k32, v32, self.u32, decay, cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)
-        else:
-            o = ops.delta_rule(r32, k32, v32, None, decay, cache.state, inputs.row_start, inputs.row_slot,
-                               inputs.num_rows, bonus32=self.u32, longest_row=inputs.plan.max_q_len)
+        # long rows over chunks of tokens, whose kernels want the decays' logarithms; the others token by token
+        d, lens, min_row = r.shape[1] // self.H, inputs.plan.row_lens, 0
+        if cache.state.stride(0) % 4 == 0 and ops.channel_chunk_ok(inputs.plan.max_q_len, T, inputs.num_rows, self.H, d, d):
+            min_row = ops.chunk_min_row(lens, ops.MIX_CHUNK_ROWS)
+        r32, k32, v32, decay, gate = ops.wkv_prep(r, k, v, g, z, self.w0_32, self.H, log2_decays=min_row,
+                                                  token_row=inputs.token_row, row_start=inputs.row_start)
+        o, rows = None, (cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)
+        if min_row:
+            o = ops.mix_chunk(r32, k32, v32, self.u32, decay, *rows, min_row=min_row)
+        if not min_row or min(lens) < min_row:
+            o = ops.delta_rule(r32, k32, v32, None, decay, *rows, bonus32=self.u32, longest_row=inputs.plan.max_q_len,
+                               max_row=min_row - 1 if min_row else 0, out=o)
         y = ops.delta_out(o, gate, self.norm32, self.eps, dt)
         return ops.linear(y, w["o"], out_dtype=dt)

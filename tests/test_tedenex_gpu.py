@@ -532,6 +532,51 @@ def test_recurrences_over_chunks_leave_earlier_tokens_alone(form, dim, vdim, whe
     assert not bool(torch.isfinite(got[bad:200]).all())
 
 
+@pytest.mark.parametrize("form", ["mix", "channel"])
+@pytest.mark.parametrize("dim", [32, 100, 128])
+def test_recurrences_of_short_rows_beside_long_ones(form, dim):
+    """Rows below a chunk of 64 tokens, single tokens among them, keep every bit of their outputs and states whatever long
+    rows share their step: decays as numbers for their tokens, as logarithms for the others', each kernel its rows."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim)
+    H, least, lens, long = 2, o.DELTA_CHUNK_MIN_ROW, [1, 64, 63, 1, 200, 17, 2], (1, 4)
+    T, starts, slots = sum(lens), np.cumsum([0] + lens), [3, 0, 7, 1, 8, 2, 5]
+    state, i32 = torch.randn(9, H * dim * dim, generator=g), dict(dtype=torch.int32, device=DEV)
+    wide, z = torch.randn(T, 4 * H * dim, generator=g), torch.randn(T, 2 * H * dim, generator=g)
+    beta_in, w0, u = torch.randn(T, H, generator=g), torch.randn(H * dim, generator=g).to(DEV), torch.randn(H, dim, generator=g).to(DEV)
+    conv = torch.zeros(3 * H * dim, 2)
+    conv[:, 1] = 1
+
+    def run(rows):
+        at = torch.cat([torch.arange(starts[r], starts[r + 1]) for r in rows])
+        n, sd = [lens[r] for r in rows], state.to(DEV)
+        token_row = torch.repeat_interleave(torch.arange(len(rows)), torch.tensor(n)).int().to(DEV)
+        row_start, row_slot = torch.tensor(np.cumsum([0] + n), **i32), torch.tensor([slots[r] for r in rows], **i32)
+        logs = least if max(n) >= least else 0
+        if form == "mix":
+            r_, k, v, gate = wide[at].to(DEV).view(len(at), 4, H * dim).unbind(1)
+            q, k, v, dec, _ = o.wkv_prep(r_, k, v, gate, z[at, :H * dim].contiguous().to(DEV), w0, H, log2_decays=logs, token_row=token_row, row_start=row_start)
+            ins, kw = (q, k, v, u, dec), dict(bonus32=u)
+        else:
+            main = torch.cat([wide[at, :3 * H * dim], beta_in[at]], 1).contiguous().to(DEV)
+            memory = torch.zeros(9, 3 * H * dim, device=DEV)
+            q, k, v, beta, dec, _ = o.delta_prep(main, z[at].contiguous().to(DEV), conv.to(DEV), memory, 0, torch.zeros(H, device=DEV), w0, token_row,
+                                                 row_start, row_slot, H, H, dim, dim, 2, log2_decays=logs)
+            ins, kw = (q, k, v, beta, dec), {}
+        rows_ = (sd, row_start, row_slot, len(rows))
+        y = (o.mix_chunk if form == "mix" else o.channel_chunk)(*ins, *rows_, min_row=least) if logs else None
+        if min(n) < least:
+            y = o.delta_rule(q, k, v, None if form == "mix" else beta, dec, *rows_, max_row=least - 1 if logs else 0, out=y, **kw)
+        return dict(zip(rows, y.cpu().split(n))), sd.cpu()
+
+    every, states = run(range(7))
+    short, short_states = run([r for r in range(7) if r not in long])
+    lone, lone_states = run(long)
+    for r, alone, alone_states in [(r, short, short_states) for r in short] + [(r, lone, lone_states) for r in long]:
+        assert torch.equal(every[r], alone[r]) and torch.equal(states[slots[r]], alone_states[slots[r]]), r
+    assert torch.equal(states[[4, 6]], state[[4, 6]]) and bool(torch.isfinite(every[2]).all())
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
 @pytest.mark.parametrize("W,off,tail,single", [(20, 7, 3, False), (20, 8, 4, False), (20, 8, 4, True), (520, 4, 0, True),
                                                (22, 8, 2, True)])
