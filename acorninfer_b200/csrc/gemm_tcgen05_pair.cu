@@ -40,7 +40,7 @@
 #define G2_B_BYTES (G2_BW * G2_BK * 2)
 #define G2_STAGE_BYTES (G2_A_BYTES + G2_B_BYTES)
 #define G2_ACC_COLS 256
-#define G2_MAX_EXPERTS 512     // matrices of a product per expert (their first tiles' numbers lie in shared memory)
+#define G2_MAX_EXPERTS 512     // matrices of a launch of products per expert (their first tiles' numbers lie in shared memory)
 #define G2_SMEM ((size_t)G2_STAGES * G2_STAGE_BYTES + (2 * G2_STAGES + 4) * 8 + 16 + 1024)
 #define G2_SMEM_GROUPED (G2_SMEM + (G2_MAX_EXPERTS + 4) * 4)
 
@@ -581,23 +581,27 @@ extern "C" int acorn_grouped_gemm_pair(const void* x, int64_t ldx, const void* w
                                        int slots, int E, int N, int K, int swiglu_pairs, float glu_limit, const float* slot_scale,
                                        int pairs, cudaStream_t stream) {
     if (slots <= 0 || E <= 0 || N <= 0) return 0;
-    if (E > G2_MAX_EXPERTS || K < 1 || K % 8 || ldx % 8 || pairs < 1 || (swiglu_pairs && N % 2) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) ||
-        (int64_t)E * N > 0x7fffffff)
+    if (K < 1 || K % 8 || ldx % 8 || pairs < 1 || (swiglu_pairs && N % 2) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) ||
+        (int64_t)(E < G2_MAX_EXPERTS ? E : G2_MAX_EXPERTS) * N > 0x7fffffff)
         return ACORN_ERR_UNSUPPORTED;
     G2Params p = {};
     p.out = out; p.ldo = ldo; p.M = slots; p.N = N; p.K = K;
     p.mode = swiglu_pairs ? G2_MODE_SWIGLU_PAIRS : G2_MODE_PLAIN;
-    p.g_offsets = offsets; p.g_experts = E; p.glu_limit = glu_limit; p.row_scale = slot_scale;
+    p.glu_limit = glu_limit; p.row_scale = slot_scale;
     p.kblocks = (K + G2_BK - 1) / G2_BK;
     p.tiles_n = (N + 2 * G2_BW - 1) / (2 * G2_BW);
-    const int64_t most = ((int64_t)slots / (2 * G2_BT) + E) * p.tiles_n;      // tiles, whatever the experts' shares
-    if (most > 0x3fffffff) return ACORN_ERR_UNSUPPORTED;
     CUtensorMap mx, mw;
     int rc = make_map(&mx, x, slots, K, ldx, G2_BK, G2_BT);
-    if (rc) return rc;
-    rc = make_map(&mw, w, (int64_t)E * N, K, K, G2_BK, G2_BW);
-    if (rc) return rc;
-    return launch_pair<true>(mx, mw, p, pairs < most ? pairs : (int)most, stream);
+    for (int e0 = 0; e0 < E && rc == 0; e0 += G2_MAX_EXPERTS) {              // a launch for as many experts as it knows
+        const int experts = E - e0 < G2_MAX_EXPERTS ? E - e0 : G2_MAX_EXPERTS;
+        const int64_t most = ((int64_t)slots / (2 * G2_BT) + experts) * p.tiles_n;      // tiles, whatever the experts' shares
+        if (most > 0x3fffffff) return ACORN_ERR_UNSUPPORTED;
+        p.g_offsets = offsets + e0;
+        p.g_experts = experts;
+        rc = make_map(&mw, reinterpret_cast<const bf16*>(w) + (int64_t)e0 * N * K, (int64_t)experts * N, K, K, G2_BK, G2_BW);
+        if (rc == 0) rc = launch_pair<true>(mx, mw, p, pairs < most ? pairs : (int)most, stream);
+    }
+    return rc;
 }
 
 // What the kernel takes: bf16 operands with K contiguous, K and the row strides multiples of 8 elements,

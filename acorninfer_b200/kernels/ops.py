@@ -2637,7 +2637,7 @@ def grouped_gemm(a: torch.Tensor, a_rows: torch.Tensor | None, w: torch.Tensor, 
         raise KernelError(f"grouped_gemm: a {tuple(a.shape)} against w {tuple(w.shape)}")
     fused = swiglu_pairs and a.data_ptr() % 16 == 0 and bool(
         lib().acorn_grouped_gemm_fuses_swiglu(N, K, a.stride(0), dtype_code(a.dtype)))
-    if (a.dtype == torch.bfloat16 and slots >= GROUPED_TCGEN05_MIN_ROWS * E and E <= 512 and K % 8 == 0 and a.stride(0) % 8 == 0
+    if (a.dtype == torch.bfloat16 and slots >= GROUPED_TCGEN05_MIN_ROWS * E and K % 8 == 0 and a.stride(0) % 8 == 0
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and (N % 2 == 0 or not swiglu_pairs)):
         # many rows an expert (a prompt's step): the paired tcgen05 kernel, operand tiles by TMA, which
         # wants an expert's rows next to one another: the tokens' rows are first copied into slot order

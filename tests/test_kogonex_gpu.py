@@ -315,6 +315,27 @@ def test_grouped_products_of_many_rows(N, K, scaled, limit, tcgen05, monkeypatch
     assert o.lib().acorn_gemm_tc_pair_error() == 0
 
 
+def test_grouped_products_of_many_experts(monkeypatch):
+    """More experts than one launch of the tcgen05 kernel knows (512): uneven shares, some empty, at and around that one."""
+    o = ops()
+    E, N, K = 1100, 40, 24
+    g = torch.Generator().manual_seed(0)
+    counts = torch.randint(0, 200, (E,), generator=g)
+    counts[[0, 511, 600, E - 1]], counts[[510, 512, 513, 1023, 1024]] = 0, torch.tensor([257, 300, 1, 5, 64])
+    slots = 64 * E
+    counts[700] += max(0, slots - int(counts.sum()))
+    slots = int(counts.sum())
+    offsets = torch.cat([torch.zeros(1, dtype=torch.int64), counts.cumsum(0)]).int().to(DEV)
+    x, w = torch.randn(slots, K, generator=g).bfloat16().to(DEV), (torch.randn(E, N, K, generator=g) * K ** -0.5).bfloat16().to(DEV)
+    monkeypatch.setattr(o.lib(), "acorn_grouped_gemm", lambda *a: 10001)                # the other kernel, for fewer rows an expert
+    out = o.grouped_gemm(x, None, w, offsets, slots)
+    off = offsets.tolist()
+    for e in range(E):
+        want = x[off[e]:off[e + 1]].double() @ w[e].double().T
+        assert ((out[off[e]:off[e + 1]].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-4).all(), e      # as above
+    assert o.lib().acorn_gemm_tc_pair_error() == 0
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-4), (torch.bfloat16, 0.15)])
 @pytest.mark.parametrize("E,T,top,min_rows", [(7, 90, 2, None), (2, 300, 2, None), (12, 5, 2, None), (3, 400, 2, 10 ** 9)])
 def test_grouped_products_take_each_experts_own_rows(dtype, tol, E, T, top, min_rows, monkeypatch):
