@@ -7,20 +7,24 @@
 // memory (7 x 16 KB at d = 448) beside two blocks of keys (56 KB each), so a block's columns come and go in groups of 128:
 // a group of the block after next is brought as soon as the value product has read the group it takes the place of.
 //   warps 0-3  softmax: thread r owns row r (= TMEM lane r): reads its 64 scores, masks, exponentiates in float32 base 2
-//              against a reference maximum, writes P (bfloat16) over them; O is rescaled only when a row's maximum outgrew
-//              its reference by 2^8.  At the end: O divided by the row's sum (and the sink's term), written out.
+//              against a reference maximum, writes P over them, as two bfloat16 numbers each (the nearest, and what that
+//              lacks); O is rescaled only when a row's maximum outgrew its reference by 2^8.  At the end: O divided by the row's sum (and the sink's term), written out.
 //   warps 4, 6, 7  producers: TMA loads of the queries (once) and, through the block table, of the keys, a third of a block's
 //              boxes each (a block is 28 boxes of a page of 16 keys by 64 entries, and one warp issues a box in about 90 ns:
 //              alone it set the pace, 3.1 us a block).
 //   warp 5     MMA issuer (converged, one elected lane), blocks in pairs: P V of two blocks, then Q K of the next two.  (Q K
 //              of block j + 1 ahead of P V of block j takes the same time.)
 // Tensor memory (512 columns): S / P of even and odd blocks at 0 and 64, O at 128 ..
+// P as one bfloat16 number was 11 % further from 64 bits than the general kernel in rows that a few keys decide (1.92e-3 and
+// 1.74e-3 of the result, scores of standard deviation 3): there a row's largest weight is a power of two and not rounded, which
+// here it is not unless O is rescaled with every new maximum.
 //
-// A block costs the tensor pipe 28 steps of N = 64 (48 clocks each, the reads of shared memory bound them) and 12 of
-// N = 128 (64 clocks): 1.1 us at d = 448, dv = 384.  Measured 2.25 us, 1.6 us at d = 192, dv = 128, with 8 tiles as with 148: a
-// block's own chain, its keys' way from L2, scores, softmax, values, is what bounds it, not the rates.
-// Measured (B200, rows of 448 with 384 values, 16 heads), the general kernel and this: 2,000 tokens under a window of 1,024
-// 311 -> 74 us, 3 x 601 tokens 131 -> 44 us, 2,048 tokens behind 6,000 2,920 -> 432 us.
+// A block costs the tensor pipe 28 steps of N = 64 (48 clocks each, the reads of shared memory bound them) and 24 of
+// N = 128 (64 clocks): 1.5 us at d = 448, dv = 384.  Measured 3.0 us, 1.95 us at d = 192, dv = 128 (56 rows of 4,000 keys; with
+// P as one number 2.65 and 1.7 us): a block's own chain, its keys' way from L2, scores, softmax, values, is what bounds it, not
+// the rates.
+// Measured (B200, launched alone, rows of 448 with 384 values, 16 heads), the general kernel and this: 2,000 tokens under a
+// window of 1,024 358 -> 97 us, 3 x 601 tokens 162 -> 54 us, 2,000 tokens behind 4,000 2,164 -> 428 us.
 // A tile in which a value row that only some of its queries read holds an infinity or no number is computed again at the end,
 // a row at a time: in a product, 0 times such a value would reach the queries that do not read it.
 // Every mbarrier wait is bounded; a wait that gives up records g_latent_tc_error and the CTA drains.
@@ -274,11 +278,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
             for (int g = 0; g < vgroups; ++g) {
                 const int n = min(2, vpieces - 2 * g);
                 const uint32_t idesc = IDESC_PV | ((uint32_t)(n * 64 >> 3) << 17);
-                // 16 keys a step: P advances 8 columns, the values 16 rows of 128 bytes
+                // 16 keys a step: P advances 8 columns, the values 16 rows of 128 bytes; then the same keys with what P lacks
 #pragma unroll
-                for (int k = 0; k < LT_KB / 16; ++k)
+                for (int k = 0; k < 2 * LT_KB / 16; ++k)
                     umma_bf16_ts_elect(tmem_o + g * 128, tmem_s + slot * 64 + 8 * k,
-                                       vlo0 + ((slot * slot_bytes + 2 * g * LT_K_PIECE + k * 16 * 128) >> 4), idesc, j > 0 || k > 0 ? 1u : 0u);
+                                       vlo0 + ((slot * slot_bytes + 2 * g * LT_K_PIECE + k % (LT_KB / 16) * 16 * 128) >> 4), idesc,
+                                       j > 0 || k > 0 ? 1u : 0u);
                 umma_commit_elect(empty0 + 8 * (slot * LT_GROUPS + g));
             }
             umma_commit_elect(o_done);
@@ -343,7 +348,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
                 }
             }
             const float neg_ref = m_ref == -INFINITY ? 0.f : -m_ref;
-            uint32_t w[32];
+            uint32_t w[32], rest[32];
             float ps[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int c = 0; c < 64; c += 2) {
@@ -351,9 +356,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_prefill_tc_kernel(const 
                 ps[(c >> 1) & 3] += a + b;
                 __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
                 w[c >> 1] = *reinterpret_cast<uint32_t*>(&v);
+                v = __floats2bfloat162_rn(a - __uint_as_float(w[c >> 1] << 16), b - __uint_as_float(w[c >> 1] & 0xffff0000u));
+                rest[c >> 1] = *reinterpret_cast<uint32_t*>(&v);
             }
             l_run += (ps[0] + ps[1]) + (ps[2] + ps[3]);
             tmem_st32_raw(my_s, w);                                      // column c holds keys 2 c and 2 c + 1
+            tmem_st32_raw(my_s + 32, rest);
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
