@@ -1535,16 +1535,19 @@ def latent_prefill_tiles(row_lens: list[int], num_heads: int) -> int:
     return sum(-(-length // n) for length in row_lens)
 
 
-def latent_prefill_wins(num_tiles: int, general_tiles: int, key_bound: int) -> bool:
+def latent_prefill_wins(num_tiles: int, general_tiles: int, key_bound: int, head_dim: int, value_dim: int) -> bool:
     """Whether the tcgen05 kernel is the faster one, for so many tiles of 128 rows or of 64 (``latent_attention_tc``) and at
-    most so many keys a row.  It needs 1.6 to 2.3 us for 64 keys whatever the number of tiles (rows of 192 and of 448 entries),
-    the other 7.5 us an SM, but shares a tile's keys out while its tiles are few.  Measured (B200, us, general / tcgen05, rows
-    of 448): 64 requests decoding at 1,000 keys 84 / 42, 32 requests 43 / 41, 8 requests 26 / 41, at 250 keys 24 / 16; a prompt
-    of 300 tokens (16 heads) 40 / 22, of 2,000 under a window of 1,024 311 / 74; rows of 192, at 4,000 keys, 56 requests
-    107 / 102, 48 requests 84 / 101, at 60 keys 300 requests 14 / 21 (two waves with next to nothing to do)."""
-    if key_bound <= 128 and num_tiles > 148:
+    most so many keys a row.  It needs 2 to 3 us for 64 keys whatever the number of tiles, the other less the narrower the rows
+    are, but for a tile on an SM at a time; with few tiles it shares their keys out.  Measured (B200, us, general / tcgen05):
+    rows of 448 with 384 values, 16 heads: 64 requests decoding at 1,000 keys 82 / 53, 56 at 4,000 300 / 189, at 250 keys 64
+    requests 27 / 18, a prompt of 300 tokens 39 / 26, of 2,000 493 / 99; rows of 192 with 128 values: 56 requests at 4,000 keys
+    104 / 123, 64 at 1,000 34 / 35, 41 at 700 beside a prompt of 200 (91 tiles) 53 / 29, a prompt of 2,000 187 / 53, at 60 keys
+    300 requests 14 / 21 (two waves with next to nothing to do); rows of 128 with 64 values, 2 heads: 64 requests at 1,000 keys
+    26 / 32, a prompt of 2,000 46 / 55, behind 4,000 120 / 154."""
+    width = head_dim + value_dim
+    if width < 256 or (key_bound <= 128 and num_tiles > 148):
         return False
-    return general_tiles >= 56 or key_bound <= 256
+    return general_tiles >= (56 if width >= 512 else 80) or key_bound <= 256
 
 
 def latent_prefill_tc(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tensor, page_base: torch.Tensor,

@@ -110,7 +110,7 @@ class LatentAttention(Mixer):
         bound = block_table.shape[1] * page_size
         if self.window:
             bound = min(bound, self.window + ops.LATENT_PREFILL_ROWS // self.H)
-        return n if ops.latent_prefill_wins(n, general_tiles, bound) else 0
+        return n if ops.latent_prefill_wins(n, general_tiles, bound, self.rank + self.rot, self.rank) else 0
 
     def forward(self, x, inputs, cache):
         if cache.write != self.own_cache:

@@ -226,3 +226,13 @@ def test_which_rows_of_a_step_run_over_chunks():
     # rows that other ones outnumber by far stay with them
     assert chunk_min_row([30] * 40 + [200], rules) == 0 and chunk_min_row([30] * 40 + [1200], rules) == 64
     assert chunk_min_row([1, 5], ((128, 1),)) == 0 and chunk_min_row([127, 128], ((128, 1),)) == 128
+
+
+def test_which_latent_steps_take_the_tcgen05_kernel():
+    from acorninfer_b200.kernels.ops import latent_prefill_wins
+
+    wide, narrow, small = (448, 384), (192, 128), (128, 64)
+    assert latent_prefill_wins(56, 56, 4096, *wide) and not latent_prefill_wins(48, 48, 4096, *wide)
+    assert latent_prefill_wins(250, 500, 2048, *narrow) and not latent_prefill_wins(64, 64, 1024, *narrow)
+    assert latent_prefill_wins(1, 1, 256, *narrow) and not latent_prefill_wins(300, 300, 128, *narrow)
+    assert not latent_prefill_wins(32, 63, 8192, *small) and not latent_prefill_wins(1, 1, 128, *small)
