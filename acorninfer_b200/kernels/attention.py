@@ -190,12 +190,13 @@ def paged_attention(qkv: torch.Tensor, inputs, group, cache, nq: int, nkv: int, 
         # a row of one token goes to the decode kernel whatever else is in the step, so that its bits stay the same
         n_single = inputs.num_tokens if inputs.plan.all_decode else int(inputs.plan.extra["attention.single_tokens"].size)
         chunks = ops.f32_decode_chunks(_key_bound(group.block_table.shape[1] * P, window, None, 0), window)
-        if n_single <= 65535 and ops.attention_f32_supported(nq, nkv, d, n_single, chunks):
+        runs = ops.f32_prefill_chunks(group.block_table.shape[1] * P, window) if n_single < inputs.num_tokens else 0
+        if n_single <= 65535 and ops.attention_f32_supported(nq, nkv, d, n_single, chunks, runs):
             out = torch.empty((inputs.num_tokens, nq * d), dtype=qkv.dtype, device=qkv.device)
             if n_single < inputs.num_tokens:
                 ops.attention_f32_prefill(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table, group.page_base,
                                           inputs.row_start, inputs.row_pos, inputs.extra["attention.q_tiles"], nq, nkv, d, scale,
-                                          window, ops.f32_prefill_chunks(group.block_table.shape[1] * P, window), out)
+                                          window, runs, out)
             if n_single:
                 ops.attention_f32_decode(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table, group.page_base,
                                          inputs.token_row, inputs.positions,

@@ -708,7 +708,7 @@ def attention_plain(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_pag
 
 F32_DECODE_KEYS = 128       # keys a block of the float32 decode kernel takes
 F32_Q_TILE = 64             # queries a tile of the float32 prefill kernel takes
-_F32_SCRATCH_MAX = 1 << 28  # floats of partial results (1 GB): beyond, the plain kernel
+_F32_SCRATCH_MAX = 1 << 24  # floats of partial results at a time (64 MB, about what a step's activations take)
 
 
 F32_PREFILL_KEYS = 512      # keys a block of the float32 prefill kernel walks
@@ -726,11 +726,14 @@ def f32_prefill_chunks(table_keys: int, window: int | None) -> int:
     return -(-keys // F32_PREFILL_KEYS) + (1 if window else 0)
 
 
-def attention_f32_supported(num_heads: int, num_kv_heads: int, head_dim: int, num_tokens: int = 0, chunks: int = 0) -> bool:
+def attention_f32_supported(num_heads: int, num_kv_heads: int, head_dim: int, num_tokens: int = 0, chunks: int = 0,
+                            prefill_chunks: int = 0) -> bool:
     """Whether the float32 prefill and decode kernels take these heads, and the decode kernel ``num_tokens`` rows of
-    ``chunks`` key blocks."""
+    ``chunks`` key blocks, the prefill kernel tiles of ``prefill_chunks`` runs of keys: what one row, or one tile, leaves in parts
+    has to fit the scratch (a tile four times it)."""
     return (bool(lib().acorn_attention_f32_supported(num_heads, num_kv_heads, head_dim)) and chunks <= 65535
-            and num_tokens * num_heads * chunks * (head_dim + 2) <= _F32_SCRATCH_MAX)
+            and min(num_tokens, 1) * num_heads * chunks * (head_dim + 2) <= _F32_SCRATCH_MAX
+            and (prefill_chunks <= 1 or F32_Q_TILE * num_heads * prefill_chunks * (head_dim + 2) <= 4 * _F32_SCRATCH_MAX))
 
 
 def attention_f32_prefill(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
@@ -765,13 +768,19 @@ def attention_f32_decode(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, 
     for t, name in ((k_pages, "k_pages"), (v_pages, "v_pages")):
         _check(t, name, torch.float32, 4)
     _check(out, "out", torch.float32, 2)
-    part_o = torch.empty((num_rows, num_heads, chunks, head_dim), dtype=torch.float32, device=q.device)
-    part_ml = torch.empty((num_rows, num_heads, chunks, 2), dtype=torch.float32, device=q.device)
-    _ok(lib().acorn_attention_f32_decode(q.data_ptr(), q_stride, out.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(),
-                                         block_table.data_ptr(), page_base.data_ptr(), block_table.stride(0), token_row.data_ptr(),
-                                         positions.data_ptr(), _ptr(token_list), num_rows, num_heads, num_kv_heads, head_dim,
-                                         k_pages.shape[2], float(scale), int(window or 0), chunks, part_o.data_ptr(),
-                                         part_ml.data_ptr(), _stream()), "attention_plain")
+    # partial results of as many rows at a time as fit the scratch
+    at_once = max(1, min(num_rows, _F32_SCRATCH_MAX // (num_heads * chunks * (head_dim + 2))))
+    part_o = torch.empty((at_once, num_heads, chunks, head_dim), dtype=torch.float32, device=q.device)
+    part_ml = torch.empty((at_once, num_heads, chunks, 2), dtype=torch.float32, device=q.device)
+    for at in range(0, num_rows, at_once):
+        first = 0 if token_list is not None else at         # listed tokens by their places in the list, others by their own
+        _ok(lib().acorn_attention_f32_decode(q.data_ptr() + 4 * first * q_stride, q_stride, out.data_ptr() + 4 * first * out.stride(0),
+                                             k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(), page_base.data_ptr(),
+                                             block_table.stride(0), token_row.data_ptr() + 4 * first, positions.data_ptr() + 4 * first,
+                                             token_list.data_ptr() + 4 * at if token_list is not None else None,
+                                             min(at_once, num_rows - at), num_heads, num_kv_heads, head_dim, k_pages.shape[2],
+                                             float(scale), int(window or 0), chunks, part_o.data_ptr(), part_ml.data_ptr(), _stream()),
+            "attention_plain")
     return out
 
 
@@ -1695,12 +1704,15 @@ def delta_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.T
 # of 128 151 / 94; time mixing of 32 heads of 64 x 64: 1 row of 64 tokens 22 / 29, of 96 32 / 25; 4 rows of 64 58 / 39.
 CHANNEL_CHUNK_ROWS = ((64, 256), (160, 160))
 MIX_CHUNK_ROWS = ((64, 128), (96, 96))
+CHANNEL_CHUNK_SCRATCH_BYTES = 1 << 29        # all that the chunks' kernels need beside inputs and result; beyond, the walk, which needs none
 
 
 def channel_chunk_ok(longest_row: int, tokens: int, num_rows: int, heads: int, dim: int, vdim: int) -> bool:
     """Whether the delta rule with decays per key channel runs over chunks (``channel_chunk``) in a step of these rows."""
     return (longest_row >= DELTA_CHUNK_MIN_ROW and bool(lib().acorn_delta_chunk_supported(dim, vdim)) and heads <= 65535
-            and num_rows <= 65535 and 4 * lib().acorn_delta_chunk_ids(tokens, num_rows, 0) * heads * dim * vdim <= DELTA_CHUNK_SCRATCH_BYTES)
+            and num_rows <= 65535
+            and 4 * heads * (lib().acorn_delta_chunk_ids(tokens, num_rows, DELTA_CHUNK_MIN_ROW) * dim * (vdim + 1)
+                             + tokens * (3 * dim + vdim + 64)) <= CHANNEL_CHUNK_SCRATCH_BYTES)
 
 
 def channel_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, log2_g: torch.Tensor, state: torch.Tensor,
@@ -2407,7 +2419,7 @@ def scan_chunk_ok(longest_row: int, num_rows: int, b: torch.Tensor, c: torch.Ten
     know (16-byte reads of b, c and x), and room for the chunks' states."""
     return (longest_row >= SCAN_CHUNK_MIN_ROW and bool(lib().acorn_scan_chunk_supported(n, v)) and num_rows <= 65535 and heads <= 65535
             and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in (b, c, x))
-            and 4 * scan_chunk_ids(x.shape[0], num_rows) * heads * n * v <= DELTA_CHUNK_SCRATCH_BYTES)
+            and 4 * scan_chunk_ids(x.shape[0], num_rows) * heads * n * v <= SCAN_SCRATCH_BYTES)
 
 
 def chunk_min_row(row_lens: list[int], rules: tuple[tuple[int, int], ...]) -> int:

@@ -294,6 +294,43 @@ def test_float32_attention_keeps_what_is_no_number_to_the_queries_that_read_it(n
     assert (got - want)[fine].abs().max() < 2e-6 * 5          # float32 sums of a few hundred weights of values up to 5
 
 
+@pytest.mark.parametrize("listed", [True, False])
+def test_float32_attention_in_as_many_launches_as_its_scratch_takes(listed, monkeypatch):
+    """Partial results for a tile or a row at a time, or a few: every bit as with room for all, and no more room than that."""
+    o, nq, nkv, d, P = ops(), 4, 2, 64, 16
+    before, qlens = [600, 0, 1200, 40, 700], [1] * 5 if not listed else [150, 700, 1, 1, 1]
+    T = sum(qlens)
+    starts = [sum(qlens[:r]) for r in range(6)]
+    NP = sum(-(-(b + n) // P) for b, n in zip(before, qlens)) + 3
+    lay = rows_layout(before, qlens, P, NP, seed=1)
+    g = torch.Generator().manual_seed(1)
+    k_pages, v_pages = (torch.randn(NP, nkv, P, d, generator=g).to(DEV) for _ in range(2))
+    q = torch.randn(T, nq * d + 8, generator=g).to(DEV)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)
+    common = (k_pages, v_pages, lay["block_table"], lay["page_base"])
+    tiles = i32([(r, q0) for r, n in enumerate(qlens) if n > 1 for q0 in range(0, n, o.F32_Q_TILE)]).view(-1, 2)
+    single = [starts[r] for r, n in enumerate(qlens) if n == 1]
+    keys = lay["block_table"].shape[1] * P
+
+    def run(room):
+        monkeypatch.setattr(o, "_F32_SCRATCH_MAX", room)
+        out = torch.full((T, nq * d), 7.0, device=DEV)
+        if len(tiles):
+            o.attention_f32_prefill(q, q.stride(0), *common, i32(starts), i32(before), tiles, nq, nkv, d, d ** -0.5, None,
+                                    o.f32_prefill_chunks(keys, None), out)
+        chunks = o.f32_decode_chunks(keys, None)
+        assert o.attention_f32_supported(nq, nkv, d, len(single), chunks) == (nq * chunks * (d + 2) <= room)
+        o.attention_f32_decode(q, q.stride(0), *common, lay["token_row"], lay["positions"], i32(single) if listed else None, len(single),
+                               nq, nkv, d, d ** -0.5, None, chunks, out)
+        return out
+
+    want = run(1 << 24)
+    one = nq * o.f32_decode_chunks(keys, None) * (d + 2)
+    for room in (one, 2 * one + 5, 64 * nq * o.f32_prefill_chunks(keys, None) * (d + 2) * 3):
+        assert torch.equal(run(room), want)
+    assert not bool((want == 7.0).any())
+
+
 def test_attention_decode_refuses_what_it_cannot_compute():
     from acorninfer_b200.kernels.ops import KernelError
     assert not ops().attention_decode_supported(34, 2, 64)       # 17 query heads a group
