@@ -373,6 +373,8 @@ __global__ void __launch_bounds__(TL_THREADS, 3) gemm_f32_tile_kernel(const floa
 
 // ------------------------------------------------------------------ host side
 
+static_assert(PL_BM == TL_BM, "the plain and the tile kernel cover the same rows a grid");
+
 template <int R, int CPL>
 static int launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
                        cudaStream_t stream) {
@@ -397,7 +399,7 @@ static int launch_tile(const float* A, int64_t lda, const float* W, int64_t ldw,
         configured.mark();
     }
     const int tn = (N + TL_BN - 1) / TL_BN, tm = (M + TL_BM - 1) / TL_BM;
-    if (tm > 65535 || (int64_t)tn * K_RANGES > 0x7fffffff) return ACORN_ERR_UNSUPPORTED;
+    if ((int64_t)tn * K_RANGES > 0x7fffffff) return ACORN_ERR_UNSUPPORTED;
     if (!SPLIT)
         return acorn_launch(gemm_f32_tile_kernel<SPLIT>, dim3(tn, tm), dim3(TL_THREADS), TL_SMEM, stream, A, lda, W, ldw,
                             C, ldc, M, N, K);
@@ -422,6 +424,11 @@ static int launch_tile(const float* A, int64_t lda, const float* W, int64_t ldw,
 extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, float* C,
                               int64_t ldc, int M, int N, int K, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
+    constexpr int most = 65535 * TL_BM;          // rows a launch's grid covers (the plain kernel's tiles have as many)
+    if (M > most) {
+        const int rc = acorn_gemm_f32(A, lda, W, ldw, C, ldc, most, N, K, stream);
+        return rc ? rc : acorn_gemm_f32(A + (int64_t)most * lda, lda, W, ldw, C + (int64_t)most * ldc, ldc, M - most, N, K, stream);
+    }
     // the faster kernels move 16 bytes at a time along K
     const bool aligned = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
     if (aligned && M <= 16) {
@@ -441,7 +448,6 @@ extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64
         return launch_tile<false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
     dim3 grid((N + PL_BN - 1) / PL_BN, (M + PL_BM - 1) / PL_BM);
-    if (grid.y > 65535) return ACORN_ERR_UNSUPPORTED;
     gemm_f32_kernel<<<grid, 256, 0, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
     return acorn_launch_status();
 }

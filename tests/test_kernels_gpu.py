@@ -172,3 +172,15 @@ def test_per_head_products_of_few_and_many_tokens(dtype, T, H, O, I):
         y1 = torch.zeros(1, H, O, device=DEV, dtype=dtype)
         ops().head_linear(x[T - 1:], w, y1)
         assert torch.equal(y1[0], y[T - 1])
+
+
+@pytest.mark.parametrize("K", [4, 3])          # tiles, and the kernel for unaligned rows
+def test_float32_product_of_more_rows_than_a_grid_covers(K):
+    o = ops()
+    M = 65535 * 64 + 70
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(5, K, generator=g, device=DEV)
+    got = o.gemm_f32(x, w)
+    for rows in (slice(0, 200), slice(M // 2, M // 2 + 200), slice(M - 200, M)):
+        assert (got[rows].double() - x[rows].double() @ w.double().T).abs().max() < 1e-5
+    assert torch.equal(got[-200:], o.gemm_f32(x[-200:].contiguous(), w))
