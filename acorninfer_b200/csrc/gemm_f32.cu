@@ -8,7 +8,7 @@
 // takes 12.5 us in dependent multiply-adds alone, where the weights of N = 2,048 columns stream in 7.6 us.
 //
 // A, W: float32 row-major, K contiguous, with row strides lda, ldw; C row stride ldc.
-//   rows kernel   up to 16 rows (decode): a block takes 16 or 32 columns and all rows, a warp one range of K with a ring
+//   rows kernel   up to 16 rows (decode; at many widths up to 32, in two launches): a block takes 16 or 32 columns and all rows, a warp one range of K with a ring
 //                 of cp.async stages of its own (no block barrier): bound by reading W once;
 //   tile kernel   more rows: 64 x 128 a block; a cluster of eight shares a tile's ranges where the tiles
 //                 alone leave the device idle: bound by the multiply-adds and the reads of shared memory that feed them;
@@ -438,6 +438,12 @@ extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64
         if (M <= 8)
             return wide ? launch_rows<4, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<4, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
         return wide ? launch_rows<8, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<8, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    }
+    if (aligned && M <= 32 && (N <= 4096 || N >= 8192)) {
+        // The weights twice through the rows kernel: 32 rows, N = 2,048, K = 6,144: 56 us, in tiles 88 us; N = 4,096, K = 1,024: 23 and
+        // 24 us; N = 12,288, K = 2,048: 79 and 93 us; between (N = 6,144, K = 1,024: 33 and 25 us) the tiles fill the device.
+        const int rc = acorn_gemm_f32(A, lda, W, ldw, C, ldc, 16, N, K, stream);
+        return rc ? rc : acorn_gemm_f32(A + 16 * lda, lda, W, ldw, C + 16 * ldc, ldc, M - 16, N, K, stream);
     }
     if (aligned) {
         // A cluster to a tile where whole tiles would leave an SM fewer than two of them (777 rows, N = 1,024, K = 2,048, 104 tiles:
