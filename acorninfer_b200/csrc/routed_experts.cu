@@ -894,7 +894,7 @@ extern "C" int acorn_moe_combine(const void* y, const void* x, const int* slot_o
                                  const void* extra, const float* extra_z, int64_t ldz, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     const uintptr_t rows = (uintptr_t)y | (uintptr_t)x | (uintptr_t)out | (uintptr_t)resid32 | (uintptr_t)norm_w | (uintptr_t)extra;
-    if (H % 8 == 0 && H <= 4096 && top <= MC_TOP && (rows & 15) == 0) {
+    if (H % 8 == 0 && H <= 4096 && top >= 1 && top <= MC_TOP && (rows & 15) == 0) {       // (its first choice is read unasked)
         ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(moe_combine_vec_kernel<T>, dim3(tokens), dim3((H / 8 + 31) / 32 * 32), 0, stream,
                                                            (const T*)y, (const T*)x, slot_of, idx, wts, (T*)out, H, top, E, resid32,
                                                            norm_w, eps, (const T*)extra, extra_z, ldz));

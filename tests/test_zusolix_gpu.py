@@ -688,3 +688,14 @@ def test_weights_on_the_experts_inputs(T, E, top, ff, width, dtype, tol):
     want = y.double()[slot_of.cpu().long()].sum(1) + torch.sigmoid(zw.double()[:, 1:2]) * extra.double()
     out = o.moe_combine(y.to(DEV), x.to(DEV), slot_of, idx.to(DEV), None, E, extra=extra.to(DEV), extra_z=zw.to(DEV)[:, 1:2])
     assert (out.double().cpu() - want).abs().max() < tol * 2
+
+
+@pytest.mark.parametrize("H", [24, 30])
+def test_combine_of_no_choices_is_what_all_tokens_take(H):
+    """No chosen expert at all: the shared row alone, or nothing."""
+    o = ops()
+    x, extra = torch.randn(5, H, device=DEV).bfloat16(), torch.randn(5, H, device=DEV).bfloat16()
+    none = torch.empty(5, 0, dtype=torch.int32, device=DEV)
+    y, wts = torch.empty(0, H, dtype=torch.bfloat16, device=DEV), torch.empty(5, 0, device=DEV)
+    assert torch.equal(o.moe_combine(y, x, none, none, wts, 3, extra=extra), extra)
+    assert not bool(o.moe_combine(y, x, none, none, wts, 3).any())
