@@ -10,8 +10,8 @@
 // temperature == 0 selects argmax (lowest index among equal maxima).
 // A row with a NaN or an infinite logit yields token -1 (the host raises).
 //
-// Two kernels.  `sample_cluster_kernel` takes every vocabulary that fits the shared memory of a cluster of eight CTAs;
-// `sample_kernel` walks the row in global memory and takes larger ones.
+// Two kernels.  `sample_cluster_kernel` takes vocabularies that fit the shared memory of a cluster of eight CTAs,
+// `sample_kernel` walks the row in global memory.  The caller chooses (acorninfer_b200/kernels/ops.py, sample_in_clusters).
 #include "common.cuh"
 
 #include <cooperative_groups.h>
@@ -527,12 +527,12 @@ static int launch_sample_cluster(const float* logits, int64_t ld, int rows, int 
 
 extern "C" int acorn_sample(const float* logits, int64_t ld, int rows, int V, const float* temperature,
                             const int* top_k, const float* top_p, const unsigned long long* seed,
-                            const unsigned long long* counter, int* token_out, float* logprob_out,
+                            const unsigned long long* counter, int* token_out, float* logprob_out, int clusters,
                             cudaStream_t stream) {
     if (rows <= 0) return 0;
     // slices are multiples of four logits, so that they start on 16 bytes where the row does
     const int slice = ((V + SC_CLUSTER - 1) / SC_CLUSTER + 3) & ~3;
-    if (slice <= SC_MAX_SLICE && rows <= 0x7fffffff / SC_CLUSTER)
+    if (clusters && slice <= SC_MAX_SLICE && rows <= 0x7fffffff / SC_CLUSTER)
         return launch_sample_cluster(logits, ld, rows, V, slice, temperature, top_k, top_p, seed, counter, token_out, logprob_out, stream);
     return acorn_launch(sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, temperature, top_k,
                         top_p, seed, counter, token_out, logprob_out);

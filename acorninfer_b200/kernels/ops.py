@@ -251,7 +251,7 @@ class _Sigs:
     acorn_gemm_tc_error = []
     acorn_gemm_f32 = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]
     acorn_sample = [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                    c_void_p, c_void_p, c_void_p]
+                    c_void_p, c_void_p, c_int, c_void_p]
     acorn_uniform = [ctypes.c_uint64, ctypes.c_uint64]
     acorn_random_fill = [c_void_p, c_int64, ctypes.c_uint64, ctypes.c_uint64, c_float, c_float, c_int, c_void_p]
     acorn_error_word_alloc = [c_void_p, c_void_p]
@@ -2755,10 +2755,20 @@ def add_row(x32: torch.Tensor, row32: torch.Tensor) -> torch.Tensor:
 # ------------------------------------------------------------------ sampling
 
 
+def sample_in_clusters(rows: int, vocab: int, greedy: bool) -> bool:
+    """Whether a cluster of CTAs takes each row, and not one CTA.  Rows that draw: by the vocabulary alone, so that a row's
+    token does not depend on the batch (the two kernels round their sums differently).  The largest logit is the same from both.
+    Measured (B200, us, one CTA / a cluster a row): 64 rows of 4,096 26 / 44 with top-k, 31 / 53 with top-p, of 32,000 88 / 49 and
+    137 / 66, without either 26 / 20; 64 rows of 151,936 716 / 123 with both; largest logits: 64 rows of 4,096 2.7 / 9.1, of
+    151,936 11 / 14, 8 rows of 151,936 11 / 5.6, 24 rows 11 / 7.6, 256 rows 28 / 66."""
+    return (vocab >= 65536 and rows <= 24) if greedy else vocab >= 20000
+
+
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,
-           seed: torch.Tensor, counter: torch.Tensor, want_logprobs: bool = False):
+           seed: torch.Tensor, counter: torch.Tensor, want_logprobs: bool = False, greedy: bool = False):
     """One token per row of float32 logits.  Per-row parameters are device tensors:
-    temperature/top_p float32, top_k int32, seed/counter int64 (used as unsigned)."""
+    temperature/top_p float32, top_k int32, seed/counter int64 (used as unsigned).  ``greedy``: the caller knows that no row
+    draws (all temperatures are 0); it decides between two kernels, not the result."""
     _check(logits, "logits", torch.float32, 2)
     R, V = logits.shape
     _check(temperature, "temperature", torch.float32, 1)
@@ -2773,7 +2783,7 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
     logprobs = torch.empty(R, dtype=torch.float32, device=logits.device) if want_logprobs else None
     _ok(lib().acorn_sample(logits.data_ptr(), logits.stride(0), R, V, temperature.data_ptr(), top_k.data_ptr(),
                            top_p.data_ptr(), seed.data_ptr(), counter.data_ptr(), tokens.data_ptr(),
-                           _ptr(logprobs), _stream()), "sample")
+                           _ptr(logprobs), int(sample_in_clusters(R, V, greedy)), _stream()), "sample")
     return tokens, logprobs
 
 

@@ -88,7 +88,8 @@ class Sampler:
         R = logits.shape[0]
         if len(params) != R or len(counters) != R:
             raise ValueError("one SamplingParams and one counter per logits row")
-        if all(p.greedy for p in params):
+        greedy = all(p.greedy for p in params)
+        if greedy:
             temperature, top_k, top_p, seeds, ctrs = self._greedy_params(R)
         else:
             # one copy to the device for all five (each copy costs the host as much as the kernel takes)
@@ -102,4 +103,4 @@ class Sampler:
             seeds, ctrs = block[:2 * R].view(torch.int64), block[2 * R:4 * R].view(torch.int64)
             temperature, top_p = block[4 * R:5 * R].view(torch.float32), block[5 * R:6 * R].view(torch.float32)
             top_k = block[6 * R:]
-        return ops.sample(logits, temperature, top_k, top_p, seeds, ctrs, want_logprobs)
+        return ops.sample(logits, temperature, top_k, top_p, seeds, ctrs, want_logprobs, greedy=greedy)

@@ -69,11 +69,15 @@ def test_draws_follow_the_distribution_and_do_not_depend_on_the_batch():
     assert alone[0] == toks[123]
 
 
-@pytest.mark.parametrize("vocab", [4095, 4096, 4097, 32771, 151936, 360448, 360449])
-def test_large_vocabularies_in_every_cut(vocab):
-    """Around the sizes where the kernel changes (one CTA, a cluster, the walk in global memory); rows of odd length, which
+@pytest.mark.parametrize("clusters", [False, True])
+@pytest.mark.parametrize("vocab", [5, 33, 4097, 19999, 20000, 32771, 151936, 360448, 360449])
+def test_large_vocabularies_in_every_cut(vocab, clusters, monkeypatch):
+    """Both kernels (one CTA a row, a cluster of eight CTAs a row) at vocabularies that leave some CTAs of a cluster without a
+    logit, at the one from which clusters are taken, at the largest that a cluster holds and one more; rows of odd length, which
     start on 16 bytes only every fourth time; a row of equal logits, one masked down to a few tokens, one with many ties."""
     from acorninfer_b200.kernels import ops
+    assert ops.sample_in_clusters(7, vocab, False) == (vocab >= 20000)
+    monkeypatch.setattr(ops, "sample_in_clusters", lambda *sizes: clusters)
     R = 7
     g = torch.Generator().manual_seed(vocab)
     x = 2.5 * torch.randn(R, vocab, generator=g)
@@ -103,3 +107,36 @@ def test_large_vocabularies_in_every_cut(vocab):
             assert abs(lps[r] - want_lp) < 1e-4
             checked += 1
     assert 0 <= toks[4] < vocab and checked >= 3
+    none = f([0.0] * R, torch.float32), f([0] * R, torch.int32), f([1.0] * R, torch.float32)
+    seeds_, counters_ = f(seeds, torch.int64), f(counters, torch.int64)
+    assert ops.sample(x.to(DEV), *none, seeds_, counters_, greedy=True)[0].tolist() == x.argmax(1).tolist()
+
+
+@pytest.mark.parametrize("k", [1, 127, 128, 129, 4000])
+def test_top_k_at_the_cut_by_the_warps_maxima(k):
+    """The cluster kernel drops keys below the least of its 128 warps' maxima for k up to 128: rows with one large logit to a
+    warp, with maxima of 0 and -0 alone, with all logits equal, and any."""
+    from acorninfer_b200.kernels import ops
+    V = 40000
+    slice_ = (V // 8 + 3) & ~3
+    x = torch.randn(4, V, generator=torch.Generator().manual_seed(k)) - 3.0
+    # vectors of four by 512 threads: warp w of a CTA starts at element 128 w of its slice
+    first = torch.tensor([cta * slice_ + 128 * w for cta in range(8) for w in range(16)])
+    x[0, first] = torch.linspace(5.0, 6.0, 128)
+    x[1] = -x[1].abs() - 1.0
+    x[1, first[::2]], x[1, first[1::2]] = 0.0, -0.0
+    x[2] = 1.5
+    n = 400
+    f = lambda v, dt: torch.full((4 * n,), v, dtype=dt, device=DEV)
+    assert ops.sample_in_clusters(4 * n, V, False)
+    toks = ops.sample(x.repeat_interleave(n, 0).to(DEV), f(1.0, torch.float32), f(k, torch.int32), f(1.0, torch.float32),
+                      f(3, torch.int64), torch.arange(4 * n, device=DEV))[0].view(4, n).cpu()
+    for r in range(4):
+        kept = x[r] >= x[r].topk(k).values[-1]
+        if r == 1 and k < 128:          # 0 ranks above -0 as a key where both are at the bound
+            kept &= ~(torch.signbit(x[r]) & (x[r] == 0)) | (k > 64)
+        assert bool(kept[toks[r].long()].all()), (r, k)
+        p = torch.where(kept, x[r].double(), torch.tensor(float("-inf")).double()).softmax(0)
+        # every token of a small kept set turns up as often as it should (four standard deviations)
+        freq = torch.bincount(toks[r].long(), minlength=V).double() / n
+        assert ((freq - p).abs() <= 4 * (p / n).sqrt() + 4 / n).all(), (r, k)
