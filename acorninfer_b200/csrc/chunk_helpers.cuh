@@ -108,3 +108,5 @@ __device__ __forceinline__ float dot4(const float4& a, const float4& b, float ac
 __device__ __forceinline__ bool not_finite(const float4& v) {
     return !(fabsf(v.x) <= FLT_MAX && fabsf(v.y) <= FLT_MAX && fabsf(v.z) <= FLT_MAX && fabsf(v.w) <= FLT_MAX);
 }
+
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }

@@ -191,7 +191,6 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(const DeltaCh
 }
 
 __device__ __forceinline__ float4 at4(const float* q) { return *reinterpret_cast<const float4*>(q); }
-__device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float4 sub4(const float4& a, const float4& b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
 __device__ __forceinline__ float4 mul4(const float4& a, const float4& b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 // 2^x for x <= 0 by the PTX instruction ex2.approx.ftz.f32: an approximation (relative error up to 2^-22), results below 2^-126
@@ -280,12 +279,18 @@ __global__ void __launch_bounds__(CC_THREADS) channel_chunk_solve_kernel(const D
     {
         const int lower = tx <= ty ? 32 * half : 32 * half + 16, upper = 64 * half + 16 - lower;
         const int i = lower + max(tx, ty), j = lower + min(tx, ty);
-        float a = 0.f, q = 0.f;
-#pragma unroll 4
-        for (int d = 0; d < DP; d += 4) {
-            const float4 k = mul4(at4(sK + j * LD + d), exp2_4(logs.between(j, i, d)));
-            a = dot4(at4(sK + i * LD + d), k, a);
-            q = dot4(at4(sQ + i * LD + d), k, q);
+        float a = 0.f, q = 0.f;                         // sums over the channels in parts of 16 (see scan_chunk.cu)
+#pragma unroll 1
+        for (int d0 = 0; d0 < DP; d0 += 16) {
+            float part_a = 0.f, part_q = 0.f;
+#pragma unroll
+            for (int d = d0; d < d0 + 16; d += 4) {
+                const float4 k = mul4(at4(sK + j * LD + d), exp2_4(logs.between(j, i, d)));
+                part_a = dot4(at4(sK + i * LD + d), k, part_a);
+                part_q = dot4(at4(sQ + i * LD + d), k, part_q);
+            }
+            a += part_a;
+            q += part_q;
         }
         sA[i * LA + j] = i > j ? sbeta[i] * a : 0.f;
         if (i < n) P[i * ldp + j] = q;
@@ -294,8 +299,13 @@ __global__ void __launch_bounds__(CC_THREADS) channel_chunk_solve_kernel(const D
         } else {                                        // the other block's diagonal
             const int o = upper + tx;
             float s = 0.f;
-#pragma unroll 4
-            for (int d = 0; d < DP; d += 4) s = dot4(at4(sQ + o * LD + d), at4(sK + o * LD + d), s);
+#pragma unroll 1
+            for (int d0 = 0; d0 < DP; d0 += 16) {
+                float part = 0.f;
+#pragma unroll
+                for (int d = d0; d < d0 + 16; d += 4) part = dot4(at4(sQ + o * LD + d), at4(sK + o * LD + d), part);
+                s += part;
+            }
             sA[o * LA + o] = 0.f;
             if (o < n) P[o * ldp + o] = s;
         }
@@ -326,11 +336,17 @@ __global__ void __launch_bounds__(CC_THREADS) channel_chunk_solve_kernel(const D
         const int i = 16 * I + ty;
         const float* rows = half == 0 ? sE + ty * LD : sQ + i * LD;      // half of the threads A, half P
         float s[3] = {0.f, 0.f, 0.f};
-#pragma unroll 4
-        for (int d = 0; d < DP; d += 4) {
-            const float4 x = at4(rows + d);
+#pragma unroll 2
+        for (int d0 = 0; d0 < DP; d0 += 16) {
+            float part[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-            for (int J = 0; J < I; ++J) s[J] = dot4(x, at4(sR + (16 * J + tx) * LD + d), s[J]);
+            for (int d = d0; d < d0 + 16; d += 4) {
+                const float4 x = at4(rows + d);
+#pragma unroll
+                for (int J = 0; J < I; ++J) part[J] = dot4(x, at4(sR + (16 * J + tx) * LD + d), part[J]);
+            }
+#pragma unroll
+            for (int J = 0; J < I; ++J) s[J] += part[J];
         }
 #pragma unroll
         for (int J = 0; J < I; ++J) {
@@ -570,16 +586,22 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_out_kernel(const DeltaChun
     auto axpy = [](float a, const float4& x, float4& y) {
         y.x = fmaf(a, x.x, y.x); y.y = fmaf(a, x.y, y.y); y.z = fmaf(a, x.z, y.z); y.w = fmaf(a, x.w, y.w);
     };
+#pragma unroll 1
+    for (int d0 = 0; d0 < DP; d0 += 32) {
+        float4 part[4] = {zero, zero, zero, zero};
 #pragma unroll 2
-    for (int d = 0; d < DP; d += 4) {
-        float4 s[4];
+        for (int d = d0; d < d0 + 32; d += 4) {
+            float4 s[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) s[q] = *reinterpret_cast<const float4*>(sS + (d + q) * LO + 4 * tx);
+            for (int q = 0; q < 4; ++q) s[q] = *reinterpret_cast<const float4*>(sS + (d + q) * LO + 4 * tx);
 #pragma unroll
-        for (int ii = 0; ii < 4; ++ii) {
-            const float4 q4 = *reinterpret_cast<const float4*>(sQ + (ty + 16 * ii) * LD + d);
-            axpy(q4.x, s[0], acc[ii]); axpy(q4.y, s[1], acc[ii]); axpy(q4.z, s[2], acc[ii]); axpy(q4.w, s[3], acc[ii]);
+            for (int ii = 0; ii < 4; ++ii) {
+                const float4 q4 = *reinterpret_cast<const float4*>(sQ + (ty + 16 * ii) * LD + d);
+                axpy(q4.x, s[0], part[ii]); axpy(q4.y, s[1], part[ii]); axpy(q4.z, s[2], part[ii]); axpy(q4.w, s[3], part[ii]);
+            }
         }
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii) acc[ii] = add4(acc[ii], part[ii]);
     }
     if (!SCALED) {
 #pragma unroll
@@ -958,19 +980,29 @@ __global__ void __launch_bounds__(256) mix_chunk_local_kernel(const DeltaChunkPa
         const int i = lower + max(tx, ty), j = lower + min(tx, ty);
         if (tx != ty) {
             float s = 0.f;
-#pragma unroll 4
-            for (int d = 0; d < DP; d += 4)
-                s = dot4(at4(sQ + i * LD + d), mul4(at4(sK + j * LD + d), exp2_4(logs.between(j, i - 1, d))), s);
+#pragma unroll 1
+            for (int d0 = 0; d0 < DP; d0 += 16) {
+                float part = 0.f;
+#pragma unroll
+                for (int d = d0; d < d0 + 16; d += 4)
+                    part = dot4(at4(sQ + i * LD + d), mul4(at4(sK + j * LD + d), exp2_4(logs.between(j, i - 1, d))), part);
+                s += part;
+            }
             if (i < n) P[i * ldp + j] = s;
             if (upper + min(tx, ty) < n) P[(upper + min(tx, ty)) * ldp + upper + max(tx, ty)] = 0.f;
         }
     }
     if (tid < DC && tid < n) {
         float s = 0.f;
-#pragma unroll 4
-        for (int d = 0; d < DP; d += 4) {
-            const float4 u = d < p.dim ? make_float4(bonus[h * p.dim + d], bonus[h * p.dim + d + 1], bonus[h * p.dim + d + 2], bonus[h * p.dim + d + 3]) : zero;
-            s = dot4(at4(sQ + tid * LD + d), mul4(at4(sK + tid * LD + d), u), s);
+#pragma unroll 1
+        for (int d0 = 0; d0 < DP; d0 += 16) {
+            float part = 0.f;
+#pragma unroll
+            for (int d = d0; d < d0 + 16; d += 4) {
+                const float4 u = d < p.dim ? make_float4(bonus[h * p.dim + d], bonus[h * p.dim + d + 1], bonus[h * p.dim + d + 2], bonus[h * p.dim + d + 3]) : zero;
+                part = dot4(at4(sQ + tid * LD + d), mul4(at4(sK + tid * LD + d), u), part);
+            }
+            s += part;
         }
         P[tid * ldp + tid] = s;
     }
@@ -994,11 +1026,17 @@ __global__ void __launch_bounds__(256) mix_chunk_local_kernel(const DeltaChunkPa
         __syncthreads();
         const int i = 16 * I + ty;
         float s[3] = {0.f, 0.f, 0.f};
-#pragma unroll 4
-        for (int d = 0; d < DP; d += 4) {
-            const float4 q = at4(sQ + i * LD + d);
+#pragma unroll 2
+        for (int d0 = 0; d0 < DP; d0 += 16) {
+            float part[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-            for (int J = 0; J < I; ++J) s[J] = dot4(q, at4(sR + (16 * J + tx) * LD + d), s[J]);
+            for (int d = d0; d < d0 + 16; d += 4) {
+                const float4 q = at4(sQ + i * LD + d);
+#pragma unroll
+                for (int J = 0; J < I; ++J) part[J] = dot4(q, at4(sR + (16 * J + tx) * LD + d), part[J]);
+            }
+#pragma unroll
+            for (int J = 0; J < I; ++J) s[J] += part[J];
         }
         if (i < n)
 #pragma unroll

@@ -1,4 +1,5 @@
-// The linear recurrence of linear_recurrence.cu over chunks of 64 tokens (float32 throughout):
+// The linear recurrence of linear_recurrence.cu over chunks of 64 tokens (float32 throughout; long sums in parts of 16 or 32
+// terms, which are then added: one chain over keys of 128 left c . b twice as far from 64 bits as the walk is):
 //     S_i = a_i S_(i-1) + b_i (w_i x_i)^T,   y_i = S_i^T c_i + skip x_i,   a number a_i per token and head.
 // With L_i the sum of log |a| up to i within the chunk (in double: differences of sums lose nothing that float32 would show),
 // and the product of the decays' signs up to i beside it,
@@ -201,17 +202,25 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
     for (int ii = 0; ii < 4; ++ii)
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) M[ii][jj] = 0.f;
-#pragma unroll 2
-    for (int d = 0; d < NP; d += 4) {
-        float4 kj[4];
+#pragma unroll 1
+    for (int d0 = 0; d0 < NP; d0 += 16) {
+        float part[4][4] = {};
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) kj[jj] = *reinterpret_cast<const float4*>(sB + (tx + 16 * jj) * LN + d);
+        for (int d = d0; d < d0 + 16; d += 4) {
+            float4 kj[4];
 #pragma unroll
-        for (int ii = 0; ii < 4; ++ii) {
-            const float4 ci = *reinterpret_cast<const float4*>(sC + (ty + 16 * ii) * LN + d);
+            for (int jj = 0; jj < 4; ++jj) kj[jj] = *reinterpret_cast<const float4*>(sB + (tx + 16 * jj) * LN + d);
 #pragma unroll
-            for (int jj = 0; jj <= ii; ++jj) M[ii][jj] = dot4(ci, kj[jj], M[ii][jj]);
+            for (int ii = 0; ii < 4; ++ii) {
+                const float4 ci = *reinterpret_cast<const float4*>(sC + (ty + 16 * ii) * LN + d);
+#pragma unroll
+                for (int jj = 0; jj <= ii; ++jj) part[ii][jj] = dot4(ci, kj[jj], part[ii][jj]);
+            }
         }
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii)
+#pragma unroll
+            for (int jj = 0; jj <= ii; ++jj) M[ii][jj] += part[ii][jj];
     }
     for (int q = 0; q < heads; ++q) {
         const int h = h0 + q;
@@ -248,16 +257,22 @@ __global__ void __launch_bounds__(256, 2) scan_chunk_out_kernel(const ScanChunkP
         float4 acc[4];
 #pragma unroll
         for (int ii = 0; ii < 4; ++ii) acc[ii] = zero;
+#pragma unroll 1
+        for (int d0 = 0; d0 < NP; d0 += 32) {
+            float4 part[4] = {zero, zero, zero, zero};
 #pragma unroll 2
-        for (int d = 0; d < NP; d += 4) {
-            float4 s[4];
+            for (int d = d0; d < d0 + 32; d += 4) {
+                float4 s[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) s[u] = *reinterpret_cast<const float4*>(sB + (d + u) * SCO_LV + 4 * tx);
+                for (int u = 0; u < 4; ++u) s[u] = *reinterpret_cast<const float4*>(sB + (d + u) * SCO_LV + 4 * tx);
 #pragma unroll
-            for (int ii = 0; ii < 4; ++ii) {
-                const float4 c4 = *reinterpret_cast<const float4*>(sC + (ty + 16 * ii) * LN + d);
-                axpy4(c4.x, s[0], acc[ii]); axpy4(c4.y, s[1], acc[ii]); axpy4(c4.z, s[2], acc[ii]); axpy4(c4.w, s[3], acc[ii]);
+                for (int ii = 0; ii < 4; ++ii) {
+                    const float4 c4 = *reinterpret_cast<const float4*>(sC + (ty + 16 * ii) * LN + d);
+                    axpy4(c4.x, s[0], part[ii]); axpy4(c4.y, s[1], part[ii]); axpy4(c4.z, s[2], part[ii]); axpy4(c4.w, s[3], part[ii]);
+                }
             }
+#pragma unroll
+            for (int ii = 0; ii < 4; ++ii) acc[ii] = add4(acc[ii], part[ii]);
         }
 #pragma unroll
         for (int ii = 0; ii < 4; ++ii) {
