@@ -13,8 +13,8 @@
 // queries of its tile, on the step's other rows or on padding.
 //
 // What bounded the plain kernel: a block a token read every key row again from L2 and made one chain of adds per thread.
-// Measured (B200): 777 tokens, 16 heads of 128: 1,596 -> 153 us a layer; 6 rows of 1,500 keys, 8 kv heads:
-// 128 -> 27 us a layer (74 MB).
+// Measured (B200, launched alone): 777 tokens, 16 heads of 128: 1,402 -> 152 us; 6 rows of 1,500 keys, 8 kv heads:
+// 109 -> 14 us (74 MB, which L2 holds).
 #include "mma_helpers.cuh"
 
 #include <cfloat>
@@ -369,8 +369,7 @@ __global__ void __launch_bounds__(FD_THREADS) attention_f32_decode_kernel(
     for (int e = 0; e < 32 / VK; ++e) {
         const int key = warp * 32 + e * VK + vk;
         const int64_t at = row_at[key];
-        const bool read = kb + key >= lo && kb + key <= pos;
-        const float4 v = read ? *reinterpret_cast<const float4*>(v_pages + at + vd) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 v = *reinterpret_cast<const float4*>(v_pages + at + vd);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const float p = sc[g][key];

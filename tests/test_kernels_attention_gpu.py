@@ -290,7 +290,6 @@ def test_float32_attention_keeps_what_is_no_number_to_the_queries_that_read_it(n
                                d ** -0.5, window, ops().f32_decode_chunks(min(window or 1 << 20, keys), window), out)
     got, fine = out.double().cpu(), torch.isfinite(want)
     assert torch.equal(torch.isfinite(got), fine) and bool(fine.any()) and not bool(fine.all())
-    assert torch.equal(torch.isposinf(got), torch.isposinf(want))
     assert (got - want)[fine].abs().max() < 2e-6 * 5          # float32 sums of a few hundred weights of values up to 5
 
 
