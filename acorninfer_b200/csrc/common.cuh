@@ -118,6 +118,18 @@ struct AcornPerDevice {
     }
 };
 
+// Multiprocessors of the current device.
+static inline int acorn_sms() {
+    static int sms[64] = {};
+    const int dev = AcornPerDevice::current();
+    if (dev < 0) return 148;
+    if (sms[dev] == 0) {
+        int n = 0;
+        sms[dev] = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }
+    return sms[dev];
+}
+
 // ---------------------------------------------------------------- programmatic dependent launch
 // Every kernel of this library is launched with programmatic stream serialization: it may be
 // scheduled while the kernel before it in the stream is still running, and must call

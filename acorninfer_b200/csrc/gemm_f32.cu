@@ -384,8 +384,8 @@ static int launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw,
         if (e != cudaSuccess) return (int)e;
         configured.mark();
     }
-    const int tiles = (N + 16 * CPL - 1) / (16 * CPL);
-    return acorn_launch(gemm_f32_rows_kernel<R, CPL>, dim3(CPL == 2 ? (tiles < 148 ? tiles : 148) : tiles), dim3(RS_THREADS), rs_smem<R, CPL>(), stream,
+    const int tiles = (N + 16 * CPL - 1) / (16 * CPL), sms = acorn_sms();
+    return acorn_launch(gemm_f32_rows_kernel<R, CPL>, dim3(CPL == 2 && sms < tiles ? sms : tiles), dim3(RS_THREADS), rs_smem<R, CPL>(), stream,
                         A, lda, W, ldw, C, ldc, M, N, K);
 }
 
@@ -450,7 +450,7 @@ extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64
         // 131 us whole, 97 us split; 2,048 rows of the same, 256 tiles: 316 and 216 us; 777 rows, N = 4,096, K = 1,024, 416
         // tiles: 164 whole, 181 split), and a range of K is worth its share of the exchange.
         const int64_t tiles = (int64_t)((N + TL_BN - 1) / TL_BN) * ((M + TL_BM - 1) / TL_BM);
-        if (tiles < 2 * 148 && K >= 256) return launch_tile<true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+        if (tiles < 2 * acorn_sms() && K >= 256) return launch_tile<true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
         return launch_tile<false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
     dim3 grid((N + PL_BN - 1) / PL_BN, (M + PL_BM - 1) / PL_BM);

@@ -12,8 +12,8 @@
 //
 // What bounds it: multiply-adds fed from shared memory (register tiles of 4 x 4 by 4 and of 8 x 4).  The walk over tokens it
 // replaces for long rows is bound by the issue of dependent instructions, twice over in its two passes.  Measured (2,048
-// tokens, B200): 64 heads of 64 columns, keys of 128, 8 groups: 492 -> 215 us; 16 heads of 128 columns, keys of 128:
-// 277 -> 135 us.
+// tokens, B200): 64 heads of 64 columns, keys of 128, 8 groups: 492 -> 216 us; 16 heads of 128 columns, keys of 128:
+// 277 -> 138 us.
 #include "chunk_helpers.cuh"
 
 #define SCO_VT 64                   // columns a block
@@ -331,13 +331,14 @@ template <int NP> static int launch_scan_chunk(const ScanChunkParams& p, int ids
     if (rc) return rc;
     rc = acorn_launch(scan_chunk_fold_kernel, dim3((p.N * (p.V / 4) + 255) / 256, p.H, walks), dim3(256), 0, stream, p);
     if (rc) return rc;
-    // The heads of a group share C B^T, about 0.4 of a head's own work, so a block wants many of them, and the 296 blocks
-    // that run at a time want to be filled: the share with the least estimated time.
+    // The heads of a group share C B^T, about 0.4 of a head's own work, so a block wants many of them, and the blocks that run
+    // at a time (two to an SM) want to be filled: the share with the least estimated time.
+    const int64_t at_once = 2 * acorn_sms();
     int best = 1;
     double best_cost = 1e30;
     for (int per = 1; per <= SCO_HEADS && per <= rep; ++per) {
         const int64_t blocks = (int64_t)ids * p.G * tiles * ((rep + per - 1) / per);
-        const double cost = (double)((blocks + 295) / 296) * (per + 0.4);
+        const double cost = (double)((blocks + at_once - 1) / at_once) * (per + 0.4);
         if (cost < best_cost - 1e-9) { best_cost = cost; best = per; }
     }
     return acorn_launch(scan_chunk_out_kernel<NP>, dim3(ids, p.G, tiles * ((rep + best - 1) / best)), dim3(256), out, stream, p, best);
