@@ -17,7 +17,7 @@
 //     A_ij = beta_i sum_d k_id k_jd exp(b_id - b_jd),   P_ij = sum_d q_id k_jd exp(b_id - b_jd),   W from diag(beta) (K exp(b)),
 //     O = (Q exp(b)) S_0 + P U,   S_end = diag(exp(b_n)) S_0 + sum_j (k_j exp(b_n - b_j)) u_j^T
 // (channel_chunk_solve in place of delta_chunk_solve; the other two kernels read its scaled q and k).  The walk over tokens that
-// it replaces for long rows is a chain of dependent instructions: 2,000 tokens, 16 heads of 128 x 128: 844 -> 340 us a layer
+// it replaces for long rows is a chain of dependent instructions: 2,000 tokens, 16 heads of 128 x 128: 847 -> 350 us a layer
 // (B200).  b is kept as sums within blocks of 16 tokens, each as two floats, and the blocks' sums: differences lose nothing to a
 // strong decay that both sides have behind them.
 //
@@ -942,8 +942,8 @@ extern "C" int acorn_linear_chunk(const void* in, int64_t ld, const float* z, in
 // and write and sees itself through the bonus.  As gated linear attention over chunks, with the sums e_i = b_(i-1) up to the token
 // before on the reading side:
 //     Q'_i = q_i exp(e_i),   P_ij = sum_d q_id k_jd exp(e_id - b_jd) for j < i,   P_ii = sum_d q_id bonus_d k_id.
-// The walk over segments that it replaces for long rows went through every token twice: 1,800 tokens of 32 heads of 64 x 64
-// 203 -> 98 us (B200).
+// The walk over segments that it replaces for long rows went through every token twice: 2,000 tokens of 32 heads of 64 x 64,
+// the kernels alone: 220 -> 148 us (B200).
 template <int DP>
 __global__ void __launch_bounds__(256) mix_chunk_local_kernel(const DeltaChunkParams p, const float* __restrict__ bonus) {
     constexpr int LD = DP + DC_PAD, LO = DC_OT + DC_PAD, DQ = DP / 4;

@@ -1704,7 +1704,7 @@ def delta_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.T
 # of 128 151 / 94; time mixing of 32 heads of 64 x 64: 1 row of 64 tokens 22 / 29, of 96 32 / 25; 4 rows of 64 58 / 39.
 CHANNEL_CHUNK_ROWS = ((64, 256), (160, 160))
 MIX_CHUNK_ROWS = ((64, 128), (96, 96))
-CHANNEL_CHUNK_SCRATCH_BYTES = 1 << 29        # all that the chunks' kernels need beside inputs and result; beyond, the walk, which needs none
+CHANNEL_CHUNK_SCRATCH_BYTES = 1 << 30        # all that the chunks' kernels need beside inputs and result (16 heads of 128: 53 KB a token); beyond, the walk
 
 
 def channel_chunk_ok(longest_row: int, tokens: int, num_rows: int, heads: int, dim: int, vdim: int) -> bool:
@@ -2760,7 +2760,7 @@ def sample_in_clusters(rows: int, vocab: int, greedy: bool) -> bool:
     token does not depend on the batch (the two kernels round their sums differently).  The largest logit is the same from both.
     Measured (B200, us, one CTA / a cluster a row): 64 rows of 4,096 26 / 44 with top-k, 31 / 53 with top-p, of 32,000 88 / 49 and
     137 / 66, without either 26 / 20; 64 rows of 151,936 716 / 123 with both; largest logits: 64 rows of 4,096 2.7 / 9.1, of
-    151,936 11 / 14, 8 rows of 151,936 11 / 5.6, 24 rows 11 / 7.6, 256 rows 28 / 66."""
+    151,936 11 / 14, 8 rows of 151,936 11 / 5.6, 24 rows 11 / 7.6, 256 rows 28 / 66.  (256 rows of 151,936 that draw without top-k and top-p: 113 / 157.)"""
     return (vocab >= 65536 and rows <= 24) if greedy else vocab >= 20000
 
 
