@@ -99,8 +99,8 @@ def test_swiglu_and_cast(dtype):
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (7, 331, 120), (130, 65, 33), (64, 64, 16), (3, 1000, 257),
                                    (16, 100, 324), (17, 40, 1028), (65, 300, 200), (300, 130, 516)])
 def test_gemm_f32_is_true_float32(M, N, K):
-    """K a multiple of 4 takes the streaming kernel (up to 64 rows) or the 128 x 128 tile kernel, other K
-    the plain one; (17, 40, 1028) runs more k-steps than the streaming kernel's ring has stages."""
+    """K a multiple of 4 takes the rows kernel (up to 16 rows, at many widths 32) or the 64 x 128 tile kernel, other K
+    the plain one; (17, 40, 1028) runs more k-steps than the rows kernel's ring has stages."""
     a = torch.randn(M, K, device=DEV)
     w = torch.randn(N, K, device=DEV)
     out = ops().gemm_f32(a, w)
@@ -111,8 +111,8 @@ def test_gemm_f32_is_true_float32(M, N, K):
 
 
 def test_gemm_f32_gives_the_same_bits_from_each_of_its_kernels():
-    """A row's result is one chain of fused multiply-adds in the order of K in every kernel: the
-    streaming kernel (8 rows), the tile kernel (200 rows) and the plain kernel (operands whose rows
+    """A row's result is the sum of eight chains of fused multiply-adds over ranges of K in every kernel: the
+    rows kernel (8 rows), the tile kernel (200 and 40 rows) and the plain kernel (operands whose rows
     are not 16-byte aligned) agree bit for bit, also where tiles end inside the matrix."""
     M, N, K = 200, 333, 712
     a = torch.randn(M, K, device=DEV)
@@ -120,7 +120,7 @@ def test_gemm_f32_gives_the_same_bits_from_each_of_its_kernels():
     tile = ops().gemm_f32(a, w)
     rows = ops().gemm_f32(a[:8].contiguous(), w)
     assert torch.equal(rows, tile[:8])
-    mid = ops().gemm_f32(a[100:140].contiguous(), w)            # 40 rows: three row blocks of the streaming kernel
+    mid = ops().gemm_f32(a[100:140].contiguous(), w)            # 40 rows: one tile of rows, partly filled
     assert torch.equal(mid, tile[100:140])
     a_odd = torch.zeros(M, K + 1, device=DEV)[:, :K]            # row stride K + 1: the plain kernel
     a_odd.copy_(a)
@@ -129,9 +129,10 @@ def test_gemm_f32_gives_the_same_bits_from_each_of_its_kernels():
     assert torch.allclose(tile.double(), a.double() @ w.double().T, atol=1e-5 * math.sqrt(K), rtol=1e-5)
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 8192, 2048), (3, 8193, 36), (8, 14208, 520), (6, 19001, 132), (16, 9500, 1028)])
+@pytest.mark.parametrize("M,N,K", [(1, 8192, 2048), (3, 8193, 36), (8, 14208, 520), (6, 19001, 132), (16, 9500, 1028),
+                                   (17, 4096, 132), (24, 300, 520), (32, 8193, 36), (31, 6000, 132)])
 def test_gemm_f32_of_few_rows_and_many_columns(M, N, K):
-    """Blocks that walk several tiles of columns, ragged last ones, ranges of K shorter than a stage or empty: the bits of
+    """Up to 16 rows in one launch, up to 32 in two (4,096 columns and fewer, 8,192 and more); blocks that walk several tiles of columns, ragged last ones, ranges of K shorter than a stage or empty: the bits of
     the tile kernel, which adds in the same order."""
     g = torch.Generator().manual_seed(N)
     a = torch.randn(40, K, generator=g).to(DEV)
