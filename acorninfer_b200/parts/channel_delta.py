@@ -87,7 +87,7 @@ class ChannelDelta(Mixer):
             min_row = ops.chunk_min_row(lens, ops.CHANNEL_CHUNK_ROWS)
         q, k, v, beta, g, gate = ops.delta_prep(main, up, self.conv32, cache.state, self.state_s, self.a_log32,
                                                 self.dt_bias32, inputs.token_row, inputs.row_start, inputs.row_slot,
-                                                self.H, self.KH, self.dim, self.vdim, self.taps, log2_decays=min_row)
+                                                self.H, self.KH, self.dim, self.vdim, self.taps, log2_decays=1 if min_row and min(lens) >= min_row else min_row)
         ops.conv_state_update(main, cache.state, self.state_s, inputs.row_start, inputs.row_slot, inputs.num_rows,
                               self.channels, self.taps)
         o, rows = None, (cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)

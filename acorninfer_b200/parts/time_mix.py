@@ -81,7 +81,7 @@ class TimeMix(Mixer):
         d, lens, min_row = r.shape[1] // self.H, inputs.plan.row_lens, 0
         if cache.state.stride(0) % 4 == 0 and ops.channel_chunk_ok(inputs.plan.max_q_len, T, inputs.num_rows, self.H, d, d):
             min_row = ops.chunk_min_row(lens, ops.MIX_CHUNK_ROWS)
-        r32, k32, v32, decay, gate = ops.wkv_prep(r, k, v, g, z, self.w0_32, self.H, log2_decays=min_row,
+        r32, k32, v32, decay, gate = ops.wkv_prep(r, k, v, g, z, self.w0_32, self.H, log2_decays=1 if min_row and min(lens) >= min_row else min_row,
                                                   token_row=inputs.token_row, row_start=inputs.row_start)
         o, rows = None, (cache.state, inputs.row_start, inputs.row_slot, inputs.num_rows)
         if min_row:
