@@ -1550,13 +1550,13 @@ def latent_prefill_wins(num_tiles: int, general_tiles: int, key_bound: int, head
     are, but for a tile on an SM at a time; with few tiles it shares their keys out.  Measured (B200, us, general / tcgen05):
     rows of 448 with 384 values, 16 heads: 64 requests decoding at 1,000 keys 82 / 53, 56 at 4,000 300 / 189, at 250 keys 64
     requests 27 / 18, a prompt of 300 tokens 39 / 26, of 2,000 493 / 99; rows of 192 with 128 values: 56 requests at 4,000 keys
-    104 / 123, 64 at 1,000 34 / 35, 41 at 700 beside a prompt of 200 (91 tiles) 53 / 29, a prompt of 2,000 187 / 53, at 60 keys
+    104 / 123, 64 at 1,000 34 / 35, a prompt of 300 (75 tiles) 20 / 14, 41 requests at 700 beside a prompt of 200 (91 tiles) 53 / 29, a prompt of 2,000 187 / 53, at 60 keys
     300 requests 14 / 21 (two waves with next to nothing to do); rows of 128 with 64 values, 2 heads: 64 requests at 1,000 keys
     26 / 32, a prompt of 2,000 46 / 55, behind 4,000 120 / 154."""
     width = head_dim + value_dim
     if width < 256 or (key_bound <= 128 and num_tiles > 148):
         return False
-    return general_tiles >= (56 if width >= 512 else 80) or key_bound <= 256
+    return general_tiles >= (56 if width >= 512 else 64 if key_bound <= 512 else 80) or key_bound <= 256
 
 
 def latent_prefill_tc(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tensor, page_base: torch.Tensor,

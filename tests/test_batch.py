@@ -234,5 +234,6 @@ def test_which_latent_steps_take_the_tcgen05_kernel():
     wide, narrow, small = (448, 384), (192, 128), (128, 64)
     assert latent_prefill_wins(56, 56, 4096, *wide) and not latent_prefill_wins(48, 48, 4096, *wide)
     assert latent_prefill_wins(250, 500, 2048, *narrow) and not latent_prefill_wins(64, 64, 1024, *narrow)
+    assert latent_prefill_wins(38, 75, 512, *narrow) and not latent_prefill_wins(40, 40, 512, *narrow)
     assert latent_prefill_wins(1, 1, 256, *narrow) and not latent_prefill_wins(300, 300, 128, *narrow)
     assert not latent_prefill_wins(32, 63, 8192, *small) and not latent_prefill_wins(1, 1, 128, *small)
