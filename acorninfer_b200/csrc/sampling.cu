@@ -181,32 +181,51 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
 // ------------------------------------------------------------------ a cluster a row, the row in shared memory
 //
 // What bounds the walk above is one SM reading its row again for each of up to 64 bisection steps (64 rows of 151,936
-// with top-k and top-p: 701 us).  Here the CTAs of a cluster hold the row in shared memory, read from HBM once, and the
-// bounds of top-k and top-p are found digit by digit (11 + 11 + 10 bits of the ordered key): a histogram of the
-// candidates a level, summed over the cluster through distributed shared memory.  Both are one question: the smallest
-// key K with weight(keys <= K) > limit, where a key weighs 1 and limit is the number of keys less k (the k-th largest), or
-// weighs its probability and limit is (1 - top_p) of the total.  Most keys are no candidates and cost no atomic: for k up
-// to the number of warps, those below the least of the warps' maxima; for top-p, those so improbable that all of them
-// together would stay within the limit.  Probabilities are summed as integers of 2^-44 of the largest one (a sum's error
-// is below that of float32 sums, and its order does not matter).
+// with top-k and top-p: 701 us).  Here the CTAs of a cluster hold the row in shared memory, read from HBM once.
+//   top-k up to the number of warps (128): the k-th largest of the warps' maxima bounds the k-th largest key from below and
+//     leaves few more than k candidates; the first CTA gathers them and ends alone (`sc_finish`), every pair compared.
+//   top-p alone: one histogram of the probabilities in equal steps of the scaled logit, summed over the cluster through
+//     distributed shared memory; the keys of the one bin that holds the bound are gathered by every CTA and compared.
+//   anything else, and rows whose candidates do not fit the lists (many equal logits): the bounds digit by digit (11 + 11 + 10
+//     bits of the ordered key), a histogram a level (`sc_select`).
+// All three ask the same: the smallest key K with weight(keys <= K) > limit, where a key weighs 1 and limit is the number of
+// keys less k (the k-th largest), or weighs its probability and limit is (1 - top_p) of the total.  Probabilities are summed
+// as integers of 2^-44 of the largest one (a sum's error is below that of float32 sums, and its order does not matter), so the
+// three answers are the same.
+// What bounds it: 64 clusters of 8 on 148 SMs are two waves (two CTAs an SM: shared memory), each a read of its slices and a
+// chain of short steps with cluster barriers between them.
 #define SC_THREADS 512
 #define SC_WARPS (SC_THREADS / 32)
 #define SC_BINS 2048
 #define SC_CLUSTER 8
+#define SC_MAXIMA (SC_CLUSTER * SC_WARPS)
+#define SC_CAND 256                 // candidates a CTA can note
+#define SC_LIST 1024                // candidates of a row that are compared in pairs
+#define SC_STEPS 128.f              // bins of the first histogram by probability to a factor of e
 #define SC_MAX_SLICE 45056          // floats of a row a CTA can hold beside the histogram
 typedef unsigned long long u64;
 
 struct alignas(16) ScShared {
     u64 sums[SC_BINS / SC_CLUSTER]; // this CTA's share of a level's bins, summed over the cluster
-    unsigned int hist[3][SC_BINS];  // a level's weights: 16-bit pieces, so that 32-bit atomics cannot overflow
+    union {
+        unsigned int hist[3][SC_BINS];  // a level's weights: 16-bit pieces, so that 32-bit atomics cannot overflow
+        struct {
+            u64 list[SC_LIST];          // gathered candidates: (key, index)
+            u64 w[SC_LIST];             // their weights
+        };
+    };
+    u64 cand[SC_CAND];              // candidates of this CTA's slice
+    u64 tops[SC_WARPS];             // its warps' maxima: (key, ~index)
+    u64 maxima[SC_MAXIMA];          // those of the whole row
+    unsigned int ncand;             // candidates met (more than SC_CAND: not all are noted)
+    unsigned int lowest;            // a bound of the k-th largest key, or the least key found
     u64 total;                      // of `sums`
     u64 kept;                       // this CTA's part of the kept set
     u64 best;                       // largest (key, ~index) of this CTA's slice
-    unsigned int low;               // key of the least of its warps' maxima
     u64 z;                          // probability of its slice
     unsigned int bad;
     u64 warp_a[SC_WARPS];
-    u64 found_cum;                  // answer of a level: weight below the bin, the bin (SC_BINS: limit not exceeded)
+    u64 left;                       // answer of a level: the limit less the weight below the bin, the bin (SC_BINS: limit not exceeded)
     unsigned int found_bin;
 };
 
@@ -233,16 +252,192 @@ __device__ __forceinline__ u64 block_sum_u64(u64 v, u64* scratch) {
     return warp_sum_u64((threadIdx.x & 31) < SC_WARPS ? scratch[threadIdx.x & 31] : 0ull);
 }
 
+__device__ __forceinline__ float key_float(unsigned int key) {
+    return __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key);
+}
+
+// Adds a probability to a bin, in pieces of 16 bits.
+__device__ __forceinline__ void sc_add_mass(ScShared& sh, int bin, u64 w) {
+    atomicAdd(&sh.hist[0][bin], (unsigned int)w & 0xffffu);
+    if (w >> 16) atomicAdd(&sh.hist[1][bin], (unsigned int)(w >> 16) & 0xffffu);
+    if (w >> 32) atomicAdd(&sh.hist[2][bin], (unsigned int)(w >> 32));
+}
+
+// Notes element i of this CTA's slice, whose logit has this key, as a candidate (index i0 + i of the row).
+__device__ __forceinline__ void sc_note(ScShared& sh, unsigned int key, int at) {
+    const unsigned int slot = atomicAdd(&sh.ncand, 1u);
+    if (slot < SC_CAND) sh.cand[slot] = ((u64)key << 32) | (unsigned int)at;
+}
+
+// The cluster has noted its candidates: brings them all into `sh.list` (of the CTAs that `take` them) and returns their number,
+// or -1 where they do not fit, the same in every CTA.  The caller's cluster barrier ends the reads of other CTAs' notes.
+__device__ int sc_gather(ScShared& sh, bool take) {
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    int first[SC_CLUSTER + 1];
+    bool fits = true;
+    first[0] = 0;
+#pragma unroll
+    for (int q = 0; q < SC_CLUSTER; ++q) {
+        const unsigned int c = *cluster.map_shared_rank(&sh.ncand, q);
+        fits = fits && c <= SC_CAND;
+        first[q + 1] = first[q] + (int)min(c, (unsigned int)SC_CAND);
+    }
+    if (!fits || first[SC_CLUSTER] > SC_LIST) return -1;
+    if (take) {
+        const int warp = threadIdx.x >> 5;       // two warps bring a CTA's notes
+        const int q = warp / (SC_WARPS / SC_CLUSTER);
+        int at = 0, c = 0;
+#pragma unroll
+        for (int i = 0; i < SC_CLUSTER; ++i)
+            if (i == q) { at = first[i]; c = first[i + 1] - first[i]; }
+        const u64* notes = cluster.map_shared_rank(&sh.cand[0], q);
+        for (int i = threadIdx.x % (SC_THREADS / SC_CLUSTER); i < c; i += SC_THREADS / SC_CLUSTER) sh.list[at + i] = notes[i];
+    }
+    __syncthreads();
+    return first[SC_CLUSTER];
+}
+
+// top-k, top-p and the draw among `n` gathered candidates that hold the row's k largest keys: one CTA, every pair compared.
+__device__ void sc_finish(ScShared& sh, int n, int k, float p_keep, unsigned int gkey, float gmax, float inv_t, int arg, u64 m, int* token,
+                          float* logprob) {
+    const int tid = threadIdx.x;
+    u64 z = 0;
+    for (int t = tid; t < n; t += SC_THREADS) {
+        const unsigned int key = (unsigned int)(sh.list[t] >> 32);
+        int greater = 0;
+        for (int j = 0; j < n; ++j) greater += (unsigned int)(sh.list[j] >> 32) > key;
+        const u64 w = greater < k ? prob_fixed(key_float(key), gmax, inv_t) : 0ull;       // kept: no less than the k-th largest
+        sh.w[t] = w;
+        z += w;
+    }
+    z = block_sum_u64(z, sh.warp_a);
+    __syncthreads();
+    if (p_keep < 1.f) {
+        const u64 bound = (u64)((double)(1.f - p_keep) * (double)z);
+        u64 own[SC_LIST / SC_THREADS] = {};
+        z = 0;
+#pragma unroll
+        for (int e = 0; e < SC_LIST / SC_THREADS; ++e) {
+            const int t = tid + e * SC_THREADS;
+            if (t >= n) break;
+            const unsigned int key = (unsigned int)(sh.list[t] >> 32);
+            u64 upto = 0;
+            for (int j = 0; j < n; ++j) upto += (unsigned int)(sh.list[j] >> 32) <= key ? sh.w[j] : 0ull;
+            own[e] = upto > bound || key >= gkey ? sh.w[t] : 0ull;                        // the largest always stays
+            z += own[e];
+        }
+        z = block_sum_u64(z, sh.warp_a);
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < SC_LIST / SC_THREADS; ++e)
+            if (tid + e * SC_THREADS < n) sh.w[tid + e * SC_THREADS] = own[e];
+        __syncthreads();
+    }
+    // u = m / 2^24: the first token whose running sum exceeds floor(m z / 2^24)
+    const u64 target = (__umul64hi(m, z) << 40) | ((m * z) >> 24);
+    for (int t = tid; t < n; t += SC_THREADS) {
+        const unsigned int at = (unsigned int)sh.list[t];
+        u64 before = 0;
+        for (int j = 0; j < n; ++j) before += (unsigned int)sh.list[j] < at ? sh.w[j] : 0ull;
+        if (target >= before && target < before + sh.w[t]) {
+            *token = (int)at;
+            if (logprob) *logprob = (key_float((unsigned int)(sh.list[t] >> 32)) - gmax) * inv_t - logf((float)((double)z * 5.684341886080802e-14));
+        }
+    }
+    if (z == 0 && tid == 0) {
+        *token = arg;
+        if (logprob) *logprob = 0.f;
+    }
+}
+
+// Sums this level's bins over the cluster and finds the first at which the weight so far exceeds the limit, which `limit_of`
+// gives from the sum of all: `sh.found_bin` (SC_BINS: none) and `sh.left`, the limit less the weight before that bin.
+// Called by all threads of the cluster after they have added to `sh.hist`.
+template <bool MASS, typename LimitOf>
+__device__ void sc_find_bin(ScShared& sh, int bins, LimitOf limit_of) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31;
+    constexpr int PIECES = MASS ? 3 : 1;
+    cluster.sync();
+    // this CTA sums its share of the bins over the cluster (all remote reads of a bin in flight at once)
+    const int share = bins / SC_CLUSTER, first = (int)cluster.block_rank() * share;
+    u64 mine = 0;
+    for (int i = tid; i < share; i += SC_THREADS) {
+        unsigned int h[SC_CLUSTER][PIECES];
+#pragma unroll
+        for (int r = 0; r < SC_CLUSTER; ++r)
+#pragma unroll
+            for (int q = 0; q < PIECES; ++q) h[r][q] = cluster.map_shared_rank(&sh.hist[q][0], r)[first + i];
+        u64 s = 0;
+#pragma unroll
+        for (int r = 0; r < SC_CLUSTER; ++r) {
+            s += h[r][0];
+            if (MASS) s += ((u64)h[r][PIECES / 2] << 16) + ((u64)h[r][PIECES - 1] << 32);
+        }
+        sh.sums[i] = s;
+        mine += s;
+    }
+    mine = block_sum_u64(mine, sh.warp_a);
+    if (tid == 0) sh.total = mine;
+    cluster.sync();
+    // one warp finds the bin: first the CTA whose share holds it, then the bin in that share
+    if (tid < 32) {
+        const u64 t = lane < SC_CLUSTER ? *cluster.map_shared_rank(&sh.total, lane) : 0ull;
+        u64 incl = t;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const u64 up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        const u64 all = __shfl_sync(0xffffffffu, incl, SC_CLUSTER - 1);
+        const u64 limit = limit_of(all);
+        const unsigned int over = __ballot_sync(0xffffffffu, lane < SC_CLUSTER && incl > limit);
+        if (over == 0) {
+            if (lane == 0) sh.found_bin = SC_BINS;
+        } else {
+            const int owner = __ffs(over) - 1;
+            u64 run = __shfl_sync(0xffffffffu, incl - t, owner);
+            const u64* sums = cluster.map_shared_rank(&sh.sums[0], owner);
+            constexpr int PER = SC_BINS / SC_CLUSTER / 32;                // a lane's bins (the last level has half as many)
+            const int per = share / 32;
+            u64 own[PER], part = 0;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) own[i] = i < per ? sums[lane * per + i] : 0ull;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) part += own[i];
+            u64 pin = part;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const u64 up = __shfl_up_sync(0xffffffffu, pin, o);
+                if (lane >= o) pin += up;
+            }
+            const int who = __ffs(__ballot_sync(0xffffffffu, run + pin > limit)) - 1;
+            if (lane == who) {
+                run += pin - part;
+                int i = 0;
+                bool on = true;
+#pragma unroll
+                for (int k = 0; k < PER; ++k) {
+                    on = on && run + own[k] <= limit;
+                    if (on) { run += own[k]; ++i; }
+                }
+                sh.found_bin = owner * share + lane * per + i;
+                sh.left = limit - run;
+            }
+        }
+    }
+    __syncthreads();
+}
+
 // The smallest key K of the row from `cut` on with weight(keys <= K) > limit; 0xffffffff if there is none.  MASS: keys from
 // lo_key on weigh their probability, the total is z, the limit (1 - top_p) z; else keys weigh 1 and the limit leaves k above
 // it.  No key below `cut` is K.  Called by all threads of the cluster with the same arguments.
 template <bool MASS>
 __device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigned int cut, float gmax, float inv_t, u64 z, u64 bound) {
-    cg::cluster_group cluster = cg::this_cluster();
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x;
     constexpr int PIECES = MASS ? 3 : 1;
     unsigned int prefix = 0;        // the digits found so far
-    u64 limit = 0;
 #pragma unroll 1
     for (int level = 0; level < 3; ++level) {
         const int shift = level == 0 ? 21 : level == 1 ? 10 : 0;
@@ -256,87 +451,13 @@ __device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigne
             const int bin = (key >> shift) & (bins - 1);
             if (MASS) {
                 const u64 w = prob_fixed(v, gmax, inv_t);
-                if (w == 0) continue;
-                atomicAdd(&sh.hist[0][bin], (unsigned int)w & 0xffffu);
-                if (w >> 16) atomicAdd(&sh.hist[1][bin], (unsigned int)(w >> 16) & 0xffffu);
-                if (w >> 32) atomicAdd(&sh.hist[2][bin], (unsigned int)(w >> 32));
+                if (w != 0) sc_add_mass(sh, bin, w);
             } else {
                 atomicAdd(&sh.hist[0][bin], 1u);
             }
         }
-        cluster.sync();
-        // this CTA sums its share of the bins over the cluster (all remote reads of a bin in flight at once)
-        const int share = bins / SC_CLUSTER, first = (int)cluster.block_rank() * share;
-        u64 mine = 0;
-        for (int i = tid; i < share; i += SC_THREADS) {
-            unsigned int h[SC_CLUSTER][PIECES];
-#pragma unroll
-            for (int r = 0; r < SC_CLUSTER; ++r)
-#pragma unroll
-                for (int q = 0; q < PIECES; ++q) h[r][q] = cluster.map_shared_rank(&sh.hist[q][0], r)[first + i];
-            u64 s = 0;
-#pragma unroll
-            for (int r = 0; r < SC_CLUSTER; ++r) {
-                s += h[r][0];
-                if (MASS) s += ((u64)h[r][PIECES / 2] << 16) + ((u64)h[r][PIECES - 1] << 32);
-            }
-            sh.sums[i] = s;
-            mine += s;
-        }
-        mine = block_sum_u64(mine, sh.warp_a);
-        if (tid == 0) sh.total = mine;
-        cluster.sync();
-        // one warp finds the bin: first the CTA whose share holds it, then the bin in that share
-        if (tid < 32) {
-            const u64 t = lane < SC_CLUSTER ? *cluster.map_shared_rank(&sh.total, lane) : 0ull;
-            u64 incl = t;
-#pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-                const u64 up = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += up;
-            }
-            const u64 all = __shfl_sync(0xffffffffu, incl, SC_CLUSTER - 1);
-            // counted from the cut on: less what lies below it
-            if (level == 0) limit = MASS ? bound - (z - all) : all - bound;
-            const unsigned int over = __ballot_sync(0xffffffffu, lane < SC_CLUSTER && incl > limit);
-            if (over == 0) {
-                if (lane == 0) sh.found_bin = SC_BINS;
-            } else {
-                const int owner = __ffs(over) - 1;
-                u64 run = __shfl_sync(0xffffffffu, incl - t, owner);
-                const u64* sums = cluster.map_shared_rank(&sh.sums[0], owner);
-                constexpr int PER = SC_BINS / SC_CLUSTER / 32;                // a lane's bins (the last level has half as many)
-                const int per = share / 32;
-                u64 own[PER], part = 0;
-#pragma unroll
-                for (int i = 0; i < PER; ++i) own[i] = i < per ? sums[lane * per + i] : 0ull;
-#pragma unroll
-                for (int i = 0; i < PER; ++i) part += own[i];
-                u64 pin = part;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const u64 up = __shfl_up_sync(0xffffffffu, pin, o);
-                    if (lane >= o) pin += up;
-                }
-                const int who = __ffs(__ballot_sync(0xffffffffu, run + pin > limit)) - 1;
-                if (lane == who) {
-                    run += pin - part;
-                    int i = 0;
-                    bool on = true;
-#pragma unroll
-                    for (int k = 0; k < PER; ++k) {
-                        on = on && run + own[k] <= limit;
-                        if (on) { run += own[k]; ++i; }
-                    }
-                    sh.found_bin = owner * share + lane * per + i;
-                    sh.found_cum = run;
-                }
-            }
-            __syncwarp();
-            limit = __shfl_sync(0xffffffffu, limit, 0);
-            if (sh.found_bin != SC_BINS) limit -= sh.found_cum;
-        }
-        __syncthreads();
+        // counted from the cut on: less what lies below it
+        sc_find_bin<MASS>(sh, bins, [&](u64 all) { return level > 0 ? sh.left : MASS ? bound - (z - all) : all - bound; });
         if (sh.found_bin == SC_BINS) return 0xffffffffu;
         prefix = (prefix << (level == 0 ? 11 : level == 1 ? 11 : 10)) | sh.found_bin;
     }
@@ -387,28 +508,26 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
         const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
         best = other > best ? other : best;
     }
-    if (tid == 0) sh.bad = 0;
-    if (lane == 0) sh.warp_a[warp] = best;
+    if (tid == 0) { sh.bad = 0; sh.ncand = 0; }
+    if (lane == 0) sh.tops[warp] = best;
     __syncthreads();
     if (bad) sh.bad = 1;
-    if (tid == 0) {
-        u64 least = best;
-        for (int w = 0; w < SC_WARPS; ++w) {
-            best = sh.warp_a[w] > best ? sh.warp_a[w] : best;
-            least = sh.warp_a[w] < least ? sh.warp_a[w] : least;
-        }
-        sh.best = best;
-        sh.low = (unsigned int)(least >> 32);
-    }
+    const int k = top_k[r];
+    const float p_keep = top_p[r];
+    const u64 m = (u64)(uniform_from(seed[r], counter[r]) * 16777216.f);       // u = m / 2^24
     cluster.sync();
+    if (tid < SC_MAXIMA) sh.maxima[tid] = cluster.map_shared_rank(&sh.tops[0], tid / SC_WARPS)[tid % SC_WARPS];
     bad = 0;
-    unsigned int low = 0xffffffffu;
 #pragma unroll
-    for (int k = 0; k < SC_CLUSTER; ++k) {
-        const u64 b = *cluster.map_shared_rank(&sh.best, k);
-        best = k == 0 || b > best ? b : best;
-        bad |= *cluster.map_shared_rank(&sh.bad, k);
-        low = min(low, *cluster.map_shared_rank(&sh.low, k));
+    for (int q = 0; q < SC_CLUSTER; ++q) bad |= *cluster.map_shared_rank(&sh.bad, q);
+    __syncthreads();
+    best = 0;
+#pragma unroll
+    for (int q = 0; q < SC_MAXIMA / 32; ++q) best = max(best, sh.maxima[lane + 32 * q]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other > best ? other : best;
     }
     const int arg = (int)~(unsigned int)best;
     if (bad || !(temp > 0.f)) {
@@ -420,32 +539,93 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
         return;
     }
     const unsigned int gkey = (unsigned int)(best >> 32);
-    const float gmax = __uint_as_float((gkey & 0x80000000u) ? gkey & 0x7fffffffu : ~gkey);
+    const float gmax = key_float(gkey);
     const float inv_t = 1.f / temp;
     unsigned int lo_key = 0u;
-    const int k = top_k[r];
-    if (k > 0 && k < V) {
-        // as many warps as k each hold a key from `low` on, so the k-th largest is one (a maximum of -0 counts as 0 there)
-        if (low == float_key(0.f)) low = float_key(-0.f);
-        lo_key = sc_select<false>(sh, row, n, k <= SC_CLUSTER * SC_WARPS ? low : 0u, 0.f, 0.f, 0ull, (u64)k);
+    const bool by_k = k > 0 && k < V;
+    if (by_k) {
+        unsigned int low = 0u;
+        if (k <= SC_MAXIMA) {
+            // The k-th largest of the warps' maxima: k warps hold a key from it on, so the k-th largest key is one (a maximum of
+            // -0 counts as 0 there).  Its rank by comparison, equal ones (warps without an element) in their order.
+            if (tid < SC_MAXIMA) {
+                const u64 own = sh.maxima[tid];
+                int before = 0;
+                for (int j = 0; j < SC_MAXIMA; ++j) before += sh.maxima[j] > own || (sh.maxima[j] == own && j < tid);
+                if (before == k - 1) sh.lowest = (unsigned int)(own >> 32);
+            }
+            __syncthreads();
+            low = sh.lowest;
+            if (low == float_key(0.f)) low = float_key(-0.f);
+            for (int i = tid; i < n; i += SC_THREADS) {
+                const unsigned int key = float_key(row[i]);
+                if (key >= low) sc_note(sh, key, i0 + i);
+            }
+            const int found = sc_gather(sh, rank == 0);
+            if (found >= 0) {
+                cluster.sync();      // the others' notes have been read
+                if (rank == 0)
+                    sc_finish(sh, found, k, p_keep, gkey, gmax, inv_t, arg, m, token_out + r, logprob_out ? logprob_out + r : nullptr);
+                return;
+            }
+        }
+        lo_key = sc_select<false>(sh, row, n, low, 0.f, 0.f, 0ull, (u64)k);
     }
-    const float p_keep = top_p[r];
     if (p_keep < 1.f) {
-        u64 part = 0;
-        for (int i = tid; i < n; i += SC_THREADS)
-            if (float_key(row[i]) >= lo_key) part += prob_fixed(row[i], gmax, inv_t);
-        part = block_sum_u64(part, sh.warp_a);
-        if (tid == 0) sh.z = part;
-        cluster.sync();
-        u64 z = 0;
+        // (1 - top_p) of all that is kept so far
+        auto limit_of = [&](u64 all) { return (u64)((double)(1.f - p_keep) * (double)all); };
+        int found = -1;
+        if (!by_k) {
+            // the bins ascend with the key: SC_STEPS a factor of e in probability, what is further down in the first
+            auto bin_of = [&](float v) { return SC_BINS - 1 - (int)fminf((gmax - v) * inv_t * SC_STEPS, (float)(SC_BINS - 1)); };
+            for (int i = tid; i < 3 * SC_BINS; i += SC_THREADS) (&sh.hist[0][0])[i] = 0;
+            __syncthreads();
+            for (int i = tid; i < n; i += SC_THREADS) {
+                const u64 w = prob_fixed(row[i], gmax, inv_t);
+                if (w != 0) sc_add_mass(sh, bin_of(row[i]), w);
+            }
+            sc_find_bin<true>(sh, SC_BINS, limit_of);
+            const int bin = (int)sh.found_bin;
+            lo_key = gkey;           // the largest always stays
+            if (bin == SC_BINS) {
+                found = 0;
+            } else {
+                for (int i = tid; i < n; i += SC_THREADS) {
+                    const float v = row[i];
+                    if (bin_of(v) == bin && prob_fixed(v, gmax, inv_t) != 0) sc_note(sh, float_key(v), i0 + i);
+                }
+                if (tid == 0) sh.lowest = gkey;
+                found = sc_gather(sh, true);
+                for (int t = tid; t < found; t += SC_THREADS) sh.w[t] = prob_fixed(key_float((unsigned int)(sh.list[t] >> 32)), gmax, inv_t);
+                __syncthreads();
+                for (int t = tid; t < found; t += SC_THREADS) {
+                    const unsigned int key = (unsigned int)(sh.list[t] >> 32);
+                    u64 upto = 0;
+                    for (int j = 0; j < found; ++j) upto += (unsigned int)(sh.list[j] >> 32) <= key ? sh.w[j] : 0ull;
+                    if (upto > sh.left) atomicMin(&sh.lowest, key);
+                }
+                __syncthreads();
+                if (found >= 0) lo_key = sh.lowest;
+                else lo_key = 0u;
+            }
+        }
+        if (found < 0) {
+            u64 part = 0;
+            for (int i = tid; i < n; i += SC_THREADS)
+                if (float_key(row[i]) >= lo_key) part += prob_fixed(row[i], gmax, inv_t);
+            part = block_sum_u64(part, sh.warp_a);
+            if (tid == 0) sh.z = part;
+            cluster.sync();
+            u64 z = 0;
 #pragma unroll
-        for (int q = 0; q < SC_CLUSTER; ++q) z += *cluster.map_shared_rank(&sh.z, q);
-        const u64 bound = (u64)((double)(1.f - p_keep) * (double)z);
-        // V keys of half of bound / V each stay within the bound
-        const float least = 0.5f * (float)((double)bound / V * 5.684341886080802e-14);
-        const unsigned int cut = least > 1e-12f ? float_key(gmax + temp * logf(least)) : 0u;
-        const unsigned int found = sc_select<true>(sh, row, n, max(cut, lo_key), gmax, inv_t, z, bound);
-        lo_key = found < gkey ? found : gkey;        // the largest always stays
+            for (int q = 0; q < SC_CLUSTER; ++q) z += *cluster.map_shared_rank(&sh.z, q);
+            const u64 bound = limit_of(z);
+            // V keys of half of bound / V each stay within the bound
+            const float least = 0.5f * (float)((double)bound / V * 5.684341886080802e-14);
+            const unsigned int cut = least > 1e-12f ? float_key(gmax + temp * logf(least)) : 0u;
+            const unsigned int key = sc_select<true>(sh, row, n, max(cut, lo_key), gmax, inv_t, z, bound);
+            lo_key = key < gkey ? key : gkey;            // the largest always stays
+        }
     }
     // inverse CDF in token order over the kept set; a thread owns a run of the slice (of odd length: no bank conflicts)
     const int seg = ((n + SC_THREADS - 1) / SC_THREADS) | 1;
@@ -477,8 +657,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
         if (q < rank) before += t;
         total += t;
     }
-    // u = m / 2^24: the first token whose running sum exceeds floor(m total / 2^24)
-    const u64 m = (u64)(uniform_from(seed[r], counter[r]) * 16777216.f);
+    // the first token whose running sum exceeds floor(m total / 2^24)
     const u64 target = (__umul64hi(m, total) << 40) | ((m * total) >> 24);
     if (target >= before && target < before + mine) {
         int i = a;

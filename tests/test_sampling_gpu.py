@@ -140,3 +140,23 @@ def test_top_k_at_the_cut_by_the_warps_maxima(k):
         # every token of a small kept set turns up as often as it should (four standard deviations)
         freq = torch.bincount(toks[r].long(), minlength=V).double() / n
         assert ((freq - p).abs() <= 4 * (p / n).sqrt() + 4 / n).all(), (r, k)
+
+
+@pytest.mark.parametrize("n,spread", [(256, False), (257, False), (1024, True), (1025, True)])
+@pytest.mark.parametrize("top_k,top_p", [(64, 1.0), (128, 0.5), (0, 0.5), (0, 0.0)])
+def test_candidates_at_the_ends_of_the_lists(n, spread, top_k, top_p):
+    """``n`` equal logits above all others, in one CTA's slice (which notes 256 candidates) or all over the row (of which
+    1,024 are compared): with ties kept whole, top-k and top-p leave exactly these, each as likely as any other."""
+    from acorninfer_b200.kernels import ops
+    V, draws = 40000, 64
+    x = torch.full((1, V), -20.0)
+    at = torch.arange(n) * (39 if spread else 1) + 3
+    x[0, at] = 7.25
+    f = lambda v, dt: torch.full((draws,), v, dtype=dt, device=DEV)
+    toks, lps = ops.sample(x.expand(draws, V).contiguous().to(DEV), f(0.8, torch.float32), f(top_k, torch.int32),
+                           f(top_p, torch.float32), f(9, torch.int64), torch.arange(draws, device=DEV), True)
+    u = [ops.uniform(9, i) for i in range(draws)]
+    # equal probabilities of 2^44 units each: the draw is exact
+    assert toks.tolist() == [int(at[int(int(v * 2 ** 24) * n // 2 ** 24)]) for v in u]
+    # -ln n in float32: one rounding of the logarithm's argument and one of its result
+    assert (lps.cpu().double() + torch.tensor(float(n)).double().log()).abs().max() < 4 * 2.0 ** -24 * 8
