@@ -12,9 +12,11 @@ import ctypes
 from ctypes import c_float, c_int, c_int64, c_void_p
 from dataclasses import dataclass
 from functools import lru_cache
+from types import SimpleNamespace
 
 import torch
 
+from . import calls
 from .build import ensure_built
 
 
@@ -38,18 +40,39 @@ def _load():
         if not torch.cuda.is_available():
             raise KernelError("acorninfer_b200 needs a CUDA device (sm_100a); none is visible and there is no CPU path")
         path = ensure_built()
-        _lib = ctypes.CDLL(str(path))
-        for name in dir(_Sigs):
-            if name.startswith("acorn_"):
-                fn = getattr(_lib, name, None)
-                if fn is None:
-                    raise KernelError(f"{path} lacks the symbol {name}: stale build?")
-                fn.argtypes = getattr(_Sigs, name)
-                fn.restype = c_int
-        _lib.acorn_uniform.restype = c_float
-        _lib.acorn_min_gru_scratch.restype = c_int64
-        _init_error_word(_lib)
+        library = ctypes.CDLL(str(path))
+        functions = {}
+        for name in _signatures():
+            fn = getattr(library, name, None)
+            if fn is None:
+                raise KernelError(f"{path} lacks the symbol {name}: stale build?")
+            fn.argtypes = getattr(_Sigs, name)
+            fn.restype = _RESULTS.get(name, c_int)
+            functions[name] = fn
+        _init_error_word(library)
+        functions.update(calls.load(_typed_signatures(), path, path.parent))
+        _lib = SimpleNamespace(**functions)
     return _lib
+
+
+# What a function returns where it is no error code.
+_RESULTS = {"acorn_uniform": c_float, "acorn_min_gru_scratch": c_int64}
+
+
+def _signatures() -> list[str]:
+    return [name for name in dir(_Sigs) if name.startswith("acorn_")]
+
+
+def _typed_signatures() -> dict[str, tuple[list, object]]:
+    """Argument and result types of the functions that the call extension takes: those whose arguments are pointers as
+    integers, integers and floats."""
+    others = {"acorn_uniform", "acorn_random_fill", "acorn_error_word_alloc"}       # 64-bit unsigned, pointers by reference
+    return {name: (getattr(_Sigs, name), _RESULTS.get(name, c_int)) for name in _signatures() if name not in others}
+
+
+def build_calls() -> None:
+    """Compiles the call extension beside the kernel library (``_load`` does so on first use)."""
+    calls.build(_typed_signatures(), ensure_built().parent)
 
 
 _error_word: ctypes.c_int | None = None       # pinned host memory that kernels write when a bounded wait gives up
