@@ -2,7 +2,7 @@
 // operands staged by TMA, accumulators in tensor memory.
 //
 // The weight matrix takes the 128-row side of the MMA ("swap-AB"): a CTA owns 128 rows of W
-// (output columns n0 .. n0+127) and MB tokens (MB = 16 .. 256), so that a decode step with few
+// (output columns n0 .. n0+127) and MB tokens (MB = 16 .. 128), so that a decode step with few
 // tokens still fills the instruction and the kernel streams W once at memory speed.  Per
 // 64-element step along K, TMA brings a [128 x 64] tile of W and a [MB x 64] tile of x into a
 // ring of shared-memory stages (128-byte swizzle, K-major); one elected thread issues four
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
     constexpr int A_BYTES = TC_BM * TC_BK * 2;           // 16 KB
     constexpr int B_BYTES = MB * TC_BK * 2;
     constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    constexpr int TMEM_COLS = MB < 32 ? 32 : MB;         // power of two >= 32 (MB is 16, 32, 64, 128 or 256)
+    constexpr int TMEM_COLS = MB < 32 ? 32 : MB == 48 ? 64 : MB;   // power of two >= 32 (MB is 16, 32, 48, 64 or 128)
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MB >> 3) << 17) |
                                ((uint32_t)(TC_BM >> 4) << 24);
 
@@ -189,17 +189,57 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
     }
     __syncwarp();
 
-    // ---- epilogue: all four warps; warp w reads TMEM lanes 32w .. 32w+31 (output column n0 + 32w + lane)
+    // ---- epilogue: all four warps; warp w reads TMEM lanes 32w .. 32w+31 (output column n0 + 32w + lane).
+    // What it needs beside the accumulator is asked for before the wait for that, so that no load's latency stands in the chain
+    // from one kernel of a step to the next (a layer's four products at Qwen3-0.6B widths, chained, with a warp a row for the
+    // rotation: 21.3 -> 20.3 us at 8 rows, 29.0 -> 23.7 at 32; at 8B widths 89.2 -> 83.5 at 32).
+    constexpr int RED_FLOATS = TC_RED_FLOATS(MB);
+    float* red = reinterpret_cast<float*>(bars + 2 * STAGES + 2);     // reduction scratch, then inv[MB]
+    float* inv_s = red + RED_FLOATS;
+    // TC_MODE_QKV_ROPE: a row's position, page and place in it, behind the 64 floats that sum up its factor
+    int* pos_s = reinterpret_cast<int*>(red + 64);
+    int* slot_s = pos_s + MB;
+    const int m_valid = min(MB, p.M - m0);
+    const int col = threadIdx.x;                                      // 128 threads = 128 columns of the tile
+    const bool n_ok = n0 + col < p.N;
+    if (p.mode == TC_MODE_QKV_ROPE && warp >= 2) {
+        // the step's own arrays (written by the host before the step): no need to wait for the kernel before this one
+        for (int m = threadIdx.x - 64; m < m_valid; m += 64) {
+            const int t = m0 + m, pos = p.positions[t];
+            pos_s[m] = pos;
+            if (p.v_pages != nullptr) {
+                const int r = p.token_row[t];
+                const int page = p.block_table[(int64_t)r * p.table_stride + (pos >> p.logP) - p.page_base[r]];
+                slot_s[2 * m] = page;
+                slot_s[2 * m + 1] = pos & ((1 << p.logP) - 1);
+            }
+        }
+    }
     pdl_wait();          // the output buffer may still be read by the kernel before this one
     pdl_trigger();
-    if (nkb > 0) ok = mbar_wait(accum_bar, 0);
-    if (!ok) tc_fail(&g_gemm_tc_error, 3, ACORN_KERNEL_GEMM_TC);
-    ok = __all_sync(0xffffffffu, ok);               // tcgen05.ld below is warp-wide
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int n = n0 + warp * 32 + lane;
-    const int m_valid = min(MB, p.M - m0);
-    const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
-
+    // Rows of x that arrive un-normalised (x = residual * norm weight): the factor rsqrt(mean(residual^2) + eps) of each row is
+    // applied to the product.  Two warps add up the partial sums while the others load and multiply.
+    if (p.ss_in != nullptr) {
+        if (warp >= 2) {
+            // 64 threads: row = t % MB, the partial sums of a row are shared out over 64 / MB threads
+            constexpr int G = MB <= 64 ? 64 / MB : 1;
+            const int m = (threadIdx.x - 64) % MB, g = (threadIdx.x - 64) / MB;
+            float ss = 0.f;
+            if (g < G && m0 + m < p.M)
+#pragma unroll 4
+                for (int q = g; q < p.ss_parts; q += G) ss += p.ss_in[(int64_t)q * p.M + m0 + m];
+            if (g < G) red[g * MB + m] = ss;
+            asm volatile("bar.sync 1, 64;" ::: "memory");
+            if (g == 0) {
+                float tot = 0.f;
+#pragma unroll
+                for (int gg = 0; gg < G; ++gg) tot += red[gg * MB + m];
+                inv_s[m] = rsqrtf(tot / (float)p.norm_width + p.eps);
+            }
+        }
+    } else if (threadIdx.x < MB) {
+        inv_s[threadIdx.x] = 1.f;
+    }
     // The output tile is finished by rows: row m by the CTA of rank m % csize of the cluster (all
     // rows by the one CTA when K is not split).  Every CTA sends its partial rows from tensor
     // memory straight into the receive buffers of their owners (remote shared-memory stores, which
@@ -208,9 +248,6 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
     // to 32 tokens the buffer lies outside the ring, because a peer may still be in its main loop
     // when rows arrive; larger tiles use the ring, and a split one says when its ring is drained
     // (its accumulator is complete: every stage has been read).
-    constexpr int RED_FLOATS = TC_RED_FLOATS(MB);
-    float* red = reinterpret_cast<float*>(bars + 2 * STAGES + 2);     // reduction scratch, then inv[MB]
-    float* inv_s = red + RED_FLOATS;
     float* recv = RECV_IN_RING ? reinterpret_cast<float*>(smem) : inv_s + MB;
     int rank = 0, csize = 1;
     if (splits > 1) {
@@ -219,6 +256,36 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
         csize = (int)cluster.num_blocks();
     }
     const int slots = (MB + csize - 1) / csize;
+    constexpr int MAX_ROWS = MB <= 64 ? MB : 1;                       // the host refuses ADD_NORM for larger tiles
+    float r_old[MAX_ROWS];
+    float nw = 0.f;
+    if (p.mode == TC_MODE_ADD_NORM) {
+        if (n_ok) nw = ld_global_now(p.norm_w + n0 + col);
+#pragma unroll
+        for (int i = 0; i < MAX_ROWS; ++i) {
+            const int m = rank + i * csize;
+            if (m >= m_valid) break;                                  // the rows of this CTA come first
+            r_old[i] = n_ok ? ld_global_now(p.resid + (int64_t)(m0 + m) * p.ldr + n0 + col) : 0.f;
+        }
+    }
+    // TC_MODE_QKV_ROPE: the tile is one head, a warp finishes a row; lane l has columns l, l + 32, l + 64, l + 96
+    const bool rope = p.mode == TC_MODE_QKV_ROPE;
+    const bool is_q = rope && (int)blockIdx.x < p.nq, is_k = rope && !is_q && (int)blockIdx.x < p.nq + p.nkv;
+    const float* hw = is_q ? p.q_w : p.k_w;
+    float wcol[4] = {1.f, 1.f, 1.f, 1.f}, freq[2] = {0.f, 0.f};
+    if (is_q || is_k) {
+        if (hw != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) wcol[j] = hw[lane + 32 * j];
+        }
+        freq[0] = p.inv_freq[lane];
+        freq[1] = p.inv_freq[lane + 32];
+    }
+    if (nkb > 0) ok = mbar_wait(accum_bar, 0);
+    if (!ok) tc_fail(&g_gemm_tc_error, 3, ACORN_KERNEL_GEMM_TC);
+    ok = __all_sync(0xffffffffu, ok);               // tcgen05.ld below is warp-wide
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
     if (splits > 1) {
         if (RECV_IN_RING) cg::this_cluster().barrier_arrive();
         cg::this_cluster().barrier_wait();
@@ -240,42 +307,6 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
                 if (c + i < m_valid) st_cluster_f32(cluster_map(mine + (uint32_t)(slot * TC_BM * 4), owner), v[i]);
                 if (++owner == csize) { owner = 0; ++slot; }
             }
-        }
-    }
-    // Rows of x that arrive un-normalised (x = residual * norm weight): the factor
-    // rsqrt(mean(residual^2) + eps) of each row is applied to the product here.
-    if (p.ss_in != nullptr) {
-        // 128 threads: row = t % MB, the partial sums of a row are shared out over 128 / MB threads
-        constexpr int G = TC_THREADS / MB;
-        const int m = threadIdx.x % MB, g = threadIdx.x / MB;
-        float ss = 0.f;
-        if (g < G && m0 + m < p.M)
-            for (int q = g; q < p.ss_parts; q += G) ss += p.ss_in[(int64_t)q * p.M + m0 + m];
-        if (g < G) red[g * MB + m] = ss;
-        __syncthreads();
-        if (threadIdx.x < MB) {
-            float tot = 0.f;
-#pragma unroll
-            for (int gg = 0; gg < G; ++gg) tot += red[gg * MB + threadIdx.x];
-            inv_s[threadIdx.x] = rsqrtf(tot / (float)p.norm_width + p.eps);
-        }
-    } else if (threadIdx.x < MB) {
-        inv_s[threadIdx.x] = 1.f;
-    }
-    const int col = threadIdx.x;                                      // 128 threads = 128 columns of the tile
-    const bool n_ok = n0 + col < p.N;
-    // What the ADD_NORM epilogue reads from global memory is requested before the cluster meets,
-    // so that it arrives while the CTAs wait for one another.
-    constexpr int MAX_ROWS = MB <= 64 ? MB : 1;                       // the host refuses ADD_NORM for larger tiles
-    float r_old[MAX_ROWS];
-    float nw = 0.f;
-    if (p.mode == TC_MODE_ADD_NORM) {
-        if (n_ok) nw = ld_global_now(p.norm_w + n0 + col);
-#pragma unroll
-        for (int i = 0; i < MAX_ROWS; ++i) {
-            const int m = rank + i * csize;
-            if (m >= m_valid) break;                                  // the rows of this CTA come first
-            r_old[i] = n_ok ? ld_global_now(p.resid + (int64_t)(m0 + m) * p.ldr + n0 + col) : 0.f;
         }
     }
     if (splits > 1) cg::this_cluster().sync();
@@ -306,57 +337,49 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
             }
         }
     } else if (p.mode == TC_MODE_SWIGLU || p.mode == TC_MODE_GEGLU) {
-        // the tile holds 64 gate columns, then the 64 up columns of the same outputs
-        for (int i = 0, m = rank; m < m_valid; ++i, m += csize) {
-            if (col < 64) {
-                const float g = tile_sum(i, col) * inv_s[m], u = tile_sum(i, col + 64) * inv_s[m];
-                const int oc = blockIdx.x * 64 + col;
-                // gelu's tanh form is g sigmoid(2 sqrt(2/pi) (g + 0.044715 g^3))
-                const float z = p.mode == TC_MODE_GEGLU ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
-                if (oc < p.N / 2)
-                    reinterpret_cast<bf16*>(p.out)[(int64_t)(m0 + m) * p.ldo + oc] =
-                        __float2bfloat16_rn(g / (1.f + expf(-z)) * u);
-            }
+        // the tile holds 64 gate columns, then the 64 up columns of the same outputs; half of the threads take every second row
+        const int c = col & 63, oc = blockIdx.x * 64 + c;
+#pragma unroll 2
+        for (int i = col >> 6, m = rank + i * csize; m < m_valid; i += 2, m += 2 * csize) {
+            const float g = tile_sum(i, c) * inv_s[m], u = tile_sum(i, c + 64) * inv_s[m];
+            // gelu's tanh form is g sigmoid(2 sqrt(2/pi) (g + 0.044715 g^3))
+            const float z = p.mode == TC_MODE_GEGLU ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
+            if (oc < p.N / 2)
+                reinterpret_cast<bf16*>(p.out)[(int64_t)(m0 + m) * p.ldo + oc] =
+                    __float2bfloat16_rn(g / (1.f + expf(-z)) * u);
         }
-    } else if (p.mode == TC_MODE_QKV_ROPE) {
-        // The tile is one head.  Query and key heads: RMSNorm over the head (float32, on the
-        // accumulator: no rounding in between), then the rotation of (x[j], x[j + 64]) by
-        // position * inv_freq[j]; keys and values go to the token's slot of its cache page.
-        const int head = blockIdx.x;
-        const bool is_q = head < p.nq, is_k = !is_q && head < p.nq + p.nkv;
-        const int kvh = is_q ? 0 : (head - p.nq) % p.nkv;
-        const float* hw = is_q ? p.q_w : p.k_w;
-        const float wcol = ((is_q || is_k) && hw != nullptr) ? hw[col] : 1.f;
-        const float freq = p.inv_freq[col & 63];
-        float* xch = red;                                             // [4] partial sums, then [128] the head
-        for (int i = 0, m = rank; m < m_valid; ++i, m += csize) {
-            float val = tile_sum(i, col) * inv_s[m];
-            const int t = m0 + m, pos = p.positions[t];
+    } else if (rope) {
+        // Query and key heads: RMSNorm over the head (float32, on the accumulator: no rounding in between), then the rotation of
+        // (x[j], x[j + 64]) by position * inv_freq[j]; keys and values go to the token's slot of its cache page.
+        const int head = blockIdx.x, kvh = is_q ? 0 : (head - p.nq) % p.nkv;
+        for (int i = warp, m = rank + warp * csize; m < m_valid; i += 4, m += 4 * csize) {
+            const int t = m0 + m;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = tile_sum(i, lane + 32 * j) * inv_s[m];
             if (is_q || is_k) {
                 if (hw != nullptr) {
-                    const float part = warp_sum(val * val);
-                    __syncthreads();                                  // the row before has been read
-                    if (lane == 0) xch[warp] = part;
-                    __syncthreads();
-                    val = val * rsqrtf((xch[0] + xch[1] + xch[2] + xch[3]) / (float)TC_BM + p.rope_eps) * wcol;
-                } else {
-                    __syncthreads();
+                    const float ss = warp_sum((v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3]));
+                    const float f = rsqrtf(ss / (float)TC_BM + p.rope_eps);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[j] = v[j] * f * wcol[j];
                 }
-                xch[4 + col] = val;
-                __syncthreads();
-                const float other = xch[4 + (col ^ 64)];
-                float sn, cs;
-                sincosf((float)pos * freq, &sn, &cs);
-                val = col < 64 ? val * cs - other * sn : val * cs + other * sn;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    float sn, cs;
+                    sincosf((float)pos_s[m] * freq[j], &sn, &cs);
+                    const float a = v[j], b = v[j + 2];
+                    v[j] = a * cs - b * sn;
+                    v[j + 2] = b * cs + a * sn;
+                }
             }
-            if (is_q) {
-                reinterpret_cast<bf16*>(p.out)[(int64_t)t * p.ldo + head * TC_BM + col] = __float2bfloat16_rn(val);
-            } else if (p.v_pages != nullptr) {
-                const int r = p.token_row[t];
-                const int page = p.block_table[(int64_t)r * p.table_stride + (pos >> p.logP) - p.page_base[r]];
-                bf16* dst = (is_k ? p.k_pages : p.v_pages) +
-                            ((((int64_t)page * p.nkv + kvh) << p.logP) + (pos & ((1 << p.logP) - 1))) * TC_BM + col;
-                *dst = __float2bfloat16_rn(val);
+            bf16* dst = nullptr;
+            if (is_q) dst = reinterpret_cast<bf16*>(p.out) + (int64_t)t * p.ldo + head * TC_BM;
+            else if (p.v_pages != nullptr)
+                dst = (is_k ? p.k_pages : p.v_pages) + ((((int64_t)slot_s[2 * m] * p.nkv + kvh) << p.logP) + slot_s[2 * m + 1]) * TC_BM;
+            if (dst != nullptr) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dst[lane + 32 * j] = __float2bfloat16_rn(v[j]);
             }
         }
     } else {
@@ -451,7 +474,7 @@ static int run_tc(const void* x, int64_t ldx, const void* w, int64_t ldw, TcPara
     if (p.ss_in != nullptr && (M > 64 || p.ss_parts < 1 || p.norm_width < 1)) return ACORN_ERR_UNSUPPORTED;
     p.kblocks = (K + TC_BK - 1) / TC_BK;
     if (splits > p.kblocks) splits = p.kblocks;
-    const int mb = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+    const int mb = M <= 16 ? 16 : M <= 32 ? 32 : M <= 48 ? 48 : M <= 64 ? 64 : 128;
     if (mb > 64) splits = 1;               // K is split only for tiles of up to 64 tokens
     CUtensorMap mw, mx;
     int rc = make_map(&mw, w, N, K, ldw, TC_BK, TC_BM);
@@ -464,6 +487,7 @@ static int run_tc(const void* x, int64_t ldx, const void* w, int64_t ldw, TcPara
     switch (mb) {
         case 16: return per_sm == 3 ? launch_tc<16, 3>(mw, mx, p, splits, stream) : launch_tc<16, 5>(mw, mx, p, splits, stream);
         case 32: return per_sm == 3 ? launch_tc<32, 2>(mw, mx, p, splits, stream) : launch_tc<32, 4>(mw, mx, p, splits, stream);
+        case 48: return per_sm == 3 ? launch_tc<48, 3>(mw, mx, p, splits, stream) : launch_tc<48, 4>(mw, mx, p, splits, stream);
         case 64: return per_sm == 3 ? launch_tc<64, 3>(mw, mx, p, splits, stream) : launch_tc<64, 4>(mw, mx, p, splits, stream);
         default: return launch_tc<128, 3>(mw, mx, p, splits, stream);
     }

@@ -309,7 +309,7 @@ class Branch:
     device idle); otherwise at once, in order.  What ``fn`` reads must stay referenced until ``join``, which returns its
     result.  Larger steps fill the device anyway; and their kernels hold so much tensor memory that two of them on one
     multiprocessor could wait for one another's (the attention of prompts takes all of it, the paired product's CTAs and
-    a cluster's wait for their partners), while a product of at most ``GEMM_TC_MAX_ROWS`` rows takes a sixteenth."""
+    a cluster's wait for their partners), while a product of few rows takes a sixteenth or an eighth."""
 
     MAX_TOKENS = 128
 
@@ -1032,7 +1032,7 @@ def gemm_tc_plan(M: int, N: int, K: int, num_sms: int = 148) -> tuple[int, int]:
     worth), while 384 half tiles, three to an SM, leave none with more than three halves (1.5).  The
     second form is taken for unsplit matrices with 1 to 1.5 tiles to an SM; where K is split
     already it gained nothing."""
-    rows = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
+    rows = 16 if M <= 16 else 32 if M <= 32 else 48 if M <= 48 else 64 if M <= 64 else 128
     tiles = -(-N // 128) * -(-M // rows)
     kblocks = -(-K // 64)
     splits = 1
@@ -1050,6 +1050,11 @@ def gemm_tc_splits(M: int, N: int, K: int) -> int:
 # At or below this many rows the tcgen05 kernel (weights on the 128-row side of the MMA) streams the
 # weight matrix at least as fast as the library product; above it the library's larger tiles win.
 GEMM_TC_MAX_ROWS = 32
+# With the residual sum and norm, SwiGLU or the rotation in its epilogue, which the library leaves to kernels of their own, it wins
+# up to this many.  Measured (B200, chained, a layer's four products, us, library / this at 41 rows): 30.0 / 28.8 at Qwen3-0.6B widths,
+# 43.5 / 41.0 at 1.7B, 63.2 / 59.1 at 4B, 91.9 / 84.6 at 8B; at 64 rows 62.8 / 81.9 at 4B: a tile of 64 rows takes as much of an
+# SM's intake as half of the weights' tile.
+GEMM_TC_FUSED_MAX_ROWS = 48
 # The paired kernel (256 x 256 tiles, a pair of SMs to a tile at a time, fused epilogues) is used from
 # this many rows on, where its tiles fill the device: see ``pair_rows_ok``.
 GEMM_PAIR_MIN_ROWS = 256
@@ -1170,7 +1175,7 @@ def gemm_tc_qkv_rope(x, w: torch.Tensor, ep: RopeKvEpilogue, out: torch.Tensor |
     if out is None:
         out = torch.empty((M, N), dtype=torch.bfloat16, device=xt.device)
     _check(out, "out", torch.bfloat16, 2)
-    if M > GEMM_TC_MAX_ROWS:
+    if M > GEMM_TC_FUSED_MAX_ROWS:
         if ep.cos_sin is not None:
             _check(ep.cos_sin, "cos_sin", torch.float32, 2)
             if tuple(ep.cos_sin.shape) != (M, 128) or not ep.cos_sin.is_contiguous():
@@ -1333,6 +1338,12 @@ def fused_rows_ok(num_rows: int, dtype: torch.dtype, widths=None, num_sms: int =
     return all(pair_rows_ok(num_rows, w, num_sms) for w in widths)
 
 
+def fused_tile_ok(num_rows: int, dtype: torch.dtype) -> bool:
+    """Whether so many rows, more than the one-CTA kernel takes for plain products, go to it where it spares a part the kernels
+    around its products (``GEMM_TC_FUSED_MAX_ROWS``)."""
+    return dtype == torch.bfloat16 and GEMM_TC_MAX_ROWS < num_rows <= GEMM_TC_FUSED_MAX_ROWS
+
+
 def linear(x, w: torch.Tensor, out_dtype: torch.dtype | None = None, epilogue: AddNormEpilogue | None = None,
            swiglu: bool = False, residual32: torch.Tensor | None = None, activation: str = "silu",
            act: str | None = None):
@@ -1344,8 +1355,8 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype | None = None, epilogue: A
     ``out_dtype=float32`` keeps the accumulator's precision (used for logits).
     A weight stored in float32 under a bfloat16 engine is multiplied in float32.
     ``x`` as ``NormedRows``, ``epilogue`` and ``swiglu`` exist on the tcgen05 kernels only: the one-CTA
-    kernel up to GEMM_TC_MAX_ROWS rows, the paired kernel above (``activation``: the gate's function under
-    ``swiglu``; callers ask ``fused_rows_ok`` whether
+    kernel up to GEMM_TC_FUSED_MAX_ROWS rows, the paired kernel above (``activation``: the gate's function under
+    ``swiglu``; callers ask ``fused_rows_ok`` and ``fused_tile_ok`` whether
     that pays for their sizes); asking for them with other operands is an error, not a silent detour.
     ``residual32`` ([T, N] float32) is an offer: where the product goes to the library it is
     added to ``residual32`` in place, in float32 (the library's C operand: the product is not
@@ -1367,7 +1378,7 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype | None = None, epilogue: A
         if not (xt.dtype == torch.bfloat16 and gemm_tc_supported(xt, w)):
             raise KernelError(f"linear: fused epilogues need a tcgen05 path (bf16, K a multiple of 8); got "
                               f"{tuple(xt.shape)} {xt.dtype} x {tuple(w.shape)} {w.dtype}")
-        if xt.shape[0] > GEMM_TC_MAX_ROWS:
+        if xt.shape[0] > GEMM_TC_FUSED_MAX_ROWS:
             return gemm_tc_pair(x, w, out_dtype, epilogue=epilogue, swiglu=swiglu, activation=activation)
         return gemm_tc(x, w, out_dtype, epilogue=epilogue, swiglu=swiglu, activation=activation)
     if w.dtype == torch.float32:

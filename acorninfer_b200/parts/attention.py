@@ -224,7 +224,8 @@ class Attention(Mixer):
 
     def _rows_fuse(self, num_rows):
         widths = ((self.nq + 2 * self.nkv) * self.d, self.hidden_size)         # of the q/k/v product and of the o product
-        return ops.fused_rows_ok(num_rows, self.ctx.dtype, widths, ops.device_sms(self.ctx.device))
+        return (ops.fused_rows_ok(num_rows, self.ctx.dtype, widths, ops.device_sms(self.ctx.device))
+                or ops.fused_tile_ok(num_rows, self.ctx.dtype))
 
     def _inner_norm_rows(self, x, inputs, cache, out_scale, out, proj):
         g, pos = inputs.groups[cache.group], self.position
@@ -273,7 +274,7 @@ class Attention(Mixer):
                 cache.k_pages if cache.write else None, cache.v_pages if cache.write else None,
                 self.q_norm32, self.k_norm32, pos.inv_freq, self.nq, self.nkv,
                 self.qk_norm_eps if self.qk_norm_eps is not None else 0.0,
-                cos_sin=pos.table(inputs) if rows > ops.GEMM_TC_MAX_ROWS and hasattr(pos, "table") else None))
+                cos_sin=pos.table(inputs) if rows > ops.GEMM_TC_FUSED_MAX_ROWS and hasattr(pos, "table") else None))
         elif self.bias or self.taps:
             if not cache.write:
                 raise ValueError("attention: biased or convolved projections need a cache of the run's own")

@@ -151,6 +151,17 @@ def test_gemm_tc_qkv_rope_epilogue(nq, nkv, K, qlens, norm, write):
     assert torch.allclose(out[:, :nq * d].double().cpu(), want, atol=3e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("M,splits", [(33, 1), (41, 8), (48, 2)])
+def test_gemm_tc_tile_of_48_rows(M, splits):
+    """33 to 48 rows: the plain product and each epilogue that the engine asks for there."""
+    test_gemm_tc_matches_float32(M, 1000, 1032, splits, torch.float32)
+    test_gemm_tc_add_norm_epilogue_and_normed_rows(M, 504, 1024, splits)
+    test_gemm_tc_swiglu_epilogue(M, 192, 1024, splits)
+    test_gemm_tc_qkv_rope_epilogue(4, 2, 256 * splits, [M - 12, 1, 11], True, True)
+    o = ops()
+    assert o.fused_tile_ok(M, torch.bfloat16) and not any(o.fused_tile_ok(m, torch.bfloat16) for m in (32, 49)) and not o.fused_tile_ok(M, torch.float32)
+
+
 # ---------------------------------------------------------------------------- the paired kernel
 
 
