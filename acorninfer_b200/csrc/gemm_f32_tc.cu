@@ -1,0 +1,417 @@
+// C[M, N] = A[M, K] * W[N, K]^T in float32 on the 5th-generation tensor cores, for many rows, many columns and long
+// sums (gemm_f32.cu says from where on): every operand is the exact sum of three bfloat16 numbers, a = a0 + a1 + a2 (8 bits of mantissa
+// each; rounding to nearest, so |a1| <= 2^-9 |a|, |a2| <= 2^-18 |a|), and a product is a0 b0 + (a0 b1 + a1 b0) + (a0 b2 + a1 b1 + a2 b0);
+// what is left out (a1 b2 + a2 b1 + a2 b2) is at most 2^-26 |a b|, a quarter of a rounding of float32.
+//
+// The tensor cores round their sums towards zero, so no sum stays there for long.  K is cut into eight ranges of ceil(K / 512) * 64
+// and a range into chunks of 64.  A chunk's three sums (the terms of each order of magnitude apart) are made in tensor memory;
+// from there float32 adds, rounded to nearest, take them: T += G0 + (G1 + G2) over a range's chunks, and T0 + T1 + ... + T7 from
+// the left.  That order does not depend on M, on the other rows or on who takes which range, so a row's bits do not either.
+// Distance from 64 bits (relative 2-norm, K = 1,024 / 2,048 / 6,144): 9.3e-8, 9.9e-8, 1.1e-7; the multiply-adds of gemm_f32.cu 2.1e-7, 2.9e-7,
+// 5.0e-7.
+//
+// A CTA takes 128 rows of W (lanes of tensor memory) and 32 tokens.  Two groups of eight warps bring 64 floats of each row, split
+// them and lay the parts out for the matrix instruction (K-major rows of 128 bytes, 128-byte swizzle; K permuted alike in both operands,
+// so that a thread's 16 bytes of parts come from two coalesced loads); one warp multiplies: per 16 of K W0 x [b0 b1 b2],
+// W1 x [b0 b1] and W2 x [b0], which reads each part of W once; eight warps add up.  Stages and accumulators are handed
+// over by mbarriers; every wait is bounded.
+//
+// What bounds it: the loading warps, a load's latency and their arithmetic in turn (a chunk of 128 x 32 takes 1.0 us, of which shared
+// memory's bytes take 0.55).  One group instead of two: 1.75 us; wider tiles of 48 and 64 tokens need registers that 25 warps do not
+// have (spills: 1.7 and 2.0 us).  The products of a prompt of 832 rows (us, multiply-adds / this): N = 4,096, K = 1,024 164 / 94;
+// N = 6,144 264 / 139; N = 1,024, K = 3,072 142 / 86; N = 12,288, K = 2,048 902 / 485 (86 TFLOP/s).
+#include <cooperative_groups.h>
+
+#include "tcgen05_helpers.cuh"
+
+namespace cg = cooperative_groups;
+
+#define F3_BM 128            // rows of W a tile
+#define F3_NT 32             // tokens a tile
+#define F3_BK 64             // floats of K a chunk
+#define F3_RANGES 8
+#define F3_GROUP 8           // warps that load and split a chunk
+#define F3_GROUPS 2          // such groups: they take turns
+#define F3_LOADERS (F3_GROUP * F3_GROUPS)
+#define F3_ADDERS 8          // warps that add up
+#define F3_STAGES 3
+#define F3_THREADS (32 * (F3_LOADERS + F3_ADDERS + 1))
+#define F3_STAGE_BYTES (3 * (F3_BM + F3_NT) * 128)
+#define F3_TOTAL_BYTES (F3_NT * F3_BM * 4)
+#define F3_SMEM (F3_STAGES * F3_STAGE_BYTES + F3_TOTAL_BYTES + 1024 + 128)
+#define F3_TMEM_COLS 256     // two accumulators of three sums of 32 columns, a power of two
+
+__device__ int g_gemm_f32_tc_error = 0;
+
+struct F3Params {
+    const float* a;
+    const float* w;
+    float* c;
+    int64_t lda, ldw, ldc;
+    int M, N, K;
+    int range;               // floats of K a range
+    int vec;                 // rows of both operands are made of aligned float4
+    int tiles_m, tiles_n;
+};
+
+// Eight columns of 32 bits of this thread's lane from three places, one wait.
+__device__ __forceinline__ void tmem_ld8x3(uint32_t at0, uint32_t at1, uint32_t at2, float (&v0)[8], float (&v1)[8], float (&v2)[8]) {
+    uint32_t r[3][8];
+    const uint32_t at[3] = {at0, at1, at2};
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                     : "=r"(r[q][0]), "=r"(r[q][1]), "=r"(r[q][2]), "=r"(r[q][3]), "=r"(r[q][4]), "=r"(r[q][5]), "=r"(r[q][6]), "=r"(r[q][7])
+                     : "r"(at[q]));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        v0[i] = __uint_as_float(r[0][i]);
+        v1[i] = __uint_as_float(r[1][i]);
+        v2[i] = __uint_as_float(r[2][i]);
+    }
+}
+
+// What float32 gives where a sum is no number: chains of fused multiply-adds over ranges of K, as in gemm_f32.cu.  An operand that is
+// infinite, NaN or beyond bfloat16's largest number makes every product of its row NaN above; such sums are made again here.
+static __device__ __noinline__ float f3_chain(const float* a, const float* w, int K) {
+    const int range = (K + 127) / 128 * 16;
+    float total = 0.f;
+    for (int k0 = 0; k0 < K; k0 += range) {
+        float acc = 0.f;
+        for (int k = k0; k < min(K, k0 + range); ++k) acc = fmaf(a[k], w[k], acc);
+        total = k0 == 0 ? acc : total + acc;
+    }
+    return total;
+}
+
+__device__ __forceinline__ void f3_store(const F3Params& p, int m, int n, float v) {
+    if (!(fabsf(v) <= 3.0e38f)) v = f3_chain(p.a + (int64_t)m * p.lda, p.w + (int64_t)n * p.ldw, p.K);
+    p.c[(int64_t)m * p.ldc + n] = v;
+}
+
+__device__ __forceinline__ uint32_t f3_pack(float lo, float hi) {        // two bfloat16, rounded to nearest
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// Pairs of floats in the packed instructions of sm_100: a - b and a + b, rounded as the single ones.
+__device__ __forceinline__ float2 f3_sub2(float2 a, float2 b) {
+    unsigned long long r, x = *reinterpret_cast<unsigned long long*>(&a), y = *reinterpret_cast<unsigned long long*>(&b);
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(y), "l"(0xbf800000bf800000ull), "l"(x));
+    return *reinterpret_cast<float2*>(&r);
+}
+__device__ __forceinline__ float2 f3_add2(float2 a, float2 b) {
+    unsigned long long r, x = *reinterpret_cast<unsigned long long*>(&a), y = *reinterpret_cast<unsigned long long*>(&b);
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return *reinterpret_cast<float2*>(&r);
+}
+__device__ __forceinline__ float2 f3_unpack(uint32_t p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)); }
+
+// The three parts of eight floats, 16 bytes each.
+__device__ __forceinline__ void f3_split(const float (&x)[8], uint4 (&part)[3]) {
+    uint32_t p[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float2 v = make_float2(x[2 * i], x[2 * i + 1]);
+        p[0][i] = f3_pack(v.x, v.y);
+        v = f3_sub2(v, f3_unpack(p[0][i]));
+        p[1][i] = f3_pack(v.x, v.y);
+        v = f3_sub2(v, f3_unpack(p[1][i]));
+        p[2][i] = f3_pack(v.x, v.y);             // exact
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) part[q] = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+}
+
+// SPLIT: a cluster of eight CTAs shares a tile, a range of K each; else a CTA walks tiles, the next one's loads under way while
+// the last sums of one are added.
+template <bool SPLIT>
+__global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const F3Params p) {
+    constexpr int NT = F3_NT, STAGES = F3_STAGES, STAGE = F3_STAGE_BYTES, ADDERS = F3_ADDERS;
+    constexpr int PART_W = F3_BM * 128, PART_A = NT * 128, COLS = F3_TMEM_COLS;
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(F3_BM >> 4) << 24);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (tc_smem(smem_raw) & 1023u)) & 1023u);
+    float* totals = reinterpret_cast<float*>(smem + STAGES * STAGE);             // the ranges' sum so far, [token][row of W]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE + F3_TOTAL_BYTES);   // full[S], empty[S], sum_full[2], sum_empty[2]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+    const uint32_t full0 = tc_smem(bars), empty0 = tc_smem(bars + STAGES), sfull0 = tc_smem(bars + 2 * STAGES),
+                   sempty0 = tc_smem(bars + 2 * STAGES + 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int part = SPLIT ? (int)(blockIdx.x % F3_RANGES) : 0;
+    const int first = SPLIT ? (int)(blockIdx.x / F3_RANGES) : (int)blockIdx.x;
+    const int step = SPLIT ? 0x40000000 : (int)gridDim.x;
+    const int tiles = p.tiles_m * p.tiles_n;
+    const int kbeg = SPLIT ? min(p.K, part * p.range) : 0, kend = SPLIT ? min(p.K, kbeg + p.range) : p.K;
+    const int chunks = (kend - kbeg + F3_BK - 1) / F3_BK;
+
+    // the first weights on their way to L2 while the kernel before this one ends (W may be its result: not read yet)
+    if (warp < F3_GROUP && chunks > 0) {
+        const int n = min(first / p.tiles_m * F3_BM + (int)(threadIdx.x >> 1), p.N - 1), k = kbeg + (threadIdx.x & 1) * 32;
+        if (k < kend) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (int64_t)n * p.ldw + k));
+        if (k + F3_BK < kend) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (int64_t)n * p.ldw + k + F3_BK));
+    }
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, F3_GROUP); mbar_init(empty0 + 8 * s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(sfull0 + 8 * b, 1); mbar_init(sempty0 + 8 * b, ADDERS); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == F3_LOADERS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     :: "r"(tc_smem(tmem_slot)), "r"((uint32_t)COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_trigger();
+
+    if (warp < F3_LOADERS) {
+        // ---- load and split.  A unit: 8 floats of a row, k = 4 j .. and 32 + 4 j .. of the chunk; a thread has units of four
+        // of the tile's W rows and of one token.  It asks for its group's next chunk as it stores this one's; the
+        // fence behind the stores waits for those loads too, so two groups take turns: one waits, one splits.
+        constexpr int WU = F3_BM / 32, UNITS = WU + 1;
+        const int group = warp / F3_GROUP, row0 = (threadIdx.x >> 3) & 31, j = threadIdx.x & 7;
+        float x[UNITS][8];
+        int off[UNITS];                            // of the units' rows in W and A (the host sees that 32 bits hold them)
+        auto place = [&](int tile) {
+            const int tn = tile / p.tiles_m, tm = tile - tn * p.tiles_m;
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u)        // rows beyond the matrix: another row's values, never written
+                off[u] = u < WU ? min(tn * F3_BM + 32 * u + row0, p.N - 1) * (int)p.ldw : min(tm * NT + row0, p.M - 1) * (int)p.lda;
+        };
+        auto fetch = [&](int u, int k, bool inner, float (&v)[8]) {
+            const float* src = (u < WU ? p.w : p.a) + off[u];
+            if (inner) {
+                const float4 lo = *reinterpret_cast<const float4*>(src + k), hi = *reinterpret_cast<const float4*>(src + k + 32);
+                v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+            } else {                               // the last chunk of a range that 64 does not divide, or unaligned rows
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int kk = k + (e & 3) + 32 * (e >> 2);
+                    v[e] = kk < kend ? src[kk] : 0.f;
+                }
+            }
+        };
+        auto inside = [&](int chunk) { return p.vec && kbeg + (chunk + 1) * F3_BK <= kend; };
+        int tile = first, chunk = 0;
+        auto advance = [&](int by) {                           // `by` chunks on, into the next tiles
+            chunk += by;
+            while (tile < tiles && chunk >= chunks) {
+                chunk -= chunks;
+                tile += step;
+            }
+        };
+        if (chunks > 0) advance(group);
+        else tile = tiles;
+        if (tile < tiles) {
+            place(tile);
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u) fetch(u, kbeg + chunk * F3_BK + 4 * j, inside(chunk), x[u]);
+        }
+        for (int it = group; tile < tiles; it += F3_GROUPS) {
+            const int s = it % STAGES;
+            bool ok = mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1);
+            if (!ok && lane == 0) tc_fail(&g_gemm_f32_tc_error, 1, ACORN_KERNEL_GEMM_F32_TC);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            const int was = tile;
+            advance(F3_GROUPS);
+            const bool more = tile < tiles, inner = inside(chunk);
+            const int k = kbeg + chunk * F3_BK + 4 * j;
+            if (more && tile != was) place(tile);
+            uint8_t* base = smem + s * STAGE + (row0 >> 3) * 1024 + (row0 & 7) * 128 + ((j ^ (row0 & 7)) << 4);
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u) {
+                uint4 parts[3];
+                f3_split(x[u], parts);
+                if (more) fetch(u, k, inner, x[u]);
+                uint8_t* dst = base + (u < WU ? 4096 * u : 3 * PART_W);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(dst + q * (u < WU ? PART_W : PART_A)) = parts[q];
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full0 + 8 * s);
+        }
+    } else if (warp == F3_LOADERS) {
+        // ---- multiply (the warp stays converged, an elected lane issues)
+        const uint32_t w0 = umma_lo(tc_smem(smem)), a0 = umma_lo(tc_smem(smem) + 3 * PART_W);
+        constexpr uint32_t I1 = IDESC | ((uint32_t)(3 * NT >> 3) << 17), I2 = IDESC | ((uint32_t)(2 * NT >> 3) << 17),
+                           I3 = IDESC | ((uint32_t)(NT >> 3) << 17);
+        int it = 0;
+        bool ok = true;
+        for (int tile = first; ok && tile < tiles; tile += step) {
+            for (int chunk = 0; chunk < chunks; ++chunk, ++it) {
+                const int s = it % STAGES, b = it & 1;
+                ok = mbar_wait(sempty0 + 8 * b, ((it >> 1) & 1) ^ 1);
+                if (ok) ok = mbar_wait(full0 + 8 * s, (it / STAGES) & 1);
+                if (!ok && lane == 0) tc_fail(&g_gemm_f32_tc_error, 2, ACORN_KERNEL_GEMM_F32_TC);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d = tmem + b * 3 * NT;
+                const uint32_t w = w0 + s * (STAGE >> 4), a = a0 + s * (STAGE >> 4);
+#pragma unroll
+                for (int k = 0; k < F3_BK / 16; ++k) {
+                    umma_bf16_elect(d, w + 2 * k, a + 2 * k, I1, k > 0 ? 1u : 0u);
+                    umma_bf16_elect(d + NT, w + 2 * k + (PART_W >> 4), a + 2 * k, I2, 1u);
+                    umma_bf16_elect(d + 2 * NT, w + 2 * k + 2 * (PART_W >> 4), a + 2 * k, I3, 1u);
+                }
+                umma_commit_elect(empty0 + 8 * s);
+                umma_commit_elect(sfull0 + 8 * b);
+            }
+        }
+    } else {
+        // ---- add up: warp w reads lanes 32 (w % 4) .. of tensor memory, its share of the tokens
+        constexpr int MINE = 4 * NT / ADDERS;                  // tokens a warp
+        const int aw = warp - F3_LOADERS - 1, quarter = warp & 3, t0 = (aw >> 2) * MINE;
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+        const int range_chunks = p.range / F3_BK;
+        int it = 0;
+        bool ok = true;
+        for (int tile = first; ok && tile < tiles; tile += step) {
+            float2 sum[MINE / 2];
+#pragma unroll
+            for (int i = 0; i < MINE / 2; ++i) sum[i] = make_float2(0.f, 0.f);
+            float* mine = totals + t0 * F3_BM + quarter * 32 + lane;
+            bool folded = false;
+            int in_range = 0;
+            for (int chunk = 0; chunk < chunks; ++chunk, ++it) {
+                if (!SPLIT && in_range == range_chunks) {
+                    in_range = 0;
+#pragma unroll
+                    for (int i = 0; i < MINE / 2; ++i) {
+                        float* at = mine + 2 * i * F3_BM;
+                        at[0] = folded ? at[0] + sum[i].x : sum[i].x;
+                        at[F3_BM] = folded ? at[F3_BM] + sum[i].y : sum[i].y;
+                        sum[i] = make_float2(0.f, 0.f);
+                    }
+                    folded = true;
+                }
+                ++in_range;
+                const int b = it & 1;
+                ok = mbar_wait(sfull0 + 8 * b, (it >> 1) & 1);
+                if (!ok && lane == 0) tc_fail(&g_gemm_f32_tc_error, 3, ACORN_KERNEL_GEMM_F32_TC);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t at = tmem + lanes + b * 3 * NT + t0;
+#pragma unroll
+                for (int c = 0; c < MINE; c += 8) {
+                    float g0[8], g1[8], g2[8];
+                    tmem_ld8x3(at + c, at + c + NT, at + c + 2 * NT, g0, g1, g2);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 lower = f3_add2(make_float2(g1[2 * i], g1[2 * i + 1]), make_float2(g2[2 * i], g2[2 * i + 1]));
+                        sum[c / 2 + i] = f3_add2(sum[c / 2 + i], f3_add2(make_float2(g0[2 * i], g0[2 * i + 1]), lower));
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sempty0 + 8 * b);
+            }
+            if (!ok) break;
+            if (SPLIT) {
+#pragma unroll
+                for (int i = 0; i < MINE; ++i) mine[i * F3_BM] = i & 1 ? sum[i / 2].y : sum[i / 2].x;
+            } else {
+                const int tn = tile / p.tiles_m, tm = tile - tn * p.tiles_m;
+                const int n = tn * F3_BM + quarter * 32 + lane, m = tm * NT + t0;
+                if (n < p.N) {
+#pragma unroll
+                    for (int i = 0; i < MINE; ++i) {
+                        const float v = i & 1 ? sum[i / 2].y : sum[i / 2].x;
+                        if (m + i < p.M) f3_store(p, m + i, n, folded ? mine[i * F3_BM] + v : v);
+                    }
+                }
+            }
+        }
+    }
+    if (SPLIT) {
+        __syncwarp();
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        const int tn = first / p.tiles_m, tm = first - tn * p.tiles_m;
+        constexpr int SHARE = NT * F3_BM / F3_RANGES;
+        for (int o = threadIdx.x; o < SHARE; o += F3_THREADS) {
+            const int at = part * SHARE + o, m = tm * NT + at / F3_BM, n = tn * F3_BM + at % F3_BM;
+            float v[F3_RANGES];
+#pragma unroll
+            for (int q = 0; q < F3_RANGES; ++q) v[q] = cluster.map_shared_rank(totals, q)[at];
+#pragma unroll
+            for (int q = 1; q < F3_RANGES; ++q) v[0] += v[q];
+            if (m < p.M && n < p.N) f3_store(p, m, n, v[0]);
+        }
+        cluster.sync();                          // a CTA's shared memory stays until all have read it
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == F3_LOADERS)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"((uint32_t)COLS) : "memory");
+}
+
+// ------------------------------------------------------------------ host side
+
+template <bool SPLIT>
+static int f3_launch(const F3Params& p, int grid, cudaStream_t stream) {
+    static AcornPerDevice configured;
+    if (!configured.seen()) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, F3_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured.mark();
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(F3_THREADS);
+    cfg.dynamicSmemBytes = F3_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = F3_RANGES;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = acorn_pdl_enabled() ? attr : attr + 1;
+    cfg.numAttrs = (acorn_pdl_enabled() ? 1 : 0) + (SPLIT ? 1 : 0);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel<SPLIT>, p);
+    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// Offsets of both operands' elements fit 32 bits.
+extern "C" int acorn_gemm_f32_tc_takes(int64_t M, int64_t N, int64_t lda, int64_t ldw) { return M * lda <= 0x7fffffff && N * ldw <= 0x7fffffff; }
+
+// split 1: a cluster of eight CTAs to a tile, 0: whole tiles, -1: chosen here.  Any alignment.
+extern "C" int acorn_gemm_f32_tc(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
+                                 int split, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || !acorn_gemm_f32_tc_takes(M, N, lda, ldw)) return ACORN_ERR_UNSUPPORTED;
+    F3Params p = {};
+    p.a = A; p.w = W; p.c = C; p.lda = lda; p.ldw = ldw; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
+    p.range = (K + F3_BK * F3_RANGES - 1) / (F3_BK * F3_RANGES) * F3_BK;
+    p.vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
+    p.tiles_m = (M + F3_NT - 1) / F3_NT;
+    p.tiles_n = (N + F3_BM - 1) / F3_BM;
+    const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n, sms = acorn_sms();
+    if (tiles * F3_RANGES > 0x3fffffff) return ACORN_ERR_UNSUPPORTED;
+    if (split < 0) {
+        // Clusters where few tiles leave SMs idle: a chunk takes 1.0 us, a cluster's start, exchange and end 7 us beside its
+        // chunks (128 rows, N = 1,024, K = 2,048, 32 tiles: 32 us whole, 23 in clusters; 256 rows: 32 and 39).
+        const int64_t chunks = (K + F3_BK - 1) / F3_BK, part = p.range / F3_BK;
+        split = K >= 4 * F3_BK && (tiles * F3_RANGES + sms - 1) / sms * (part + 7) < (tiles + sms - 1) / sms * chunks;
+    }
+    return split ? f3_launch<true>(p, (int)tiles * F3_RANGES, stream) : f3_launch<false>(p, (int)(tiles < sms ? tiles : sms), stream);
+}
+
+// Reads and clears the flag that a bounded wait sets when it gives up (0 = no error).
+extern "C" int acorn_gemm_f32_tc_error() {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_gemm_f32_tc_error, sizeof(int)) != cudaSuccess) return -1;
+    if (v != 0) cudaMemcpyToSymbol(g_gemm_f32_tc_error, &zero, sizeof(int));
+    return v;
+}
+
+ACORN_ERROR_WORD_SETTER(acorn_gemm_f32_tc_set_error_word)

@@ -77,7 +77,7 @@ def build_calls() -> None:
 
 _error_word: ctypes.c_int | None = None       # pinned host memory that kernels write when a bounded wait gives up
 _KERNEL_NAMES = {1: "gemm_tcgen05", 2: "attention_prefill_tc", 3: "attention_decode_tma", 4: "gemm_tcgen05_pair",
-                 5: "latent_prefill_tc", 9: "error-word self-test"}
+                 5: "latent_prefill_tc", 6: "gemm_f32_tc", 9: "error-word self-test"}
 
 
 def _init_error_word(library) -> None:
@@ -88,7 +88,7 @@ def _init_error_word(library) -> None:
         raise KernelError(f"could not allocate the kernels' error word: CUDA error {code}")
     for setter in ("acorn_gemm_tc_set_error_word", "acorn_attention_tc_set_error_word",
                    "acorn_attention_decode_tma_set_error_word", "acorn_selftest_set_error_word",
-                   "acorn_gemm_tc_pair_set_error_word", "acorn_latent_prefill_tc_set_error_word"):
+                   "acorn_gemm_tc_pair_set_error_word", "acorn_latent_prefill_tc_set_error_word", "acorn_gemm_f32_tc_set_error_word"):
         code = getattr(library, setter)(dev)
         if code != 0:
             raise KernelError(f"{setter}: CUDA error {code}")
@@ -102,7 +102,7 @@ def raise_on_kernel_error() -> None:
         return
     word = _error_word.value
     _error_word.value = 0
-    for getter in (gemm_tc_error, attention_tc_error, attention_decode_tma_error, gemm_tc_pair_error, latent_prefill_tc_error):   # clear the kernels' own flags
+    for getter in (gemm_tc_error, attention_tc_error, attention_decode_tma_error, gemm_tc_pair_error, latent_prefill_tc_error, gemm_f32_tc_error):   # clear the kernels' own flags
         getter()
     raise KernelError(f"kernel {_KERNEL_NAMES.get(word // 100, word // 100)} gave up a bounded wait at point "
                       f"{word % 100}: the results of the step are not valid")
@@ -273,6 +273,9 @@ class _Sigs:
     acorn_gemm_tc_pair_error = []
     acorn_gemm_tc_error = []
     acorn_gemm_f32 = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]
+    acorn_gemm_f32_tc = [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p]
+    acorn_gemm_f32_tc_error = []
+    acorn_gemm_f32_tc_set_error_word = [c_void_p]
     acorn_sample = [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                     c_void_p, c_void_p, c_int, c_void_p]
     acorn_uniform = [ctypes.c_uint64, ctypes.c_uint64]
@@ -987,7 +990,9 @@ def attention_tc_error() -> int:
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """a [M, K] @ w [N, K]^T in true float32 (CUDA cores)."""
+    """a [M, K] @ w [N, K]^T in true float32: multiply-adds on the CUDA cores; from 65 rows on, for at least 1,024 columns and K of
+    512, operands as sums of three bfloat16 numbers on the tensor cores (``csrc/gemm_f32_tc.cu``), which is nearer to the exact
+    product.  Within either kind a row's bits do not depend on the other rows."""
     _check(w, "w", torch.float32, 2)
     if a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1:
         raise KernelError("a must be float32 [M, K] with contiguous K")
@@ -1001,6 +1006,24 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
     _ok(lib().acorn_gemm_f32(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(),
                              out.stride(0), M, N, K, _stream()), "gemm_f32", f"{M}x{N}x{K}")
     return out
+
+
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, split: bool | None = None) -> torch.Tensor:
+    """``gemm_f32`` on the tcgen05 kernel whatever the sizes; ``split``: a cluster of eight CTAs to a tile (None: as ``gemm_f32``
+    has it), which does not change a bit of the result."""
+    _check(w, "w", torch.float32, 2)
+    if a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1 or a.shape[1] != w.shape[1]:
+        raise KernelError("a must be float32 [M, K] with contiguous K, w [N, K]")
+    M, K = a.shape
+    out = torch.empty((M, w.shape[0]), dtype=torch.float32, device=a.device)
+    _ok(lib().acorn_gemm_f32_tc(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, w.shape[0], K,
+                                -1 if split is None else int(split), _stream()), "gemm_f32_tc", f"{M}x{w.shape[0]}x{K}")
+    return out
+
+
+def gemm_f32_tc_error() -> int:
+    """0, or where a bounded wait inside the float32 product on tcgen05 gave up since the last call (clears it)."""
+    return int(lib().acorn_gemm_f32_tc_error())
 
 
 def gemm_tc_supported(x: torch.Tensor, w: torch.Tensor) -> bool:

@@ -145,6 +145,47 @@ def test_gemm_f32_of_few_rows_and_many_columns(M, N, K):
     assert ((tile[:M].double() - ref).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("M,N,K,pad", [(1, 128, 64, 0), (130, 1025, 516, 0), (300, 1100, 1028, 0), (333, 1024, 515, 0), (129, 1030, 2048, 3)])
+def test_float32_product_on_tcgen05(M, N, K, pad):
+    """Operands as three bfloat16 numbers each: tiles whole and shared by a cluster give the same bits, also where
+    tiles end inside the matrix, ranges of K are empty or rows are not aligned; no further from 64 bits than the multiply-adds."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    a = torch.randn(M, K + pad, device=DEV, generator=g)[:, :K]
+    w = torch.randn(N, K, device=DEV, generator=g)
+    out = o.gemm_f32_tc(a, w)
+    for split in (False, True):
+        assert torch.equal(o.gemm_f32_tc(a, w, split), out), split
+    assert torch.equal(o.gemm_f32_tc(a[M // 2:], w), out[M // 2:]) and o.gemm_f32_tc_error() == 0
+    want = a.double() @ w.double().T
+    # per product: at most 2^-26 left out by the split; per chunk of 64: four sums in tensor memory cut off at 2^-23 of the sum at
+    # most (twice a rounding), then one float32 sum; eight ranges
+    steps = 4 * 2 + -(-K // 64) + 8
+    assert ((out.double() - want).abs() <= (a.abs().double() @ w.abs().double().T) * steps * 2.0 ** -24).all()
+    if K >= 512:
+        chains = torch.cat([o.gemm_f32(a[i:i + 16].contiguous(), w) for i in range(0, M, 16)])       # few rows: multiply-adds
+        assert (out.double() - want).norm() <= (chains.double() - want).norm()
+    assert torch.equal(o.gemm_f32(a, w), out) == (M > 64 and N >= 1024 and K >= 512)
+
+
+def test_float32_product_on_tcgen05_with_numbers_that_do_not_split():
+    """Infinities, NaN, numbers that bfloat16 rounds to infinity and sums that overflow: what the multiply-adds give, in the rows and
+    columns that hold them and in no others; small numbers keep their 24 bits."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(3)
+    a, w = torch.randn(140, 512, device=DEV, generator=g), torch.randn(200, 512, device=DEV, generator=g)
+    a[3, 5], a[4, 7], w[9, 100], a[5] = float("inf"), float("nan"), float("-inf"), 3.0e38
+    a[7], a[7, 0] = 0.0, 3.399e38
+    new, old = o.gemm_f32_tc(a, w), torch.cat([o.gemm_f32(a[i:i + 16].contiguous(), w) for i in range(0, 140, 16)])
+    assert torch.equal(new.isnan(), old.isnan()) and torch.equal(new.isinf(), old.isinf()) and not bool(new.isfinite().all())
+    assert torch.equal(new[new.isinf()], old[new.isinf()])
+    fine = new.isfinite()
+    assert bool(((new - old).abs()[fine] <= 2.0 ** -13 * (a.abs().nan_to_num(0, 0) @ w.abs().nan_to_num(0, 0).T)[fine]).all())
+    for scale in (1.0, 2.0 ** -90, 2.0 ** 120):
+        x = torch.randn(64, 128, device=DEV, generator=g) * scale
+        assert torch.equal(o.gemm_f32_tc(x, torch.eye(128, device=DEV)), x)
+
+
 def test_gemm_f32_shows_what_a_reduced_precision_mode_would_hide():
     # 1 + 2^-12 is lost by a product that rounds its inputs to 10 mantissa bits (TF32) or to bfloat16
     a = torch.full((4, 8), 1 + 2 ** -12, device=DEV)
