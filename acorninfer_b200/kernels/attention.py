@@ -105,6 +105,42 @@ def decode_splits(rows: int, num_kv_heads: int, key_bound: int, head_dim: int, n
     return best
 
 
+# How the TMA decode kernel's launches share the work (measured: 1 to 64 rows of 8 kv heads at contexts of 300, 900 and 1,700, equal
+# and of 35 to 100 %, every number of splits).  Clusters run in one wave only as long as they fill no more than seven
+# eighths of the CTAs that single ones would (5 rows of 900 keys: 6 splits, 240 CTAs, 9.1 us; 7 splits, 280 CTAs, 15.4; 12 rows: 2
+# splits 13.9, 3 splits, 288 CTAs, 21.6), pairs of CTAs fill all of them, clusters of sixteen half; and a second wave of
+# clusters costs more than its splits bring (41 rows of 900: unsplit 43.7, 3 splits 50.7).
+_START_US, _CLUSTER_US = 3.5, 1.5
+
+
+def _wave(splits: int, num_sms: int) -> int:
+    """CTAs that run at once where a (row, kv head) has so many."""
+    return 2 * num_sms if splits <= 2 or splits > 16 else 2 * num_sms * 7 // 8 if splits <= 8 else num_sms
+
+
+@lru_cache(maxsize=4096)
+def decode_plan(rows: int, num_kv_heads: int, key_bound: int, num_sms: int = B200_SMS, merge_limit: int = 16) -> int:
+    """For the TMA decode kernel (head size 128, ``merge_limit`` splits merged inside it): splits of the key range, or 0 where the keys
+    of all rows should be shared out evenly instead (``ops.attention_decode_stream``): where whole (row, kv head)s leave
+    the last of several waves of CTAs less than four fifths full, as 41 rows of 8 do on 148 SMs (us, unsplit / even shares at 900 keys:
+    43.7 / 35.7, of 35 to 100 % as many 28.5 / 27.5; 48 rows 44.1 / 38.2; 64 rows, 0.86 full, 46.6 / 47.6)."""
+    pairs, wave = rows * num_kv_heads, 2 * num_sms
+    if pairs > wave:
+        return 0 if pairs < 0.8 * wave * -(-pairs // wave) and key_bound > 2 * _CHUNK else 1
+    most = max(1, -(-key_bound // _CHUNK))
+    pair_kb = key_bound * 128 * 4 / 1e3                             # K and V of one pair, bfloat16, in KB
+    best, best_us = 1, None
+    for s in (1, 2, 3, 4, 5, 6, 7, 8, 16, 24, 32):
+        if s > most or (s > 1 and pairs * s > _wave(s, num_sms)):
+            continue
+        us = _START_US + pair_kb / s / min(_CTA_GBS, _HBM_GBS / (pairs * s))
+        if s > 1:
+            us += _CLUSTER_US if merged_in_kernel(s, merge_limit) else _WAVE_US + _MERGE_US
+        if best_us is None or us <= best_us + 1e-9:                  # equal estimates: more CTAs in flight
+            best, best_us = s, us
+    return best
+
+
 _MERGE_FREE: dict = {}
 
 
@@ -115,6 +151,20 @@ def _merge_free(nq: int, nkv: int, d: int, P: int) -> int:
         _MERGE_FREE[key] = (ops.lib().acorn_attention_decode_tma_merges(nq, nkv)
                             if ops.lib().acorn_attention_decode_tma_supported(nq, nkv, d, P) else 1)
     return _MERGE_FREE[key]
+
+
+def _decode(qkv, inputs, group, cache, nq, nkv, d, P, scale, window, bound, n, windowed_only, mask, token_list=None, out=None):
+    """The step's ``n`` single-token rows (``token_list``, or all tokens) on a decode kernel."""
+    args = (qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table, group.page_base, inputs.token_row, inputs.positions,
+            inputs.num_tokens, nq, nkv, d, scale, window)
+    limit = _merge_free(nq, nkv, d, P) if windowed_only else 1
+    if limit > 1:                                                    # the TMA kernel takes these sizes
+        splits = decode_plan(n, nkv, bound, sm_count(qkv.device), limit)
+        if splits == 0 and ops.attention_decode_stream_supported(nq, nkv, d, P, n):
+            return ops.attention_decode_stream(*args, token_list=token_list, out=out)
+        return ops.attention_decode(*args, max(splits, 1), token_list=token_list, out=out, **mask)
+    return ops.attention_decode(*args, decode_splits(n, nkv, bound, d, sm_count(qkv.device), limit), token_list=token_list, out=out,
+                                **mask)
 
 
 def _key_bound(table_keys: int, window: int | None, chunk: int | None, keep_first: int) -> int:
@@ -151,11 +201,7 @@ def paged_attention(qkv: torch.Tensor, inputs, group, cache, nq: int, nkv: int, 
     if qkv.dtype == torch.bfloat16 and (value_dim is None or value_dim == d):
         if inputs.plan.all_decode and ops.attention_decode_supported(nq, nkv, d) and inputs.num_tokens <= 65535:
             bound = _key_bound(group.block_table.shape[1] * P, window, chunk, keep_first)
-            splits = decode_splits(inputs.num_rows, nkv, bound, d, sm_count(qkv.device),
-                                   _merge_free(nq, nkv, d, P) if windowed_only else 1)
-            return ops.attention_decode(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table,
-                                        group.page_base, inputs.token_row, inputs.positions, inputs.num_tokens,
-                                        nq, nkv, d, scale, window, splits, **mask)
+            return _decode(qkv, inputs, group, cache, nq, nkv, d, P, scale, window, bound, inputs.num_rows, windowed_only, mask)
         x, hx = inputs.extra, inputs.plan.extra
         n_single = int(hx["attention.single_tokens"].size)
         if ops.attention_prefill_supported(nq, nkv, d) and (n_single == 0 or (
@@ -179,12 +225,8 @@ def paged_attention(qkv: torch.Tensor, inputs, group, cache, nq: int, nkv: int, 
                                       inputs.num_tokens, nq, nkv, d, scale, window, out=out, **mask)
             if n_single:
                 bound = _key_bound(group.block_table.shape[1] * P, window, chunk, keep_first)
-                ops.attention_decode(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table,
-                                     group.page_base, inputs.token_row, inputs.positions, inputs.num_tokens,
-                                     nq, nkv, d, scale, window,
-                                     decode_splits(n_single, nkv, bound, d, sm_count(qkv.device),
-                                                   _merge_free(nq, nkv, d, P) if windowed_only else 1),
-                                     token_list=x["attention.single_tokens"], out=out, **mask)
+                _decode(qkv, inputs, group, cache, nq, nkv, d, P, scale, window, bound, n_single, windowed_only, mask,
+                        token_list=x["attention.single_tokens"], out=out)
             return out
     if qkv.dtype == torch.float32 and (value_dim is None or value_dim == d) and windowed_only and cache.k_pages.shape == cache.v_pages.shape:
         # a row of one token goes to the decode kernel whatever else is in the step, so that its bits stay the same
