@@ -15,6 +15,7 @@
 #include "common.cuh"
 
 #include <cooperative_groups.h>
+#include <cstring>
 namespace cg = cooperative_groups;
 
 #define SAMPLE_THREADS 1024
@@ -37,6 +38,24 @@ __host__ __device__ __forceinline__ float uniform_from(unsigned long long seed, 
     return (float)(z >> 40) * (1.0f / 16777216.0f);
 }
 
+// A row's parameters: arrays in device memory, or the values themselves among the launch's arguments, which spares a step the
+// copy of a block that the host has just made.
+struct SampleArrays {
+    const float* temperature;
+    const int* top_k;
+    const float* top_p;
+    const unsigned long long* seed;
+    const unsigned long long* counter;
+};
+
+#define SAMPLE_INLINE_ROWS 128
+
+struct SampleInline {
+    unsigned long long seed[SAMPLE_INLINE_ROWS], counter[SAMPLE_INLINE_ROWS];
+    float temperature[SAMPLE_INLINE_ROWS], top_p[SAMPLE_INLINE_ROWS];
+    int top_k[SAMPLE_INLINE_ROWS];
+};
+
 __device__ __forceinline__ unsigned int block_sum_u32(unsigned int v, unsigned int* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -48,11 +67,10 @@ __device__ __forceinline__ unsigned int block_sum_u32(unsigned int v, unsigned i
     return t;
 }
 
+template <typename Rows>
 __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
-    const float* __restrict__ logits, int64_t ld, int V, const float* __restrict__ temperature,
-    const int* __restrict__ top_k, const float* __restrict__ top_p,
-    const unsigned long long* __restrict__ seed, const unsigned long long* __restrict__ counter,
-    int* __restrict__ token_out, float* __restrict__ logprob_out) {
+    const float* __restrict__ logits, int64_t ld, int V, const __grid_constant__ Rows rows, int* __restrict__ token_out,
+    float* __restrict__ logprob_out) {
     __shared__ float fscratch[32];
     __shared__ unsigned int uscratch[32];
     __shared__ float seg_prefix[SAMPLE_THREADS / 32];
@@ -61,7 +79,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
     pdl_trigger();
     const int r = blockIdx.x, tid = threadIdx.x;
     const float* x = logits + (int64_t)r * ld;
-    const float temp = temperature[r];
+    const float temp = rows.temperature[r];
 
     // pass 1: max (first index among equals) and finiteness
     float best = -INFINITY;
@@ -93,7 +111,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
     const float inv_t = 1.f / temp;
     // keys of the kept set: key >= lo_key
     unsigned int lo_key = 0u;
-    int k = top_k[r];
+    int k = rows.top_k[r];
     if (k > 0 && k < V) {
         // largest K with count(key >= K) >= k  ==  key of the k-th largest logit
         unsigned int lo = 0u, hi = 0xffffffffu;
@@ -106,7 +124,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
         }
         lo_key = lo;
     }
-    const float p_keep = top_p[r];
+    const float p_keep = rows.top_p[r];
     if (p_keep < 1.f) {
         float z = 0.f;
         for (int i = tid; i < V; i += SAMPLE_THREADS)
@@ -155,7 +173,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
     __syncthreads();
     const float total = fscratch[0];
     const float excl = seg_prefix[tid >> 5] + (incl - mine);
-    const float target = uniform_from(seed[r], counter[r]) * total;
+    const float target = uniform_from(rows.seed[r], rows.counter[r]) * total;
     if (mine > 0.f && target >= excl && target < excl + mine) {
         float run = excl;
         int pick = -1, last_kept = -1;
@@ -185,7 +203,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
 //   top-k up to the number of warps (128): the k-th largest of the warps' maxima bounds the k-th largest key from below and
 //     leaves few more than k candidates; the first CTA gathers them and ends alone (`sc_finish`), every pair compared.
 //   top-p alone: one histogram of the probabilities in equal steps of the scaled logit, summed over the cluster through
-//     distributed shared memory; the keys of the one bin that holds the bound are gathered by every CTA and compared.
+//     distributed shared memory; the keys of the one bin that holds the bound are gathered by every CTA, which compares an eighth.
 //   anything else, and rows whose candidates do not fit the lists (many equal logits): the bounds digit by digit (11 + 11 + 10
 //     bits of the ordered key), a histogram a level (`sc_select`).
 // All three ask the same: the smallest key K with weight(keys <= K) > limit, where a key weighs 1 and limit is the number of
@@ -193,7 +211,8 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
 // as integers of 2^-44 of the largest one (a sum's error is below that of float32 sums, and its order does not matter), so the
 // three answers are the same.
 // What bounds it: 64 clusters of 8 on 148 SMs are two waves (two CTAs an SM: shared memory), each a read of its slices and a
-// chain of short steps with cluster barriers between them.
+// chain of short steps with cluster barriers between them; rows with top-p alone, whose probabilities are all made twice, take
+// longest.  64 rows of 151,936, parameters mixed: 63 us a call.  (Slices left in L2, so that all 64 run at once: 77 us.)
 #define SC_THREADS 512
 #define SC_WARPS (SC_THREADS / 32)
 #define SC_BINS 2048
@@ -202,6 +221,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
 #define SC_CAND 256                 // candidates a CTA can note
 #define SC_LIST 1024                // candidates of a row that are compared in pairs
 #define SC_STEPS 128.f              // bins of the first histogram by probability to a factor of e
+#define SC_GROUPS 16                // parts of a warp's share whose sums it keeps for the draw
 #define SC_MAX_SLICE 45056          // floats of a row a CTA can hold beside the histogram
 typedef unsigned long long u64;
 
@@ -215,13 +235,13 @@ struct alignas(16) ScShared {
         };
     };
     u64 cand[SC_CAND];              // candidates of this CTA's slice
-    u64 tops[SC_WARPS];             // its warps' maxima: (key, ~index)
-    u64 maxima[SC_MAXIMA];          // those of the whole row
+    unsigned int tops[SC_WARPS];    // its warps' maxima (keys)
+    unsigned int maxima[SC_MAXIMA]; // those of the whole row
+    unsigned int first;             // least index of a largest logit in its slice
     unsigned int ncand;             // candidates met (more than SC_CAND: not all are noted)
     unsigned int lowest;            // a bound of the k-th largest key, or the least key found
     u64 total;                      // of `sums`
     u64 kept;                       // this CTA's part of the kept set
-    u64 best;                       // largest (key, ~index) of this CTA's slice
     u64 z;                          // probability of its slice
     unsigned int bad;
     u64 warp_a[SC_WARPS];
@@ -299,7 +319,7 @@ __device__ int sc_gather(ScShared& sh, bool take) {
 }
 
 // top-k, top-p and the draw among `n` gathered candidates that hold the row's k largest keys: one CTA, every pair compared.
-__device__ void sc_finish(ScShared& sh, int n, int k, float p_keep, unsigned int gkey, float gmax, float inv_t, int arg, u64 m, int* token,
+__device__ void sc_finish(ScShared& sh, int n, int k, float p_keep, unsigned int gkey, float gmax, float inv_t, u64 m, int* token,
                           float* logprob) {
     const int tid = threadIdx.x;
     u64 z = 0;
@@ -345,10 +365,28 @@ __device__ void sc_finish(ScShared& sh, int n, int k, float p_keep, unsigned int
             if (logprob) *logprob = (key_float((unsigned int)(sh.list[t] >> 32)) - gmax) * inv_t - logf((float)((double)z * 5.684341886080802e-14));
         }
     }
-    if (z == 0 && tid == 0) {
-        *token = arg;
+    if (z == 0 && tid == 0) {                    // the first of the largest (-0 and 0 are equal), all of which are candidates
+        unsigned int first = 0xffffffffu;
+        for (int j = 0; j < n; ++j)
+            if (key_float((unsigned int)(sh.list[j] >> 32)) == gmax) first = min(first, (unsigned int)sh.list[j]);
+        *token = (int)first;
         if (logprob) *logprob = 0.f;
     }
+}
+
+// The row's first index among its largest logits (in every thread).  Called by all threads of the cluster.
+__device__ int sc_first(ScShared& sh, const float* row, int n, int i0, float gmax) {
+    cg::cluster_group cluster = cg::this_cluster();
+    if (threadIdx.x == 0) sh.first = 0x7fffffffu;
+    __syncthreads();
+    unsigned int first = 0x7fffffffu;
+    for (int i = threadIdx.x; i < n; i += SC_THREADS)
+        if (row[i] == gmax) first = min(first, (unsigned int)(i0 + i));
+    if (first != 0x7fffffffu) atomicMin(&sh.first, first);
+    cluster.sync();
+#pragma unroll
+    for (int q = 0; q < SC_CLUSTER; ++q) first = min(first, *cluster.map_shared_rank(&sh.first, q));
+    return (int)first;
 }
 
 // Sums this level's bins over the cluster and finds the first at which the weight so far exceeds the limit, which `limit_of`
@@ -464,10 +502,10 @@ __device__ unsigned int sc_select(ScShared& sh, const float* row, int n, unsigne
     return prefix;
 }
 
+template <typename Rows>
 __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
-    const float* __restrict__ logits, int64_t ld, int V, int slice, const float* __restrict__ temperature,
-    const int* __restrict__ top_k, const float* __restrict__ top_p, const u64* __restrict__ seed,
-    const u64* __restrict__ counter, int* __restrict__ token_out, float* __restrict__ logprob_out) {
+    const float* __restrict__ logits, int64_t ld, int V, int slice, const __grid_constant__ Rows rows, int* __restrict__ token_out,
+    float* __restrict__ logprob_out) {
     extern __shared__ __align__(16) unsigned char sc_smem[];
     ScShared& sh = *reinterpret_cast<ScShared*>(sc_smem);
     float* row = reinterpret_cast<float*>(sc_smem + sizeof(ScShared));
@@ -478,68 +516,58 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     pdl_trigger();
     const int i0 = min(V, rank * slice), n = min(V, i0 + slice) - i0;
     const float* x = logits + (int64_t)r * ld + i0;
-    const float temp = temperature[r];
+    const float temp = rows.temperature[r];
 
-    // the slice into shared memory; largest logit (first index among equals) and finiteness on the way
-    float top = -INFINITY;
-    int top_i = -1;
-    unsigned int bad = 0;
-    auto take = [&](float v, int i) {
-        if (!(fabsf(v) <= 3.0e38f)) bad = 1;
-        if (v > top) { top = v; top_i = i; }
-        row[i] = v;
+    // the slice into shared memory; its largest logit, and finiteness: NaN and infinities make a NaN of their product with 0
+    float top = -INFINITY, size = 0.f, zero = 0.f;
+    auto take = [&](float v) {
+        top = fmaxf(top, v);
+        size = fmaxf(size, fabsf(v));
+        zero = fmaf(v, 0.f, zero);
     };
     if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
         const int n4 = n >> 2;
 #pragma unroll 8
         for (int i = tid; i < n4; i += SC_THREADS) {
             const float4 v = reinterpret_cast<const float4*>(x)[i];
-            take(v.x, 4 * i); take(v.y, 4 * i + 1); take(v.z, 4 * i + 2); take(v.w, 4 * i + 3);
+            take(v.x); take(v.y); take(v.z); take(v.w);
+            reinterpret_cast<float4*>(row)[i] = v;
         }
-        for (int i = 4 * n4 + tid; i < n; i += SC_THREADS) take(x[i], i);
+        for (int i = 4 * n4 + tid; i < n; i += SC_THREADS) { take(x[i]); row[i] = x[i]; }
     } else {
 #pragma unroll 8
-        for (int i = tid; i < n; i += SC_THREADS) take(x[i], i);
+        for (int i = tid; i < n; i += SC_THREADS) { const float v = x[i]; take(v); row[i] = v; }
     }
-    // -0 and 0 are equal: the first of them wins
-    u64 best = top_i < 0 ? 0ull : ((u64)float_key(top == 0.f ? 0.f : top) << 32) | (unsigned int)~(i0 + top_i);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
-        best = other > best ? other : best;
-    }
+    unsigned int bad = !(size <= 3.0e38f) || zero != 0.f;
+    top = warp_max(top);
     if (tid == 0) { sh.bad = 0; sh.ncand = 0; }
-    if (lane == 0) sh.tops[warp] = best;
+    if (lane == 0) sh.tops[warp] = float_key(top == 0.f ? 0.f : top);        // -0 and 0 are equal
     __syncthreads();
     if (bad) sh.bad = 1;
-    const int k = top_k[r];
-    const float p_keep = top_p[r];
-    const u64 m = (u64)(uniform_from(seed[r], counter[r]) * 16777216.f);       // u = m / 2^24
+    const int k = rows.top_k[r];
+    const float p_keep = rows.top_p[r];
+    const u64 m = (u64)(uniform_from(rows.seed[r], rows.counter[r]) * 16777216.f);       // u = m / 2^24
     cluster.sync();
     if (tid < SC_MAXIMA) sh.maxima[tid] = cluster.map_shared_rank(&sh.tops[0], tid / SC_WARPS)[tid % SC_WARPS];
     bad = 0;
 #pragma unroll
     for (int q = 0; q < SC_CLUSTER; ++q) bad |= *cluster.map_shared_rank(&sh.bad, q);
     __syncthreads();
-    best = 0;
+    unsigned int gkey = 0;
 #pragma unroll
-    for (int q = 0; q < SC_MAXIMA / 32; ++q) best = max(best, sh.maxima[lane + 32 * q]);
+    for (int q = 0; q < SC_MAXIMA / 32; ++q) gkey = max(gkey, sh.maxima[lane + 32 * q]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
-        best = other > best ? other : best;
-    }
-    const int arg = (int)~(unsigned int)best;
+    for (int o = 16; o > 0; o >>= 1) gkey = max(gkey, __shfl_xor_sync(0xffffffffu, gkey, o));
+    const float gmax = key_float(gkey);
     if (bad || !(temp > 0.f)) {
+        const int arg = bad ? -1 : sc_first(sh, row, n, i0, gmax);
         if (rank == 0 && tid == 0) {
-            token_out[r] = bad ? -1 : arg;
+            token_out[r] = arg;
             if (logprob_out) logprob_out[r] = 0.f;
         }
         cluster.sync();              // a CTA's shared memory stays until all have read it
         return;
     }
-    const unsigned int gkey = (unsigned int)(best >> 32);
-    const float gmax = key_float(gkey);
     const float inv_t = 1.f / temp;
     unsigned int lo_key = 0u;
     const bool by_k = k > 0 && k < V;
@@ -549,23 +577,33 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
             // The k-th largest of the warps' maxima: k warps hold a key from it on, so the k-th largest key is one (a maximum of
             // -0 counts as 0 there).  Its rank by comparison, equal ones (warps without an element) in their order.
             if (tid < SC_MAXIMA) {
-                const u64 own = sh.maxima[tid];
+                const unsigned int own = sh.maxima[tid];
                 int before = 0;
                 for (int j = 0; j < SC_MAXIMA; ++j) before += sh.maxima[j] > own || (sh.maxima[j] == own && j < tid);
-                if (before == k - 1) sh.lowest = (unsigned int)(own >> 32);
+                if (before == k - 1) sh.lowest = own;
             }
             __syncthreads();
             low = sh.lowest;
             if (low == float_key(0.f)) low = float_key(-0.f);
-            for (int i = tid; i < n; i += SC_THREADS) {
-                const unsigned int key = float_key(row[i]);
-                if (key >= low) sc_note(sh, key, i0 + i);
+            // as keys and as numbers the same: low is not the key of 0
+            const float least = key_float(low);
+            const int n4 = n >> 2;
+            for (int i = tid; i < n4; i += SC_THREADS) {
+                const float4 v = reinterpret_cast<const float4*>(row)[i];
+                if (fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) >= least) {
+                    if (v.x >= least) sc_note(sh, float_key(v.x), i0 + 4 * i);
+                    if (v.y >= least) sc_note(sh, float_key(v.y), i0 + 4 * i + 1);
+                    if (v.z >= least) sc_note(sh, float_key(v.z), i0 + 4 * i + 2);
+                    if (v.w >= least) sc_note(sh, float_key(v.w), i0 + 4 * i + 3);
+                }
             }
+            for (int i = 4 * n4 + tid; i < n; i += SC_THREADS)
+                if (row[i] >= least) sc_note(sh, float_key(row[i]), i0 + i);
             const int found = sc_gather(sh, rank == 0);
             if (found >= 0) {
                 cluster.sync();      // the others' notes have been read
                 if (rank == 0)
-                    sc_finish(sh, found, k, p_keep, gkey, gmax, inv_t, arg, m, token_out + r, logprob_out ? logprob_out + r : nullptr);
+                    sc_finish(sh, found, k, p_keep, gkey, gmax, inv_t, m, token_out + r, logprob_out ? logprob_out + r : nullptr);
                 return;
             }
         }
@@ -598,13 +636,15 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
                 found = sc_gather(sh, true);
                 for (int t = tid; t < found; t += SC_THREADS) sh.w[t] = prob_fixed(key_float((unsigned int)(sh.list[t] >> 32)), gmax, inv_t);
                 __syncthreads();
-                for (int t = tid; t < found; t += SC_THREADS) {
+                // an eighth of the candidates to each CTA; the least key at which the sum exceeds the limit is told to all
+                for (int t = rank + SC_CLUSTER * tid; t < found; t += SC_CLUSTER * SC_THREADS) {
                     const unsigned int key = (unsigned int)(sh.list[t] >> 32);
                     u64 upto = 0;
                     for (int j = 0; j < found; ++j) upto += (unsigned int)(sh.list[j] >> 32) <= key ? sh.w[j] : 0ull;
-                    if (upto > sh.left) atomicMin(&sh.lowest, key);
+                    if (upto > sh.left && key < gkey)
+                        for (int q = 0; q < SC_CLUSTER; ++q) atomicMin(cluster.map_shared_rank(&sh.lowest, q), key);
                 }
-                __syncthreads();
+                cluster.sync();
                 if (found >= 0) lo_key = sh.lowest;
                 else lo_key = 0u;
             }
@@ -627,12 +667,19 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
             lo_key = key < gkey ? key : gkey;            // the largest always stays
         }
     }
-    // inverse CDF in token order over the kept set; a thread owns a run of the slice (of odd length: no bank conflicts)
-    const int seg = ((n + SC_THREADS - 1) / SC_THREADS) | 1;
-    const int a = min(n, tid * seg), b = min(n, a + seg);
+    // inverse CDF in token order over the kept set: a warp owns a run of the slice, in SC_GROUPS groups; lane g keeps the sum of
+    // group g
+    const int group = (n + SC_WARPS * SC_GROUPS - 1) / (SC_WARPS * SC_GROUPS);
+    const int run0 = warp * SC_GROUPS * group;
+    auto weigh = [&](int i) -> u64 { return float_key(row[i]) >= lo_key ? prob_fixed(row[i], gmax, inv_t) : 0ull; };
     u64 mine = 0;
-    for (int i = a; i < b; ++i)
-        if (float_key(row[i]) >= lo_key) mine += prob_fixed(row[i], gmax, inv_t);
+    for (int g = 0; g < SC_GROUPS; ++g) {
+        const int a = min(n, run0 + g * group), b = min(n, a + group);
+        u64 part = 0;
+        for (int i = a + lane; i < b; i += 32) part += weigh(i);
+        part = warp_sum_u64(part);
+        if (lane == g) mine = part;
+    }
     u64 incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -642,12 +689,12 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     __syncthreads();
     if (lane == 31) sh.warp_a[warp] = incl;
     __syncthreads();
-    u64 before = incl - mine;
-    u64 here = 0;
+    u64 before = 0, here = 0;                    // of the row up to this warp's run
     for (int w = 0; w < SC_WARPS; ++w) {
         if (w < warp) before += sh.warp_a[w];
         here += sh.warp_a[w];
     }
+    const u64 own = sh.warp_a[warp];
     if (tid == 0) sh.kept = here;
     cluster.sync();
     u64 total = 0;
@@ -659,34 +706,56 @@ __global__ void __launch_bounds__(SC_THREADS, 2) sample_cluster_kernel(
     }
     // the first token whose running sum exceeds floor(m total / 2^24)
     const u64 target = (__umul64hi(m, total) << 40) | ((m * total) >> 24);
-    if (target >= before && target < before + mine) {
-        int i = a;
-        for (;; ++i) {
-            if (float_key(row[i]) < lo_key) continue;
-            before += prob_fixed(row[i], gmax, inv_t);
-            if (before > target) break;
+    if (target >= before && target < before + own) {         // one warp of the cluster
+        const int g = __ffs(__ballot_sync(0xffffffffu, before + incl > target)) - 1;
+        before += __shfl_sync(0xffffffffu, incl - mine, g);
+        const int a = min(n, run0 + g * group), b = min(n, a + group);
+        for (int at = a; at < b; at += 32) {
+            const int i = at + lane;
+            const u64 w = i < b ? weigh(i) : 0ull;
+            u64 upto = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const u64 up = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += up;
+            }
+            const unsigned int over = __ballot_sync(0xffffffffu, before + upto > target);
+            if (over != 0) {
+                if (lane == __ffs(over) - 1) {
+                    token_out[r] = i0 + i;
+                    if (logprob_out) logprob_out[r] = (row[i] - gmax) * inv_t - logf((float)((double)total * 5.684341886080802e-14));
+                }
+                break;
+            }
+            before += __shfl_sync(0xffffffffu, upto, 31);
         }
-        token_out[r] = i0 + i;
-        if (logprob_out) logprob_out[r] = (row[i] - gmax) * inv_t - logf((float)((double)total * 5.684341886080802e-14));
-    } else if (total == 0 && rank == 0 && tid == 0) {
-        token_out[r] = arg;
-        if (logprob_out) logprob_out[r] = 0.f;
+    }
+    if (total == 0) {
+        const int arg = sc_first(sh, row, n, i0, gmax);
+        if (rank == 0 && tid == 0) {
+            token_out[r] = arg;
+            if (logprob_out) logprob_out[r] = 0.f;
+        }
     }
     cluster.sync();
 }
 
-static int launch_sample_cluster(const float* logits, int64_t ld, int rows, int V, int slice, const float* temperature,
-                                 const int* top_k, const float* top_p, const u64* seed, const u64* counter, int* token_out,
-                                 float* logprob_out, cudaStream_t stream) {
+template <typename Rows>
+static int launch_sample(const float* logits, int64_t ld, int n, int V, const Rows& rows, int* token_out, float* logprob_out, int clusters,
+                         cudaStream_t stream) {
+    // slices are multiples of four logits, so that they start on 16 bytes where the row does
+    const int slice = ((V + SC_CLUSTER - 1) / SC_CLUSTER + 3) & ~3;
+    if (!clusters || slice > SC_MAX_SLICE || n > 0x7fffffff / SC_CLUSTER)
+        return acorn_launch(sample_kernel<Rows>, dim3(n), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, rows, token_out, logprob_out);
     static AcornPerDevice configured;
     if (!configured.seen()) {
         const int most = (int)(sizeof(ScShared) + SC_MAX_SLICE * sizeof(float));
-        cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel<Rows>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return (int)e;
         configured.mark();
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(rows * SC_CLUSTER));
+    cfg.gridDim = dim3((unsigned)(n * SC_CLUSTER));
     cfg.blockDim = dim3(SC_THREADS);
     cfg.dynamicSmemBytes = sizeof(ScShared) + (size_t)slice * sizeof(float);
     cfg.stream = stream;
@@ -699,8 +768,7 @@ static int launch_sample_cluster(const float* logits, int64_t ld, int rows, int 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = acorn_pdl_enabled() ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel, logits, ld, V, slice, temperature, top_k, top_p, seed, counter,
-                                       token_out, logprob_out);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<Rows>, logits, ld, V, slice, rows, token_out, logprob_out);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -709,12 +777,28 @@ extern "C" int acorn_sample(const float* logits, int64_t ld, int rows, int V, co
                             const unsigned long long* counter, int* token_out, float* logprob_out, int clusters,
                             cudaStream_t stream) {
     if (rows <= 0) return 0;
-    // slices are multiples of four logits, so that they start on 16 bytes where the row does
-    const int slice = ((V + SC_CLUSTER - 1) / SC_CLUSTER + 3) & ~3;
-    if (clusters && slice <= SC_MAX_SLICE && rows <= 0x7fffffff / SC_CLUSTER)
-        return launch_sample_cluster(logits, ld, rows, V, slice, temperature, top_k, top_p, seed, counter, token_out, logprob_out, stream);
-    return acorn_launch(sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, temperature, top_k,
-                        top_p, seed, counter, token_out, logprob_out);
+    const SampleArrays r = {temperature, top_k, top_p, seed, counter};
+    return launch_sample(logits, ld, rows, V, r, token_out, logprob_out, clusters, stream);
+}
+
+// The same with the parameters in host memory: one after the other `rows` seeds, counters (64 bits each), temperatures, top_p
+// (float32) and top_k (int32).  At most SAMPLE_INLINE_ROWS rows; `block` is free again when this returns.
+extern "C" int acorn_sample_inline(const float* logits, int64_t ld, int rows, int V, const void* block, int* token_out, float* logprob_out,
+                                   int clusters, cudaStream_t stream) {
+    if (rows <= 0) return 0;
+    if (rows > SAMPLE_INLINE_ROWS || block == nullptr) return ACORN_ERR_UNSUPPORTED;
+    SampleInline r = {};
+    const unsigned char* at = (const unsigned char*)block;
+    auto part = [&](void* to, size_t bytes) {
+        memcpy(to, at, bytes);
+        at += bytes;
+    };
+    part(r.seed, 8 * (size_t)rows);
+    part(r.counter, 8 * (size_t)rows);
+    part(r.temperature, 4 * (size_t)rows);
+    part(r.top_p, 4 * (size_t)rows);
+    part(r.top_k, 4 * (size_t)rows);
+    return launch_sample(logits, ld, rows, V, r, token_out, logprob_out, clusters, stream);
 }
 
 // Host copy of the generator, for callers that need the same uniforms off the device.

@@ -9,6 +9,7 @@ to fall back to.  Tensors are passed as raw device pointers.
 from __future__ import annotations
 
 import ctypes
+from array import array
 from ctypes import c_float, c_int, c_int64, c_void_p
 from dataclasses import dataclass
 from functools import lru_cache
@@ -287,6 +288,7 @@ class _Sigs:
     acorn_gemm_f32_tc_set_error_word = [c_void_p]
     acorn_sample = [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                     c_void_p, c_void_p, c_int, c_void_p]
+    acorn_sample_inline = [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
     acorn_uniform = [ctypes.c_uint64, ctypes.c_uint64]
     acorn_random_fill = [c_void_p, c_int64, ctypes.c_uint64, ctypes.c_uint64, c_float, c_float, c_int, c_void_p]
     acorn_error_word_alloc = [c_void_p, c_void_p]
@@ -2886,6 +2888,25 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
     _ok(lib().acorn_sample(logits.data_ptr(), logits.stride(0), R, V, temperature.data_ptr(), top_k.data_ptr(),
                            top_p.data_ptr(), seed.data_ptr(), counter.data_ptr(), tokens.data_ptr(),
                            _ptr(logprobs), int(sample_in_clusters(R, V, greedy)), _stream()), "sample")
+    return tokens, logprobs
+
+
+SAMPLE_INLINE_ROWS = 128          # rows whose parameters travel among a launch's arguments
+
+
+def sample_inline(logits: torch.Tensor, seeds: list[int], counters: list[int], temperatures: list[float], top_ps: list[float],
+                  top_ks: list[int], want_logprobs: bool = False, greedy: bool = False):
+    """``sample`` with the rows' parameters still on the host (at most ``SAMPLE_INLINE_ROWS`` rows): no copy to the device before
+    the launch, which took the host longer than the launch."""
+    _check(logits, "logits", torch.float32, 2)
+    R, V = logits.shape
+    if R > SAMPLE_INLINE_ROWS or not (len(seeds) == len(counters) == len(temperatures) == len(top_ps) == len(top_ks) == R):
+        raise KernelError(f"sample_inline takes at most {SAMPLE_INLINE_ROWS} rows and one entry a row of every parameter")
+    block = array("q", [*seeds, *counters]).tobytes() + array("f", [*temperatures, *top_ps]).tobytes() + array("i", top_ks).tobytes()
+    tokens = torch.empty(R, dtype=torch.int32, device=logits.device)
+    logprobs = torch.empty(R, dtype=torch.float32, device=logits.device) if want_logprobs else None
+    _ok(lib().acorn_sample_inline(logits.data_ptr(), logits.stride(0), R, V, ctypes.cast(block, c_void_p).value, tokens.data_ptr(),
+                                  _ptr(logprobs), int(sample_in_clusters(R, V, greedy)), _stream()), "sample")
     return tokens, logprobs
 
 

@@ -91,6 +91,9 @@ class Sampler:
         greedy = all(p.greedy for p in params)
         if greedy:
             temperature, top_k, top_p, seeds, ctrs = self._greedy_params(R)
+        elif R <= ops.SAMPLE_INLINE_ROWS:
+            return ops.sample_inline(logits, [p.seed & (2 ** 63 - 1) for p in params], counters, [p.temperature for p in params],
+                                     [p.top_p for p in params], [p.top_k for p in params], want_logprobs)
         else:
             # one copy to the device for all five (each copy costs the host as much as the kernel takes)
             block = np.empty(7 * R, dtype=np.int32)

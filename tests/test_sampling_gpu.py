@@ -160,3 +160,24 @@ def test_candidates_at_the_ends_of_the_lists(n, spread, top_k, top_p):
     assert toks.tolist() == [int(at[int(int(v * 2 ** 24) * n // 2 ** 24)]) for v in u]
     # -ln n in float32: one rounding of the logarithm's argument and one of its result
     assert (lps.cpu().double() + torch.tensor(float(n)).double().log()).abs().max() < 4 * 2.0 ** -24 * 8
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 50), (128, 700), (128, 20001), (129, 700)])
+def test_parameters_among_the_launch_arguments(rows, vocab):
+    """Up to 128 rows carry their parameters in the launch, more in device memory: the same tokens and log-probabilities."""
+    from acorninfer_b200 import SamplingParams
+    from acorninfer_b200.kernels import ops
+    from acorninfer_b200.sampling.sampler import Sampler
+    g = torch.Generator().manual_seed(rows)
+    x = (2 * torch.randn(rows, vocab, generator=g)).to(DEV)
+    params = [SamplingParams(temperature=(0.7, 0.0, 1e39, 1.3)[i % 4], top_p=(1.0, 0.4, 0.9)[i % 3], top_k=(0, 7, 1000000, 150)[i % 4],
+                             seed=(1 << 62) + 5 * i) for i in range(rows)]
+    counters = [i << 33 for i in range(rows)]
+    f = lambda v, dt: torch.tensor(v, dtype=dt, device=DEV)
+    want = ops.sample(x, f([p.temperature for p in params], torch.float64).float(), f([p.top_k for p in params], torch.int32),
+                      f([p.top_p for p in params], torch.float32), f([p.seed for p in params], torch.int64), f(counters, torch.int64), True)
+    got = Sampler(DEV).launch(x, params, counters, True)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    if rows > ops.SAMPLE_INLINE_ROWS:
+        with pytest.raises(ops.KernelError):
+            ops.sample_inline(x, [0] * rows, [0] * rows, [1.0] * rows, [1.0] * rows, [0] * rows)
