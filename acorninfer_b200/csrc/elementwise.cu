@@ -218,6 +218,27 @@ __global__ void swiglu_bf16x8_kernel(const bf16* __restrict__ gu, bf16* __restri
     }
 }
 
+// float32 rows whose block width is a multiple of four, as above: 16-byte loads and stores, no 64-bit division by the row width an
+// element.
+__global__ void swiglu_f32x4_kernel(const float* __restrict__ gu, float* __restrict__ out, int I4, int b4, int act, float limit) {
+    pdl_wait();
+    pdl_trigger();
+    const float4* row = reinterpret_cast<const float4*>(gu) + (int64_t)blockIdx.y * I4 * 2;
+    float4* orow = reinterpret_cast<float4*>(out) + (int64_t)blockIdx.y * I4;
+    auto one = [&](float g, float u) -> float {
+        if (act == 2) {
+            g = fminf(g, limit);
+            u = fminf(fmaxf(u, -limit), limit) + 1.f;
+        }
+        return glu_act(g, act) * u;
+    };
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < I4; i += gridDim.x * blockDim.x) {
+        const int gi = (i / b4) * 2 * b4 + i % b4;
+        const float4 g = row[gi], u = row[gi + b4];
+        orow[i] = make_float4(one(g.x, u.x), one(g.y, u.y), one(g.z, u.z), one(g.w, u.w));
+    }
+}
+
 extern "C" int acorn_swiglu(const void* gu, void* out, int tokens, int I, int block, int dtype, int act, float limit,
                             cudaStream_t stream) {
     const int64_t total = (int64_t)tokens * I;
@@ -236,6 +257,9 @@ extern "C" int acorn_swiglu(const void* gu, void* out, int tokens, int I, int bl
         return acorn_launch(swiglu_bf16x8_kernel<0>, dim3(bx, tokens), dim3(256), 0, stream, (const bf16*)gu, (bf16*)out,
                             I8, block / 8, limit);
     }
+    if (dtype == ACORN_DTYPE_F32 && block % 4 == 0 && tokens <= 65535 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0)
+        return acorn_launch(swiglu_f32x4_kernel, dim3((I / 4 + 255) / 256, tokens), dim3(256), 0, stream, (const float*)gu, (float*)out,
+                            I / 4, block / 4, act, limit);
     int64_t blocks = (total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     ACORN_DISPATCH_DTYPE(dtype, T, return acorn_launch(swiglu_kernel<T>, dim3((int)blocks), dim3(256), 0, stream,

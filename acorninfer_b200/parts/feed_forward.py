@@ -58,7 +58,7 @@ class SwiGLU(FeedForward):
     def fusable(self, num_rows):
         widths = (2 * self.intermediate_size, self.hidden_size)                 # of the gate/up product and of the down product
         return (self.epilogue_act and (ops.fused_rows_ok(num_rows, self.ctx.dtype, widths, ops.device_sms(self.ctx.device))
-                                       or ops.fused_tile_ok(num_rows, self.ctx.dtype))
+                                       or (ops.fused_tile_ok(num_rows, self.ctx.dtype) and not self._gate_up_fuses(num_rows)))
                 and self.w_gate_up.dtype == torch.bfloat16
                 and self.w_down.dtype == torch.bfloat16 and self.hidden_size % 8 == 0
                 and self.intermediate_size % 8 == 0)
