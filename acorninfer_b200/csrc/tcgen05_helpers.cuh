@@ -17,7 +17,6 @@
 #define ACORN_KERNEL_GEMM_PAIR 4
 #define ACORN_KERNEL_LATENT_PREFILL_TC 5
 #define ACORN_KERNEL_GEMM_F32_TC 6
-#define ACORN_KERNEL_ATTN_DECODE_STREAM 7
 #define ACORN_KERNEL_SELFTEST 9
 
 static __device__ int* g_error_word = nullptr;

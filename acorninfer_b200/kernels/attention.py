@@ -109,7 +109,8 @@ def decode_splits(rows: int, num_kv_heads: int, key_bound: int, head_dim: int, n
 # and of 35 to 100 %, every number of splits).  Clusters run in one wave only as long as they fill no more than seven
 # eighths of the CTAs that single ones would (5 rows of 900 keys: 6 splits, 240 CTAs, 9.1 us; 7 splits, 280 CTAs, 15.4; 12 rows: 2
 # splits 13.9, 3 splits, 288 CTAs, 21.6), pairs of CTAs fill all of them, clusters of sixteen half; and a second wave of
-# clusters costs more than its splits bring (41 rows of 900: unsplit 43.7, 3 splits 50.7).
+# clusters costs more than its splits bring (41 rows of 900: unsplit 43.7, 3 splits 50.7; a step of 41 rows of 600 to 1,700 keys at
+# Qwen3-4B: 3,866 and 4,280 us).
 _START_US, _CLUSTER_US = 3.5, 1.5
 
 
@@ -120,13 +121,10 @@ def _wave(splits: int, num_sms: int) -> int:
 
 @lru_cache(maxsize=4096)
 def decode_plan(rows: int, num_kv_heads: int, key_bound: int, num_sms: int = B200_SMS, merge_limit: int = 16) -> int:
-    """For the TMA decode kernel (head size 128, ``merge_limit`` splits merged inside it): splits of the key range, or 0 where the keys
-    of all rows should be shared out evenly instead (``ops.attention_decode_stream``): where whole (row, kv head)s leave
-    the last of several waves of CTAs less than four fifths full, as 41 rows of 8 do on 148 SMs (us, unsplit / even shares at 900 keys:
-    43.7 / 35.7, of 35 to 100 % as many 28.5 / 27.5; 48 rows 44.1 / 38.2; 64 rows, 0.86 full, 46.6 / 47.6)."""
+    """Splits of the key range for the TMA decode kernel (head size 128, ``merge_limit`` splits merged inside it)."""
     pairs, wave = rows * num_kv_heads, 2 * num_sms
     if pairs > wave:
-        return 0 if pairs < 0.8 * wave * -(-pairs // wave) and key_bound > 2 * _CHUNK else 1
+        return 1
     most = max(1, -(-key_bound // _CHUNK))
     pair_kb = key_bound * 128 * 4 / 1e3                             # K and V of one pair, bfloat16, in KB
     best, best_us = 1, None
@@ -155,15 +153,11 @@ def _merge_free(nq: int, nkv: int, d: int, P: int) -> int:
 
 def _decode(qkv, inputs, group, cache, nq, nkv, d, P, scale, window, bound, n, windowed_only, mask, token_list=None, out=None):
     """The step's ``n`` single-token rows (``token_list``, or all tokens) on a decode kernel."""
-    args = (qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table, group.page_base, inputs.token_row, inputs.positions,
-            inputs.num_tokens, nq, nkv, d, scale, window)
     limit = _merge_free(nq, nkv, d, P) if windowed_only else 1
-    if limit > 1:                                                    # the TMA kernel takes these sizes
-        splits = decode_plan(n, nkv, bound, sm_count(qkv.device), limit)
-        if splits == 0 and ops.attention_decode_stream_supported(nq, nkv, d, P, n):
-            return ops.attention_decode_stream(*args, token_list=token_list, out=out)
-        return ops.attention_decode(*args, max(splits, 1), token_list=token_list, out=out, **mask)
-    return ops.attention_decode(*args, decode_splits(n, nkv, bound, d, sm_count(qkv.device), limit), token_list=token_list, out=out,
+    # (a limit above 1: the TMA kernel takes these sizes)
+    splits = decode_plan(n, nkv, bound, sm_count(qkv.device), limit) if limit > 1 else decode_splits(n, nkv, bound, d, sm_count(qkv.device))
+    return ops.attention_decode(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table, group.page_base, inputs.token_row,
+                                inputs.positions, inputs.num_tokens, nq, nkv, d, scale, window, splits, token_list=token_list, out=out,
                                 **mask)
 
 

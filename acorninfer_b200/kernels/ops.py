@@ -78,8 +78,7 @@ def build_calls() -> None:
 
 _error_word: ctypes.c_int | None = None       # pinned host memory that kernels write when a bounded wait gives up
 _KERNEL_NAMES = {1: "gemm_tcgen05", 2: "attention_prefill_tc", 3: "attention_decode_tma", 4: "gemm_tcgen05_pair",
-                 5: "latent_prefill_tc", 6: "gemm_f32_tc", 7: "attention_decode_stream",
-                 9: "error-word self-test"}
+                 5: "latent_prefill_tc", 6: "gemm_f32_tc", 9: "error-word self-test"}
 
 
 def _init_error_word(library) -> None:
@@ -90,8 +89,7 @@ def _init_error_word(library) -> None:
         raise KernelError(f"could not allocate the kernels' error word: CUDA error {code}")
     for setter in ("acorn_gemm_tc_set_error_word", "acorn_attention_tc_set_error_word",
                    "acorn_attention_decode_tma_set_error_word", "acorn_selftest_set_error_word",
-                   "acorn_gemm_tc_pair_set_error_word", "acorn_latent_prefill_tc_set_error_word", "acorn_gemm_f32_tc_set_error_word",
-                   "acorn_attention_decode_stream_set_error_word"):
+                   "acorn_gemm_tc_pair_set_error_word", "acorn_latent_prefill_tc_set_error_word", "acorn_gemm_f32_tc_set_error_word"):
         code = getattr(library, setter)(dev)
         if code != 0:
             raise KernelError(f"{setter}: CUDA error {code}")
@@ -105,8 +103,7 @@ def raise_on_kernel_error() -> None:
         return
     word = _error_word.value
     _error_word.value = 0
-    for getter in (gemm_tc_error, attention_tc_error, attention_decode_tma_error, gemm_tc_pair_error, latent_prefill_tc_error, gemm_f32_tc_error,
-                   attention_decode_stream_error):   # clear the kernels' own flags
+    for getter in (gemm_tc_error, attention_tc_error, attention_decode_tma_error, gemm_tc_pair_error, latent_prefill_tc_error, gemm_f32_tc_error):   # clear the kernels' own flags
         getter()
     raise KernelError(f"kernel {_KERNEL_NAMES.get(word // 100, word // 100)} gave up a bounded wait at point "
                       f"{word % 100}: the results of the step are not valid")
@@ -247,12 +244,6 @@ class _Sigs:
     acorn_attention_decode_tma_supported = [c_int, c_int, c_int, c_int]
     acorn_attention_decode_tma_merges = [c_int, c_int]
     acorn_attention_decode_tma_error = []
-    acorn_attention_decode_stream = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p,
-                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p,
-                                     c_void_p]
-    acorn_attention_decode_stream_supported = [c_int, c_int, c_int, c_int, c_int]
-    acorn_attention_decode_stream_error = []
-    acorn_attention_decode_stream_set_error_word = [c_void_p]
     acorn_attention_decode_merge = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     acorn_attention_prefill = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
@@ -910,42 +901,6 @@ def attention_decode(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_pa
                                         _ptr(slopes32), _ptr(sink32), float(softcap or 0.0), int(maps), _stream()),
         "attention_decode")
     return out
-
-
-def attention_decode_stream_supported(num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, rows: int) -> bool:
-    return bool(lib().acorn_attention_decode_stream_supported(num_heads, num_kv_heads, head_dim, page_size, rows))
-
-
-def attention_decode_stream(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
-                            page_base: torch.Tensor, token_row: torch.Tensor, positions: torch.Tensor, num_tokens: int,
-                            num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int | None,
-                            token_list: torch.Tensor | None = None, out: torch.Tensor | None = None, ctas: int | None = None) -> torch.Tensor:
-    """Decode attention (bfloat16, head size 128) of single-token rows as ``attention_decode``, the keys of all rows shared out
-    evenly over the device (``csrc/attention_decode_stream.cu``): for many rows, above all of unequal lengths.  ``ctas``: shares
-    (two to a multiprocessor if not given)."""
-    _check(k_pages, "k_pages", torch.bfloat16, 4)
-    _check(v_pages, "v_pages", torch.bfloat16, 4)
-    _check(block_table, "block_table", torch.int32, 2)
-    n, P = num_tokens if token_list is None else token_list.numel(), k_pages.shape[2]
-    if q.dtype != torch.bfloat16 or not attention_decode_stream_supported(num_heads, num_kv_heads, head_dim, P, n):
-        raise KernelError(f"attention_decode_stream does not take {n} rows, nq={num_heads}, nkv={num_kv_heads}, d={head_dim}, pages of {P}, {q.dtype}")
-    if out is None:
-        out = torch.empty((num_tokens, num_heads * head_dim), dtype=q.dtype, device=q.device)
-    if ctas is None:
-        ctas = 2 * device_sms(q.device)
-    rep = num_heads // num_kv_heads
-    parts = torch.empty(2 * ctas * rep * (head_dim + 1), dtype=torch.float32, device=q.device)      # results, then log-sums
-    _ok(lib().acorn_attention_decode_stream(
-        q.data_ptr(), q_stride, out.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0], block_table.data_ptr(),
-        page_base.data_ptr(), block_table.stride(0), token_row.data_ptr(), positions.data_ptr(), _ptr(token_list), n, num_heads,
-        num_kv_heads, head_dim, P, float(scale), int(window or 0), ctas, parts.data_ptr(),
-        parts.data_ptr() + 2 * ctas * rep * head_dim * 4, _stream()), "attention_decode_stream")
-    return out
-
-
-def attention_decode_stream_error() -> int:
-    """0, or where a bounded wait inside the evenly shared decode attention gave up since the last call (clears it)."""
-    return int(lib().acorn_attention_decode_stream_error())
 
 
 def attention_decode_tma_error() -> int:

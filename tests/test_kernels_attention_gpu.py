@@ -240,27 +240,6 @@ def test_attention_decode_kernel(nq, nkv, d, P, window, splits):
     assert torch.equal(out, again)
 
 
-@pytest.mark.parametrize("nq,nkv,P,window", [(32, 8, 16, None), (8, 1, 8, None), (6, 2, 8, 300), (8, 8, 128, 64), (5, 5, 32, 129)])
-@pytest.mark.parametrize("ctas", [1, 7, 50, None])
-def test_attention_decode_in_even_shares(nq, nkv, P, window, ctas):
-    """The keys of all rows in one line, cut into shares: one share for everything, borders within rows and heads, shares that lie
-    within one head, more shares than chunks; listed tokens, and rows that are not listed."""
-    before = [0, 1, 63, 64, 65, 700, 127, 2000, 5, 640]
-    lay, wide, k_pages, v_pages, _, _, _, want = build_case(before, [1] * len(before), nq, nkv, 128, P, window, 400, 3, standout_row=5)
-
-    def run(**more):
-        return ops().attention_decode_stream(wide, wide.stride(0), k_pages, v_pages, lay["block_table"], lay["page_base"], lay["token_row"],
-                                             lay["positions"], len(before), nq, nkv, 128, 128 ** -0.5, window, ctas=ctas, **more)
-    out = run()
-    assert torch.allclose(out.double().cpu(), want, **BF16_TOL)
-    assert torch.equal(out, run()) and ops().attention_decode_stream_error() == 0
-    chosen = [7, 1, 4]
-    part = torch.full_like(out, 7.0)
-    run(token_list=torch.tensor(chosen, dtype=torch.int32, device=DEV), out=part)
-    assert torch.allclose(part[chosen].double().cpu(), want[chosen], **BF16_TOL)
-    assert bool((part[[r for r in range(len(before)) if r not in chosen]] == 7.0).all())
-
-
 def test_attention_decode_token_list_leaves_other_rows():
     nq, nkv, d, P = 8, 2, 64, 16
     before, qlens = [10, 300, 77, 5], [1, 1, 1, 1]

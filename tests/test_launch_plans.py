@@ -32,16 +32,16 @@ def test_decode_splits_follow_the_measured_cases():
 def test_decode_plans_of_the_tma_kernel():
     """One wave of clusters or none; the measured cases; what the kernels take."""
     from acorninfer_b200.kernels.attention import decode_plan
-    want = {1: 16, 2: 8, 3: 8, 5: 6, 6: 5, 7: 4, 8: 4, 9: 3, 10: 3, 11: 2, 12: 2, 16: 2, 19: 1, 32: 1, 37: 1, 41: 0, 48: 0, 64: 1}
+    want = {1: 16, 2: 8, 3: 8, 5: 6, 6: 5, 7: 4, 8: 4, 9: 3, 10: 3, 11: 2, 12: 2, 16: 2, 19: 1, 32: 1, 37: 1, 41: 1, 64: 1}
     assert {r: decode_plan(r, 8, 2048) for r in want} == want
-    assert decode_plan(41, 8, 128) == 1 and decode_plan(1, 8, 48) == 1 and decode_plan(1, 1, 1 << 20) == 32
+    assert decode_plan(1, 8, 48) == 1 and decode_plan(1, 1, 1 << 20) == 32
     rng = random.Random(2)
     for _ in range(2000):
         rows, nkv, bound = rng.randint(1, 4096), rng.choice([1, 2, 3, 5, 8, 16, 32]), rng.choice([1, 63, 64, 65, 1000, 4096, 40000, 1 << 20])
         limit = rng.choice([2, 8, 16])
         s = decode_plan(rows, nkv, bound, 148, limit)
-        assert 0 <= s <= 32 and s <= max(1, -(-bound // 64))
-        assert s <= 1 or rows * nkv * s <= 296
+        assert 1 <= s <= 32 and s <= max(1, -(-bound // 64))
+        assert s == 1 or rows * nkv * s <= 296
 
 
 def test_gemm_plans_are_valid_for_any_shape():
