@@ -1080,6 +1080,9 @@ GEMM_TC_MAX_ROWS = 32
 # 43.5 / 41.0 at 1.7B, 63.2 / 59.1 at 4B, 91.9 / 84.6 at 8B; at 64 rows 62.8 / 81.9 at 4B: a tile of 64 rows takes as much of an
 # SM's intake as half of the weights' tile.
 GEMM_TC_FUSED_MAX_ROWS = 48
+# ... and the smallest hidden size where that was measured to pay (41 rows: 1,024 to 4,096); below it the products are small enough
+# for the library and the launches beside them to cost the same.
+GEMM_TC_FUSED_MIN_WIDTH = 1024
 # The paired kernel (256 x 256 tiles, a pair of SMs to a tile at a time, fused epilogues) is used from
 # this many rows on, where its tiles fill the device: see ``pair_rows_ok``.
 GEMM_PAIR_MIN_ROWS = 256
@@ -1363,10 +1366,10 @@ def fused_rows_ok(num_rows: int, dtype: torch.dtype, widths=None, num_sms: int =
     return all(pair_rows_ok(num_rows, w, num_sms) for w in widths)
 
 
-def fused_tile_ok(num_rows: int, dtype: torch.dtype) -> bool:
+def fused_tile_ok(num_rows: int, dtype: torch.dtype, hidden: int) -> bool:
     """Whether so many rows, more than the one-CTA kernel takes for plain products, go to it where it spares a part the kernels
-    around its products (``GEMM_TC_FUSED_MAX_ROWS``)."""
-    return dtype == torch.bfloat16 and GEMM_TC_MAX_ROWS < num_rows <= GEMM_TC_FUSED_MAX_ROWS
+    around its products (``GEMM_TC_FUSED_MAX_ROWS``), in a model of this hidden size (``GEMM_TC_FUSED_MIN_WIDTH``)."""
+    return dtype == torch.bfloat16 and GEMM_TC_MAX_ROWS < num_rows <= GEMM_TC_FUSED_MAX_ROWS and hidden >= GEMM_TC_FUSED_MIN_WIDTH
 
 
 def linear(x, w: torch.Tensor, out_dtype: torch.dtype | None = None, epilogue: AddNormEpilogue | None = None,

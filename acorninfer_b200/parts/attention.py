@@ -225,7 +225,7 @@ class Attention(Mixer):
     def _rows_fuse(self, num_rows):
         widths = ((self.nq + 2 * self.nkv) * self.d, self.hidden_size)         # of the q/k/v product and of the o product
         return (ops.fused_rows_ok(num_rows, self.ctx.dtype, widths, ops.device_sms(self.ctx.device))
-                or ops.fused_tile_ok(num_rows, self.ctx.dtype))
+                or ops.fused_tile_ok(num_rows, self.ctx.dtype, self.hidden_size))
 
     def _inner_norm_rows(self, x, inputs, cache, out_scale, out, proj):
         g, pos = inputs.groups[cache.group], self.position

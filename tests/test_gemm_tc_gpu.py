@@ -159,7 +159,8 @@ def test_gemm_tc_tile_of_48_rows(M, splits):
     test_gemm_tc_swiglu_epilogue(M, 192, 1024, splits)
     test_gemm_tc_qkv_rope_epilogue(4, 2, 256 * splits, [M - 12, 1, 11], True, True)
     o = ops()
-    assert o.fused_tile_ok(M, torch.bfloat16) and not any(o.fused_tile_ok(m, torch.bfloat16) for m in (32, 49)) and not o.fused_tile_ok(M, torch.float32)
+    assert o.fused_tile_ok(M, torch.bfloat16, 1024) and not any(o.fused_tile_ok(m, torch.bfloat16, 1024) for m in (32, 49))
+    assert not o.fused_tile_ok(M, torch.float32, 1024) and not o.fused_tile_ok(M, torch.bfloat16, 1023)
 
 
 # ---------------------------------------------------------------------------- the paired kernel
