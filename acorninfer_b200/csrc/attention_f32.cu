@@ -13,8 +13,14 @@
 // queries of its tile, on the step's other rows or on padding.
 //
 // What bounded the plain kernel: a block a token read every key row again from L2 and made one chain of adds per thread.
-// Measured (B200, launched alone): 777 tokens, 16 heads of 128: 1,402 -> 152 us; 6 rows of 1,500 keys, 8 kv heads:
+// Measured (B200, launched alone): 777 tokens, 16 heads of 128: 1,402 -> 141 us; 6 rows of 1,500 keys, 8 kv heads:
 // 109 -> 14 us (74 MB, which L2 holds).
+//
+// What bounds the prefill kernel: shared memory, whose reads into registers (8 of 16 bytes a lane for 32 packed multiply-adds of the
+// scores, 3 for 16 of the sum) take 1.75 times the multiply-adds' time; 8,000 tokens run at half the multiply-adds' rate.  Eight
+// queries a thread, which need a quarter fewer reads on half the warps, were no faster: 141 -> 148 us at 777 tokens, 31 -> 38 at 130.
+// Short steps end with their longest blocks, so those of all heads come first (heads along the grid's first axis): 151 -> 141 us at 777
+// tokens, 198 -> 161 at 1,000, 564 -> 529 at 2,000, 31 at 130 and 7,150 at 8,000 either way.
 #include "mma_helpers.cuh"
 
 #include <cfloat>
@@ -73,9 +79,9 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
     constexpr int DC = D / 64;                      // runs of 64 dimensions; a thread holds four of each
     pdl_wait();
     pdl_trigger();
-    const int tile = n_tiles - 1 - blockIdx.x;      // later tiles of a row read more keys: they start first
+    const int tile = n_tiles - 1 - blockIdx.y;      // later tiles of a row read more keys: of all heads they start first
     const int r = tiles[2 * tile], q0 = tiles[2 * tile + 1];
-    const int h = blockIdx.y, kvh = h / (nq / nkv);
+    const int h = blockIdx.x, kvh = h / (nq / nkv);
     const int t0 = row_start[r] + q0, n = min(FP_Q, row_start[r + 1] - t0), p0 = row_pos[r] + q0;
     const int* table = block_table + (int64_t)r * table_stride - page_base[r];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -422,9 +428,14 @@ static int launch_prefill(const float* q, int64_t q_stride, float* out, const fl
         if (e != cudaSuccess) return (int)e;
         configured.mark();
     }
-    const int code = acorn_launch(attention_f32_prefill_kernel<D>, dim3(n_tiles, nq, chunks), dim3(FP_THREADS), fp_smem<D>(), stream, q,
-                                  q_stride, out, k_pages, v_pages, block_table, page_base, table_stride, row_start, row_pos, tiles, n_tiles,
-                                  nq, nkv, P, scale, window, chunks, part_o, part_ml);
+    int code = 0;                                   // 65,535 tiles a launch: what the grid's second axis takes
+    for (int at = 0; at < n_tiles && code == 0; at += 65535) {
+        const int n = min(n_tiles - at, 65535);
+        const int64_t slots = (int64_t)at * FP_Q * nq * chunks;
+        code = acorn_launch(attention_f32_prefill_kernel<D>, dim3(nq, n, chunks), dim3(FP_THREADS), fp_smem<D>(), stream, q, q_stride, out,
+                            k_pages, v_pages, block_table, page_base, table_stride, row_start, row_pos, tiles + 2 * at, n, nq, nkv, P,
+                            scale, window, chunks, chunks > 1 ? part_o + slots * D : part_o, chunks > 1 ? part_ml + slots * 2 : part_ml);
+    }
     if (code != 0 || chunks == 1) return code;
     return acorn_launch(attention_f32_prefill_merge_kernel<D>, dim3(n_tiles * FP_Q, nq), dim3(D), 0, stream, part_o, part_ml, out, row_start,
                         row_pos, tiles, nq, window, chunks);
