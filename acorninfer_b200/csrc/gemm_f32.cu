@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
 #define RS_THREADS (32 * K_RANGES)
 
 // R rows and CPL columns a lane, 2 R rows and 16 CPL columns a block.
-template <int R, int CPL> constexpr int rs_stages() { return R == 8 && CPL == 2 ? 3 : 4; }     // what shared memory holds
+template <int R, int CPL> constexpr int rs_stages() { return R >= 7 && CPL == 2 ? 3 : 4; }     // what shared memory holds
 template <int R, int CPL> constexpr int rs_ring() { return K_RANGES * rs_stages<R, CPL>() * (16 * CPL + 2 * R) * RS_LD; }
 // the ranges' sums: with one column a lane in the place of the rings, with two behind them, for two tiles
 template <int R, int CPL> constexpr int rs_smem() {
@@ -101,9 +101,10 @@ template <int R, int CPL> constexpr int rs_smem() {
 // A block then walks the tiles of its share one behind the other, and the next tile's weights are under way while the ranges'
 // sums of the one before are added: a block that ends with its tile spends a third of its time on filling and emptying its
 // rings (6 rows, N = 12,288, K = 2,048: 31 -> 25 us).
-// Measured (B200): the 113 products of a decode step of 6 rows at Qwen3-1.7B sizes (6.9 GB), with one block for 32 columns and
-// 16 rows whose four warps walked K together 5.64 ms, this 1.9 ms.  At 6 rows the reads of A and W from shared memory that feed
-// the multiply-adds set the pace (4.0 TB/s at N = 12,288, 4.9 at N = 151,936; at one row 4.9 and 6.2).
+// The reads of A and W from shared memory that feed the multiply-adds set the pace (R + CPL reads of 16 bytes a lane for 4 R CPL
+// multiply-adds), so there is a form for each number of rows a lane, and none reads rows that are not there.  Measured (B200, us, forms
+// for 4, 8 and 16 rows only / this), 6 rows: N = 4,096, K = 2,048 11.5 / 8.5; N = 2,048, K = 6,144 19.6 / 14.2; N = 12,288, K = 2,048
+// 26.4 / 24.9 (4.0 TB/s); N = 151,936, K = 1,024 134 / 122 (5.1 TB/s); one row of the last 107 / 98 (6.4 TB/s).
 template <int R, int CPL>
 __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* __restrict__ A, int64_t lda,
                                                                    const float* __restrict__ W, int64_t ldw,
@@ -124,8 +125,9 @@ __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* 
             const int n0 = ((int)blockIdx.x + ltile * (int)gridDim.x) * BN;
             float* dst = ring + fill * STAGE;
 #pragma unroll
-            for (int e = 0; e < ROWS / 4; ++e) {                 // rows of W, then of A; 8 lanes take 128 bytes of a row
+            for (int e = 0; e < (ROWS + 3) / 4; ++e) {           // rows of W, then of A; 8 lanes take 128 bytes of a row
                 const int row = e * 4 + (lane >> 3), seg = (lane & 7) * 4, k = kbeg + lkb * RS_BK + seg;
+                if (ROWS % 4 != 0 && row >= ROWS) break;         // in the last turn
                 const bool of_w = e < BN / 4;
                 const bool valid = k < kend && (of_w ? n0 + row < N : row - BN < M);
                 const float* src = of_w ? W + (int64_t)(n0 + row) * ldw + k : A + (int64_t)(row - BN) * lda + k;
@@ -376,18 +378,25 @@ __global__ void __launch_bounds__(TL_THREADS, 3) gemm_f32_tile_kernel(const floa
 
 static_assert(PL_BM == TL_BM, "the plain and the tile kernel cover the same rows a grid");
 
+// Shared memory that leaves no room for a second block on the SM.  A launch of no more blocks than SMs asks for it: its blocks come
+// while those of the kernel before it end, and two would go to the SMs that are free first, while others stay without (a decode step
+// of 6 rows at Qwen3-1.7B sizes: 3,042 -> 2,938 us).
+#define RS_ALONE (116 * 1024)
+
 template <int R, int CPL>
 static int launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
                        cudaStream_t stream) {
     static AcornPerDevice configured;
     if (!configured.seen()) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<R, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, rs_smem<R, CPL>());
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<R, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             rs_smem<R, CPL>() < RS_ALONE ? RS_ALONE : rs_smem<R, CPL>());
         if (e != cudaSuccess) return (int)e;
         configured.mark();
     }
     const int tiles = (N + 16 * CPL - 1) / (16 * CPL), sms = acorn_sms();
-    return acorn_launch(gemm_f32_rows_kernel<R, CPL>, dim3(CPL == 2 && sms < tiles ? sms : tiles), dim3(RS_THREADS), rs_smem<R, CPL>(), stream,
-                        A, lda, W, ldw, C, ldc, M, N, K);
+    const int smem = tiles <= sms && rs_smem<R, CPL>() < RS_ALONE ? RS_ALONE : rs_smem<R, CPL>();
+    return acorn_launch(gemm_f32_rows_kernel<R, CPL>, dim3(CPL == 2 && sms < tiles ? sms : tiles), dim3(RS_THREADS), smem, stream, A,
+                         lda, W, ldw, C, ldc, M, N, K);
 }
 
 template <bool SPLIT>
@@ -443,18 +452,27 @@ extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64
     // the faster kernels move 16 bytes at a time along K
     const bool aligned = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
     if (aligned && M <= 16) {
-        const bool wide = N >= 8192;             // blocks of 32 columns still cover the device
-        if (M <= 4)
-            return wide ? launch_rows<2, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<2, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-        if (M <= 8)
-            return wide ? launch_rows<4, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<4, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-        return wide ? launch_rows<8, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) : launch_rows<8, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+        // Blocks of 32 columns read a row of A half as often for each weight: taken where they still cover the device, or give every
+        // SM one where blocks of 16 give some SMs two (2,369 to 4,736 columns of 148 SMs).  N = 4,096, K = 2,048, blocks of 16 / 32:
+        // one row 8.0 / 7.2 us, 6 rows 9.9 / 8.5, 16 rows 18.0 / 13.4; N = 6,144 would give 44 SMs two of 32.
+        const int sms = acorn_sms();
+        const bool wide = N >= 8192 || (N > 16 * sms && N <= 32 * sms);
+        // As few rows a lane as hold them, since the reads of A set the pace.  (Two rows: one row a lane was slower, N = 6,144,
+        // K = 1,024 8.5 us instead of 7.9, since both halves of a warp then read as much of W as of A.)
+        switch (M == 2 ? 2 : (M + 1) / 2) {
+#define ROWS(R) case R: return wide ? launch_rows<R, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream) \
+                                    : launch_rows<R, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream)
+            ROWS(1); ROWS(2); ROWS(3); ROWS(4); ROWS(5); ROWS(6); ROWS(7); ROWS(8);
+#undef ROWS
+        }
     }
     if (aligned && M <= 32 && (N <= 4096 || N >= 8192)) {
-        // The weights twice through the rows kernel: 32 rows, N = 2,048, K = 6,144: 56 us, in tiles 88 us; N = 4,096, K = 1,024: 23 and
-        // 24 us; N = 12,288, K = 2,048: 79 and 93 us; between (N = 6,144, K = 1,024: 33 and 25 us) the tiles fill the device.
-        const int rc = acorn_gemm_f32(A, lda, W, ldw, C, ldc, 16, N, K, stream);
-        return rc ? rc : acorn_gemm_f32(A + 16 * lda, lda, W, ldw, C + 16 * ldc, ldc, M - 16, N, K, stream);
+        // The weights twice through the rows kernel, half of the rows each: 32 rows, N = 2,048, K = 6,144: 54 us, in tiles 88 us;
+        // N = 4,096, K = 1,024: 15 and 24 us; N = 12,288, K = 2,048: 77 and 93 us; between (N = 6,144, K = 1,024: 30 and 25 us) the
+        // tiles fill the device.
+        const int half = (M + 1) / 2;
+        const int rc = acorn_gemm_f32(A, lda, W, ldw, C, ldc, half, N, K, stream);
+        return rc ? rc : acorn_gemm_f32(A + half * lda, lda, W, ldw, C + half * ldc, ldc, M - half, N, K, stream);
     }
     if (aligned) {
         // A cluster to a tile where whole tiles would leave an SM fewer than two of them (777 rows, N = 1,024, K = 2,048, 104 tiles:

@@ -129,6 +129,18 @@ def test_gemm_f32_gives_the_same_bits_from_each_of_its_kernels():
     assert torch.allclose(tile.double(), a.double() @ w.double().T, atol=1e-5 * math.sqrt(K), rtol=1e-5)
 
 
+@pytest.mark.parametrize("N,K", [(40, 132), (2368, 516), (2400, 260), (4736, 64), (4800, 132), (8200, 1028)])
+def test_gemm_f32_rows_of_every_number(N, K):
+    """1 to 20 rows, in blocks of 16 and of 32 columns on either side of where one gives way to the other: the bits of the kernel
+    for operands that are not 16-byte aligned, and nothing beyond the rows."""
+    w = torch.randn(N, K, device=DEV)
+    for M in range(1, 21):
+        a, out = torch.randn(M, K, device=DEV), torch.full((M + 2, N), 7.0, device=DEV)
+        apart = torch.empty(M, K + 3, device=DEV)[:, 1:K + 1].copy_(a)
+        ops().gemm_f32(a, w, out=out[:M])
+        assert torch.equal(out[:M], ops().gemm_f32(apart, w)) and bool((out[M:] == 7.0).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8192, 2048), (3, 8193, 36), (8, 14208, 520), (6, 19001, 132), (16, 9500, 1028),
                                    (17, 4096, 132), (24, 300, 520), (32, 8193, 36), (31, 6000, 132)])
 def test_gemm_f32_of_few_rows_and_many_columns(M, N, K):
