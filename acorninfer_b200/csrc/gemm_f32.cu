@@ -9,8 +9,9 @@
 // takes 12.5 us in dependent multiply-adds alone, where the weights of N = 2,048 columns stream in 7.6 us.
 //
 // A, W: float32 row-major, K contiguous, with row strides lda, ldw; C row stride ldc.
-//   rows kernel   up to 16 rows (decode; at many widths up to 32, in two launches): a block takes 16 or 32 columns and all rows, a warp one range of K with a ring
-//                 of cp.async stages of its own (no block barrier): bound by reading W once;
+//   rows kernel   up to 16 rows (decode; at many widths up to 32, in two launches): a block takes up to 16 or 32 columns and all
+//                 rows, a warp one range of K with a ring of cp.async stages of its own (no block barrier): bound by reading W
+//                 once and by the reads of shared memory;
 //   tile kernel   more rows: 64 x 128 a block; a cluster of eight shares a tile's ranges where the tiles
 //                 alone leave the device idle: bound by the multiply-adds and the reads of shared memory that feed them;
 //   plain kernel  64 x 64 a block, scalar loads: operands that are not 16-byte aligned.
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
 #define RS_LD (RS_BK + 4)       // row stride in shared memory: 16-byte reads of 8 neighbouring rows hit 8 groups of banks
 #define RS_THREADS (32 * K_RANGES)
 
-// R rows and CPL columns a lane, 2 R rows and 16 CPL columns a block.
+// R rows and CPL columns a lane, 2 R rows and 16 CPL columns a block, of which a tile of the NARROW form uses `width`.
 template <int R, int CPL> constexpr int rs_stages() { return R >= 7 && CPL == 2 ? 3 : 4; }     // what shared memory holds
 template <int R, int CPL> constexpr int rs_ring() { return K_RANGES * rs_stages<R, CPL>() * (16 * CPL + 2 * R) * RS_LD; }
 // the ranges' sums: with one column a lane in the place of the rings, with two behind them, for two tiles
@@ -105,31 +106,32 @@ template <int R, int CPL> constexpr int rs_smem() {
 // multiply-adds), so there is a form for each number of rows a lane, and none reads rows that are not there.  Measured (B200, us, forms
 // for 4, 8 and 16 rows only / this), 6 rows: N = 4,096, K = 2,048 11.5 / 8.5; N = 2,048, K = 6,144 19.6 / 14.2; N = 12,288, K = 2,048
 // 26.4 / 24.9 (4.0 TB/s); N = 151,936, K = 1,024 134 / 122 (5.1 TB/s); one row of the last 107 / 98 (6.4 TB/s).
-template <int R, int CPL>
+template <int R, int CPL, bool NARROW>
 __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* __restrict__ A, int64_t lda,
                                                                    const float* __restrict__ W, int64_t ldw,
-                                                                   float* __restrict__ C, int64_t ldc, int M, int N, int K) {
+                                                                   float* __restrict__ C, int64_t ldc, int M, int N, int K, int width) {
     extern __shared__ __align__(16) float rs_buf[];
     constexpr int BN = 16 * CPL, ROWS = BN + 2 * R, STAGE = ROWS * RS_LD, STAGES = rs_stages<R, CPL>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int col = lane & 15, row0 = (lane >> 4) * R;
     const int range = k_range(K), kbeg = min(K, warp * range), kend = min(K, kbeg + range);
     const int nk = (kend - kbeg + RS_BK - 1) / RS_BK;
-    const int tiles = (N + BN - 1) / BN;
+    const int step = NARROW ? width : BN;        // columns from a tile to the next
+    const int tiles = (int)(((unsigned int)N + step - 1) / step);
     const int mine = CPL == 2 ? (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1;   // tiles of this block
     float* ring = rs_buf + warp * STAGES * STAGE;
 
     int ltile = 0, lkb = 0, fill = 0;            // the next stage to load: of which tile of this block, where in K, into which slot
     auto load = [&]() {
         if (ltile < mine && nk > 0) {
-            const int n0 = ((int)blockIdx.x + ltile * (int)gridDim.x) * BN;
+            const int n0 = ((int)blockIdx.x + ltile * (int)gridDim.x) * step, cols = NARROW ? min(width, N - n0) : N - n0;
             float* dst = ring + fill * STAGE;
 #pragma unroll
             for (int e = 0; e < (ROWS + 3) / 4; ++e) {           // rows of W, then of A; 8 lanes take 128 bytes of a row
                 const int row = e * 4 + (lane >> 3), seg = (lane & 7) * 4, k = kbeg + lkb * RS_BK + seg;
                 if (ROWS % 4 != 0 && row >= ROWS) break;         // in the last turn
                 const bool of_w = e < BN / 4;
-                const bool valid = k < kend && (of_w ? n0 + row < N : row - BN < M);
+                const bool valid = k < kend && (of_w ? (NARROW ? row < cols : n0 + row < N) : row - BN < M);
                 const float* src = of_w ? W + (int64_t)(n0 + row) * ldw + k : A + (int64_t)(row - BN) * lda + k;
                 cp_async_16(smem_addr(dst + row * RS_LD + seg), valid ? src : W, valid);
             }
@@ -142,15 +144,15 @@ __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* 
     // the first weights on their way to L2 while the kernel before this one ends (W may be its result: not read yet)
 #pragma unroll
     for (int e = 0; e < CPL * (STAGES - 1) / 2; ++e) {
-        const int n = (int)blockIdx.x * BN + (lane + 32 * e) % BN, k = kbeg + ((lane + 32 * e) / BN) * RS_BK;
-        if (k < kend && n < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (int64_t)n * ldw + k));
+        const int c = (lane + 32 * e) % BN, n = (int)blockIdx.x * step + c, k = kbeg + ((lane + 32 * e) / BN) * RS_BK;
+        if (k < kend && (!NARROW || c < width) && n < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (int64_t)n * ldw + k));
     }
     pdl_wait();
     pdl_trigger();
     for (int s = 0; s < STAGES - 1; ++s) load();
     int stage = 0;
     for (int it = 0; it < mine; ++it) {
-        const int n0 = ((int)blockIdx.x + it * (int)gridDim.x) * BN;
+        const int n0 = ((int)blockIdx.x + it * (int)gridDim.x) * step, cols = NARROW ? min(width, N - n0) : N - n0;
         float acc[R][CPL];
 #pragma unroll
         for (int i = 0; i < R; ++i)
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* 
         __syncthreads();                         // the one barrier of a tile: its sums were read before the next tile's barrier
         for (int o = threadIdx.x; o < 2 * R * BN; o += RS_THREADS) {
             const int r = o / BN, c = o % BN;
-            if (r >= M || n0 + c >= N) continue;
+            if (r >= M || (NARROW ? c >= cols : n0 + c >= N)) continue;
             float v = parts[o];
 #pragma unroll
             for (int q = 1; q < K_RANGES; ++q) v += parts[q * 2 * R * BN + o];
@@ -383,20 +385,36 @@ static_assert(PL_BM == TL_BM, "the plain and the tile kernel cover the same rows
 // of 6 rows at Qwen3-1.7B sizes: 3,042 -> 2,938 us).
 #define RS_ALONE (116 * 1024)
 
-template <int R, int CPL>
-static int launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
-                       cudaStream_t stream) {
+template <int R, int CPL, bool NARROW>
+static int launch_rows_of(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K, int width,
+                          cudaStream_t stream) {
     static AcornPerDevice configured;
     if (!configured.seen()) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<R, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<R, CPL, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              rs_smem<R, CPL>() < RS_ALONE ? RS_ALONE : rs_smem<R, CPL>());
         if (e != cudaSuccess) return (int)e;
         configured.mark();
     }
-    const int tiles = (N + 16 * CPL - 1) / (16 * CPL), sms = acorn_sms();
+    const int sms = acorn_sms(), tiles = (int)(((int64_t)N + width - 1) / width);
     const int smem = tiles <= sms && rs_smem<R, CPL>() < RS_ALONE ? RS_ALONE : rs_smem<R, CPL>();
-    return acorn_launch(gemm_f32_rows_kernel<R, CPL>, dim3(CPL == 2 && sms < tiles ? sms : tiles), dim3(RS_THREADS), smem, stream, A,
-                         lda, W, ldw, C, ldc, M, N, K);
+    return acorn_launch(gemm_f32_rows_kernel<R, CPL, NARROW>, dim3(CPL == 2 && sms < tiles ? sms : tiles), dim3(RS_THREADS), smem, stream, A,
+                        lda, W, ldw, C, ldc, M, N, K, width);
+}
+
+template <int R, int CPL>
+static int launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
+                       cudaStream_t stream) {
+    // Tiles of all columns that a block can take, or, where they would leave a fifth of the SMs' turns empty, of fewer: as many for
+    // every SM, alike in width.  One row / 6 / 12 rows, us, whole tiles (at the second of 16 columns) / these: N = 2,560, K = 9,728 28.5, 36.4,
+    // 49.5 / 25.4, 32.2, 42.7; N = 6,144, K = 1,024 8.1, 10.4, 12.8 / 6.5, 8.8, 10.4; N = 1,024, K = 3,072 6.2, 7.5, 11.7 / 5.3, 7.5, 10.9.
+    // At fuller turns the columns that a warp leaves unused cost what the SMs gain (N = 4,096, K = 2,048 7.3, 8.5, 11.5 / 7.2, 8.6,
+    // 12.1), and the form that knows its width at compile time is 2 to 7 % faster.
+    const int sms = acorn_sms();
+    const int64_t full = ((int64_t)N + 16 * CPL - 1) / (16 * CPL), turns = (full + sms - 1) / sms;
+    const int even = (int)((N + turns * sms - 1) / (turns * sms));
+    if (5 * full < 4 * turns * sms)
+        return launch_rows_of<R, CPL, true>(A, lda, W, ldw, C, ldc, M, N, K, even < 4 ? 4 : even, stream);
+    return launch_rows_of<R, CPL, false>(A, lda, W, ldw, C, ldc, M, N, K, 16 * CPL, stream);
 }
 
 template <bool SPLIT>
@@ -452,11 +470,10 @@ extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64
     // the faster kernels move 16 bytes at a time along K
     const bool aligned = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
     if (aligned && M <= 16) {
-        // Blocks of 32 columns read a row of A half as often for each weight: taken where they still cover the device, or give every
-        // SM one where blocks of 16 give some SMs two (2,369 to 4,736 columns of 148 SMs).  N = 4,096, K = 2,048, blocks of 16 / 32:
-        // one row 8.0 / 7.2 us, 6 rows 9.9 / 8.5, 16 rows 18.0 / 13.4; N = 6,144 would give 44 SMs two of 32.
-        const int sms = acorn_sms();
-        const bool wide = N >= 8192 || (N > 16 * sms && N <= 32 * sms);
+        // Blocks of 32 columns read a row of A half as often for each weight: taken where blocks of 16 would give some SMs two or more
+        // (more than 2,368 columns of 148 SMs).  N = 4,096, K = 2,048, blocks of 16 / 32: one row 8.0 / 7.2 us, 6 rows 9.9 / 8.5, 16
+        // rows 18.0 / 13.4.
+        const bool wide = N > 16 * acorn_sms();
         // As few rows a lane as hold them, since the reads of A set the pace.  (Two rows: one row a lane was slower, N = 6,144,
         // K = 1,024 8.5 us instead of 7.9, since both halves of a warp then read as much of W as of A.)
         switch (M == 2 ? 2 : (M + 1) / 2) {
@@ -468,7 +485,7 @@ extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64
     }
     if (aligned && M <= 32 && (N <= 4096 || N >= 8192)) {
         // The weights twice through the rows kernel, half of the rows each: 32 rows, N = 2,048, K = 6,144: 54 us, in tiles 88 us;
-        // N = 4,096, K = 1,024: 15 and 24 us; N = 12,288, K = 2,048: 77 and 93 us; between (N = 6,144, K = 1,024: 30 and 25 us) the
+        // N = 4,096, K = 1,024: 15 and 24 us; N = 12,288, K = 2,048: 77 and 93 us; between (N = 6,144, K = 1,024: 27 and 25 us) the
         // tiles fill the device.
         const int half = (M + 1) / 2;
         const int rc = acorn_gemm_f32(A, lda, W, ldw, C, ldc, half, N, K, stream);

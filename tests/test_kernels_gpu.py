@@ -129,7 +129,7 @@ def test_gemm_f32_gives_the_same_bits_from_each_of_its_kernels():
     assert torch.allclose(tile.double(), a.double() @ w.double().T, atol=1e-5 * math.sqrt(K), rtol=1e-5)
 
 
-@pytest.mark.parametrize("N,K", [(40, 132), (2368, 516), (2400, 260), (4736, 64), (4800, 132), (8200, 1028)])
+@pytest.mark.parametrize("N,K", [(3, 36), (40, 132), (1000, 260), (2368, 516), (2400, 260), (4736, 64), (6000, 132), (8200, 1028)])
 def test_gemm_f32_rows_of_every_number(N, K):
     """1 to 20 rows, in blocks of 16 and of 32 columns on either side of where one gives way to the other: the bits of the kernel
     for operands that are not 16-byte aligned, and nothing beyond the rows."""
