@@ -90,7 +90,10 @@ __device__ __forceinline__ float ld_global_now(const float* p) {
 
 // ------------------------------------------------------------------ the kernel
 
-template <int MB, int STAGES>
+// FUSED: the modes ADD_NORM, SWIGLU, GEGLU and QKV_ROPE; the others' code is a kernel of its own.  In one kernel a plain product carried
+// the registers and the code of all (a decode step of 16 rows with ten plain products a layer: 783 -> 766 us; one row of Qwen3-0.6B,
+// whose output matrix alone is plain: 691 -> 685).
+template <int MB, int STAGES, bool FUSED>
 __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                   const __grid_constant__ CUtensorMap map_x,
                                                                   const TcParams p) {
@@ -152,7 +155,9 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
     // The kernel after this one may start now that every CTA has its tensor memory: where a short ring leaves room on the SMs its
     // first weights stream under this kernel's work.  (It reads nothing of this one's before this one has ended.)  A layer's four
     // products at Qwen3-0.6B widths, chained: 18.8 -> 17.2 us at one row, 28.8 -> 26.6 at 41; wider ones fill the SMs either way.
-    pdl_trigger();
+    // Not after a plain product, which a kernel without weights to fetch follows: its blocks would take places on the SMs (780 us
+    // for the step named above, 776 without).
+    if (FUSED) pdl_trigger();
     bool ok = true;
 
     if (warp == 0) {
@@ -207,7 +212,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
     const int m_valid = min(MB, p.M - m0);
     const int col = threadIdx.x;                                      // 128 threads = 128 columns of the tile
     const bool n_ok = n0 + col < p.N;
-    if (p.mode == TC_MODE_QKV_ROPE && warp >= 2) {
+    if (FUSED && p.mode == TC_MODE_QKV_ROPE && warp >= 2) {
         // the step's own arrays (written by the host before the step): no need to wait for the kernel before this one
         for (int m = threadIdx.x - 64; m < m_valid; m += 64) {
             const int t = m0 + m, pos = p.positions[t];
@@ -221,6 +226,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
         }
     }
     pdl_wait();          // the output buffer may still be read by the kernel before this one
+    if (!FUSED) pdl_trigger();
     // Rows of x that arrive un-normalised (x = residual * norm weight): the factor rsqrt(mean(residual^2) + eps) of each row is
     // applied to the product.  Two warps add up the partial sums while the others load and multiply.
     if (p.ss_in != nullptr) {
@@ -263,7 +269,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
     constexpr int MAX_ROWS = MB <= 64 ? MB : 1;                       // the host refuses ADD_NORM for larger tiles
     float r_old[MAX_ROWS];
     float nw = 0.f;
-    if (p.mode == TC_MODE_ADD_NORM) {
+    if (FUSED && p.mode == TC_MODE_ADD_NORM) {
         if (n_ok) nw = ld_global_now(p.norm_w + n0 + col);
 #pragma unroll
         for (int i = 0; i < MAX_ROWS; ++i) {
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
         }
     }
     // TC_MODE_QKV_ROPE: the tile is one head, a warp finishes a row; lane l has columns l, l + 32, l + 64, l + 96
-    const bool rope = p.mode == TC_MODE_QKV_ROPE;
+    const bool rope = FUSED && p.mode == TC_MODE_QKV_ROPE;
     const bool is_q = rope && (int)blockIdx.x < p.nq, is_k = rope && !is_q && (int)blockIdx.x < p.nq + p.nkv;
     const float* hw = is_q ? p.q_w : p.k_w;
     float wcol[4] = {1.f, 1.f, 1.f, 1.f}, freq[2] = {0.f, 0.f};
@@ -325,7 +331,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
         for (int q = 1; q < 8; ++q) acc += v[q];
         return acc;
     };
-    if (p.mode == TC_MODE_PLAIN || p.mode == TC_MODE_RELU2 || p.mode == TC_MODE_TANH || p.mode == TC_MODE_GELU_ROWS) {
+    if (!FUSED) {
         for (int i = 0, m = rank; m < m_valid; ++i, m += csize) {
             float val = tile_sum(i, col) * inv_s[m];
             if (p.mode == TC_MODE_RELU2) { val = fmaxf(val, 0.f); val *= val; }
@@ -428,8 +434,8 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
 
 // ------------------------------------------------------------------ host side
 
-template <int MB, int STAGES>
-static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, TcParams& p, int splits, cudaStream_t stream) {
+template <int MB, int STAGES, bool FUSED>
+static int launch_tc_of(const CUtensorMap& mw, const CUtensorMap& mx, TcParams& p, int splits, cudaStream_t stream) {
     constexpr int STAGE_BYTES = TC_BM * TC_BK * 2 + MB * TC_BK * 2;
     const int steps = (p.kblocks + splits - 1) / splits;
     p.ring = steps < STAGES ? steps : STAGES;
@@ -442,7 +448,7 @@ static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, TcParams& p, 
     const size_t smem = ring + rest, most = (size_t)STAGES * STAGE_BYTES + rest;
     static AcornPerDevice configured;
     if (!configured.seen()) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<MB, STAGES>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<MB, STAGES, FUSED>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         if (e != cudaSuccess) return (int)e;
         configured.mark();
@@ -461,8 +467,14 @@ static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, TcParams& p, 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = acorn_pdl_enabled() ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<MB, STAGES>, mw, mx, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<MB, STAGES, FUSED>, mw, mx, p);
     return e != cudaSuccess ? (int)e : acorn_launch_status();
+}
+
+template <int MB, int STAGES>
+static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, TcParams& p, int splits, cudaStream_t stream) {
+    const bool plain = p.mode == TC_MODE_PLAIN || p.mode == TC_MODE_RELU2 || p.mode == TC_MODE_TANH || p.mode == TC_MODE_GELU_ROWS;
+    return plain ? launch_tc_of<MB, STAGES, false>(mw, mx, p, splits, stream) : launch_tc_of<MB, STAGES, true>(mw, mx, p, splits, stream);
 }
 
 // What the kernel takes: bf16 operands with K contiguous, K and both row strides multiples of 8
