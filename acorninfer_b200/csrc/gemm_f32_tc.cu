@@ -4,17 +4,20 @@
 // what is left out (a1 b2 + a2 b1 + a2 b2) is at most 2^-26 |a b|, a quarter of a rounding of float32.
 //
 // The tensor cores round their sums towards zero, so no sum stays there for long.  K is cut into eight ranges of ceil(K / 512) * 64
-// and a range into chunks of 64.  A chunk's three sums (the terms of each order of magnitude apart) are made in tensor memory;
-// from there float32 adds, rounded to nearest, take them: T += G0 + (G1 + G2) over a range's chunks, and T0 + T1 + ... + T7 from
-// the left.  That order does not depend on M, on the other rows or on who takes which range, so a row's bits do not either.
+// and a range into chunks of 64.  A chunk's six sums (one a product of parts) are made in tensor memory;
+// from there float32 adds, rounded to nearest, take them, the smaller ones first: T += G over a range's chunks, and
+// T0 + T1 + ... + T7 from the left.  That order does not depend on M, on the other rows or on who takes which range, so a row's
+// bits do not either.
 // Distance from 64 bits (relative 2-norm, K = 1,024 / 2,048 / 6,144): 9.3e-8, 9.9e-8, 1.1e-7; the multiply-adds of gemm_f32.cu 2.1e-7, 2.9e-7,
 // 5.0e-7.
 //
 // A CTA takes 128 rows of W (lanes of tensor memory) and 32 tokens.  Two groups of eight warps bring 64 floats of each row, split
 // them and lay the parts out for the matrix instruction (K-major rows of 128 bytes, 128-byte swizzle; K permuted alike in both operands,
 // so that a thread's 16 bytes of parts come from two coalesced loads); one warp multiplies: per 16 of K W0 x [b0 b1 b2],
-// W1 x [b0 b1] and W2 x [b0], which reads each part of W once; eight warps add up.  Stages and accumulators are handed
-// over by mbarriers; every wait is bounded.
+// W1 x [b0 b1] and W2 x [b0], which reads each part of W once; eight warps add up.  The three instructions differ in shape, and only
+// those of one shape on one accumulator are sure to run in the order they are issued in: each shape has columns of its own (777 rows,
+// N = 4,096, K = 1,024: 95 -> 98 us).  A CTA holds all of tensor memory; its 197 KB of shared memory leave no room on the SM for a kernel
+// that needs some, so that nobody waits for columns there.  Stages and accumulators are handed over by mbarriers; every wait is bounded.
 //
 // What bounds it: the loading warps, a load's latency and their arithmetic in turn (a chunk of 128 x 32 takes 1.0 us, of which shared
 // memory's bytes take 0.55).  One group instead of two: 1.75 us; wider tiles of 48 and 64 tokens need registers that 25 warps do not
@@ -39,7 +42,8 @@ namespace cg = cooperative_groups;
 #define F3_STAGE_BYTES (3 * (F3_BM + F3_NT) * 128)
 #define F3_TOTAL_BYTES (F3_NT * F3_BM * 4)
 #define F3_SMEM (F3_STAGES * F3_STAGE_BYTES + F3_TOTAL_BYTES + 1024 + 128)
-#define F3_TMEM_COLS 256     // two accumulators of three sums of 32 columns, a power of two
+#define F3_SUMS (6 * F3_NT)   // columns of a chunk's sums: W0 x [b0 b1 b2], W1 x [b0 b1] and W2 x [b0], each in columns of its own
+#define F3_TMEM_COLS 512     // two chunks' sums, a power of two
 
 __device__ int g_gemm_f32_tc_error = 0;
 
@@ -54,22 +58,19 @@ struct F3Params {
     int tiles_m, tiles_n;
 };
 
-// Eight columns of 32 bits of this thread's lane from three places, one wait.
-__device__ __forceinline__ void tmem_ld8x3(uint32_t at0, uint32_t at1, uint32_t at2, float (&v0)[8], float (&v1)[8], float (&v2)[8]) {
-    uint32_t r[3][8];
-    const uint32_t at[3] = {at0, at1, at2};
+// Eight columns of 32 bits of this thread's lane from six places F3_NT columns apart, one wait.
+__device__ __forceinline__ void tmem_ld8x6(uint32_t at, float (&v)[6][8]) {
+    uint32_t r[6][8];
 #pragma unroll
-    for (int q = 0; q < 3; ++q)
+    for (int q = 0; q < 6; ++q)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                      : "=r"(r[q][0]), "=r"(r[q][1]), "=r"(r[q][2]), "=r"(r[q][3]), "=r"(r[q][4]), "=r"(r[q][5]), "=r"(r[q][6]), "=r"(r[q][7])
-                     : "r"(at[q]));
+                     : "r"(at + q * F3_NT));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        v0[i] = __uint_as_float(r[0][i]);
-        v1[i] = __uint_as_float(r[1][i]);
-        v2[i] = __uint_as_float(r[2][i]);
-    }
+    for (int q = 0; q < 6; ++q)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[q][i] = __uint_as_float(r[q][i]);
 }
 
 // What float32 gives where a sum is no number: chains of fused multiply-adds over ranges of K, as in gemm_f32.cu.  An operand that is
@@ -252,13 +253,13 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const F3Para
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t d = tmem + b * 3 * NT;
+                const uint32_t d = tmem + b * F3_SUMS;
                 const uint32_t w = w0 + s * (STAGE >> 4), a = a0 + s * (STAGE >> 4);
 #pragma unroll
                 for (int k = 0; k < F3_BK / 16; ++k) {
                     umma_bf16_elect(d, w + 2 * k, a + 2 * k, I1, k > 0 ? 1u : 0u);
-                    umma_bf16_elect(d + NT, w + 2 * k + (PART_W >> 4), a + 2 * k, I2, 1u);
-                    umma_bf16_elect(d + 2 * NT, w + 2 * k + 2 * (PART_W >> 4), a + 2 * k, I3, 1u);
+                    umma_bf16_elect(d + 3 * NT, w + 2 * k + (PART_W >> 4), a + 2 * k, I2, k > 0 ? 1u : 0u);
+                    umma_bf16_elect(d + 5 * NT, w + 2 * k + 2 * (PART_W >> 4), a + 2 * k, I3, k > 0 ? 1u : 0u);
                 }
                 umma_commit_elect(empty0 + 8 * s);
                 umma_commit_elect(sfull0 + 8 * b);
@@ -298,15 +299,16 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const F3Para
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t at = tmem + lanes + b * 3 * NT + t0;
+                const uint32_t at = tmem + lanes + b * F3_SUMS + t0;
 #pragma unroll
                 for (int c = 0; c < MINE; c += 8) {
-                    float g0[8], g1[8], g2[8];
-                    tmem_ld8x3(at + c, at + c + NT, at + c + 2 * NT, g0, g1, g2);
+                    float g[6][8];                             // W0 b0, W0 b1, W0 b2; W1 b0, W1 b1; W2 b0
+                    tmem_ld8x6(at + c, g);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const float2 lower = f3_add2(make_float2(g1[2 * i], g1[2 * i + 1]), make_float2(g2[2 * i], g2[2 * i + 1]));
-                        sum[c / 2 + i] = f3_add2(sum[c / 2 + i], f3_add2(make_float2(g0[2 * i], g0[2 * i + 1]), lower));
+                        auto two = [&](int q) { return make_float2(g[q][2 * i], g[q][2 * i + 1]); };
+                        const float2 lower = f3_add2(f3_add2(two(1), two(3)), f3_add2(f3_add2(two(2), two(4)), two(5)));
+                        sum[c / 2 + i] = f3_add2(sum[c / 2 + i], f3_add2(two(0), lower));
                     }
                 }
                 tc_fence_before();
