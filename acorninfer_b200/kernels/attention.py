@@ -74,18 +74,15 @@ def merged_in_kernel(splits: int, limit: int) -> bool:
 
 
 @lru_cache(maxsize=4096)        # asked by every layer of a step, with the same sizes
-def decode_splits(rows: int, num_kv_heads: int, key_bound: int, head_dim: int, num_sms: int = B200_SMS,
-                  merge_free_upto: int = 1) -> int:
-    """Splits of the key range.  ``key_bound`` bounds the keys any row reads; it changes only with
-    the table stride, so a captured step keeps its grid.
+def decode_splits(rows: int, num_kv_heads: int, key_bound: int, head_dim: int, num_sms: int = B200_SMS) -> int:
+    """Splits of the key range for the decode kernels that end in a merge pass (``decode_plan`` has the TMA kernel's).
+    ``key_bound`` bounds the keys any row reads; it changes only with the table stride, so a captured step keeps its grid.
 
     Two CTAs of the decode kernel fit on an SM: ``2 * num_sms`` (296 on a B200) run at a time, in waves.  A CTA is bound by
     its own streaming rate, a full wave by the memory.  So few (row, kv head) pairs want many
     splits (more CTAs in flight); a count just above a multiple of 296 wants splits too (a last
-    wave of few long CTAs takes as long as one CTA takes alone: 40 rows of 8 kv heads, unsplit,
-    take 149 us against 123 us in three splits); a count that fills its last wave well wants
-    none.  The splits with the least estimated time are taken.  ``merge_free_upto``: up to this many
-    splits cost no merge pass (the TMA kernel merges up to sixteen inside itself)."""
+    wave of few long CTAs takes as long as one CTA takes alone); a count that fills its last wave well wants
+    none.  The splits with the least estimated time are taken."""
     _TARGET_CTAS = 2 * num_sms
     pairs = max(1, rows * num_kv_heads)
     most = max(1, min(-(-key_bound // _CHUNK), 32))
@@ -98,20 +95,27 @@ def decode_splits(rows: int, num_kv_heads: int, key_bound: int, head_dim: int, n
         us = full * (max(alone_us, _TARGET_CTAS * kb / _HBM_GBS) + _WAVE_US)
         if rest:
             us += max(alone_us, rest * kb / _HBM_GBS) + _WAVE_US
-        if not merged_in_kernel(s, merge_free_upto):
+        if s > 1:
             us += _MERGE_US
         if best_us is None or us <= best_us + 1e-9:                  # equal estimates: more CTAs in flight
             best, best_us = s, us
     return best
 
 
-# How the TMA decode kernel's launches share the work (measured: 1 to 64 rows of 8 kv heads at contexts of 300, 900 and 1,700, equal
-# and of 35 to 100 %, every number of splits).  Clusters run in one wave only as long as they fill no more than seven
+# How the TMA decode kernel's launches share the work (measured: 1 to 90 rows of 8 kv heads and 40 to 90 of 4 at contexts of 300 to
+# 16,384, equal and of 35 to 100 %, every number of splits).  Clusters run in one wave only as long as they fill no more than seven
 # eighths of the CTAs that single ones would (5 rows of 900 keys: 6 splits, 240 CTAs, 9.1 us; 7 splits, 280 CTAs, 15.4; 12 rows: 2
-# splits 13.9, 3 splits, 288 CTAs, 21.6), pairs of CTAs fill all of them, clusters of sixteen half; and a second wave of
-# clusters costs more than its splits bring (41 rows of 900: unsplit 43.7, 3 splits 50.7; a step of 41 rows of 600 to 1,700 keys at
-# Qwen3-4B: 3,866 and 4,280 us).
+# splits 13.9, 3 splits, 288 CTAs, 21.6), pairs of CTAs fill all of them, clusters of sixteen half.  At short contexts a second
+# wave of clusters costs more than its splits bring (41 rows of 900: unsplit 43.7, 3 splits 50.7; of 1,700: 69 and 67; a step of 41
+# rows of 600 to 1,700 keys at Qwen3-4B: 3,866 and 4,280 us).
 _START_US, _CLUSTER_US = 3.5, 1.5
+# From here on the keys of a row that is left whole take longer than another wave's start: ``_waves_us`` has the choice for more
+# rows than two splits of each fit one wave.  40 rows of 8 kv heads, equal / ragged, us, whole and in the splits it takes: 4,096 keys
+# 149 / 93 and 131 / 86 (2), 8,192 289 / 176 and 222 / 154 (3), 16,384 569 / 342 and 406 / 281 (4); 20 rows of 16,384 250 / 226 and
+# 204 / 158 (3); 48 of 8,192 294 / 208 and 247 / 180 (2); 80 of 16,384 902 / 586 and 800 / 548 (2); 64 rows, which fill two waves
+# well, stay whole (16,384 keys: 610 / 507, in 4 splits 650 / 441).  The table is a power of two of pages wide, so a bound of 4,096
+# stands for contexts from 2,049 on: those of 2,500 gain less (40 rows 95 / 60 and 89 / 60) and lose at 76 rows (147 / 96 and 150 / 103).
+_LONG_KEYS = 2048
 
 
 def _wave(splits: int, num_sms: int) -> int:
@@ -119,13 +123,27 @@ def _wave(splits: int, num_sms: int) -> int:
     return 2 * num_sms if splits <= 2 or splits > 16 else 2 * num_sms * 7 // 8 if splits <= 8 else num_sms
 
 
+def _waves_us(pairs: int, keys: float, splits: int, num_sms: int) -> float:
+    """Estimated time of the TMA decode kernel over several waves, fitted to the measurements above (2.3 % above the best choice on
+    average): a lone CTA streams 40 GB/s and two on an SM 33 each, all together 6.8 TB/s; a wave's start takes 2 us, of clusters of
+    three and more 6."""
+    kb, wave, start = keys * 128 * 4 / 1e3 / splits, _wave(splits, num_sms), 2.0 if splits <= 2 else 6.0
+    full, rest = divmod(pairs * splits, wave)
+    us = full * (max(kb / 33.0, wave * kb / 6800.0) + start)
+    return us + (max(kb / (40.0 if rest <= num_sms else 33.0), rest * kb / 6800.0) + start if rest else 0.0)
+
+
 @lru_cache(maxsize=4096)
 def decode_plan(rows: int, num_kv_heads: int, key_bound: int, num_sms: int = B200_SMS, merge_limit: int = 16) -> int:
     """Splits of the key range for the TMA decode kernel (head size 128, ``merge_limit`` splits merged inside it)."""
     pairs, wave = rows * num_kv_heads, 2 * num_sms
+    most = max(1, -(-key_bound // _CHUNK))
+    if key_bound > _LONG_KEYS and 2 * pairs > wave:
+        # contexts are anywhere between half of the bound and all of it: the sum of two estimates
+        return min(range(1, min(merge_limit, 8) + 1),
+                   key=lambda s: (_waves_us(pairs, key_bound, s, num_sms) + _waves_us(pairs, 0.75 * key_bound, s, num_sms), s))
     if pairs > wave:
         return 1
-    most = max(1, -(-key_bound // _CHUNK))
     pair_kb = key_bound * 128 * 4 / 1e3                             # K and V of one pair, bfloat16, in KB
     best, best_us = 1, None
     for s in (1, 2, 3, 4, 5, 6, 7, 8, 16, 24, 32):
@@ -151,11 +169,16 @@ def _merge_free(nq: int, nkv: int, d: int, P: int) -> int:
     return _MERGE_FREE[key]
 
 
+def choose_splits(rows: int, nq: int, nkv: int, d: int, P: int, key_bound: int, windowed_only: bool, num_sms: int) -> int:
+    """Splits for the decode kernel that takes these sizes."""
+    limit = _merge_free(nq, nkv, d, P) if windowed_only else 1
+    # (a limit above 1: the TMA kernel takes them)
+    return decode_plan(rows, nkv, key_bound, num_sms, limit) if limit > 1 else decode_splits(rows, nkv, key_bound, d, num_sms)
+
+
 def _decode(qkv, inputs, group, cache, nq, nkv, d, P, scale, window, bound, n, windowed_only, mask, token_list=None, out=None):
     """The step's ``n`` single-token rows (``token_list``, or all tokens) on a decode kernel."""
-    limit = _merge_free(nq, nkv, d, P) if windowed_only else 1
-    # (a limit above 1: the TMA kernel takes these sizes)
-    splits = decode_plan(n, nkv, bound, sm_count(qkv.device), limit) if limit > 1 else decode_splits(n, nkv, bound, d, sm_count(qkv.device))
+    splits = choose_splits(n, nq, nkv, d, P, bound, windowed_only, sm_count(qkv.device))
     return ops.attention_decode(qkv, qkv.stride(0), cache.k_pages, cache.v_pages, group.block_table, group.page_base, inputs.token_row,
                                 inputs.positions, inputs.num_tokens, nq, nkv, d, scale, window, splits, token_list=token_list, out=out,
                                 **mask)

@@ -30,7 +30,7 @@ def test_decode_splits_follow_the_measured_cases():
 
 
 def test_decode_plans_of_the_tma_kernel():
-    """One wave of clusters or none; the measured cases; what the kernels take."""
+    """One wave of clusters or none up to 2,048 keys, several waves of longer rows; the measured cases; what the kernels take."""
     from acorninfer_b200.kernels.attention import decode_plan
     want = {1: 16, 2: 8, 3: 8, 5: 6, 6: 5, 7: 4, 8: 4, 9: 3, 10: 3, 11: 2, 12: 2, 16: 2, 19: 1, 32: 1, 37: 1, 41: 1, 64: 1}
     assert {r: decode_plan(r, 8, 2048) for r in want} == want
@@ -41,7 +41,12 @@ def test_decode_plans_of_the_tma_kernel():
         limit = rng.choice([2, 8, 16])
         s = decode_plan(rows, nkv, bound, 148, limit)
         assert 1 <= s <= 32 and s <= max(1, -(-bound // 64))
-        assert s == 1 or rows * nkv * s <= 296
+        assert s == 1 or rows * nkv * s <= 296 or (bound > 2048 and rows * nkv > 148 and s <= min(limit, 8))
+    # rows beyond a wave, and rows whose second split does not fit one, at long contexts: the last wave of whole rows takes longer
+    assert decode_plan(64, 8, 4096) == 1 and decode_plan(37, 8, 16384) == 1 and decode_plan(40, 8, 2048) == 1
+    for rows in (38, 40, 44, 48, 76, 80):
+        assert all(decode_plan(rows, 8, bound) > 1 for bound in (4096, 8192, 16384)), rows
+    assert decode_plan(20, 8, 4096) == 3 and decode_plan(40, 8, 16384, merge_limit=2) == 2
 
 
 def test_gemm_plans_are_valid_for_any_shape():
