@@ -123,5 +123,15 @@ def ensure_built(verbose: bool = True) -> Path:
     return out / LIB_NAME
 
 
+def own_folder(lib: Path) -> Path:
+    """Where files that go with the library are kept: beside it, but for a library that ``ACORN_KERNEL_LIB`` names, whose folder is
+    not this package's to write to."""
+    if not os.environ.get("ACORN_KERNEL_LIB"):
+        return lib.parent
+    out = build_dir()
+    _writable_dir(out)
+    return out
+
+
 if __name__ == "__main__":
     print(ensure_built())

@@ -3,7 +3,8 @@
 A call of 25 to 40 arguments costs ctypes 3 to 4 us, as much as the launch behind it: a step of a few hundred tokens that is not
 replayed from a graph makes 100 to 300 of them and is bound by the host.  ``load`` makes a small extension module from the
 functions' signatures (one typed call each, compiled with the Python headers) and returns its functions by name; an
-argument costs 5 to 10 ns there.  Without those headers or a C++ compiler it returns nothing and ctypes does the calls.
+argument costs 5 to 10 ns there.  Without those headers or a C++ compiler, or where the compiler or the import fails (which a warning
+says), it returns nothing and ctypes does the calls.
 Steps of 27 decoded rows and 3 prompts at Qwen3-0.6B sizes: 4.83 -> 4.29 ms; three prompts of a design with 185 launches 3.15 -> 2.91 ms.
 """
 
@@ -17,6 +18,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from pathlib import Path
 
 _TYPES = {ctypes.c_void_p: "void*", ctypes.c_int: "int", ctypes.c_int64: "long long", ctypes.c_float: "float"}
@@ -81,7 +83,8 @@ def source(signatures: dict[str, tuple[list, object]]) -> str:
 
 
 def build(signatures: dict[str, tuple[list, object]], folder: Path) -> Path | None:
-    """Compiles the extension into ``folder`` if it is not there yet; None where that is not possible."""
+    """Compiles the extension into ``folder`` if it is not there yet; None without a compiler, headers or a folder that can be
+    written; a compiler that fails raises."""
     text, suffix = source(signatures), sysconfig.get_config_var("EXT_SUFFIX")
     include, gxx = sysconfig.get_paths()["include"], shutil.which("g++")
     digest = hashlib.sha256((text + sys.version).encode()).hexdigest()[:16]
@@ -110,12 +113,17 @@ def build(signatures: dict[str, tuple[list, object]], folder: Path) -> Path | No
 
 
 def load(signatures: dict[str, tuple[list, object]], library: Path, folder: Path) -> dict[str, object]:
-    """The library's functions by name as the extension calls them (``library`` is loaded); empty where it cannot be built."""
-    path = build(signatures, folder)
-    if path is None:
+    """The library's functions by name as the extension calls them (``library`` is loaded); empty where it cannot be built or
+    imported."""
+    try:
+        path = build(signatures, folder)
+        if path is None:
+            return {}
+        spec = importlib.util.spec_from_file_location("acorn_calls", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except (RuntimeError, ImportError, OSError) as e:
+        warnings.warn(f"kernels are called through ctypes, which is slower: no call extension ({e})", RuntimeWarning, stacklevel=2)
         return {}
-    spec = importlib.util.spec_from_file_location("acorn_calls", path)
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
     module.bind(str(library))
     return {name: getattr(module, name) for name in signatures}

@@ -18,7 +18,7 @@ from types import SimpleNamespace
 import torch
 
 from . import calls
-from .build import ensure_built
+from .build import ensure_built, own_folder
 
 
 class KernelError(RuntimeError):
@@ -51,7 +51,7 @@ def _load():
             fn.restype = _RESULTS.get(name, c_int)
             functions[name] = fn
         _init_error_word(library)
-        functions.update(calls.load(_typed_signatures(), path, path.parent))
+        functions.update(calls.load(_typed_signatures(), path, own_folder(path)))
         _lib = SimpleNamespace(**functions)
     return _lib
 
@@ -73,7 +73,7 @@ def _typed_signatures() -> dict[str, tuple[list, object]]:
 
 def build_calls() -> None:
     """Compiles the call extension beside the kernel library (``_load`` does so on first use)."""
-    calls.build(_typed_signatures(), ensure_built().parent)
+    calls.build(_typed_signatures(), own_folder(ensure_built()))
 
 
 _error_word: ctypes.c_int | None = None       # pinned host memory that kernels write when a bounded wait gives up

@@ -35,3 +35,42 @@ def test_calls_convert_and_refuse_arguments(tmp_path):
     assert calls.load(signatures, lib, tmp_path)["none"]() == -7          # built once
     with pytest.raises(RuntimeError):
         calls.load({"other": ([], ctypes.c_int)}, lib, tmp_path)
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="no C++ compiler")
+def test_a_compiler_or_an_import_that_fails_leaves_the_calls_to_ctypes(tmp_path, monkeypatch):
+    src, lib = tmp_path / "small.cpp", tmp_path / "libsmall.so"
+    src.write_text(SOURCE)
+    subprocess.run(["g++", "-shared", "-fPIC", str(src), "-o", str(lib)], check=True)
+    signatures = {"none": ([], ctypes.c_int)}
+    loaded = ctypes.CDLL(str(lib))
+    path = calls.build(signatures, tmp_path)
+    if path is None:
+        pytest.skip("no Python headers")
+    path.write_bytes(b"not an extension")
+    with pytest.warns(RuntimeWarning, match="ctypes"):
+        assert calls.load(signatures, lib, tmp_path) == {}
+    path.unlink()
+    tools = tmp_path / "tools"
+    tools.mkdir()
+    (tools / "g++").write_text("#!/bin/sh\necho unknown standard c++17 >&2\nexit 1\n")
+    (tools / "g++").chmod(0o755)
+    monkeypatch.setenv("PATH", str(tools), prepend=":")
+    with pytest.warns(RuntimeWarning, match="unknown standard"):
+        assert calls.load(signatures, lib, tmp_path) == {}
+    with pytest.raises(RuntimeError):               # the build step itself says so
+        calls.build(signatures, tmp_path)
+    assert loaded.none() == -7 and not list(tmp_path.glob("acorn_calls*"))
+
+
+def test_a_given_library_keeps_its_folder(tmp_path, monkeypatch):
+    from acorninfer_b200.kernels import build
+    given, own = tmp_path / "given", tmp_path / "own"
+    given.mkdir()
+    lib = given / "lib.so"
+    lib.write_bytes(b"")
+    monkeypatch.delenv("ACORN_KERNEL_LIB", raising=False)
+    monkeypatch.setenv("ACORN_BUILD_DIR", str(own))
+    assert build.own_folder(lib) == given
+    monkeypatch.setenv("ACORN_KERNEL_LIB", str(lib))
+    assert build.own_folder(build.ensure_built()) == own and own.is_dir() and list(given.iterdir()) == [lib]
