@@ -1,7 +1,9 @@
 // C[M, N] = A[M, K] * W[N, K]^T in float32 on the 5th-generation tensor cores, for many rows, many columns and long
-// sums (gemm_f32.cu says from where on): every operand is the exact sum of three bfloat16 numbers, a = a0 + a1 + a2 (8 bits of mantissa
-// each; rounding to nearest, so |a1| <= 2^-9 |a|, |a2| <= 2^-18 |a|), and a product is a0 b0 + (a0 b1 + a1 b0) + (a0 b2 + a1 b1 + a2 b0);
-// what is left out (a1 b2 + a2 b1 + a2 b2) is at most 2^-26 |a b|, a quarter of a rounding of float32.
+// sums (gemm_f32.cu says from where on): every operand, times 2^16, is the exact sum of three bfloat16 numbers, a = a0 + a1 + a2 (8 bits
+// of mantissa each; rounding to nearest, so |a1| <= 2^-9 |a|, |a2| <= 2^-18 |a|), and a product is
+// a0 b0 + (a0 b1 + a1 b0) + (a0 b2 + a1 b1 + a2 b0); what is left out (a1 b2 + a2 b1 + a2 b2) is at most 2^-26 |a b|, a quarter of a
+// rounding of float32.  The scale takes float32's least number, 2^-149, to bfloat16's, 2^-133, so that no bit falls below: without it the
+// parts of an operand of 2^-117 lost 4e-6 of it, of 2^-126 2e-3.  Operands from 2^112 and sums from 2^96 on overflow and go to f3_chain.
 //
 // The tensor cores round their sums towards zero, so no sum stays there for long.  K is cut into eight ranges of ceil(K / 512) * 64
 // and a range into chunks of 64.  A chunk's six sums (one a product of parts) are made in tensor memory;
@@ -33,6 +35,7 @@ namespace cg = cooperative_groups;
 #define F3_NT 32             // tokens a tile
 #define F3_BK 64             // floats of K a chunk
 #define F3_RANGES 8
+#define F3_SCALE 65536.f     // operands are split at this scale
 #define F3_GROUP 8           // warps that load and split a chunk
 #define F3_GROUPS 2          // such groups: they take turns
 #define F3_LOADERS (F3_GROUP * F3_GROUPS)
@@ -73,8 +76,9 @@ __device__ __forceinline__ void tmem_ld8x6(uint32_t at, float (&v)[6][8]) {
         for (int i = 0; i < 8; ++i) v[q][i] = __uint_as_float(r[q][i]);
 }
 
-// What float32 gives where a sum is no number: chains of fused multiply-adds over ranges of K, as in gemm_f32.cu.  An operand that is
-// infinite, NaN or beyond bfloat16's largest number makes every product of its row NaN above; such sums are made again here.
+// What float32 gives where a scaled sum is no number: chains of fused multiply-adds over ranges of K, as in gemm_f32.cu.  An operand that
+// is infinite, NaN or, scaled, beyond bfloat16's largest number (2^112) makes every product of its row NaN above, and a sum from 2^96 on is
+// infinite; such sums are made again here.
 static __device__ __noinline__ float f3_chain(const float* a, const float* w, int K) {
     const int range = (K + 127) / 128 * 16;
     float total = 0.f;
@@ -87,8 +91,8 @@ static __device__ __noinline__ float f3_chain(const float* a, const float* w, in
 }
 
 __device__ __forceinline__ void f3_store(const F3Params& p, int m, int n, float v) {
-    if (!(fabsf(v) <= 3.0e38f)) v = f3_chain(p.a + (int64_t)m * p.lda, p.w + (int64_t)n * p.ldw, p.K);
-    p.c[(int64_t)m * p.ldc + n] = v;
+    const bool fine = fabsf(v) <= 3.0e38f;
+    p.c[(int64_t)m * p.ldc + n] = fine ? v * (1.f / (F3_SCALE * F3_SCALE)) : f3_chain(p.a + (int64_t)m * p.lda, p.w + (int64_t)n * p.ldw, p.K);
 }
 
 __device__ __forceinline__ uint32_t f3_pack(float lo, float hi) {        // two bfloat16, rounded to nearest
@@ -96,29 +100,39 @@ __device__ __forceinline__ uint32_t f3_pack(float lo, float hi) {        // two 
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// Pairs of floats in the packed instructions of sm_100: a - b and a + b, rounded as the single ones.
-__device__ __forceinline__ float2 f3_sub2(float2 a, float2 b) {
-    unsigned long long r, x = *reinterpret_cast<unsigned long long*>(&a), y = *reinterpret_cast<unsigned long long*>(&b);
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(y), "l"(0xbf800000bf800000ull), "l"(x));
-    return *reinterpret_cast<float2*>(&r);
-}
+// Pairs of floats in the packed instructions of sm_100: a + b and F3_SCALE a, rounded as the single ones.
 __device__ __forceinline__ float2 f3_add2(float2 a, float2 b) {
     unsigned long long r, x = *reinterpret_cast<unsigned long long*>(&a), y = *reinterpret_cast<unsigned long long*>(&b);
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
     return *reinterpret_cast<float2*>(&r);
 }
-__device__ __forceinline__ float2 f3_unpack(uint32_t p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)); }
+__device__ __forceinline__ float2 f3_scale2(float2 a) {
+    const float2 b = make_float2(F3_SCALE, F3_SCALE);
+    unsigned long long r, x = *reinterpret_cast<unsigned long long*>(&a), y = *reinterpret_cast<const unsigned long long*>(&b);
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return *reinterpret_cast<float2*>(&r);
+}
 
-// The three parts of eight floats, 16 bytes each.
+// What two floats leave beyond the bfloat16 numbers in p (exact): fused multiply-adds of mixed precision, p times -1 (0xbf80) on the floats.
+// Unpacking p for a subtraction in float32 takes twice the instructions (777 rows, N = 12,288, K = 2,048: 512 us, unpacked 604).
+__device__ __forceinline__ float2 f3_rest(float2 v, uint32_t p) {
+    float2 r;
+    asm("{\n .reg .b16 lo, hi, minus;\n mov.b32 {lo, hi}, %4;\n mov.b16 minus, 0xbf80;\n"
+        " fma.rn.f32.bf16 %0, lo, minus, %2;\n fma.rn.f32.bf16 %1, hi, minus, %3;\n}\n"
+        : "=f"(r.x), "=f"(r.y) : "f"(v.x), "f"(v.y), "r"(p));
+    return r;
+}
+
+// The three parts of eight floats times F3_SCALE, 16 bytes each.
 __device__ __forceinline__ void f3_split(const float (&x)[8], uint4 (&part)[3]) {
     uint32_t p[3][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        float2 v = make_float2(x[2 * i], x[2 * i + 1]);
+        float2 v = f3_scale2(make_float2(x[2 * i], x[2 * i + 1]));
         p[0][i] = f3_pack(v.x, v.y);
-        v = f3_sub2(v, f3_unpack(p[0][i]));
+        v = f3_rest(v, p[0][i]);
         p[1][i] = f3_pack(v.x, v.y);
-        v = f3_sub2(v, f3_unpack(p[1][i]));
+        v = f3_rest(v, p[1][i]);
         p[2][i] = f3_pack(v.x, v.y);             // exact
     }
 #pragma unroll

@@ -198,6 +198,22 @@ def test_float32_product_on_tcgen05_with_numbers_that_do_not_split():
         assert torch.equal(o.gemm_f32_tc(x, torch.eye(128, device=DEV)), x)
 
 
+@pytest.mark.parametrize("e", [-100, -110, -117, -126, -135, -149])
+def test_float32_product_on_tcgen05_keeps_small_operands(e):
+    """Down to float32's least number an operand's three parts are the operand: products with 1 are exact on either side, and
+    sums keep float32's error where the other operand makes them large again."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(-e)
+    x = (torch.randn(64, 128, device=DEV, generator=g).double() * 2.0 ** e).float()
+    one = torch.eye(128, device=DEV)
+    assert torch.equal(o.gemm_f32_tc(x, one), x) and torch.equal(o.gemm_f32_tc(one, x), x.T)
+    w = torch.randn(256, 128, device=DEV, generator=g) * 2.0 ** 100
+    steps = 4 * 2 + 2 + 8                                      # as above
+    bound = (x.abs().double() @ w.abs().double().T) * steps * 2.0 ** -24
+    assert ((o.gemm_f32_tc(x, w).double() - x.double() @ w.double().T).abs() <= bound).all()
+    assert ((o.gemm_f32_tc(w, x).double() - w.double() @ x.double().T).abs() <= bound.T).all()
+
+
 def test_gemm_f32_shows_what_a_reduced_precision_mode_would_hide():
     # 1 + 2^-12 is lost by a product that rounds its inputs to 10 mantissa bits (TF32) or to bfloat16
     a = torch.full((4, 8), 1 + 2 ** -12, device=DEV)
