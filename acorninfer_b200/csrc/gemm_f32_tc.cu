@@ -6,25 +6,27 @@
 // parts of an operand of 2^-117 lost 4e-6 of it, of 2^-126 2e-3.  Operands from 2^112 and sums from 2^96 on overflow and go to f3_chain.
 //
 // The tensor cores round their sums towards zero, so no sum stays there for long.  K is cut into eight ranges of ceil(K / 512) * 64
-// and a range into chunks of 64.  A chunk's six sums (one a product of parts) are made in tensor memory;
-// from there float32 adds, rounded to nearest, take them, the smaller ones first: T += G over a range's chunks, and
-// T0 + T1 + ... + T7 from the left.  That order does not depend on M, on the other rows or on who takes which range, so a row's
-// bits do not either.
-// Distance from 64 bits (relative 2-norm, K = 1,024 / 2,048 / 6,144): 9.3e-8, 9.9e-8, 1.1e-7; the multiply-adds of gemm_f32.cu 2.1e-7, 2.9e-7,
-// 5.0e-7.
+// and a range into chunks of 64.  A chunk's sums are made in tensor memory: a0 b0 for every 16 of K apart, a single instruction each
+// (added up there, the cut-off bits of sums of one sign had one sign, too: -6.6e-8 of the sum on average, now -1.3e-8), the lower
+// products by their order of magnitude.  From there float32 adds, rounded to nearest, take them, the smaller ones apart: T += G over a
+// range's chunks, and T0 + T1 + ... + T7 from the left.  That order does not depend on M, on the other rows or on who takes which
+// range, so a row's bits do not either.
+// Distance from 64 bits (relative 2-norm, K = 512 / 1,024 / 2,048 / 6,144), normally distributed operands: 7.5e-8, 8.0e-8, 8.6e-8,
+// 1.0e-7 (the multiply-adds of gemm_f32.cu 1.6e-7, 2.1e-7, 2.9e-7, 5.0e-7); uniform in [0, 1): 5.0e-8, 5.2e-8, 5.0e-8, 5.2e-8 (6.1e-8,
+// 7.3e-8, 9.0e-8, 1.5e-7).
 //
 // A CTA takes 128 rows of W (lanes of tensor memory) and 32 tokens.  Two groups of eight warps bring 64 floats of each row, split
 // them and lay the parts out for the matrix instruction (K-major rows of 128 bytes, 128-byte swizzle; K permuted alike in both operands,
-// so that a thread's 16 bytes of parts come from two coalesced loads); one warp multiplies: per 16 of K W0 x [b0 b1 b2],
-// W1 x [b0 b1] and W2 x [b0], which reads each part of W once; eight warps add up.  The three instructions differ in shape, and only
-// those of one shape on one accumulator are sure to run in the order they are issued in: each shape has columns of its own (777 rows,
-// N = 4,096, K = 1,024: 95 -> 98 us).  A CTA holds all of tensor memory; its 197 KB of shared memory leave no room on the SM for a kernel
+// so that a thread's 16 bytes of parts come from two coalesced loads); one warp multiplies: per 16 of K W0 x [b0], W0 x [b1 b2],
+// W1 x [b0 b1] and W2 x [b0]; eight warps add up.  Only instructions of one shape on one accumulator are sure to run in the order they
+// are issued in: columns that several add into belong to one shape (777 rows, N = 4,096, K = 1,024: 95 us with columns that shapes
+// shared, 101 now).  A CTA holds all of tensor memory; its 197 KB of shared memory leave no room on the SM for a kernel
 // that needs some, so that nobody waits for columns there.  Stages and accumulators are handed over by mbarriers; every wait is bounded.
 //
 // What bounds it: the loading warps, a load's latency and their arithmetic in turn (a chunk of 128 x 32 takes 1.0 us, of which shared
 // memory's bytes take 0.55).  One group instead of two: 1.75 us; wider tiles of 48 and 64 tokens need registers that 25 warps do not
-// have (spills: 1.7 and 2.0 us).  The products of a prompt of 832 rows (us, multiply-adds / this): N = 4,096, K = 1,024 164 / 94;
-// N = 6,144 264 / 139; N = 1,024, K = 3,072 142 / 86; N = 12,288, K = 2,048 902 / 485 (86 TFLOP/s).
+// have (spills: 1.7 and 2.0 us).  The products of a prompt of 777 rows (us, multiply-adds / this): N = 4,096, K = 1,024 164 / 101;
+// N = 6,144 263 / 148; N = 1,024, K = 3,072 141 / 91; N = 12,288, K = 2,048 901 / 512 (76 TFLOP/s).
 #include <cooperative_groups.h>
 
 #include "tcgen05_helpers.cuh"
@@ -45,7 +47,7 @@ namespace cg = cooperative_groups;
 #define F3_STAGE_BYTES (3 * (F3_BM + F3_NT) * 128)
 #define F3_TOTAL_BYTES (F3_NT * F3_BM * 4)
 #define F3_SMEM (F3_STAGES * F3_STAGE_BYTES + F3_TOTAL_BYTES + 1024 + 128)
-#define F3_SUMS (6 * F3_NT)   // columns of a chunk's sums: W0 x [b0 b1 b2], W1 x [b0 b1] and W2 x [b0], each in columns of its own
+#define F3_SUMS (7 * F3_NT)   // columns of a chunk's sums: W0 x b0 for every 16 of K, W0 x [b1 b2] + W1 x [b0 b1], W2 x b0
 #define F3_TMEM_COLS 512     // two chunks' sums, a power of two
 
 __device__ int g_gemm_f32_tc_error = 0;
@@ -61,17 +63,17 @@ struct F3Params {
     int tiles_m, tiles_n;
 };
 
-// Eight columns of 32 bits of this thread's lane from six places F3_NT columns apart, one wait.
-__device__ __forceinline__ void tmem_ld8x6(uint32_t at, float (&v)[6][8]) {
-    uint32_t r[6][8];
+// Eight columns of 32 bits of this thread's lane from seven places F3_NT columns apart, one wait.
+__device__ __forceinline__ void tmem_ld8x7(uint32_t at, float (&v)[7][8]) {
+    uint32_t r[7][8];
 #pragma unroll
-    for (int q = 0; q < 6; ++q)
+    for (int q = 0; q < 7; ++q)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                      : "=r"(r[q][0]), "=r"(r[q][1]), "=r"(r[q][2]), "=r"(r[q][3]), "=r"(r[q][4]), "=r"(r[q][5]), "=r"(r[q][6]), "=r"(r[q][7])
                      : "r"(at + q * F3_NT));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int q = 0; q < 6; ++q)
+    for (int q = 0; q < 7; ++q)
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[q][i] = __uint_as_float(r[q][i]);
 }
@@ -254,8 +256,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const F3Para
     } else if (warp == F3_LOADERS) {
         // ---- multiply (the warp stays converged, an elected lane issues)
         const uint32_t w0 = umma_lo(tc_smem(smem)), a0 = umma_lo(tc_smem(smem) + 3 * PART_W);
-        constexpr uint32_t I1 = IDESC | ((uint32_t)(3 * NT >> 3) << 17), I2 = IDESC | ((uint32_t)(2 * NT >> 3) << 17),
-                           I3 = IDESC | ((uint32_t)(NT >> 3) << 17);
+        constexpr uint32_t I1 = IDESC | ((uint32_t)(NT >> 3) << 17), I2 = IDESC | ((uint32_t)(2 * NT >> 3) << 17);
         int it = 0;
         bool ok = true;
         for (int tile = first; ok && tile < tiles; tile += step) {
@@ -271,9 +272,10 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const F3Para
                 const uint32_t w = w0 + s * (STAGE >> 4), a = a0 + s * (STAGE >> 4);
 #pragma unroll
                 for (int k = 0; k < F3_BK / 16; ++k) {
-                    umma_bf16_elect(d, w + 2 * k, a + 2 * k, I1, k > 0 ? 1u : 0u);
-                    umma_bf16_elect(d + 3 * NT, w + 2 * k + (PART_W >> 4), a + 2 * k, I2, k > 0 ? 1u : 0u);
-                    umma_bf16_elect(d + 5 * NT, w + 2 * k + 2 * (PART_W >> 4), a + 2 * k, I3, k > 0 ? 1u : 0u);
+                    umma_bf16_elect(d + k * NT, w + 2 * k, a + 2 * k, I1, 0u);
+                    umma_bf16_elect(d + 4 * NT, w + 2 * k, a + 2 * k + (PART_A >> 4), I2, k > 0 ? 1u : 0u);
+                    umma_bf16_elect(d + 4 * NT, w + 2 * k + (PART_W >> 4), a + 2 * k, I2, 1u);
+                    umma_bf16_elect(d + 6 * NT, w + 2 * k + 2 * (PART_W >> 4), a + 2 * k, I1, k > 0 ? 1u : 0u);
                 }
                 umma_commit_elect(empty0 + 8 * s);
                 umma_commit_elect(sfull0 + 8 * b);
@@ -316,13 +318,14 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const F3Para
                 const uint32_t at = tmem + lanes + b * F3_SUMS + t0;
 #pragma unroll
                 for (int c = 0; c < MINE; c += 8) {
-                    float g[6][8];                             // W0 b0, W0 b1, W0 b2; W1 b0, W1 b1; W2 b0
-                    tmem_ld8x6(at + c, g);
+                    float g[7][8];                             // W0 b0 four times; W0 b1 + W1 b0, W0 b2 + W1 b1; W2 b0
+                    tmem_ld8x7(at + c, g);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         auto two = [&](int q) { return make_float2(g[q][2 * i], g[q][2 * i + 1]); };
-                        const float2 lower = f3_add2(f3_add2(two(1), two(3)), f3_add2(f3_add2(two(2), two(4)), two(5)));
-                        sum[c / 2 + i] = f3_add2(sum[c / 2 + i], f3_add2(two(0), lower));
+                        const float2 lower = f3_add2(two(4), f3_add2(two(5), two(6)));
+                        const float2 first = f3_add2(f3_add2(two(0), two(1)), f3_add2(two(2), two(3)));
+                        sum[c / 2 + i] = f3_add2(sum[c / 2 + i], f3_add2(first, lower));
                     }
                 }
                 tc_fence_before();

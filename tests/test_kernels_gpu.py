@@ -214,6 +214,22 @@ def test_float32_product_on_tcgen05_keeps_small_operands(e):
     assert ((o.gemm_f32_tc(w, x).double() - w.double() @ x.double().T).abs() <= bound.T).all()
 
 
+@pytest.mark.parametrize("K", [512, 1024, 6144])
+@pytest.mark.parametrize("left", ["uniform", "relu"])
+def test_float32_product_on_tcgen05_of_operands_of_one_sign(left, K):
+    """Sums whose cut-off bits all have one sign are no further from 64 bits than the multiply-adds'."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(K)
+    a = torch.rand(192, K, device=DEV, generator=g) if left == "uniform" else torch.randn(192, K, device=DEV, generator=g).relu()
+    w = torch.rand(1024, K, device=DEV, generator=g)
+    want = a.double() @ w.double().T
+    chains = torch.cat([o.gemm_f32(a[i:i + 16].contiguous(), w) for i in range(0, 192, 16)])
+    error = o.gemm_f32_tc(a, w).double() - want
+    assert error.norm() <= (chains.double() - want).norm()
+    # cut off once for every 16 of K: on average well below half of a float32 rounding (it was 2^-23.9 of the sum)
+    assert (error / want).mean().abs() <= 2.0 ** -25.5
+
+
 def test_gemm_f32_shows_what_a_reduced_precision_mode_would_hide():
     # 1 + 2^-12 is lost by a product that rounds its inputs to 10 mantissa bits (TF32) or to bfloat16
     a = torch.full((4, 8), 1 + 2 ** -12, device=DEV)
