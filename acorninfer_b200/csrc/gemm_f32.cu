@@ -1,6 +1,6 @@
 // C[M, N] = A[M, K] * W[N, K]^T in true float32: FMA on the CUDA cores, no tensor-core
-// mode of reduced precision.  It is the matrix product of the float32 path, but for many rows of wide matrices, which
-// gemm_f32_tc.cu takes (exact splits of the operands on the tensor cores; see the dispatch at the end).
+// mode of reduced precision.  It is the matrix product of the float32 path, but for the tokens of longer rows, whose wide products
+// gemm_f32_tc.cu takes (exact splits of the operands on the tensor cores; the caller chooses, acorninfer_b200/kernels/ops.py).
 //
 // Every kernel of this file sums an output element in one order: K is cut into eight ranges of ceil(K / 128) * 16, a range is a
 // chain acc = fma(a[k], w[k], acc) from 0 in the order of k, and the result is T0 + T1 + ... + T7 from the left.  So a
@@ -449,19 +449,9 @@ static int launch_tile(const float* A, int64_t lda, const float* W, int64_t ldw,
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-extern "C" int acorn_gemm_f32_tc_takes(int64_t M, int64_t N, int64_t lda, int64_t ldw);
-extern "C" int acorn_gemm_f32_tc(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
-                                 int split, cudaStream_t stream);
-
 extern "C" int acorn_gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, float* C,
                               int64_t ldc, int M, int N, int K, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    // Many rows of long sums on the tensor cores.  The line at 64 rows keeps steps of decoded tokens with the multiply-adds, whose
-    // bits do not depend on the kernel; narrower matrices and shorter sums leave that kernel's SMs idle or end before its
-    // chunks overlap.  Measured (B200, us, multiply-adds / tensor cores): 128 rows, N = 4,096, K = 1,024 40 / 19; N = 1,024, K = 3,072
-    // 49 / 28; 832 rows 164 / 94 and 142 / 86; 2,048 rows of N = 12,288, K = 2,048 2,072 / 1,200.
-    if (M > 64 && N >= 1024 && K >= 512 && acorn_gemm_f32_tc_takes(M, N, lda, ldw))
-        return acorn_gemm_f32_tc(A, lda, W, ldw, C, ldc, M, N, K, -1, stream);
     constexpr int most = 65535 * TL_BM;          // rows a launch's grid covers (the plain kernel's tiles have as many)
     if (M > most) {
         const int rc = acorn_gemm_f32(A, lda, W, ldw, C, ldc, most, N, K, stream);

@@ -1,5 +1,5 @@
-// C[M, N] = A[M, K] * W[N, K]^T in float32 on the 5th-generation tensor cores, for many rows, many columns and long
-// sums (gemm_f32.cu says from where on): every operand, times 2^16, is the exact sum of three bfloat16 numbers, a = a0 + a1 + a2 (8 bits
+// C[M, N] = A[M, K] * W[N, K]^T in float32 on the 5th-generation tensor cores, for prompts, many columns and long
+// sums (acorninfer_b200/kernels/ops.py, gemm_f32_step): every operand, times 2^16, is the exact sum of three bfloat16 numbers, a = a0 + a1 + a2 (8 bits
 // of mantissa each; rounding to nearest, so |a1| <= 2^-9 |a|, |a2| <= 2^-18 |a|), and a product is
 // a0 b0 + (a0 b1 + a1 b0) + (a0 b2 + a1 b1 + a2 b0); what is left out (a1 b2 + a2 b1 + a2 b2) is at most 2^-26 |a b|, a quarter of a
 // rounding of float32.  The scale takes float32's least number, 2^-149, to bfloat16's, 2^-133, so that no bit falls below: without it the
@@ -401,13 +401,13 @@ static int f3_launch(const F3Params& p, int grid, cudaStream_t stream) {
 }
 
 // Offsets of both operands' elements fit 32 bits.
-extern "C" int acorn_gemm_f32_tc_takes(int64_t M, int64_t N, int64_t lda, int64_t ldw) { return M * lda <= 0x7fffffff && N * ldw <= 0x7fffffff; }
+static bool f3_takes(int64_t M, int64_t N, int64_t lda, int64_t ldw) { return M * lda <= 0x7fffffff && N * ldw <= 0x7fffffff; }
 
 // split 1: a cluster of eight CTAs to a tile, 0: whole tiles, -1: chosen here.  Any alignment.
 extern "C" int acorn_gemm_f32_tc(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K,
                                  int split, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || !acorn_gemm_f32_tc_takes(M, N, lda, ldw)) return ACORN_ERR_UNSUPPORTED;
+    if (K <= 0 || !f3_takes(M, N, lda, ldw)) return ACORN_ERR_UNSUPPORTED;
     F3Params p = {};
     p.a = A; p.w = W; p.c = C; p.lda = lda; p.ldw = ldw; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
     p.range = (K + F3_BK * F3_RANGES - 1) / (F3_BK * F3_RANGES) * F3_BK;

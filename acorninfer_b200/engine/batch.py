@@ -23,6 +23,7 @@ upload and reach the part as ``StepInputs.extra[name]`` (device) and ``StepPlan.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
+from functools import cached_property
 
 import numpy as np
 
@@ -75,6 +76,21 @@ class StepPlan:
     @property
     def num_logits(self) -> int:
         return int(self.logit_tokens.size)
+
+    @cached_property
+    def longer_rows(self) -> tuple[tuple[int, int], list[tuple[int, int]]] | None:
+        """The span of tokens from the first row of several tokens to the end of the last one, and the runs of tokens that are
+        alone in their rows (those inside the span among them); None where every row is a single token."""
+        singles, first, last, at = [], None, 0, 0
+        for n in self.row_lens:
+            if n > 1:
+                first, last = at if first is None else first, at + n
+            elif singles and singles[-1][1] == at:
+                singles[-1] = (singles[-1][0], at + 1)
+            else:
+                singles.append((at, at + 1))
+            at += n
+        return None if first is None else ((first, last), singles)
 
 
 def _table_stride(pages: int) -> int:

@@ -992,9 +992,8 @@ def attention_tc_error() -> int:
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """a [M, K] @ w [N, K]^T in true float32: multiply-adds on the CUDA cores; from 65 rows on, for at least 1,024 columns and K of
-    512, operands as sums of three bfloat16 numbers on the tensor cores (``csrc/gemm_f32_tc.cu``), which is nearer to the exact
-    product.  Within either kind a row's bits do not depend on the other rows."""
+    """a [M, K] @ w [N, K]^T in true float32: multiply-adds on the CUDA cores.  A row's bits depend on K alone, not on the other
+    rows or on their number."""
     _check(w, "w", torch.float32, 2)
     if a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1:
         raise KernelError("a must be float32 [M, K] with contiguous K")
@@ -1010,14 +1009,17 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
     return out
 
 
-def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, split: bool | None = None) -> torch.Tensor:
-    """``gemm_f32`` on the tcgen05 kernel whatever the sizes; ``split``: a cluster of eight CTAs to a tile (None: as ``gemm_f32``
-    has it), which does not change a bit of the result."""
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, split: bool | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+    """a [M, K] @ w [N, K]^T in true float32 on the tensor cores: operands as sums of three bfloat16 numbers
+    (``csrc/gemm_f32_tc.cu``), nearer to the exact product than ``gemm_f32``.  A row's bits depend on K alone, but are not those of
+    ``gemm_f32``.  ``split``: a cluster of eight CTAs to a tile (None: chosen by the sizes), which does not change a bit."""
     _check(w, "w", torch.float32, 2)
     if a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1 or a.shape[1] != w.shape[1]:
         raise KernelError("a must be float32 [M, K] with contiguous K, w [N, K]")
     M, K = a.shape
-    out = torch.empty((M, w.shape[0]), dtype=torch.float32, device=a.device)
+    if out is None:
+        out = torch.empty((M, w.shape[0]), dtype=torch.float32, device=a.device)
+    _check(out, "out", torch.float32, 2)
     _ok(lib().acorn_gemm_f32_tc(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, w.shape[0], K,
                                 -1 if split is None else int(split), _stream()), "gemm_f32_tc", f"{M}x{w.shape[0]}x{K}")
     return out
@@ -1026,6 +1028,29 @@ def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, split: bool | None = None) -> 
 def gemm_f32_tc_error() -> int:
     """0, or where a bounded wait inside the float32 product on tcgen05 gave up since the last call (clears it)."""
     return int(lib().acorn_gemm_f32_tc_error())
+
+
+def gemm_f32_step(x: torch.Tensor, w: torch.Tensor, plan) -> torch.Tensor:
+    """The float32 product of a step's tokens (rows of ``x``; ``plan``: the step's ``StepPlan``): tokens that are alone in their row,
+    decoded ones above all, by ``gemm_f32``, those of longer rows by ``gemm_f32_tc`` where the matrix is wide and deep enough.  So a
+    token's bits depend on its own row, as attention's do, and not on what else is in the step or on how many rows there are.
+
+    Measured (B200, us, multiply-adds / tensor cores): N = 4,096, K = 1,024 at 32 rows 21 / 20, 128 40 / 20, 777 164 / 101; N = 1,024,
+    K = 3,072 28 / 10, 48 / 30, 141 / 91; N = 12,288, K = 2,048 75 / 40, 175 / 100, 901 / 512; operands that are not 16-byte aligned:
+    N = 4,096, K = 1,023 at 128 rows 122 / 26, at 777 333 / 117.  Decoded tokens lose by the tensor cores (8 rows 8 / 21, 11 / 10, 26 / 39);
+    narrower matrices and shorter sums leave that kernel's SMs idle or end before its chunks overlap."""
+    M, (N, K) = x.shape[0], w.shape
+    longer = None if plan is None or plan.num_tokens != M or N < 1024 or K < 512 else plan.longer_rows
+    if longer is None or N * w.stride(0) > 0x7fffffff:            # the tcgen05 kernel's offsets have 32 bits
+        return gemm_f32(x, w)
+    (first, last), singles = longer
+    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    most = 0x7fffffff // max(1, x.stride(0), N // 32)              # ... and its number of tiles
+    for at in range(first, last, most):
+        gemm_f32_tc(x[at:min(at + most, last)], w, out=out[at:min(at + most, last)])
+    for a, b in singles:                   # among the longer rows, too: the later launch overwrites
+        gemm_f32(x[a:b], w, out=out[a:b])
+    return out
 
 
 def gemm_tc_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -1374,10 +1399,11 @@ def fused_tile_ok(num_rows: int, dtype: torch.dtype, hidden: int) -> bool:
 
 def linear(x, w: torch.Tensor, out_dtype: torch.dtype | None = None, epilogue: AddNormEpilogue | None = None,
            swiglu: bool = False, residual32: torch.Tensor | None = None, activation: str = "silu",
-           act: str | None = None):
+           act: str | None = None, inputs=None):
     """x [T, K] times w [N, K] transposed.
 
-    float32 operands: the CUDA-core kernel (no reduced-precision matrix mode).
+    float32 operands: multiply-adds on the CUDA cores, or exact three-way splits on the tensor cores (no reduced-precision
+    matrix mode): the latter for the tokens of longer rows where ``inputs`` says which step's tokens ``x``'s rows are (``gemm_f32_step``).
     bfloat16 operands: up to GEMM_TC_MAX_ROWS rows the one-CTA tcgen05/TMA kernel of this library,
     above that the library matrix product (cuBLAS); float32 accumulation either way, and
     ``out_dtype=float32`` keeps the accumulator's precision (used for logits).
@@ -1398,7 +1424,7 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype | None = None, epilogue: A
         if (act in TC_EPILOGUE_ACTS and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
                 and x.shape[0] <= GEMM_TC_MAX_ROWS and gemm_tc_supported(x, w) and (out_dtype or x.dtype) == torch.bfloat16):
             return gemm_tc(x, w, torch.bfloat16, act=act)
-        return activation_rows(linear(x, w, out_dtype), act)
+        return activation_rows(linear(x, w, out_dtype, inputs=inputs), act)
     fused = isinstance(x, NormedRows) or epilogue is not None or swiglu
     xt = x.x if isinstance(x, NormedRows) else x
     out_dtype = out_dtype or xt.dtype
@@ -1410,7 +1436,7 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype | None = None, epilogue: A
             return gemm_tc_pair(x, w, out_dtype, epilogue=epilogue, swiglu=swiglu, activation=activation)
         return gemm_tc(x, w, out_dtype, epilogue=epilogue, swiglu=swiglu, activation=activation)
     if w.dtype == torch.float32:
-        y = gemm_f32(cast(x, torch.float32) if x.dtype != torch.float32 else x, w)
+        y = gemm_f32_step(cast(x, torch.float32) if x.dtype != torch.float32 else x, w, inputs.plan if inputs is not None else None)
         return y if out_dtype == torch.float32 else cast(y, out_dtype)
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise KernelError(f"linear: unsupported dtypes x={x.dtype}, w={w.dtype}")
@@ -2099,10 +2125,11 @@ def activation(x: torch.Tensor, kind: str) -> torch.Tensor:
     return out
 
 
-def side_gate_linear(x: torch.Tensor, w: torch.Tensor, token_ids: torch.Tensor, table: torch.Tensor, col0: int) -> torch.Tensor:
+def side_gate_linear(x: torch.Tensor, w: torch.Tensor, token_ids: torch.Tensor, table: torch.Tensor, col0: int,
+                     inputs=None) -> torch.Tensor:
     """``gelu_tanh(x w^T)[t] * table[token_ids[t], col0 : col0 + n]`` for x [T, K], w [n, K]: the gate as the epilogue
     of the one-CTA tcgen05 product where that runs (bfloat16, at most GEMM_TC_MAX_ROWS rows: the product is not
-    rounded before the gate), else the product followed by ``side_gate``."""
+    rounded before the gate), else the product followed by ``side_gate``.  ``inputs``: as for ``linear``."""
     _check(table, "table", x.dtype, 2)
     _check(token_ids, "token_ids", torch.int32, 1)
     T, n = x.shape[0], w.shape[0]
@@ -2110,7 +2137,7 @@ def side_gate_linear(x: torch.Tensor, w: torch.Tensor, token_ids: torch.Tensor, 
         raise KernelError(f"side_gate_linear: x {tuple(x.shape)} / w {tuple(w.shape)} / table {tuple(table.shape)} / "
                           f"first column {col0} do not fit")
     if not (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and T <= GEMM_TC_MAX_ROWS and gemm_tc_supported(x, w)):
-        return side_gate(linear(x, w, out_dtype=x.dtype), token_ids, table, col0)
+        return side_gate(linear(x, w, out_dtype=x.dtype, inputs=inputs), token_ids, table, col0)
     K = x.shape[1]
     splits, per_sm = gemm_tc_plan(T, n, K, device_sms(x.device))
     out = torch.empty((T, n), dtype=torch.bfloat16, device=x.device)

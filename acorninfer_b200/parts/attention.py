@@ -232,7 +232,7 @@ class Attention(Mixer):
         if not cache.write:
             raise ValueError("attention: a q/k norm over whole rows needs a cache of the run's own")
         if proj is None:
-            proj = ops.linear(x, self.w_qkv, out_dtype=self.ctx.dtype)
+            proj = ops.linear(x, self.w_qkv, out_dtype=self.ctx.dtype, inputs=inputs)
         q = torch.empty((proj.shape[0], self.nq * self.d), dtype=self.ctx.dtype, device=proj.device)
         conv = None
         if self.taps:
@@ -278,7 +278,7 @@ class Attention(Mixer):
         elif self.bias or self.taps:
             if not cache.write:
                 raise ValueError("attention: biased or convolved projections need a cache of the run's own")
-            proj = ops.linear(x, self.w_qkv, out_dtype=self.ctx.dtype)
+            proj = ops.linear(x, self.w_qkv, out_dtype=self.ctx.dtype, inputs=inputs)
             qkv = torch.empty((rows, self.nq * self.d), dtype=self.ctx.dtype, device=proj.device)      # the queries
             conv = None
             if self.taps:
@@ -296,7 +296,7 @@ class Attention(Mixer):
                 ops.conv_state_update(proj, cache.state, self.state_base, inputs.row_start, inputs.row_slot, inputs.num_rows,
                                       self.channels, self.taps, bias32=self.bias32, skip_single=True)
         else:
-            qkv = ops.linear(x, self.w_qkv, out_dtype=self.ctx.dtype)
+            qkv = ops.linear(x, self.w_qkv, out_dtype=self.ctx.dtype, inputs=inputs)
             ops.qk_rope_kv(qkv, self.q_norm32, self.k_norm32,
                            pos.inv_freq if pos is not None else _no_freq(self.ctx.device),
                            inputs.positions, inputs.token_row, g.block_table, g.page_base,
@@ -316,7 +316,7 @@ class Attention(Mixer):
 
     def forward(self, x, inputs, cache, epilogue=None, residual32=None):
         return ops.linear(self.inner(x, inputs, cache), self.w_o, out_dtype=self.ctx.dtype, epilogue=epilogue,
-                          residual32=residual32 if epilogue is None else None)
+                          residual32=residual32 if epilogue is None else None, inputs=inputs)
 
 
 _NO_FREQ: dict = {}

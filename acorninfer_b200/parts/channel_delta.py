@@ -79,8 +79,8 @@ class ChannelDelta(Mixer):
 
     def forward(self, x, inputs, cache):
         dt = self.ctx.dtype
-        main = ops.linear(x, self.w_main, out_dtype=dt)
-        up = ops.linear(ops.linear(x, self.w_low, out_dtype=dt), self.w_up, out_dtype=torch.float32)
+        main = ops.linear(x, self.w_main, out_dtype=dt, inputs=inputs)
+        up = ops.linear(ops.linear(x, self.w_low, out_dtype=dt, inputs=inputs), self.w_up, out_dtype=torch.float32, inputs=inputs)
         # long rows over chunks of tokens, whose kernels want the decays' logarithms; the others token by token
         lens, min_row = inputs.plan.row_lens, 0
         if ops.channel_chunk_ok(inputs.plan.max_q_len, main.shape[0], inputs.num_rows, self.H, self.dim, self.vdim):
@@ -96,4 +96,4 @@ class ChannelDelta(Mixer):
         if not min_row or min(lens) < min_row:
             o = ops.delta_rule(q, k, v, beta, g, *rows, max_row=min_row - 1 if min_row else 0, out=o)
         y = ops.delta_out(o, gate, self.norm32, self.eps, dt)
-        return ops.linear(y, self.w_o, out_dtype=dt)
+        return ops.linear(y, self.w_o, out_dtype=dt, inputs=inputs)

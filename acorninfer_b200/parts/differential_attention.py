@@ -118,7 +118,7 @@ class DifferentialAttention(Mixer):
             raise ValueError("differential attention keeps a cache of its own")
         g = inputs.groups[cache.group]
         D = 2 * self.d
-        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)
+        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, inputs=inputs)
         nq = 2 * self.H if self.spread else self.H          # query heads of a key row's width in a projected row
         q = torch.empty((proj.shape[0], nq * D), dtype=self.ctx.dtype, device=proj.device)
         ops.qk_rope_kv(proj, None, None, _no_freq(self.ctx.device), inputs.positions, inputs.token_row, g.block_table,
@@ -130,7 +130,7 @@ class DifferentialAttention(Mixer):
         gate_col = self.q_cols + self.G * (D + self.dv)
         o = ops.diff_combine(pairs, proj[:, gate_col:], self.H, self.dv, self.lam, 1.0 - self.diff, self.eps)
         return ops.linear(o, self.w_o, out_dtype=self.ctx.dtype, epilogue=epilogue,
-                          residual32=residual32 if epilogue is None else None)
+                          residual32=residual32 if epilogue is None else None, inputs=inputs)
 
 
 _NO_FREQ: dict = {}

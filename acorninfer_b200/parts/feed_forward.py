@@ -82,10 +82,10 @@ class SwiGLU(FeedForward):
         elif self.block == 64 and self._gate_up_fuses(rows):
             h = ops.gemm_tc_pair(x, self.w_gate_up, self.ctx.dtype, swiglu=True, activation=self.activation)
         else:
-            gu = ops.linear(x, self.w_gate_up, out_dtype=self.ctx.dtype)
+            gu = ops.linear(x, self.w_gate_up, out_dtype=self.ctx.dtype, inputs=inputs)
             h = ops.swiglu(gu, block=self.block, activation=self.activation, limit=self.limit)
         return ops.linear(h, self.w_down, out_dtype=self.ctx.dtype, epilogue=epilogue,
-                          residual32=residual32 if epilogue is None else None)
+                          residual32=residual32 if epilogue is None else None, inputs=inputs)
 
 
 @FEED_FORWARDS.register("dense")
@@ -112,5 +112,5 @@ class DenseFeedForward(FeedForward):
         self.w_down = tensors[self.names["down"]].contiguous()
 
     def forward(self, x, inputs, residual32=None):
-        h = ops.linear(x, self.w_up, out_dtype=self.ctx.dtype, act=self.activation)
-        return ops.linear(h, self.w_down, out_dtype=self.ctx.dtype, residual32=residual32)
+        h = ops.linear(x, self.w_up, out_dtype=self.ctx.dtype, act=self.activation, inputs=inputs)
+        return ops.linear(h, self.w_down, out_dtype=self.ctx.dtype, residual32=residual32, inputs=inputs)

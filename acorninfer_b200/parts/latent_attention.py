@@ -120,11 +120,11 @@ class LatentAttention(Mixer):
         pos = self.position
         kv_rows = None
         if self.q_rank is None:
-            proj = ops.linear(x, self.w_in, out_dtype=dt)
+            proj = ops.linear(x, self.w_in, out_dtype=dt, inputs=inputs)
         else:
-            cq = ops.add_rmsnorm(ops.linear(x, self.w_dq, out_dtype=torch.float32), None, self.q_norm32, self.eps, dt)
-            proj = ops.linear(cq, self.w_uq, out_dtype=dt)
-            kv_rows = ops.linear(x, self.w_in, out_dtype=dt) if cache.write else None
+            cq = ops.add_rmsnorm(ops.linear(x, self.w_dq, out_dtype=torch.float32, inputs=inputs), None, self.q_norm32, self.eps, dt)
+            proj = ops.linear(cq, self.w_uq, out_dtype=dt, inputs=inputs)
+            kv_rows = ops.linear(x, self.w_in, out_dtype=dt, inputs=inputs) if cache.write else None
         qcat = torch.empty((T, H, self.rank + self.rot), dtype=dt, device=x.device)
         ops.latent_prep(proj, qcat, self.c_norm32, pos.inv_freq if pos is not None else _no_freq(x.device),
                         pos.magnitude if pos is not None else 1.0, inputs.positions, inputs.token_row, g.block_table,
@@ -147,7 +147,7 @@ class LatentAttention(Mixer):
                                     self.window, value_dim=self.rank, sink32=self.sink32)
         v = torch.empty((T, H, self.vdim), dtype=dt, device=x.device)
         ops.head_linear(o.view(T, H, self.rank), self.w_uv, v)
-        return ops.linear(v.view(T, H * self.vdim), self.w_o, out_dtype=dt)
+        return ops.linear(v.view(T, H * self.vdim), self.w_o, out_dtype=dt, inputs=inputs)
 
 
 _NO_FREQ: dict = {}

@@ -40,7 +40,7 @@ class _RecurrentMixer(Mixer):
     state_base = 0
 
     def forward(self, x, inputs, cache, residual32=None):
-        return ops.linear(self.inner(x, inputs, cache), self.w_o, out_dtype=self.ctx.dtype, residual32=residual32)
+        return ops.linear(self.inner(x, inputs, cache), self.w_o, out_dtype=self.ctx.dtype, residual32=residual32, inputs=inputs)
 
 
 @MIXERS.register("state_space")
@@ -84,7 +84,7 @@ class StateSpace(_RecurrentMixer):
 
     def inner(self, x, inputs, cache, out_scale: float = 1.0, out=None):
         I, GN, C = self.inner_size, self.G * self.N, self.channels
-        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)             # [z | x | B | C | dt]
+        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, inputs=inputs)             # [z | x | B | C | dt]
         conv_off = self.state_base + self.state_s
         act, dt, decay = ops.ssm_prep(proj, I, I + C, self.conv32, self.conv_b32, cache.state, conv_off, self.a_log32,
                                       self.dt_bias32, inputs.token_row, inputs.row_start, inputs.row_slot, self.taps,
@@ -136,7 +136,7 @@ class DecayLinearAttention(_RecurrentMixer):
 
     def inner(self, x, inputs, cache, out_scale: float = 1.0, out=None):
         Hd, Hv = self.H * self.dim, self.H * self.V
-        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)             # [q | k | v | g]
+        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, inputs=inputs)             # [q | k | v | g]
         act = ops.silu_rows(proj[:, :2 * Hd + Hv])
         y = ops.linear_scan(act[:, Hd:2 * Hd], act[:, :Hd], act[:, 2 * Hd:], self._decay32, None, None, cache.state,
                             self.state_base, inputs.row_start, inputs.row_slot, inputs.num_rows, self.H, self.H,

@@ -51,7 +51,7 @@ class MinGRU(Mixer):
         return CacheNeeds(state=StateNeeds((self.width,)))
 
     def forward(self, x, inputs, cache, residual32=None):
-        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)
+        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, inputs=inputs)
         y = ops.min_gru(proj, self.bias32, cache.state, self.state_base, inputs.row_start, inputs.row_slot, inputs.num_rows,
                         longest_row=inputs.plan.max_q_len)
-        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, residual32=residual32)
+        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, residual32=residual32, inputs=inputs)

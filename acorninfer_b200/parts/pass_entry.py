@@ -35,5 +35,5 @@ class MixIn(PassEntry):
         if not (0 <= pass_index < self.passes):
             raise ValueError(f"pass {pass_index} of {self.passes}")
         both = ops.pair_rows(resid32, entered32, self.ctx.dtype)
-        y32 = ops.linear(both, self.w_in, out_dtype=torch.float32)
+        y32 = ops.linear(both, self.w_in, out_dtype=torch.float32, inputs=inputs)
         return ops.add_row(y32, self.step32[pass_index])

@@ -57,13 +57,13 @@ class _HeadsMixer(Mixer):
         self.norm_heads32 = self.norm32.repeat(self.H).contiguous()           # the same for the kernel that norms rows of heads
 
     def forward(self, x, inputs, cache):
-        return ops.linear(self.inner(x, inputs, cache), self.w_o, out_dtype=self.ctx.dtype)
+        return ops.linear(self.inner(x, inputs, cache), self.w_o, out_dtype=self.ctx.dtype, inputs=inputs)
 
     def inner(self, x, inputs, cache, out_scale: float = 1.0, out=None, proj=None):
         """The heads' rows before the output projection, times ``out_scale``, into ``out`` if given; ``proj``: the rows of
         ``w_in``'s product where the caller has made it (beside another mixer's)."""
         if proj is None:
-            proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)
+            proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, inputs=inputs)
         if out is None:
             out = torch.empty((proj.shape[0], self.H * self.vdim), dtype=self.ctx.dtype, device=proj.device)
         return self._run(proj, inputs, cache, out_scale, out)
@@ -161,7 +161,7 @@ class GatedLinearAttention(_HeadsMixer):
 
     def _run(self, proj, inputs, cache, out_scale, out):
         low = proj[:, self.a1_col:self.a1_col + self.rank]
-        z = ops.linear(low if low.dtype == self.w_a2.dtype else low.contiguous(), self.w_a2, out_dtype=torch.float32)
+        z = ops.linear(low if low.dtype == self.w_a2.dtype else low.contiguous(), self.w_a2, out_dtype=torch.float32, inputs=inputs)
         gate = proj[:, self.gate_col:self.gate_col + self.H * self.vdim]
         if self._steps(inputs, cache, (proj, gate, out)) and (self.H * self.dim) % 2 == 0 and z.stride(0) % 4 == 0:
             return ops.recurrent_step(cache.state, self.state_base, inputs.row_slot, gate, self.norm32, self.eps, out, self.H,

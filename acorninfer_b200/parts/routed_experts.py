@@ -117,7 +117,7 @@ class RoutedExperts(FeedForward):
     def forward(self, x, inputs, add_normed=None, defer=False):
         T, n = x.shape[0], self.E + self.I
         beside = ops.Branch(lambda: self.shared_ff.forward(x, inputs), inputs) if self.shared_ff is not None else None
-        z = ops.linear(x, self.w_router, out_dtype=torch.float32)
+        z = ops.linear(x, self.w_router, out_dtype=torch.float32, inputs=inputs)
         idx, wts, offsets, slot_of, slot_token, slot_wts = ops.moe_route_plan(
             z[:, :n], self.correction32, self.top, self.groups, self.keep, self.normalize, self.scoring,
             by_slot=self.weight_on == "input", bias32=self.bias32)

@@ -80,9 +80,9 @@ class SideBySide(Mixer):
         rows = torch.empty((x.shape[0], sum(self.widths)), dtype=self.ctx.dtype, device=x.device)
         a, b = {}, {}
         if self.w_in is not None:
-            proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)
+            proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, inputs=inputs)
             a["proj"], b["proj"] = proj[:, :self.first_in], proj[:, self.first_in:]
         beside = ops.Branch(lambda: right.inner(x, inputs, cache, out_scale=self.scales[1], out=rows[:, self.widths[0]:], **b), inputs)
         left.inner(x, inputs, cache, out_scale=self.scales[0], out=rows[:, :self.widths[0]], **a)
         beside.join()
-        return ops.linear(rows, self.w_o, out_dtype=self.ctx.dtype, residual32=residual32)
+        return ops.linear(rows, self.w_o, out_dtype=self.ctx.dtype, residual32=residual32, inputs=inputs)

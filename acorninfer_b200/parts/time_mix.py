@@ -76,7 +76,7 @@ class TimeMix(Mixer):
         T = x.shape[0]
         r, k, v, g = ops.grouped_gemm(mixes[:4].view(4 * T, self.hidden_size), None, self.w_rkvg,
                                       inputs.extra["time_mix.blend_rows"], 4 * T).view(4, T, -1).unbind(0)
-        z = ops.linear(ops.linear(mixes[4], w["w1"], out_dtype=dt, act="tanh"), w["w2"], out_dtype=torch.float32)
+        z = ops.linear(ops.linear(mixes[4], w["w1"], out_dtype=dt, act="tanh", inputs=inputs), w["w2"], out_dtype=torch.float32, inputs=inputs)
         # long rows over chunks of tokens, whose kernels want the decays' logarithms; the others token by token
         d, lens, min_row = r.shape[1] // self.H, inputs.plan.row_lens, 0
         if cache.state.stride(0) % 4 == 0 and ops.channel_chunk_ok(inputs.plan.max_q_len, T, inputs.num_rows, self.H, d, d):
@@ -90,4 +90,4 @@ class TimeMix(Mixer):
             o = ops.delta_rule(r32, k32, v32, None, decay, *rows, bonus32=self.u32, longest_row=inputs.plan.max_q_len,
                                max_row=min_row - 1 if min_row else 0, out=o)
         y = ops.delta_out(o, gate, self.norm32, self.eps, dt)
-        return ops.linear(y, w["o"], out_dtype=dt)
+        return ops.linear(y, w["o"], out_dtype=dt, inputs=inputs)

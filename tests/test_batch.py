@@ -237,3 +237,13 @@ def test_which_latent_steps_take_the_tcgen05_kernel():
     assert latent_prefill_wins(38, 75, 512, *narrow) and not latent_prefill_wins(40, 40, 512, *narrow)
     assert latent_prefill_wins(1, 1, 256, *narrow) and not latent_prefill_wins(300, 300, 128, *narrow)
     assert not latent_prefill_wins(32, 63, 8192, *small) and not latent_prefill_wins(1, 1, 128, *small)
+
+
+@pytest.mark.parametrize("lens,want", [((1, 1), None), ((3,), ((0, 3), [])), ((1, 1, 4), ((2, 6), [(0, 2)])), ((2, 1, 1), ((0, 2), [(2, 4)])),
+                                       ((1, 2, 1, 3, 1), ((1, 7), [(0, 1), (3, 4), (7, 8)]))])
+def test_where_a_steps_longer_rows_lie(lens, want):
+    m = manager()
+    entries = [StepEntry(m.open(i), list(range(n)), []) for i, n in enumerate(lens)]
+    for e in entries:
+        m.extend(e.cache, len(e.tokens))
+    assert plan_step(entries, m, STEP_ARRAYS).longer_rows == want

@@ -4,6 +4,7 @@ of 16, odd head counts).  float32 inputs catch indexing faults (tolerance 1e-5);
 inputs are compared at bfloat16's resolution."""
 
 import math
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -177,7 +178,9 @@ def test_float32_product_on_tcgen05(M, N, K, pad):
     if K >= 512:
         chains = torch.cat([o.gemm_f32(a[i:i + 16].contiguous(), w) for i in range(0, M, 16)])       # few rows: multiply-adds
         assert (out.double() - want).norm() <= (chains.double() - want).norm()
-    assert torch.equal(o.gemm_f32(a, w), out) == (M > 64 and N >= 1024 and K >= 512)
+    # the tokens of a step's longer rows take it where the matrix is wide and deep enough, whatever their number
+    whole = SimpleNamespace(num_tokens=M, longer_rows=((0, M), []))
+    assert torch.equal(o.gemm_f32_step(a, w, whole), out if N >= 1024 and K >= 512 else o.gemm_f32(a, w))
 
 
 def test_float32_product_on_tcgen05_with_numbers_that_do_not_split():
@@ -196,6 +199,23 @@ def test_float32_product_on_tcgen05_with_numbers_that_do_not_split():
     for scale in (1.0, 2.0 ** -90, 2.0 ** 120):
         x = torch.randn(64, 128, device=DEV, generator=g) * scale
         assert torch.equal(o.gemm_f32_tc(x, torch.eye(128, device=DEV)), x)
+
+
+def test_float32_product_of_a_step_by_the_kind_of_its_tokens():
+    """Decoded tokens anywhere among prompts: their bits those of the multiply-adds, the others' those of the tensor cores."""
+    from acorninfer_b200.engine.batch import StepPlan
+    o = ops()
+    lens = [1, 1, 7, 1, 1, 1, 60, 2, 1, 1]
+    kinds = torch.tensor([n > 1 for n in lens for _ in range(n)], device=DEV)
+    T = len(kinds)
+    plan = StepPlan(T, len(lens), *([None] * 8), lens, max(lens), False)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x, w = torch.randn(T, 640, device=DEV, generator=g), torch.randn(1100, 640, device=DEV, generator=g)
+    want = torch.where(kinds[:, None], o.gemm_f32_tc(x, w), o.gemm_f32(x, w))
+    assert torch.equal(o.gemm_f32_step(x, w, plan), want)
+    assert torch.equal(o.linear(x, w, inputs=SimpleNamespace(plan=plan)), want)
+    assert torch.equal(o.linear(x, w), o.gemm_f32(x, w)) and torch.equal(o.gemm_f32_step(x[:9], w, plan), o.gemm_f32(x[:9], w))
+    assert torch.equal(o.gemm_f32_step(x, w[:1000], plan), o.gemm_f32(x, w[:1000]))
 
 
 @pytest.mark.parametrize("e", [-100, -110, -117, -126, -135, -149])
