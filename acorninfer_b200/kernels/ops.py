@@ -1100,12 +1100,14 @@ def gemm_tc_splits(M: int, N: int, K: int) -> int:
 # At or below this many rows the tcgen05 kernel (weights on the 128-row side of the MMA) streams the
 # weight matrix at least as fast as the library product; above it the library's larger tiles win.
 GEMM_TC_MAX_ROWS = 32
-# With the residual sum and norm, SwiGLU or the rotation in its epilogue, which the library leaves to kernels of their own, it wins
-# up to this many.  Measured (B200, chained, a layer's four products, us, library / this at 41 rows): 30.0 / 28.8 at Qwen3-0.6B widths,
-# 43.5 / 41.0 at 1.7B, 63.2 / 59.1 at 4B, 91.9 / 84.6 at 8B; at 64 rows 62.8 / 81.9 at 4B: a tile of 64 rows takes as much of an
-# SM's intake as half of the weights' tile.
+# In a layer whose products take all of the residual sums and norms, SwiGLU and the rotation into their epilogues, which the library
+# leaves to kernels of their own, it wins up to this many.  Measured (B200, replayed decode steps of 8 to 12 layers, us, library / this
+# at 36, 40 and 48 rows): Qwen3-0.6B widths 639 / 597, 707 / 654, 719 / 680; 4B 1,100 / 1,041, 1,170 / 1,115, 1,185 / 1,159; 8B 1,531 / 1,440,
+# 1,597 / 1,497, 1,613 / 1,561; 14B 2,163 / 1,994, 2,227 / 2,055, 2,232 / 2,100; 32B the same.  At 64 rows 62.8 / 81.9 for the four
+# products of a layer at 4B: a tile of 64 rows takes as much of an SM's intake as half of the weights' tile.  A gate/up product with
+# SwiGLU alone loses (Vagulorn, width 1,024 and 2,048, at 40 rows: 502 / 519 and 832 / 858; Zusolix, width 2,048: 772 / 787).
 GEMM_TC_FUSED_MAX_ROWS = 48
-# ... and the smallest hidden size where that was measured to pay (41 rows: 1,024 to 4,096); below it the products are small enough
+# ... and the smallest hidden size where that was measured to pay; below it the products are small enough
 # for the library and the launches beside them to cost the same.
 GEMM_TC_FUSED_MIN_WIDTH = 1024
 # The paired kernel (256 x 256 tiles, a pair of SMs to a tile at a time, fused epilogues) is used from
@@ -1392,8 +1394,8 @@ def fused_rows_ok(num_rows: int, dtype: torch.dtype, widths=None, num_sms: int =
 
 
 def fused_tile_ok(num_rows: int, dtype: torch.dtype, hidden: int) -> bool:
-    """Whether so many rows, more than the one-CTA kernel takes for plain products, go to it where it spares a part the kernels
-    around its products (``GEMM_TC_FUSED_MAX_ROWS``), in a model of this hidden size (``GEMM_TC_FUSED_MIN_WIDTH``)."""
+    """Whether so many rows, more than the one-CTA kernel takes for plain products, go to it where it spares a layer all of the
+    kernels around its products (``GEMM_TC_FUSED_MAX_ROWS``), in a model of this hidden size (``GEMM_TC_FUSED_MIN_WIDTH``)."""
     return dtype == torch.bfloat16 and GEMM_TC_MAX_ROWS < num_rows <= GEMM_TC_FUSED_MAX_ROWS and hidden >= GEMM_TC_FUSED_MIN_WIDTH
 
 

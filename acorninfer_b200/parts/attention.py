@@ -219,13 +219,20 @@ class Attention(Mixer):
 
     def fusable(self, num_rows):
         # (the options only change what runs between the two products, which take the fused forms either way)
-        return (not self.norm_rows and self._rows_fuse(num_rows) and self.w_qkv.dtype == torch.bfloat16
+        return (not self.norm_rows and (self._rows_fuse(num_rows) or self._tile_fuses(num_rows)) and self.w_qkv.dtype == torch.bfloat16
                 and self.w_o.dtype == torch.bfloat16 and self.hidden_size % 8 == 0 and (self.nq * self.d) % 8 == 0)
 
     def _rows_fuse(self, num_rows):
         widths = ((self.nq + 2 * self.nkv) * self.d, self.hidden_size)         # of the q/k/v product and of the o product
-        return (ops.fused_rows_ok(num_rows, self.ctx.dtype, widths, ops.device_sms(self.ctx.device))
-                or ops.fused_tile_ok(num_rows, self.ctx.dtype, self.hidden_size))
+        return ops.fused_rows_ok(num_rows, self.ctx.dtype, widths, ops.device_sms(self.ctx.device))
+
+    def _rope_fuses(self, num_rows):
+        pos = self.position
+        return self.plain and pos is not None and ops.rope_kv_fusable(num_rows, self.ctx.dtype, self.d, pos.rotary_dim, pos.interleaved)
+
+    def _tile_fuses(self, num_rows):
+        """Whether the one-CTA kernel's tile for more rows pays here: in a layer all of whose products fuse, the rotation among them."""
+        return self._rope_fuses(num_rows) and ops.fused_tile_ok(num_rows, self.ctx.dtype, self.hidden_size)
 
     def _inner_norm_rows(self, x, inputs, cache, out_scale, out, proj):
         g, pos = inputs.groups[cache.group], self.position
@@ -255,19 +262,20 @@ class Attention(Mixer):
     state_base = 0
     w_in = None            # the projection of x where its product may be made by the caller (``inner(proj=...)``)
 
-    def inner(self, x, inputs, cache, out_scale: float = 1.0, out=None, proj=None):
+    def inner(self, x, inputs, cache, out_scale: float = 1.0, out=None, proj=None, fused: bool = False):
         """Everything before the output projection: the heads' outputs [T, nq * dv] (gated, times ``out_scale``),
-        into ``out`` if given (rows of a wider buffer).  ``proj``: the rows of ``w_in``'s product, if the caller made it."""
+        into ``out`` if given (rows of a wider buffer).  ``proj``: the rows of ``w_in``'s product, if the caller made it;
+        ``fused``: the layer's other products fuse."""
         if self.norm_rows:
             return self._inner_norm_rows(x, inputs, cache, out_scale, out, proj)
         g = inputs.groups[cache.group]
         pos = self.position
         rows = x.x.shape[0] if isinstance(x, ops.NormedRows) else x.shape[0]
         proj = None                 # the projected rows where the queries do not stay among them
-        if (self.plain and pos is not None and self.w_qkv.dtype == torch.bfloat16 and ops.gemm_tc_supported(
+        fused = fused or isinstance(x, ops.NormedRows)
+        if (self._rope_fuses(rows) and self.w_qkv.dtype == torch.bfloat16 and ops.gemm_tc_supported(
                 x.x if isinstance(x, ops.NormedRows) else x, self.w_qkv)
-                and self._rows_fuse(rows)
-                and ops.rope_kv_fusable(rows, self.ctx.dtype, self.d, pos.rotary_dim, pos.interleaved)):
+                and (self._rows_fuse(rows) or (fused and self._tile_fuses(rows)))):
             # few rows or very many, head size 128: norm, rotation and the cache write are the epilogue of the product
             qkv = ops.gemm_tc_qkv_rope(x, self.w_qkv, ops.RopeKvEpilogue(
                 inputs.positions, inputs.token_row, g.block_table, g.page_base,
@@ -315,7 +323,7 @@ class Attention(Mixer):
         return heads
 
     def forward(self, x, inputs, cache, epilogue=None, residual32=None):
-        return ops.linear(self.inner(x, inputs, cache), self.w_o, out_dtype=self.ctx.dtype, epilogue=epilogue,
+        return ops.linear(self.inner(x, inputs, cache, fused=epilogue is not None), self.w_o, out_dtype=self.ctx.dtype, epilogue=epilogue,
                           residual32=residual32 if epilogue is None else None, inputs=inputs)
 
 

@@ -77,7 +77,8 @@ class SwiGLU(FeedForward):
 
     def forward(self, x, inputs, epilogue=None, residual32=None):
         rows = x.x.shape[0] if isinstance(x, ops.NormedRows) else x.shape[0]
-        if self.block == 64 and self.fusable(rows):
+        fused = isinstance(x, ops.NormedRows) or epilogue is not None        # the layer's other products fuse, too
+        if self.block == 64 and self.fusable(rows) and (fused or not ops.fused_tile_ok(rows, self.ctx.dtype, self.hidden_size)):
             h = ops.linear(x, self.w_gate_up, out_dtype=self.ctx.dtype, swiglu=True, activation=self.activation)
         elif self.block == 64 and self._gate_up_fuses(rows):
             h = ops.gemm_tc_pair(x, self.w_gate_up, self.ctx.dtype, swiglu=True, activation=self.activation)

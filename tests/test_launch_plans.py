@@ -97,3 +97,29 @@ def test_paired_kernel_is_asked_for_where_its_tiles_fill_the_device():
     assert fused_rows_ok(1024, torch.bfloat16, 4096) and not fused_rows_ok(1024, torch.bfloat16, (6144, 4096))
     assert fused_rows_ok(2048, torch.bfloat16, (6144, 4096)) and fused_rows_ok(2048, torch.bfloat16, (24576, 4096))
     assert not fused_rows_ok(2048, torch.float32, 4096)
+
+
+def test_tile_of_48_rows_is_for_layers_that_fuse_throughout(monkeypatch):
+    """33 to 48 rows: gate/up products take the one-CTA kernel's tile between fused neighbours only, layers whose rotation is not in
+    the epilogue of their q/k/v product do not ask for it."""
+    import torch
+    from acorninfer_b200.kernels import ops
+    from acorninfer_b200.parts.attention import Attention
+    from acorninfer_b200.parts.base import POSITION_ENCODINGS, BuildContext, PartSpec, build_part
+    from acorninfer_b200.parts.feed_forward import SwiGLU
+    monkeypatch.setattr(ops, "device_sms", lambda device: 148)
+    taken = []
+    monkeypatch.setattr(ops, "linear", lambda x, w, **kw: taken.append(kw.get("swiglu", False)) or torch.zeros(1, w.shape[0]))
+    monkeypatch.setattr(ops, "swiglu", lambda gu, **kw: gu)
+    ctx = BuildContext(dtype=torch.bfloat16, device=torch.device("cpu"), page_size=16)
+    ff = SwiGLU(ctx, 1024, 64)
+    ff.bind({n: torch.zeros(s.shape, dtype=torch.bfloat16) for n, s in ff.tensor_specs().items()})
+    x = torch.zeros(40, 1024, dtype=torch.bfloat16)
+    for rows, between in ((x, object()), (ops.NormedRows(x, None, 1e-6, 1024), None), (x, None), (x[:32], None)):
+        ff.forward(rows, None, epilogue=between)
+    assert taken == [True, False, True, False, False, False, True, False]       # of the gate/up and the down product in turn
+    for rotary in (128, 64):
+        ctx.positions["rope"] = build_part(POSITION_ENCODINGS, PartSpec("rope", {"head_dim": 128, "theta": 1e6, "rotary_dim": rotary}, ""), ctx)
+        att = Attention(ctx, hidden_size=1024, num_heads=8, num_kv_heads=2, head_dim=128, position="rope", scale=128 ** -0.5)
+        att.bind({n: torch.zeros(s.shape, dtype=torch.bfloat16) for n, s in att.tensor_specs().items()})
+        assert att.fusable(40) == (rotary == 128) and att.fusable(32) and not att.fusable(49)
