@@ -104,6 +104,19 @@ def test_gemm_tc_swiglu_epilogue(M, I, K, splits):
     assert ops().gemm_tc_error() == 0
 
 
+@pytest.mark.parametrize("M,I,K,splits", [(5, 64, 64, 1), (32, 192, 1024, 2), (33, 128, 520, 1), (41, 192, 1024, 4), (48, 64, 512, 8)])
+def test_gemm_tc_geglu_epilogue(M, I, K, splits):
+    """gelu's tanh form times up, in tiles of 16, 32 and 48 rows, against float64."""
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x = torch.randn(M, K, device=DEV, generator=g).to(torch.bfloat16)
+    gate, up = ((torch.randn(I, K, device=DEV, generator=g) / K ** 0.5).to(torch.bfloat16) for _ in range(2))
+    w = torch.stack([gate.view(I // 64, 64, K), up.view(I // 64, 64, K)], dim=1).reshape(2 * I, K).contiguous()
+    out = ops().gemm_tc(x, w, torch.bfloat16, splits=splits, swiglu=True, activation="gelu_tanh")
+    want = torch.nn.functional.gelu(x.double() @ gate.double().T, approximate="tanh") * (x.double() @ up.double().T)
+    # one rounding to bfloat16 (2^-9) beside float32 sums of K terms
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all() and ops().gemm_tc_error() == 0
+
+
 @pytest.mark.parametrize("nq,nkv,K,qlens,norm,write", [(4, 2, 256, [7, 1, 5], True, True), (6, 1, 520, [1, 1, 1, 1], True, True),
                                                        (2, 2, 128, [30], False, True), (8, 4, 1024, [3, 20], True, False)])
 def test_gemm_tc_qkv_rope_epilogue(nq, nkv, K, qlens, norm, write):
