@@ -80,13 +80,18 @@ __device__ __forceinline__ void tmem_ld8x7(uint32_t at, float (&v)[7][8]) {
 
 // What float32 gives where a scaled sum is no number: chains of fused multiply-adds over ranges of K, as in gemm_f32.cu.  An operand that
 // is infinite, NaN or, scaled, beyond bfloat16's largest number (2^112) makes every product of its row NaN above, and a sum from 2^96 on is
-// infinite; such sums are made again here.
+// infinite; such sums are made again here, up to the first NaN, which stays one
+// (777 rows of nothing else, N = 4,096, K = 1,024: 13.8 ms to the end of K, 0.35 so; the multiply-adds 0.19).
 static __device__ __noinline__ float f3_chain(const float* a, const float* w, int K) {
     const int range = (K + 127) / 128 * 16;
     float total = 0.f;
     for (int k0 = 0; k0 < K; k0 += range) {
         float acc = 0.f;
-        for (int k = k0; k < min(K, k0 + range); ++k) acc = fmaf(a[k], w[k], acc);
+        const int end = min(K, k0 + range);
+        for (int k1 = k0; k1 < end; k1 += 16) {
+            for (int k = k1; k < min(end, k1 + 16); ++k) acc = fmaf(a[k], w[k], acc);
+            if (acc != acc) return acc;
+        }
         total = k0 == 0 ? acc : total + acc;
     }
     return total;
