@@ -103,8 +103,8 @@ template <int R, int CPL> constexpr int rs_smem() {
 // sums of the one before are added: a block that ends with its tile spends a third of its time on filling and emptying its
 // rings (6 rows, N = 12,288, K = 2,048: 31 -> 25 us).
 // The reads of A and W from shared memory that feed the multiply-adds set the pace (R + CPL reads of 16 bytes a lane for 4 R CPL
-// multiply-adds), so there is a form for each number of rows a lane, and none reads rows that are not there.  Measured (B200, us, forms
-// for 4, 8 and 16 rows only / this), 6 rows: N = 4,096, K = 2,048 11.5 / 8.5; N = 2,048, K = 6,144 19.6 / 14.2; N = 12,288, K = 2,048
+// multiply-adds), so there is a form for each number of rows a lane: at most one row is read that is not there (two for two rows).
+// Measured (B200, us, forms for 4, 8 and 16 rows only / this), 6 rows: N = 4,096, K = 2,048 11.5 / 8.5; N = 2,048, K = 6,144 19.6 / 14.2; N = 12,288, K = 2,048
 // 26.4 / 24.9 (4.0 TB/s); N = 151,936, K = 1,024 134 / 122 (5.1 TB/s); one row of the last 107 / 98 (6.4 TB/s).
 template <int R, int CPL, bool NARROW>
 __global__ void __launch_bounds__(RS_THREADS) gemm_f32_rows_kernel(const float* __restrict__ A, int64_t lda,

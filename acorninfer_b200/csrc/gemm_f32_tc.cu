@@ -1,6 +1,6 @@
 // C[M, N] = A[M, K] * W[N, K]^T in float32 on the 5th-generation tensor cores, for prompts, many columns and long
-// sums (acorninfer_b200/kernels/ops.py, gemm_f32_step): every operand, times 2^16, is the exact sum of three bfloat16 numbers, a = a0 + a1 + a2 (8 bits
-// of mantissa each; rounding to nearest, so |a1| <= 2^-9 |a|, |a2| <= 2^-18 |a|), and a product is
+// sums (acorninfer_b200/kernels/ops.py, gemm_f32_step): every operand, times 2^16, is the exact sum of three bfloat16 numbers,
+// a = a0 + a1 + a2 (8 bits of mantissa each; rounding to nearest, so |a1| <= 2^-9 |a|, |a2| <= 2^-18 |a|), and a product is
 // a0 b0 + (a0 b1 + a1 b0) + (a0 b2 + a1 b1 + a2 b0); what is left out (a1 b2 + a2 b1 + a2 b2) is at most 2^-26 |a b|, a quarter of a
 // rounding of float32.  The scale takes float32's least number, 2^-149, to bfloat16's, 2^-133, so that no bit falls below: without it the
 // parts of an operand of 2^-117 lost 4e-6 of it, of 2^-126 2e-3.  Operands from 2^112 and sums from 2^96 on overflow and go to f3_chain.
@@ -26,7 +26,7 @@
 // What bounds it: the loading warps, a load's latency and their arithmetic in turn (a chunk of 128 x 32 takes 1.0 us, of which shared
 // memory's bytes take 0.55).  One group instead of two: 1.75 us; wider tiles of 48 and 64 tokens need registers that 25 warps do not
 // have (spills: 1.7 and 2.0 us).  The products of a prompt of 777 rows (us, multiply-adds / this): N = 4,096, K = 1,024 164 / 101;
-// N = 6,144 263 / 148; N = 1,024, K = 3,072 141 / 91; N = 12,288, K = 2,048 901 / 512 (76 TFLOP/s).
+// N = 6,144 263 / 149; N = 1,024, K = 3,072 141 / 93; N = 12,288, K = 2,048 900 / 518 (75 TFLOP/s).
 #include <cooperative_groups.h>
 
 #include "tcgen05_helpers.cuh"

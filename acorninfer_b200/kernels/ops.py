@@ -1035,9 +1035,9 @@ def gemm_f32_step(x: torch.Tensor, w: torch.Tensor, plan) -> torch.Tensor:
     decoded ones above all, by ``gemm_f32``, those of longer rows by ``gemm_f32_tc`` where the matrix is wide and deep enough.  So a
     token's bits depend on its own row, as attention's do, and not on what else is in the step or on how many rows there are.
 
-    Measured (B200, us, multiply-adds / tensor cores): N = 4,096, K = 1,024 at 32 rows 21 / 20, 128 40 / 20, 777 164 / 101; N = 1,024,
-    K = 3,072 28 / 10, 48 / 30, 141 / 91; N = 12,288, K = 2,048 75 / 40, 175 / 100, 901 / 512; operands that are not 16-byte aligned:
-    N = 4,096, K = 1,023 at 128 rows 122 / 26, at 777 333 / 117.  Decoded tokens lose by the tensor cores (8 rows 8 / 21, 11 / 10, 26 / 39);
+    Measured (B200, us, multiply-adds / tensor cores): N = 4,096, K = 1,024 at 32 rows 15 / 20, 128 39 / 21, 777 164 / 101; N = 1,024,
+    K = 3,072 26 / 10, 46 / 30, 141 / 93; N = 12,288, K = 2,048 75 / 38, 175 / 97, 900 / 518; operands that are not 16-byte aligned:
+    N = 4,096, K = 1,023 at 128 rows 129 / 25, at 777 332 / 119.  Decoded tokens lose by the tensor cores (8 rows 5 / 19, 10 / 10, 26 / 37);
     narrower matrices and shorter sums leave that kernel's SMs idle or end before its chunks overlap."""
     M, (N, K) = x.shape[0], w.shape
     longer = None if plan is None or plan.num_tokens != M or N < 1024 or K < 512 else plan.longer_rows

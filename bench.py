@@ -461,7 +461,7 @@ def long_context(steps: int, warmup: int, pk: dict, torch) -> dict:
 
 def float32_path(pk: dict, torch) -> dict:
     """The true 32-bit path at Qwen3-8B layer sizes with 4 of the 36 layers (float32 weights, cache
-    and products on the CUDA cores): a decode step at batch 8, context 4,096, and a 2,048-token
+    and products, exact splits on the tensor cores for the prompt): a decode step at batch 8, context 4,096, and a 2,048-token
     prefill, device-timed.  It is the correctness path; the figures say how long a check takes."""
     from acorninfer_b200.config.model_config import Qwen3Config
     from acorninfer_b200.engine.runner import ModelRunner
